@@ -7,6 +7,8 @@ Both fail loudly (ImportError) when the library has not been built: nothing fall
 slower path.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -27,7 +29,7 @@ EXPORTS = (
 )
 
 _core = None
-_ops_loaded = False
+_ops = None
 
 _i64 = ctypes.c_int64
 _vp = ctypes.c_void_p
@@ -86,9 +88,10 @@ def load_core():
 
 
 def load_ops():
-    global _ops_loaded
-    if _ops_loaded:
-        return
+    """Registers torch.ops.lfw / torch.ops.dfw and returns the extension module with the autograd entry points."""
+    global _ops
+    if _ops is not None:
+        return _ops
     import torch
 
     if not os.path.exists(OPS_PATH):
@@ -96,4 +99,21 @@ def load_ops():
             "t2fw_b200: %s is missing; build it with `python -m t2fw_b200.build`" % OPS_PATH)
     load_core()
     torch.ops.load_library(OPS_PATH)
-    _ops_loaded = True
+    loader = importlib.machinery.ExtensionFileLoader("t2fw_torch_ops", OPS_PATH)
+    spec = importlib.util.spec_from_file_location("t2fw_torch_ops", OPS_PATH, loader=loader)
+    _ops = importlib.util.module_from_spec(spec)
+    loader.exec_module(_ops)
+    return _ops
+
+
+# which of set_fallback()'s slots belongs to which class
+LFW, DFW, FUSED = range(3)
+
+
+def bind_apply(cls, which, native):
+    """Replaces cls.apply by the native entry point; what is not the plain case (and every subclass, which may
+    override forward or backward) goes through torch.autograd.Function.apply as before."""
+    python_apply = cls.apply
+    load_ops().set_fallback(which, python_apply)
+    cls.apply = native
+    cls.__init_subclass__ = classmethod(lambda sub, **kw: setattr(sub, "apply", classmethod(python_apply.__func__)))

@@ -2,7 +2,8 @@
 
   lib/libt2fw_b200.so     CUDA kernels + the C ABI (include/t2fw_b200.h); nvcc, sm_100a only
   lib/t2fw_torch_ops.so   the PyTorch operator library (torch.ops.lfw / torch.ops.dfw), a thin
-                          C++ adapter that links against the former
+                          C++ adapter that links against the former; also the Python extension
+                          module with the autograd entry points
 
 Run `python -m t2fw_b200.build` (add --force to rebuild everything).  nvcc cross-compiles
 without a GPU.  Nothing is JIT-compiled at import time: the .so files must exist.
@@ -11,6 +12,7 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -76,19 +78,19 @@ def build_ops(force=False, verbose=False):
     import torch
     from torch.utils import cpp_extension
 
-    src = os.path.join(CSRC, "torch_ops.cpp")
-    deps = [src, os.path.join(ROOT, "include", "t2fw_b200.h")]
+    srcs = [os.path.join(CSRC, "torch_ops.cpp"), os.path.join(CSRC, "torch_bind.cpp")]
+    deps = srcs + [os.path.join(CSRC, "torch_ops.h"), os.path.join(ROOT, "include", "t2fw_b200.h")]
     if not force and _newer(OPS_LIB, deps) and _newer(OPS_LIB, [CORE_LIB]):
         return OPS_LIB
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    inc = []
+    inc = ["-isystem", sysconfig.get_paths()["include"]]
     for p in cpp_extension.include_paths(device_type="cuda"):
         inc += ["-isystem", p]
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=%d" % abi,
-            "-DTORCH_API_INCLUDE_EXTENSION_H", src, "-o", OPS_LIB, "-I", os.path.join(ROOT, "include")]
+            "-DTORCH_API_INCLUDE_EXTENSION_H"] + srcs + ["-o", OPS_LIB, "-I", os.path.join(ROOT, "include")]
            + inc + ["-L", tlib, "-L", LIB_DIR, "-L", "/usr/local/cuda/lib64",
-                    "-lt2fw_b200", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
+                    "-lt2fw_b200", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
                     "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + tlib])
     if verbose:
         print(" ".join(cmd))

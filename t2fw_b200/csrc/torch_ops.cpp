@@ -5,6 +5,8 @@
 // stream, and forwards raw pointers to the C ABI in include/t2fw_b200.h.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 
@@ -12,6 +14,9 @@
 #include <vector>
 
 #include "t2fw_b200.h"
+#include "torch_ops.h"
+
+namespace t2fw_ops {
 
 namespace {
 
@@ -47,16 +52,24 @@ int64_t ckpt_interval(int64_t T, int64_t D, int64_t K, int dtype) {
   return t2fw_lfw_default_ckpt_every(T, D, K, dtype);
 }
 
-at::Tensor make_scratch(size_t bytes, const at::Tensor &like) {
-  if (bytes == 0) return at::Tensor();
-  return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte));
+// Uninitialised tensors of `like`'s device straight from the caching allocator: a call makes up to seven
+// of them, and each trip through the dispatcher costs about as much host time as a kernel launch.
+at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dtype, const at::Tensor &like) {
+  return at::Tensor(at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt));
+}
+at::Tensor new_like(const at::Tensor &t) { return new_tensor(t.sizes(), t.scalar_type(), t); }
+
+// Scratch of one call: freed when the call returns, which the caching allocator orders on the stream.
+c10::DataPtr make_scratch(size_t bytes) {
+  if (bytes == 0) return c10::DataPtr();
+  return c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
 }
 
-void *ptr_or_null(const at::Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; }
+}  // namespace
 
 // ---- decay rule ---------------------------------------------------------------------------
-std::vector<at::Tensor> lfw_forward(at::Tensor x, at::Tensor f, at::Tensor query, at::Tensor key,
-                                    at::Tensor f_key, at::Tensor state) {
+std::vector<at::Tensor> lfw_forward(const at::Tensor &x, const at::Tensor &f, const at::Tensor &query, const at::Tensor &key,
+                                    const at::Tensor &f_key, const at::Tensor &state) {
   T2FW_CHECK_INPUT(x);
   T2FW_CHECK_INPUT(f);
   T2FW_CHECK_INPUT(query);
@@ -77,23 +90,23 @@ std::vector<at::Tensor> lfw_forward(at::Tensor x, at::Tensor f, at::Tensor query
   const int dt = dtype_code(x);
   const int64_t C = ckpt_interval(T, D, K, dt);
   const int64_t slots = t2fw_lfw_ckpt_slots(T, C);
-  at::Tensor outputs = at::empty({B, T, D}, x.options());
-  at::Tensor ckpt = at::empty({B, slots, D, K}, x.options());
+  at::Tensor outputs = new_tensor({B, T, D}, x.scalar_type(), x);
+  at::Tensor ckpt = new_tensor({B, slots, D, K}, x.scalar_type(), x);
   const size_t sb = t2fw_lfw_forward_scratch_bytes(B, T, D, K, dt, C);
-  at::Tensor scratch = make_scratch(sb, x);
+  const c10::DataPtr scratch = make_scratch(sb);
   auto stream = at::cuda::getCurrentCUDAStream();
   check_status(t2fw_lfw_forward(x.data_ptr(), f.data_ptr(), query.data_ptr(), key.data_ptr(),
                                 f_key.data_ptr(), state.data_ptr(), outputs.data_ptr(),
-                                ckpt.data_ptr(), B, T, D, K, dt, C, ptr_or_null(scratch), sb,
+                                ckpt.data_ptr(), B, T, D, K, dt, C, scratch.get(), sb,
                                 stream.stream()),
                "lfw.forward");
   return {outputs, ckpt};
 }
 
-std::vector<at::Tensor> lfw_backward(at::Tensor grad_output, at::Tensor grad_state,
-                                     at::Tensor value, at::Tensor forget, at::Tensor query,
-                                     at::Tensor key, at::Tensor f_key, at::Tensor outputs,
-                                     at::Tensor state, at::Tensor ckpt_states) {
+std::vector<at::Tensor> lfw_backward(const at::Tensor &grad_output, const at::Tensor &grad_state,
+                                     const at::Tensor &value, const at::Tensor &forget, const at::Tensor &query,
+                                     const at::Tensor &key, const at::Tensor &f_key, const at::Tensor &outputs,
+                                     const at::Tensor &state, const at::Tensor &ckpt_states) {
   T2FW_CHECK_INPUT(grad_output);
   T2FW_CHECK_INPUT(grad_state);
   T2FW_CHECK_INPUT(value);
@@ -126,18 +139,18 @@ std::vector<at::Tensor> lfw_backward(at::Tensor grad_output, at::Tensor grad_sta
               "ckpt_states does not match the checkpoint interval in use");
   // separate allocations: views of one buffer would be flagged by autograd when a caller later
   // modifies a gradient in place
-  at::Tensor d_x = at::empty_like(value), d_f = at::empty_like(forget);
-  at::Tensor d_q = at::empty_like(query), d_k = at::empty_like(key), d_fk = at::empty_like(f_key);
-  at::Tensor d_s = at::empty_like(state);
+  at::Tensor d_x = new_like(value), d_f = new_like(forget);
+  at::Tensor d_q = new_like(query), d_k = new_like(key), d_fk = new_like(f_key);
+  at::Tensor d_s = new_like(state);
   const size_t sb = t2fw_lfw_backward_scratch_bytes(B, T, D, K, dt, C);
-  at::Tensor scratch = make_scratch(sb, value);
+  const c10::DataPtr scratch = make_scratch(sb);
   auto stream = at::cuda::getCurrentCUDAStream();
   check_status(t2fw_lfw_backward(grad_output.data_ptr(), grad_state.data_ptr(), value.data_ptr(),
                                  forget.data_ptr(), query.data_ptr(), key.data_ptr(),
                                  f_key.data_ptr(), state.data_ptr(), ckpt_states.data_ptr(),
                                  d_x.data_ptr(), d_f.data_ptr(), d_q.data_ptr(), d_k.data_ptr(),
                                  d_fk.data_ptr(), d_s.data_ptr(), B, T, D, K, dt, C,
-                                 ptr_or_null(scratch), sb, stream.stream()),
+                                 scratch.get(), sb, stream.stream()),
                "lfw.backward");
   return {d_x, d_f, d_q, d_k, d_fk, d_s};
 }
@@ -146,8 +159,8 @@ std::vector<at::Tensor> lfw_backward(at::Tensor grad_output, at::Tensor grad_sta
 // written, nothing is allocated, so a loop that alternates two state buffers can be captured in a
 // CUDA graph and replayed.  Additive: the reference has no counterpart (its recurrent use is
 // LFWFunction.apply with the returned state fed back, t2fw/functional_lfw.py:65).
-void lfw_decode_step(at::Tensor x, at::Tensor f, at::Tensor query, at::Tensor key, at::Tensor f_key,
-                     at::Tensor state_in, at::Tensor state_out, at::Tensor outputs) {
+void lfw_decode_step(const at::Tensor &x, const at::Tensor &f, const at::Tensor &query, const at::Tensor &key, const at::Tensor &f_key,
+                     const at::Tensor &state_in, const at::Tensor &state_out, const at::Tensor &outputs) {
   T2FW_CHECK_INPUT(x);
   T2FW_CHECK_INPUT(f);
   T2FW_CHECK_INPUT(query);
@@ -180,7 +193,7 @@ void lfw_decode_step(at::Tensor x, at::Tensor f, at::Tensor query, at::Tensor ke
 
 // Fused decay-rule layer (d_head = 64): heads are read in place from the projection output
 // qkvg [B,T,4*H*64] = query | key | value | gate; returns {outputs [B,T,H*64], ckpt_states}.
-std::vector<at::Tensor> lfw_fused_forward(at::Tensor qkvg, at::Tensor state, int64_t n_head) {
+std::vector<at::Tensor> lfw_fused_forward(const at::Tensor &qkvg, const at::Tensor &state, int64_t n_head) {
   T2FW_CHECK_INPUT(qkvg);
   T2FW_CHECK_INPUT(state);
   TORCH_CHECK(qkvg.dim() == 3 && state.dim() == 3 && n_head > 0, "expected qkvg [B,T,4*H*64], state [B*H,64,64]");
@@ -191,19 +204,19 @@ std::vector<at::Tensor> lfw_fused_forward(at::Tensor qkvg, at::Tensor state, int
   TORCH_CHECK(B > 0 && T > 0, "empty tensors are not supported");
   const c10::cuda::CUDAGuard guard(qkvg.device());
   const int dt = dtype_code(qkvg);
-  at::Tensor outputs = at::empty({B, T, H * 64}, qkvg.options());
-  at::Tensor ckpt = at::empty({B * H, t2fw_lfw_ckpt_slots(T, 64), 64, 64}, qkvg.options());
+  at::Tensor outputs = new_tensor({B, T, H * 64}, qkvg.scalar_type(), qkvg);
+  at::Tensor ckpt = new_tensor({B * H, t2fw_lfw_ckpt_slots(T, 64), 64, 64}, qkvg.scalar_type(), qkvg);
   const size_t sb = t2fw_lfw_fused_scratch_bytes(B, T, H, dt);
-  at::Tensor scratch = make_scratch(sb, qkvg);
+  const c10::DataPtr scratch = make_scratch(sb);
   auto stream = at::cuda::getCurrentCUDAStream();
   check_status(t2fw_lfw_fused_forward(qkvg.data_ptr(), state.data_ptr(), outputs.data_ptr(), ckpt.data_ptr(), B, T, H,
-                                      dt, ptr_or_null(scratch), sb, stream.stream()),
+                                      dt, scratch.get(), sb, stream.stream()),
                "lfw.fused_forward");
   return {outputs, ckpt};
 }
 
-std::vector<at::Tensor> lfw_fused_backward(at::Tensor grad_output, at::Tensor grad_state, at::Tensor qkvg,
-                                           at::Tensor state, at::Tensor ckpt_states, int64_t n_head) {
+std::vector<at::Tensor> lfw_fused_backward(const at::Tensor &grad_output, const at::Tensor &grad_state, const at::Tensor &qkvg,
+                                           const at::Tensor &state, const at::Tensor &ckpt_states, int64_t n_head) {
   T2FW_CHECK_INPUT(grad_output);
   T2FW_CHECK_INPUT(grad_state);
   T2FW_CHECK_INPUT(qkvg);
@@ -224,24 +237,24 @@ std::vector<at::Tensor> lfw_fused_backward(at::Tensor grad_output, at::Tensor gr
   check_same(state, qkvg, "state"); check_same(ckpt_states, qkvg, "ckpt_states");
   const c10::cuda::CUDAGuard guard(qkvg.device());
   const int dt = dtype_code(qkvg);
-  at::Tensor d_qkvg = at::empty_like(qkvg), d_state = at::empty_like(state);
+  at::Tensor d_qkvg = new_like(qkvg), d_state = new_like(state);
   const size_t sb = t2fw_lfw_fused_scratch_bytes(B, T, H, dt);
-  at::Tensor scratch = make_scratch(sb, qkvg);
+  const c10::DataPtr scratch = make_scratch(sb);
   auto stream = at::cuda::getCurrentCUDAStream();
   check_status(t2fw_lfw_fused_backward(grad_output.data_ptr(), grad_state.data_ptr(), qkvg.data_ptr(), state.data_ptr(),
                                        ckpt_states.data_ptr(), d_qkvg.data_ptr(), d_state.data_ptr(), B, T, H, dt,
-                                       ptr_or_null(scratch), sb, stream.stream()),
+                                       scratch.get(), sb, stream.stream()),
                "lfw.fused_backward");
   return {d_qkvg, d_state};
 }
 
 // ---- delta rule ---------------------------------------------------------------------------
-at::ScalarType acc_type(const at::Tensor &t) {
+static at::ScalarType acc_type(const at::Tensor &t) {
   return t.scalar_type() == at::kDouble ? at::kDouble : at::kFloat;
 }
 
-std::vector<at::Tensor> dfw_forward(at::Tensor query, at::Tensor key, at::Tensor value,
-                                    at::Tensor state) {
+std::vector<at::Tensor> dfw_forward(const at::Tensor &query, const at::Tensor &key, const at::Tensor &value,
+                                    const at::Tensor &state) {
   T2FW_CHECK_INPUT(query);
   T2FW_CHECK_INPUT(key);
   T2FW_CHECK_INPUT(value);
@@ -255,24 +268,23 @@ std::vector<at::Tensor> dfw_forward(at::Tensor query, at::Tensor key, at::Tensor
 
   const c10::cuda::CUDAGuard guard(value.device());
   const int dt = dtype_code(value);
-  at::Tensor outputs = at::empty_like(value);
-  at::Tensor final_state = at::empty_like(state);
-  at::Tensor delta = at::empty({B, T, D}, value.options().dtype(acc_type(value)));
+  at::Tensor outputs = new_like(value);
+  at::Tensor final_state = new_like(state);
+  at::Tensor delta = new_tensor({B, T, D}, acc_type(value), value);
   auto stream = at::cuda::getCurrentCUDAStream();
   const size_t sb = t2fw_dfw_forward_scratch_bytes(B, T, D, M, dt);
-  at::Tensor scratch;
-  if (sb) scratch = at::empty({(int64_t)sb}, value.options().dtype(at::kByte));
+  const c10::DataPtr scratch = make_scratch(sb);
   check_status(t2fw_dfw_forward_ws(query.data_ptr(), key.data_ptr(), value.data_ptr(),
                                    state.data_ptr(), outputs.data_ptr(), final_state.data_ptr(),
-                                   delta.data_ptr(), B, T, D, M, dt, sb ? scratch.data_ptr() : nullptr, sb,
+                                   delta.data_ptr(), B, T, D, M, dt, scratch.get(), sb,
                                    stream.stream()),
                "dfw.forward");
   return {outputs, final_state, delta};
 }
 
-std::vector<at::Tensor> dfw_backward(at::Tensor grad_output, at::Tensor grad_state,
-                                     at::Tensor query, at::Tensor key, at::Tensor delta_value,
-                                     at::Tensor final_state) {
+std::vector<at::Tensor> dfw_backward(const at::Tensor &grad_output, const at::Tensor &grad_state,
+                                     const at::Tensor &query, const at::Tensor &key, const at::Tensor &delta_value,
+                                     const at::Tensor &final_state) {
   T2FW_CHECK_INPUT(grad_output);
   T2FW_CHECK_INPUT(grad_state);
   T2FW_CHECK_INPUT(query);
@@ -295,15 +307,15 @@ std::vector<at::Tensor> dfw_backward(at::Tensor grad_output, at::Tensor grad_sta
 
   const c10::cuda::CUDAGuard guard(query.device());
   const int dt = dtype_code(query);
-  at::Tensor d_q = at::empty_like(query), d_k = at::empty_like(key);
-  at::Tensor d_v = at::empty_like(grad_output), d_s = at::empty_like(final_state);
+  at::Tensor d_q = new_like(query), d_k = new_like(key);
+  at::Tensor d_v = new_like(grad_output), d_s = new_like(final_state);
   const size_t sb = t2fw_dfw_backward_scratch_bytes(B, T, D, M, dt);
-  at::Tensor scratch = make_scratch(sb, query);
+  const c10::DataPtr scratch = make_scratch(sb);
   auto stream = at::cuda::getCurrentCUDAStream();
   check_status(t2fw_dfw_backward(grad_output.data_ptr(), grad_state.data_ptr(), query.data_ptr(),
                                  key.data_ptr(), delta_value.data_ptr(), final_state.data_ptr(),
                                  d_q.data_ptr(), d_k.data_ptr(), d_v.data_ptr(), d_s.data_ptr(), B,
-                                 T, D, M, dt, ptr_or_null(scratch), sb, stream.stream()),
+                                 T, D, M, dt, scratch.get(), sb, stream.stream()),
                "dfw.backward");
   return {d_q, d_k, d_v, d_s};
 }
@@ -311,7 +323,7 @@ std::vector<at::Tensor> dfw_backward(at::Tensor grad_output, at::Tensor grad_sta
 // What a sequence segment does to the state (backward = false: inputs value, forget, key, f_key) or
 // to the state gradient (backward = true: grad_output, forget, query, f_key), D = K = 64, 16-bit:
 // {end_state [B,64,64], decay_d [B,64] fp32, decay_k [B,64] fp32}.  See t2fw_lfw_segment_summary.
-std::vector<at::Tensor> lfw_segment_summary(at::Tensor val_d, at::Tensor gate_d, at::Tensor val_k, at::Tensor gate_k,
+std::vector<at::Tensor> lfw_segment_summary(const at::Tensor &val_d, const at::Tensor &gate_d, const at::Tensor &val_k, const at::Tensor &gate_k,
                                             bool backward) {
   T2FW_CHECK_INPUT(val_d);
   T2FW_CHECK_INPUT(gate_d);
@@ -328,16 +340,16 @@ std::vector<at::Tensor> lfw_segment_summary(at::Tensor val_d, at::Tensor gate_d,
   TORCH_CHECK(B > 0 && T > 0, "empty tensors are not supported");
   const c10::cuda::CUDAGuard guard(val_d.device());
   const int dt = dtype_code(val_d);
-  at::Tensor end_state = at::empty({B, D, K}, val_d.options());
-  at::Tensor decay_d = at::empty({B, D}, val_d.options().dtype(at::kFloat));
-  at::Tensor decay_k = at::empty({B, K}, val_d.options().dtype(at::kFloat));
+  at::Tensor end_state = new_tensor({B, D, K}, val_d.scalar_type(), val_d);
+  at::Tensor decay_d = new_tensor({B, D}, at::kFloat, val_d);
+  at::Tensor decay_k = new_tensor({B, K}, at::kFloat, val_d);
   const size_t sb = t2fw_lfw_segment_summary_scratch_bytes(B, T, D, K, dt);
   TORCH_CHECK(sb != 0, "lfw.segment_summary: D = K = 64 and fp16 / bf16 only");
-  at::Tensor scratch = make_scratch(sb, val_d);
+  const c10::DataPtr scratch = make_scratch(sb);
   auto stream = at::cuda::getCurrentCUDAStream();
   check_status(t2fw_lfw_segment_summary(backward ? 1 : 0, val_d.data_ptr(), gate_d.data_ptr(), val_k.data_ptr(),
                                         gate_k.data_ptr(), end_state.data_ptr(), decay_d.data_ptr<float>(),
-                                        decay_k.data_ptr<float>(), B, T, D, K, dt, ptr_or_null(scratch), sb,
+                                        decay_k.data_ptr<float>(), B, T, D, K, dt, scratch.get(), sb,
                                         stream.stream()),
                "lfw.segment_summary");
   return {end_state, decay_d, decay_k};
@@ -346,7 +358,7 @@ std::vector<at::Tensor> lfw_segment_summary(at::Tensor val_d, at::Tensor gate_d,
 // Fold of gathered segment summaries [n][B][D*K+D+K] (fp32) over `start` [B,D,K] (fp32):
 // {state entering segment `segment`, state after the last segment} (backward = false) or
 // {state gradient at the end of `segment`} (backward = true).  See t2fw_lfw_fold_summaries.
-std::vector<at::Tensor> lfw_fold_summaries(at::Tensor gathered, at::Tensor start, int64_t segment, bool backward) {
+std::vector<at::Tensor> lfw_fold_summaries(const at::Tensor &gathered, const at::Tensor &start, int64_t segment, bool backward) {
   T2FW_CHECK_INPUT(gathered);
   T2FW_CHECK_INPUT(start);
   TORCH_CHECK(gathered.scalar_type() == at::kFloat && start.scalar_type() == at::kFloat,
@@ -357,8 +369,8 @@ std::vector<at::Tensor> lfw_fold_summaries(at::Tensor gathered, at::Tensor start
               "fold_summaries: tensor shapes or devices do not agree");
   TORCH_CHECK(n > 0 && n < (1 << 20) && segment >= 0 && segment < n, "fold_summaries: segment out of range");
   const c10::cuda::CUDAGuard guard(start.device());
-  at::Tensor at_seg = at::empty_like(start);
-  at::Tensor total = backward ? at::Tensor() : at::empty_like(start);
+  at::Tensor at_seg = new_like(start);
+  at::Tensor total = backward ? at::Tensor() : new_like(start);
   auto stream = at::cuda::getCurrentCUDAStream();
   check_status(t2fw_lfw_fold_summaries(backward ? 1 : 0, gathered.data_ptr<float>(), start.data_ptr<float>(),
                                        at_seg.data_ptr<float>(), backward ? nullptr : total.data_ptr<float>(), (int)n,
@@ -368,7 +380,9 @@ std::vector<at::Tensor> lfw_fold_summaries(at::Tensor gathered, at::Tensor start
   return {at_seg, total};
 }
 
-}  // namespace
+}  // namespace t2fw_ops
+
+using namespace t2fw_ops;
 
 TORCH_LIBRARY(lfw, m) {
   m.def("forward", lfw_forward);

@@ -16,13 +16,14 @@ import torch
 
 from . import _lib
 
-_lib.load_ops()
+_ops = _lib.load_ops()
 
 
 def lfw_decode_step(x, f, query, key, f_key, state_in, state_out, outputs):
     """o = S' q with S' = (f f_key^T) * S + x key^T; writes `outputs` [B,1,D] and `state_out` [B,D,K].
     `state_out` must be a different buffer from `state_in`."""
-    torch.ops.lfw.decode_step(x, f, query, key, f_key, state_in, state_out, outputs)
+    if _ops.decode_step(x, f, query, key, f_key, state_in, state_out, outputs) is NotImplemented:
+        torch.ops.lfw.decode_step(x, f, query, key, f_key, state_in, state_out, outputs)
     return outputs, state_out
 
 

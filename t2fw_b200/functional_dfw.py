@@ -14,7 +14,7 @@ import torch
 
 from . import _lib
 
-_lib.load_ops()
+_ops = _lib.load_ops()
 
 
 class DFWFunction(torch.autograd.Function):
@@ -38,3 +38,6 @@ class DFWFunction(torch.autograd.Function):
         grads = torch.ops.dfw.backward(grad_output.contiguous(), grad_state.contiguous(),
                                        query, key, delta_value, final_state)
         return tuple(grads)
+
+
+_lib.bind_apply(DFWFunction, _lib.DFW, _ops.dfw_apply)

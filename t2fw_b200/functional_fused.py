@@ -15,7 +15,7 @@ import torch
 
 from . import _lib
 
-_lib.load_ops()
+_ops = _lib.load_ops()
 
 GATE_FLOOR = 0.125
 
@@ -39,6 +39,9 @@ class LFWFusedFunction(torch.autograd.Function):
         d_qkvg, d_state = torch.ops.lfw.fused_backward(grad_output.contiguous(), grad_state.contiguous(), qkvg,
                                                        state, ckpt, ctx.n_head)
         return d_qkvg, d_state, None
+
+
+_lib.bind_apply(LFWFusedFunction, _lib.FUSED, _ops.fused_apply)
 
 
 def unfused_reference(qkvg, state, n_head):

@@ -15,7 +15,7 @@ import torch
 
 from . import _lib
 
-_lib.load_ops()
+_ops = _lib.load_ops()
 
 
 class LFWFunction(torch.autograd.Function):
@@ -43,3 +43,6 @@ class LFWFunction(torch.autograd.Function):
                                        value, forget, query, key, f_key, outputs, state,
                                        ckpt_states)
         return tuple(grads)
+
+
+_lib.bind_apply(LFWFunction, _lib.LFW, _ops.lfw_apply)
