@@ -95,6 +95,14 @@ int t2fw_lfw_forward(const void *x, const void *f, const void *q, const void *k,
                      int64_t B, int64_t T, int64_t D, int64_t K, int dtype, int64_t ckpt_every,
                      void *scratch, size_t scratch_bytes, void *stream);
 
+/* n chained decode steps (T = 1 calls that feed the state on, each rounding it to the storage type) in one launch:
+ * x, f, outputs [n, B, D], q, k, f_key [n, B, K], state and new_state [B, D, K] (new_state may be state).
+ * 16-bit storage, K = 32, 64 or 128, D a multiple of 8, 16-byte aligned pointers; T2FW_ERR_UNSUPPORTED otherwise.
+ * Bit-identical to n t2fw_lfw_forward calls with T = 1.  Additive: the reference loops over its T = 1 call. */
+int t2fw_lfw_decode_steps(const void *x, const void *f, const void *q, const void *k, const void *f_key,
+                          const void *state, void *outputs, void *new_state, int64_t n, int64_t B, int64_t D,
+                          int64_t K, int dtype, void *stream);
+
 /*
  * Decay rule backward: all six gradients in forward-argument order.
  * Replaces torch.ops.lfw.backward = lfw_backward (t2fw/csrc/lfw.cpp:50-96), i.e. the reverse

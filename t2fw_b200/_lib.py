@@ -21,7 +21,7 @@ EXPORTS = (
     "t2fw_lfw_default_ckpt_every", "t2fw_lfw_ckpt_slots",
     "t2fw_lfw_forward_scratch_bytes", "t2fw_lfw_backward_scratch_bytes",
     "t2fw_dfw_backward_scratch_bytes",
-    "t2fw_lfw_forward", "t2fw_lfw_backward", "t2fw_dfw_forward", "t2fw_dfw_backward",
+    "t2fw_lfw_forward", "t2fw_lfw_decode_steps", "t2fw_lfw_backward", "t2fw_dfw_forward", "t2fw_dfw_backward",
     "t2fw_dfw_forward_ws", "t2fw_dfw_forward_scratch_bytes",
     "t2fw_dfw_backward_noalloc_max_elems", "t2fw_dfw_backward_noalloc",
     "t2fw_lfw_fused_scratch_bytes", "t2fw_lfw_fused_forward", "t2fw_lfw_fused_backward",
@@ -67,6 +67,8 @@ def load_core():
     lib.t2fw_dfw_forward_ws.argtypes = [_vp] * 7 + [_i64] * 4 + [_int, _vp, _sz, _vp]
     lib.t2fw_lfw_forward.restype = _int
     lib.t2fw_lfw_forward.argtypes = [_vp] * 8 + [_i64] * 4 + [_int, _i64, _vp, _sz, _vp]
+    lib.t2fw_lfw_decode_steps.restype = _int
+    lib.t2fw_lfw_decode_steps.argtypes = [_vp] * 8 + [_i64] * 4 + [_int, _vp]
     lib.t2fw_lfw_backward.restype = _int
     lib.t2fw_lfw_backward.argtypes = [_vp] * 15 + [_i64] * 4 + [_int, _i64, _vp, _sz, _vp]
     lib.t2fw_dfw_forward.restype = _int

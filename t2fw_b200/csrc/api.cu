@@ -127,6 +127,17 @@ static bool aligned16(std::initializer_list<const void *> ps) {
   return (acc & 15u) == 0;
 }
 
+// Longest sequences that are walked step by step (steps.cu) instead of in 64-step chunks, measured over 1 to 4096
+// rows: below a whole chunk the decay rule's three chunk kernels never win (96 x 48: 19.8 us against 14.5, 2048 x 48:
+// 205 against 105), and a whole chunk is left to them so that their ragged tail stays the only other case; the delta
+// rule's step waits for a row sum, so its one-chunk kernels catch up at about 48 steps (16.4 us both at 96 rows).
+constexpr int64_t kLfwStepsMax = 63;
+constexpr int64_t kDfwStepsMax = 48;
+// Largest state (elements) for which a single decode step takes the step kernel: while state and vectors come from
+// L2 its many small CTAs start faster (96 rows of 128 x 128: 2.6 us against 5.2), beyond that the bulk-copy ring
+// streams better (4096 rows of 64 x 64 from HBM: 14.1 us against 16.0).
+constexpr int64_t kOneStepMaxElems = 8ll << 20;
+
 static int check_common(int64_t B, int64_t T, int64_t D, int64_t K, int dtype) {
   T2FW_CHECK_ARG(dtype_size(dtype) != 0, "unknown dtype %d", dtype);
   T2FW_CHECK_ARG(B > 0 && T > 0 && D > 0 && K > 0, "sizes must be positive (B=%lld T=%lld D=%lld K=%lld)",
@@ -147,6 +158,9 @@ int t2fw_lfw_forward(const void *x, const void *f, const void *q, const void *k,
   T2FW_CHECK_ARG(x && f && q && k && f_key && state && outputs && ckpt_states, "null pointer argument");
   T2FW_CHECK_ARG(ckpt_every > 0, "ckpt_every must be positive");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (T == 1 && B * D * K <= kOneStepMaxElems && steps_supported(B, D, K, dtype) && decode_bulk_enabled() &&
+      aligned16({x, f, q, k, f_key, state, outputs, ckpt_states}))
+    return lfw_steps_forward(x, f, q, k, f_key, state, outputs, ckpt_states, B, T, D, K, dtype, st);
   if (T == 1) {
     const bool al = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(f) |
                       reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
@@ -161,6 +175,10 @@ int t2fw_lfw_forward(const void *x, const void *f, const void *q, const void *k,
       if (rc != T2FW_ERR_UNSUPPORTED) return rc;
     }
   }
+  // one checkpoint slot and few steps: no chunk to build
+  if (T > 1 && T <= kLfwStepsMax && ckpt_every >= T && chunk_path_enabled() && steps_supported(B, D, K, dtype) &&
+      aligned16({x, f, q, k, f_key, state, outputs, ckpt_states}))
+    return lfw_steps_forward(x, f, q, k, f_key, state, outputs, ckpt_states, B, T, D, K, dtype, st);
   const size_t need = t2fw_lfw_forward_scratch_bytes(B, T, D, K, dtype, ckpt_every);
   if (need != 0 && aligned16({x, f, q, k, f_key, state, outputs, ckpt_states, scratch})) {
     if (scratch == nullptr || scratch_bytes < need) {
@@ -181,6 +199,20 @@ int t2fw_lfw_forward(const void *x, const void *f, const void *q, const void *k,
   }
   return lfw_scan_forward(x, f, q, k, f_key, state, outputs, ckpt_states, B, T, D, K, dtype,
                           ckpt_every, st);
+}
+
+int t2fw_lfw_decode_steps(const void *x, const void *f, const void *q, const void *k, const void *f_key,
+                          const void *state, void *outputs, void *new_state, int64_t n, int64_t B, int64_t D,
+                          int64_t K, int dtype, void *stream) {
+  int rc = check_common(B, n, D, K, dtype);
+  if (rc != T2FW_OK) return rc;
+  T2FW_CHECK_ARG(x && f && q && k && f_key && state && outputs && new_state, "null pointer argument");
+  if (n >= (1ll << 31) || !steps_supported(B, D, K, dtype) || !aligned16({x, f, q, k, f_key, state, outputs, new_state})) {
+    set_error("decode steps: 16-bit storage, K = 32, 64 or 128, D a multiple of 8 and 16-byte aligned pointers only "
+              "(D=%lld K=%lld dtype %d)", (long long)D, (long long)K, dtype);
+    return T2FW_ERR_UNSUPPORTED;
+  }
+  return lfw_steps_ring(x, f, q, k, f_key, state, outputs, new_state, n, B, D, K, dtype, static_cast<cudaStream_t>(stream));
 }
 
 int t2fw_lfw_backward(const void *grad_output, const void *grad_state, const void *x,
@@ -294,6 +326,9 @@ int t2fw_lfw_fused_forward(const void *qkvg, const void *state, void *outputs, v
     set_error("lfw fused forward: all pointers must be 16-byte aligned");
     return T2FW_ERR_UNSUPPORTED;
   }
+  // same rule as the plain forward, whose results this entry point repeats bit for bit
+  if (T <= kLfwStepsMax && chunk_path_enabled() && steps_supported(B * H, 64, 64, dtype))
+    return lfw_steps_fused(qkvg, state, outputs, ckpt_states, B, T, (int)H, dtype, static_cast<cudaStream_t>(stream));
   return lfw_fused_forward(qkvg, state, outputs, ckpt_states, B, T, (int)H, dtype, scratch,
                            static_cast<cudaStream_t>(stream));
 }
@@ -335,6 +370,10 @@ int t2fw_dfw_forward_ws(const void *q, const void *k, const void *v, const void 
   int rc = check_common(B, T, D, M, dtype);
   if (rc != T2FW_OK) return rc;
   T2FW_CHECK_ARG(q && k && v && state && outputs && final_state && delta, "null pointer argument");
+  if (T <= kDfwStepsMax && dfw_chunk_enabled() && steps_supported(B, D, M, dtype) &&
+      aligned16({q, k, v, state, outputs, final_state, delta}))
+    return dfw_steps_forward(q, k, v, state, outputs, final_state, delta, B, T, D, M, dtype,
+                             static_cast<cudaStream_t>(stream));
   const size_t need = t2fw_dfw_forward_scratch_bytes(B, T, D, M, dtype);
   if (need != 0 && aligned16({q, k, v, state, outputs, final_state, delta, scratch})) {
     if (scratch == nullptr || scratch_bytes < need) {

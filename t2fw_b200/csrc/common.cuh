@@ -181,6 +181,16 @@ int lfw_decode_bulk_forward(const void *x, const void *f, const void *q, const v
                             const void *fk, const void *state, void *out, void *new_state,
                             int64_t B, int64_t D, int64_t K, int dtype, cudaStream_t st);
 int lfw_decode_bulk_status();
+// sequences walked step by step with the state in registers (steps.cu), 16-bit storage
+bool steps_supported(int64_t B, int64_t D, int64_t K, int dtype);
+int lfw_steps_ring(const void *x, const void *f, const void *q, const void *k, const void *fk, const void *state,
+                   void *out, void *next, int64_t n, int64_t B, int64_t D, int64_t K, int dtype, cudaStream_t st);
+int lfw_steps_forward(const void *x, const void *f, const void *q, const void *k, const void *fk, const void *state,
+                      void *out, void *next, int64_t B, int64_t T, int64_t D, int64_t K, int dtype, cudaStream_t st);
+int lfw_steps_fused(const void *qkvg, const void *state, void *out, void *next, int64_t B, int64_t T, int H, int dtype,
+                    cudaStream_t st);
+int dfw_steps_forward(const void *q, const void *k, const void *v, const void *state, void *out, void *fin, void *delta,
+                      int64_t B, int64_t T, int64_t D, int64_t M, int dtype, cudaStream_t st);
 bool lfw_decode_supported(int64_t D, int64_t K, int dtype);
 int lfw_decode_forward(const void *x, const void *f, const void *q, const void *k, const void *fk,
                        const void *state, void *out, void *new_state, int64_t B, int64_t D,

@@ -10,7 +10,7 @@
 //
 // Every wait on an mbarrier is bounded: if it does not complete within kSpinLimit polls the CTA
 // records the failure in *status and leaves after draining its own outstanding copies.
-#include "common.cuh"
+#include "steps.cuh"
 
 namespace t2fw {
 
@@ -69,44 +69,6 @@ __device__ __forceinline__ void bulk_wait_read() {
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-template <typename T> struct Cvt8;
-template <> struct Cvt8<__half> {
-  static __device__ __forceinline__ void unpack(const uint4 &u, float (&v)[8]) {
-    const __half2 *h = reinterpret_cast<const __half2 *>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 p = __half22float2(h[i]);
-      v[2 * i] = p.x;
-      v[2 * i + 1] = p.y;
-    }
-  }
-  static __device__ __forceinline__ uint4 pack(const float (&v)[8]) {
-    uint4 u;
-    __half2 *h = reinterpret_cast<__half2 *>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-    return u;
-  }
-};
-template <> struct Cvt8<__nv_bfloat16> {
-  static __device__ __forceinline__ void unpack(const uint4 &u, float (&v)[8]) {
-    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 p = __bfloat1622float2(h[i]);
-      v[2 * i] = p.x;
-      v[2 * i + 1] = p.y;
-    }
-  }
-  static __device__ __forceinline__ uint4 pack(const float (&v)[8]) {
-    uint4 u;
-    __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-    return u;
-  }
-};
-
 // Stage layout (bytes): state [D*K*2] | fk [K*2] | k [K*2] | q [K*2] | x [D*2] | f [D*2] | out [D*2]
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
@@ -132,6 +94,7 @@ lfw_decode_bulk_kernel(const T *__restrict__ x, const T *__restrict__ f, const T
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  dependency_wait();      // a chain of steps: this launch's prologue overlaps the step before
 
   auto issue_load = [&](int item) {
     const int64_t b = (int64_t)blockIdx.x + (int64_t)item * gridDim.x;
@@ -165,23 +128,18 @@ lfw_decode_bulk_kernel(const T *__restrict__ x, const T *__restrict__ f, const T
     const T *sf = reinterpret_cast<const T *>(st + sbytes + 3 * kbytes + dbytes);
     T *so = reinterpret_cast<T *>(st + sbytes + 3 * kbytes + 2 * dbytes);
 
-    float g[8], kk[8], qq[8];
-    Cvt8<T>::unpack(reinterpret_cast<const uint4 *>(sfk)[kc], g);
-    Cvt8<T>::unpack(reinterpret_cast<const uint4 *>(sk)[kc], kk);
-    Cvt8<T>::unpack(reinterpret_cast<const uint4 *>(sq)[kc], qq);
+    steps::f2 g[4], kk[4], qq[4];
+    steps::Oct<T>::unpack(reinterpret_cast<const uint4 *>(sfk)[kc], g);
+    steps::Oct<T>::unpack(reinterpret_cast<const uint4 *>(sk)[kc], kk);
+    steps::Oct<T>::unpack(reinterpret_cast<const uint4 *>(sq)[kc], qq);
     for (int base = 0; base < D; base += RP) {
       const int row = base + rr;
       const bool in = row < D;
-      float sv[8];
-      Cvt8<T>::unpack(in ? sst[row * KT + kc] : make_uint4(0, 0, 0, 0), sv);
+      steps::f2 sv[4];
+      steps::Oct<T>::unpack(in ? sst[row * KT + kc] : make_uint4(0, 0, 0, 0), sv);
       const float xs = in ? Elem<T>::ld(sx + row) : 0.f, as = in ? Elem<T>::ld(sf + row) : 0.f;
-      float acc = 0.f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        sv[e] = sv[e] * (as * g[e]) + xs * kk[e];
-        acc += sv[e] * qq[e];
-      }
-      if (in) sst[row * KT + kc] = Cvt8<T>::pack(sv);
+      float acc = steps::decay_step8(sv, g, kk, qq, steps::pack2(xs, xs), steps::pack2(as, as));
+      if (in) sst[row * KT + kc] = steps::Oct<T>::pack(sv);
       for (int o = KT >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
       if (in && kc == 0) Elem<T>::st(so + row, acc);
     }
@@ -260,17 +218,13 @@ int lfw_decode_bulk_forward(const void *x, const void *f, const void *q, const v
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     g_attr_set[dev][ti] = true;
   }
-  if (dtype == T2FW_F16) {
-    lfw_decode_bulk_kernel<__half><<<(unsigned)grid, kThreads, smem, st>>>(
-        (const __half *)x, (const __half *)f, (const __half *)q, (const __half *)k,
-        (const __half *)fk, (const __half *)state, (__half *)out, (__half *)new_state, (int)B,
-        (int)D, (int)K, stage, status);
-  } else {
-    lfw_decode_bulk_kernel<__nv_bfloat16><<<(unsigned)grid, kThreads, smem, st>>>(
-        (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)f, (const __nv_bfloat16 *)q,
-        (const __nv_bfloat16 *)k, (const __nv_bfloat16 *)fk, (const __nv_bfloat16 *)state,
-        (__nv_bfloat16 *)out, (__nv_bfloat16 *)new_state, (int)B, (int)D, (int)K, stage, status);
-  }
+#define T2FW_LAUNCH(TT)                                                                                         \
+  T2FW_CHECK_CUDA(launch_dependent(lfw_decode_bulk_kernel<TT>, dim3((unsigned)grid), dim3(kThreads), smem, st,   \
+                                   (const TT *)x, (const TT *)f, (const TT *)q, (const TT *)k, (const TT *)fk,   \
+                                   (const TT *)state, (TT *)out, (TT *)new_state, (int)B, (int)D, (int)K, stage, \
+                                   status))
+  if (dtype == T2FW_F16) T2FW_LAUNCH(__half); else T2FW_LAUNCH(__nv_bfloat16);
+#undef T2FW_LAUNCH
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;
 }

@@ -234,6 +234,22 @@ PyObject *py_decode_step(PyObject *, PyObject *const *args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// decode_ring(x, f, query, key, f_key, state, outputs): whether the whole ring was done in one launch
+PyObject *py_decode_ring(PyObject *, PyObject *const *args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  bool ok = n == 7 && plain_mode();
+  for (int i = 0; ok && i < 7; ++i) ok = plain_tensor(args[i]);
+  if (!ok) Py_RETURN_FALSE;
+  const Tensor *t[7];
+  for (int i = 0; i < 7; ++i) t[i] = &THPVariable_Unpack(args[i]);
+  {
+    pybind11::gil_scoped_release no_gil;
+    ok = t2fw_ops::lfw_decode_ring(*t[0], *t[1], *t[2], *t[3], *t[4], *t[5], *t[6]);
+  }
+  return PyBool_FromLong(ok);
+  END_HANDLE_TH_ERRORS
+}
+
 // set_fallback(which, callable): 0 LFWFunction, 1 DFWFunction, 2 LFWFusedFunction
 PyObject *py_set_fallback(PyObject *, PyObject *const *args, Py_ssize_t n) {
   const long w = n == 2 ? PyLong_AsLong(args[0]) : -1;
@@ -252,6 +268,7 @@ PyMethodDef g_methods[] = {
     T2FW_METHOD("dfw_apply", py_dfw_apply, "apply(query, key, value, state) -> (outputs, final_state)"),
     T2FW_METHOD("fused_apply", py_fused_apply, "apply(qkvg, state, n_head) -> (outputs, next_state)"),
     T2FW_METHOD("decode_step", py_decode_step, "decode_step(x, f, query, key, f_key, state_in, state_out, outputs)"),
+    T2FW_METHOD("decode_ring", py_decode_ring, "decode_ring(x, f, query, key, f_key, state, outputs) -> bool"),
     T2FW_METHOD("set_fallback", py_set_fallback, "set_fallback(which, callable)"),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "t2fw_torch_ops", "Autograd entry points of t2fw_b200.", -1, g_methods,

@@ -191,6 +191,37 @@ void lfw_decode_step(const at::Tensor &x, const at::Tensor &f, const at::Tensor 
                "lfw.decode_step");
 }
 
+// n decode steps in one launch: x, f, outputs [n,B,1,D], query, key, f_key [n,B,1,K]; `state` [B,D,K] is
+// advanced in place.  Returns false, having done nothing, for shapes and types that go step by step.
+bool lfw_decode_ring(const at::Tensor &x, const at::Tensor &f, const at::Tensor &query, const at::Tensor &key,
+                     const at::Tensor &f_key, const at::Tensor &state, const at::Tensor &outputs) {
+  T2FW_CHECK_INPUT(x);
+  T2FW_CHECK_INPUT(f);
+  T2FW_CHECK_INPUT(query);
+  T2FW_CHECK_INPUT(key);
+  T2FW_CHECK_INPUT(f_key);
+  T2FW_CHECK_INPUT(state);
+  T2FW_CHECK_INPUT(outputs);
+  TORCH_CHECK(x.dim() == 4 && x.size(2) == 1 && query.dim() == 4 && state.dim() == 3,
+              "expected x [n,B,1,D], query [n,B,1,K], state [B,D,K]");
+  const int64_t n = x.size(0), B = x.size(1), D = x.size(3), K = query.size(3);
+  TORCH_CHECK(f.sizes() == x.sizes() && outputs.sizes() == x.sizes(), "f and outputs must have x's shape");
+  TORCH_CHECK(query.size(0) == n && query.size(1) == B && query.size(2) == 1, "query must be [n,B,1,K]");
+  TORCH_CHECK(key.sizes() == query.sizes() && f_key.sizes() == query.sizes(), "key and f_key must have query's shape");
+  TORCH_CHECK(state.size(0) == B && state.size(1) == D && state.size(2) == K, "state must be [B,D,K]");
+  check_same(f, x, "f"); check_same(query, x, "query"); check_same(key, x, "key"); check_same(f_key, x, "f_key");
+  check_same(state, x, "state"); check_same(outputs, x, "outputs");
+  TORCH_CHECK(n > 0 && B > 0 && D > 0 && K > 0, "empty tensors are not supported");
+  const c10::cuda::CUDAGuard guard(x.device());
+  auto stream = at::cuda::getCurrentCUDAStream();
+  const int rc = t2fw_lfw_decode_steps(x.data_ptr(), f.data_ptr(), query.data_ptr(), key.data_ptr(), f_key.data_ptr(),
+                                       state.data_ptr(), outputs.data_ptr(), state.data_ptr(), n, B, D, K, dtype_code(x),
+                                       stream.stream());
+  if (rc == T2FW_ERR_UNSUPPORTED) return false;
+  check_status(rc, "lfw.decode_ring");
+  return true;
+}
+
 // Fused decay-rule layer (d_head = 64): heads are read in place from the projection output
 // qkvg [B,T,4*H*64] = query | key | value | gate; returns {outputs [B,T,H*64], ckpt_states}.
 std::vector<at::Tensor> lfw_fused_forward(const at::Tensor &qkvg, const at::Tensor &state, int64_t n_head) {

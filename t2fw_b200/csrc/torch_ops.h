@@ -18,6 +18,8 @@ std::vector<at::Tensor> lfw_backward(const at::Tensor &grad_output, const at::Te
 void lfw_decode_step(const at::Tensor &x, const at::Tensor &f, const at::Tensor &query, const at::Tensor &key,
                      const at::Tensor &f_key, const at::Tensor &state_in, const at::Tensor &state_out,
                      const at::Tensor &outputs);
+bool lfw_decode_ring(const at::Tensor &x, const at::Tensor &f, const at::Tensor &query, const at::Tensor &key,
+                     const at::Tensor &f_key, const at::Tensor &state, const at::Tensor &outputs);
 std::vector<at::Tensor> lfw_fused_forward(const at::Tensor &qkvg, const at::Tensor &state, int64_t n_head);
 std::vector<at::Tensor> lfw_fused_backward(const at::Tensor &grad_output, const at::Tensor &grad_state,
                                            const at::Tensor &qkvg, const at::Tensor &state,

@@ -6,9 +6,9 @@ That call allocates its outputs, so the state changes address every step.  The a
 the addresses fixed:
 
   lfw_decode_step(...)   one step into caller-owned `outputs` and `state_out`
-  LFWDecodeLoop          two alternating state buffers, a ring of input slots, and a CUDA graph
-                         over one trip round the ring, so that a decode loop costs one graph
-                         launch per `ring` steps
+  LFWDecodeLoop          a ring of input slots; one trip round the ring is one launch: a kernel that keeps
+                         the state in registers over the ring where it fits (16-bit storage, K = 32, 64
+                         or 128), else a CUDA graph of single steps over two alternating state buffers
 
 A state produced by a T > 1 call (prefill) is handed over by passing it to the constructor.
 """
@@ -28,12 +28,12 @@ def lfw_decode_step(x, f, query, key, f_key, state_in, state_out, outputs):
 
 
 class LFWDecodeLoop:
-    """Graph-replayed decode loop.
+    """Decode loop with one launch per `ring` steps.
 
     `ring` (even) input slots x, f [ring,B,1,D] and query, key, f_key [ring,B,1,K] are filled by the
     caller; `run_ring()` advances the state by `ring` steps (slot 0 first) and leaves the outputs of
-    every step in `outputs` [ring,B,1,D].  The first call runs eagerly and captures the graph; later
-    calls replay it.  `state` is the current state (a view of one of the two internal buffers)."""
+    every step in `outputs` [ring,B,1,D].  Shapes outside the one-kernel trip run eagerly in the first
+    call, which captures the graph that later calls replay.  `state` is the current state (a view of one of the two internal buffers)."""
 
     def __init__(self, state, ring=2):
         if ring < 2 or ring % 2:
@@ -64,6 +64,12 @@ class LFWDecodeLoop:
                             self._s[i & 1], self._s[(i + 1) & 1], self.outputs[i])
 
     def run_ring(self):
+        # One launch for the whole trip where the state fits a CTA's registers; launching that kernel costs
+        # the host half of what replaying a graph with one node does.
+        if self._graph is None and _ops.decode_ring(self.x, self.f, self.query, self.key, self.f_key, self._s[0],
+                                                    self.outputs):
+            self.steps += self.ring
+            return self.outputs
         if self._graph is None:
             self._trip()                                   # eager: also the warm-up before capture
             side = torch.cuda.Stream(self.x.device)
