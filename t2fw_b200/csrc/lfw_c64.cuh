@@ -62,6 +62,13 @@ __device__ __forceinline__ float rna_tf32(float v) {
 // so adding half a unit of the last kept place is enough and the mask can be left out.
 __device__ __forceinline__ float bias_tf32(float v) { return __uint_as_float(__float_as_uint(v) + 0x1000u); }
 
+// 1 / v as the hardware's approximation (about 1 ulp; denormals count as zero, which every caller has excluded)
+__device__ __forceinline__ float rcp_fast(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 __device__ __forceinline__ float sanitize_gate(float g) {
   return fabsf(g) < kTinyState ? copysignf(kTinyState, g) : g;
 }

@@ -64,6 +64,15 @@ __device__ __forceinline__ void fill_block(T *blk, float v, int tid, int nthread
   const T tv = (T)v;
   for (int i = tid; i < 64 * 64; i += nthreads) blk[i] = tv;
 }
+template <typename T>
+__device__ __forceinline__ float round_to(float v) {
+  const T r = (T)v;
+  return Elem<T>::ld(&r);
+}
+template <typename T>
+__device__ __forceinline__ float sigmoid_gate(float g) {
+  return round_to<T>(fmaxf(__fdividef(1.f, 1.f + __expf(-g)), kGateFloor));
+}
 // gate = max(sigmoid(g), 1/8), rounded to the storage type (what a separate elementwise pass
 // followed by the plain operator would have fed the kernel)
 template <typename T>
