@@ -79,6 +79,10 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
+constexpr uint32_t kIdesc64 = umma::make_idesc_tf32(64, 64, false, false);
+// descriptor offset of k-step ks (eight contraction columns) of a tile
+__device__ __forceinline__ uint64_t kstep(int ks) { return (uint64_t)(((ks >> 2) * kColBlock + (ks & 3) * 32) >> 4); }
+
 // D[64 x 32] (+)= A[64 x 64] * B[rows n0 .. n0+31][64]^T over the 64 contraction columns (8 steps of 8).
 // da, db are the descriptors of the two tiles (desc_sw128 of the tile base); a k-step or a row
 // offset only moves the start-address field, which is the low word in units of 16 bytes.
@@ -184,6 +188,32 @@ __device__ __forceinline__ Item split_item(int64_t ci, int64_t nc, int heads) {
   it.h = it.bh - it.b * heads;
   return it;
 }
+
+// Chunk indices first, first + stride, ... of a persistent CTA as (problem row, chunk), stepped without divisions.
+struct ItemWalk {
+  int bh, c;             // problem row, chunk
+  int step_bh, step_c, nc;
+  __device__ __forceinline__ ItemWalk(uint32_t first, uint32_t stride, int64_t nc_) {
+    nc = (int)nc_;
+    bh = (int)(first / (uint32_t)nc);
+    c = (int)first - bh * nc;
+    step_bh = (int)(stride / (uint32_t)nc);
+    step_c = (int)stride - step_bh * nc;
+  }
+  __device__ __forceinline__ void step() {
+    bh += step_bh;
+    c += step_c;
+    if (c >= nc) {
+      c -= nc;
+      ++bh;
+    }
+  }
+  // batch item and head of the problem row
+  __device__ __forceinline__ void row(int heads, int *b, int *h) const {
+    *b = heads == 1 ? bh : (int)((uint32_t)bh / (uint32_t)heads);
+    *h = heads == 1 ? 0 : bh - *b * heads;
+  }
+};
 
 __device__ __forceinline__ void sync_all() {
   umma::fence_before_sync();

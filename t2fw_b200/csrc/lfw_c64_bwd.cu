@@ -83,9 +83,6 @@ constexpr int cS2 = 0, cR2 = 64, cVw = 128, cMw = 192;
 constexpr int cZ = 256, cT2 = 256, cTQ1 = 320, cTQ2 = 384, cT7 = 448;
 constexpr int kTmemCols = 512;
 
-constexpr uint32_t kIdesc64 = umma::make_idesc_tf32(64, 64, false, false);
-__device__ __forceinline__ uint64_t kstep(int ks) { return (uint64_t)(((ks >> 2) * kColBlock + (ks & 3) * 32) >> 4); }
-
 // kFused = false: the plain operator (no activation flags, query scale 1), decided at compile time.
 template <typename T, bool kFused>
 __global__ void __launch_bounds__(kThreadsB, 1)
@@ -120,9 +117,10 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   const bool unit_forget = kFused && (mp.flags & seq::kUnitForget) != 0;
   const bool sigmoid_gate = kFused && (mp.flags & seq::kSigmoidGate) != 0;
   const float q_scale = kFused ? mp.q_scale : 1.f;
-  auto issue_raw = [&](int64_t ci) {     // thread 0 only: one copy per tensor
-    const Item w = split_item(ci, nc, mp.heads);
-    const int row = (int)(w.b * T_ + w.c * kC), hc = w.h;
+  auto issue_raw = [&](const ItemWalk &w) {     // thread 0 only: one copy per tensor
+    int b, hc;
+    w.row(mp.heads, &b, &hc);
+    const int row = (int)(b * T_ + w.c * kC);
     const int nv = (int)((T_ - (int64_t)w.c * kC < kC) ? T_ - (int64_t)w.c * kC : kC);
     const uint32_t per = (mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes;
     acp::mbar_expect_tx(&barRaw, (unit_forget ? 5u : 6u) * per);
@@ -132,18 +130,17 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   };
   // fused layer: the gate pre-activations once more, into the block that the constant forget gate leaves free.
   // The epilogue reads them, after the raw blocks have been handed to the next chunk.
-  auto issue_preact = [&](int64_t ci) {
-    const Item w = split_item(ci, nc, mp.heads);
+  auto issue_preact = [&](const ItemWalk &w) {
+    int b, hc;
+    w.row(mp.heads, &b, &hc);
     const int nv = (int)((T_ - (int64_t)w.c * kC < kC) ? T_ - (int64_t)w.c * kC : kC);
     acp::mbar_expect_tx(&barG, (mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
-    seq::fetch_block<T>(mp, 4, sm + oRaw + kRawBytes, (int)(w.b * T_ + w.c * kC), w.h, nv, &barG);
+    seq::fetch_block<T>(mp, 4, sm + oRaw + kRawBytes, (int)(b * T_ + w.c * kC), hc, nv, &barG);
   };
   // start state (16-bit, 8 KB) and end state gradient (fp32, 16 KB) of a chunk into the padded
   // landing zones: three 16-byte asynchronous copies per thread
-  auto issue_state = [&](int64_t ci) {   // every thread
-    const Item w = split_item(ci, nc, mp.heads);
-    const int64_t b = w.bh, c = w.c;
-    const T *s0p = (c == 0) ? state + (size_t)b * kDim * kDim : ckpt + ((size_t)b * nc + (c - 1)) * kDim * kDim;
+  auto issue_state = [&](const ItemWalk &w, int64_t ci) {   // every thread
+    const T *s0p = (w.c == 0) ? state + (size_t)w.bh * kDim * kDim : ckpt + (size_t)(ci - 1) * kDim * kDim;
     const float *rp = Rend + (size_t)ci * kDim * kDim;
     cp_async16(sm + oS0L + (tid >> 3) * kS0Ld + (tid & 7) * 16, s0p + (tid >> 3) * kDim + (tid & 7) * 8);
 #pragma unroll
@@ -165,35 +162,54 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     s_bad2[0] = s_bad2[1] = fix_n2[0] = fix_n2[1] = fix_rows_n = 0;
   }
   if (tid < 2 * kDim) fix_mask[tid] = 0ull;
+  for (int i = tid; i < 4 * kTile / 16; i += kThreadsB)      // the blocks above the diagonal of Z are never written again
+    *reinterpret_cast<float4 *>(sm + oZ + 16 * i) = make_float4(0.f, 0.f, 0.f, 0.f);
   if (warp == 0) umma::tmem_alloc(&tmem_slot, kTmemCols);
   sync_all();
   dependency_wait();
   const uint32_t tb = __shfl_sync(0xffffffffu, tmem_slot, 0);
   const uint32_t tl = umma::tmem_addr(tb, 32 * q4, 0);
   bool raw_pending = false, pre_pending = false;      // thread 0
+  ItemWalk wi(blockIdx.x, gridDim.x, nc), wn = wi;           // this chunk and the next one
   if ((int64_t)blockIdx.x < total) {
     if (tid == 0) {
-      issue_raw(blockIdx.x);
+      issue_raw(wi);
       raw_pending = true;
     }
-    issue_state(blockIdx.x);
+    issue_state(wi, blockIdx.x);
   }
   const uint32_t aT = umma::smem_u32(sm);
   // tile column offset of the own feature: row r of the swizzled tile adds r * 128 and XORs r % 8 into bits 4-6
   const int tcol = (feat >> 5) * kColBlock + ((feat & 3) << 2), tswz = ((feat >> 2) & 7) << 4;
+  // Z tiles of the own side: row 16 q4 + fl, columns t0 .. (16-byte pieces XOR-ed with the row); and column
+  // 16 q4 + fl of the transposed tile, rows t0 .., the second half warp four rows on
+  const int zt_row = 16 * q4 + fl;
+  unsigned char *const zrow = sm + oZ + h * 2 * kTile + (t0 >> 5) * kColBlock + zt_row * 128;
+  const int zsw = (((t0 >> 2) & 7) ^ (zt_row & 7)) << 4;
+  unsigned char *const zt_lo = sm + oZ + (h * 2 + 1) * kTile + (zt_row >> 5) * kColBlock + t0 * 128 + ((zt_row & 3) << 2) + 512 * h;
+  unsigned char *const zt_hi = zt_lo - 1024 * h;
+  const int ztsw = (((zt_row >> 2) & 7) ^ (4 * h)) << 4;
   const T *gcol = raw + (h ? 1 : 4) * kC * kDim + t0 * kDim + feat;
   const T *mcol = raw + (h ? 5 : 2) * kC * kDim + t0 * kDim + feat;
   const T *vcol = raw + (h ? 0 : 3) * kC * kDim + t0 * kDim + feat;
 
   uint32_t it = 0;
   for (int64_t ci = blockIdx.x; ci < total; ci += gridDim.x, ++it) {
-    const Item wi = split_item(ci, nc, mp.heads);
+    wi = wn;
+    wn.step();
     const int64_t t0c = (int64_t)wi.c * kC;
     const int nvalid = (int)((T_ - t0c < kC) ? T_ - t0c : kC);
     // first row and column window of the chunk in the output arrays
     const bool by_row = (mp.flags & seq::kOutByRow) != 0;
-    const int64_t row0 = (by_row ? wi.bh : wi.b) * T_ + t0c;
-    const int hcol = by_row ? 0 : wi.h * kDim;
+    int64_t row0 = wi.bh;
+    int hcol = 0;
+    if (!by_row) {
+      int b, hh;
+      wi.row(mp.heads, &b, &hh);
+      row0 = b;
+      hcol = hh * kDim;
+    }
+    row0 = row0 * T_ + t0c;
     int &fix_n = fix_n2[it & 1], &s_bad = s_bad2[it & 1];
 
     if (!acp::mbar_wait(&barRaw, it & 1u)) s_fail = 1;
@@ -331,7 +347,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       __syncwarp();
     }
     if (kFused && sigmoid_gate && tid == 0) {      // every thread is past the epilogue of the chunk before
-      issue_preact(ci);
+      issue_preact(wi);
       pre_pending = true;
     }
     if (fix_n > 0 && fix_mask[h * kDim + feat] != 0ull) {      // rare: the direct pair sums of this feature read its operand rows
@@ -415,10 +431,10 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     }
     if (ci + gridDim.x < total) {      // the next chunk's inputs and state blocks
       if (tid == 0) {
-        issue_raw(ci + gridDim.x);
+        issue_raw(wn);
         raw_pending = true;
       }
-      issue_state(ci + gridDim.x);
+      issue_state(wn, ci + gridDim.x);
     }
     if (tid == 0) {
       if (s_bad) atomicExch(rowflag + wi.bh, 1);      // the scan kernels redo this batch row
@@ -426,27 +442,28 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       fix_n2[(it & 1) ^ 1] = 0;
     }
 
-    // ---- Z: mask, round, store as [t][s] and [s][t] ----
+    // ---- Z: mask, round, store as [t][s] and [s][t].  A warp holds rows 16 q4 .. + 15 and columns t0 .. t0 + 15: on
+    //      the diagonal it masks, below it nothing is masked, above it the blocks stay zero ----
     if (!umma::mbar_wait(&barZ, it & 1u)) s_fail = 1;
     umma::fence_after_sync();
-    {
-      const int t = 16 * q4 + fl;
+    if (tq <= q4) {
       float v[16];
       umma::tmem_ld16(tl + cZ + t0, v);
       umma::tmem_ld_wait();
+      if (tq == q4) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = (t0 + j <= t) ? bias_tf32(v[j]) : 0.f;
-      unsigned char *z = sm + oZ + h * 2 * kTile, *zt = z + kTile;
+        for (int j = 0; j < 16; ++j) v[j] = j <= fl ? bias_tf32(v[j]) : 0.f;
+      } else {
 #pragma unroll
-      for (int j = 0; j < 16; j += 4)
-        *reinterpret_cast<float4 *>(z + toff(t, t0 + j)) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        for (int j = 0; j < 16; ++j) v[j] = bias_tf32(v[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4 *>(zrow + (zsw ^ (j << 4))) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
       // transposed: the half warps take rows four apart, which lie in different halves of the swizzle
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float w = h ? v[j ^ 4] : v[j];
-        const int s = t0 + (j ^ (h << 2));
-        *reinterpret_cast<float *>(zt + toff(s, t)) = w;
-      }
+      for (int j = 0; j < 16; ++j)
+        *reinterpret_cast<float *>(((j & 4) ? zt_hi : zt_lo) + j * 128 + (ztsw ^ ((j & 7) << 4))) = h ? v[j ^ 4] : v[j];
     }
     umma::fence_async_smem();
     sync_all();
@@ -536,6 +553,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     T *p_mu = dq.p + (size_t)(row0 + t0) * dq.ld + dq.col + hcol + feat;
     T *p_dv = o_dv.p + (size_t)(row0 + t0) * o_dv.ld + o_dv.col + hcol + feat;
     const int n_own = nvalid - t0;      // valid own steps (may be negative)
+    const bool full = n_own >= 16;
 
     if (!umma::mbar_wait(&barM2, it & 1u)) s_fail = 1;
     umma::fence_after_sync();
@@ -566,7 +584,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         const float ip = rcp_fast(pm[jj]);
         const float dmu = pm[jj] * fmaf(up, tq1[j], tq2[j]), ddv = ip * fmaf(after, t7[j], t2[j]);
         pm[jj] = (jj > 0 ? pm[jj > 0 ? jj - 1 : 0] : pm_prev) * ip;      // from here on: 1 / gate of the step
-        if (jj < n_own) {
+        if (full || jj < n_own) {
           if (h == 0) p_mu[jj * ld_mu] = (T)(kFused ? dmu * q_scale : dmu);
           p_dv[jj * ld_dv] = (T)ddv;
         }
@@ -622,7 +640,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
             const float e = __expf(-Elem<T>::ld(pre + j * kDim)), sg = rcp_fast(1.f + e);
             dg *= sg > seq::kGateFloor ? sg * sg * e : 0.f;      // s (1 - s) = s^2 e^{-g}
           }
-          if (j < n_own) p_gt[j * ld_gt] = (T)dg;
+          if (full || j < n_own) p_gt[j * ld_gt] = (T)dg;
         }
       }
       __syncwarp();

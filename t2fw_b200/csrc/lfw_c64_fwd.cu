@@ -5,21 +5,28 @@
 //
 // Per chunk, with S0 the state at the chunk start (the caller's state or the 16-bit checkpoint the
 // carry wrote; notation of lfw_c64.cuh):
-//     P   = tril( (q pm_g) (k / pm_g)^T )                       in-chunk decays, k side
-//     O^  = (q G_t) (A_REF .* S0)^T  +  P (x / pm_a)            [t][d]
-//     o_t = pm_a[t] .* O^_t
-// i.e. three 64 x 64 x 64 contractions, all on TF32 operand tiles in shared memory with fp32
-// accumulators in tensor memory.
+//     P   = tril( (q pm_g) (k / pm_g)^T )      [t][s]  in-chunk decays, k side
+//     O1  = (G_REF .* S0) (q pm_g)^T           [d][t]  to be scaled by A_REF
+//     O2  = (x / pm_a)^T P^T                   [d][t]
+//     o_t = pm_a[t] .* (A_REF O1 + O2)_t
+// i.e. three 64 x 64 x 64 contractions.  The state carries the k side's anchor product only and the d
+// side's scales the result, so the mid-anchored query tile serves P and O1 (no operand is scaled by two
+// 32-step products).
 //
-// One persistent CTA of 16 warps per SM.  The five raw 8 KB input blocks of a chunk arrive by bulk
-// asynchronous copies into one of two buffers (the next chunk is fetched while this one is
-// computed); thread (gate side, 16-step quarter, feature) walks its steps with a running gate
-// product (stage 1: ratio tables), then the operand tiles are written element-wise with 16-byte
-// stores (stage 2); one elected lane issues the MMAs; the accumulators come
-// back time-major (a thread owns one step and eight features), so the 16-bit outputs leave as
-// 16-byte stores.
-#include <type_traits>
-
+// A CTA works on TWO chunks at a time.  An M = 64 accumulator takes 16 lanes of every 32-lane quarter of
+// tensor memory; chunk 0 of the pair uses one lane set and chunk 1 the other, so a thread's lane decides its
+// chunk and every operand and every result exists once.  Thread (chunk, feature, 16-step quarter) walks the
+// k-side gates of its feature (operand tiles [step][feature] in shared memory), then the d-side gates
+// (operand x / pm_a straight into tensor memory, row = feature), and reads the outputs of its own feature
+// and steps back, so that the ratios never leave its registers.  Odd chunk lanes are rotated by 16 features
+// so that the half warps touch different banks.
+//
+// What bounds it: instruction issue and the latency of its phases (shared-memory loads, two barriers, the two
+// product rounds); against the one-chunk version with ratio tables in shared memory, config B*H = 96,
+// T = 1024 (1536 chunks): 12.7 k -> 7 k warp instructions per chunk, FWD_US.
+//
+// One persistent CTA of 16 warps per SM.  The raw 8 KB input blocks of the next pair are requested as soon as
+// this pair's operands are built.  Every wait is bounded.
 #include "lfw_c64.cuh"
 #include "seq_layout.cuh"
 
@@ -33,293 +40,365 @@ int lfw_chunk_sm_count(int *out);
 namespace {
 
 constexpr int kThreadsF = 512;
-constexpr int kPmLd = 68;                          // row stride (floats) of the padded ratio tables
-// shared-memory map (bytes from the 1024-byte aligned base)
-constexpr int oT = 0;                              // tiles: 0 Qmid -> P, 1 Kmid, 2 Qstart, 3 Xmid (feature-major), 4 S0'
-constexpr int oPmk = oT + 5 * kTile;               // pm_g[t][k]
-constexpr int oPmF = oPmk + kC * kDim * 4;         // pm_a[d][t]
-constexpr int oPmA = oPmF + kDim * kPmLd * 4;      // pm_a[t][d]
-constexpr int oQt = oPmA + kC * kPmLd * 4;         // quarter products [2 sides][4][64]
 constexpr int kS0Ld = 144;                         // row stride (bytes) of the start-state landing zone
-constexpr int oS0L = oQt + 2 * 4 * kDim * 4;       // start state of a chunk, [64][kS0Ld] 16-bit
-constexpr int oRaw = oS0L + kDim * kS0Ld;           // [2 buffers] x, f, q, k, fk
+// shared-memory map (bytes from the 1024-byte aligned base), everything once per chunk of the pair
+constexpr int oT = 0;                              // [chunk][2] tiles [step][feature]: q pm_g, k / pm_g -> P
+constexpr int oS0L = oT + 4 * kTile;               // [chunk] start state, [64][kS0Ld] 16-bit
+constexpr int oQt = oS0L + 2 * kDim * kS0Ld;       // [chunk][side][4][64] products of the quarters
+constexpr int oRaw = oQt + 2 * 2 * 4 * kDim * 4;   // [chunk] x, f, q, k, fk
 constexpr int kSmemF = oRaw + 2 * 5 * kRawBytes + 1024;   // + slack for the 1024-byte alignment
 static_assert(oRaw % 128 == 0 && oS0L % 16 == 0, "copy destination alignment");
 static_assert(kSmemF + 256 <= 227 * 1024, "shared memory limit");
 
-constexpr int cP = 0, cO = 32;                     // tensor-memory columns
+// tensor-memory columns, one lane set per chunk
+constexpr int cS2 = 0, cX = 64, cP = 128, cO1 = 192, cO2 = 256;
+constexpr int kTmemColsF = 512;
 
-template <typename T>
+template <typename T, bool kFused>
 __global__ void __launch_bounds__(kThreadsF, 1)
 lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ state, const T *__restrict__ ckpt,
                    const seq::Out<T> out, int *__restrict__ rowflag, int *__restrict__ status, int64_t T_,
                    int64_t nc, int64_t total) {
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);   // swizzle atoms are 1024-byte aligned
-  __shared__ __align__(8) uint64_t barRaw[2], barP, barO;
+  __shared__ __align__(8) uint64_t barRaw, barP, barO;
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_fail, s_bad;
+  __shared__ int s_fail, s_bad2[2][2];
 
   const int tid = threadIdx.x, warp = uniform_warp_idx(), lane = tid & 31;
-  // stage 1: gate side (0: k side, 1: d side), quarter of the chunk, feature
-  const int gs = warp >> 3, tq = (warp >> 1) & 3, feat = (warp & 1) * 32 + lane;
-  // accumulator read-out: lane quarter, column part, column half (lane set), row in the quarter
-  const int q4 = warp & 3, part = warp >> 2, h = lane >> 4, fl = lane & 15;
-  // state tile: row d, eight columns
-  const int sr = tid & 63, sc0 = (tid >> 6) * 8;
-
-  float *pmk = reinterpret_cast<float *>(sm + oPmk);
-  float *pmF = reinterpret_cast<float *>(sm + oPmF);
-  float *pmA = reinterpret_cast<float *>(sm + oPmA);
-  float *qtot = reinterpret_cast<float *>(sm + oQt);
+  // lane quarter of tensor memory, 16-step quarter of the chunk, chunk of the pair, row in the quarter
+  const int q4 = warp & 3, tq = warp >> 2, h = lane >> 4, fl = lane & 15;
+  const int feat = 16 * ((q4 + h) & 3) + fl;       // own feature, both sides
+  const int t0 = 16 * tq;
+  float *qtot = reinterpret_cast<float *>(sm + oQt) + h * 2 * 4 * kDim;      // of the own chunk
 
   // tensors: 0 x, 1 f, 2 q, 3 k, 4 fk
-  const bool unit_forget = (mp.flags & seq::kUnitForget) != 0;
-  auto issue_raw = [&](int64_t ci, int buf) {     // thread 0 only: one copy per tensor
-    const Item w = split_item(ci, nc, mp.heads);
-    const int row = (int)(w.b * T_ + w.c * kC), hc = w.h;
-    const int nv = (int)((T_ - (int64_t)w.c * kC < kC) ? T_ - (int64_t)w.c * kC : kC);
-    unsigned char *r = sm + oRaw + buf * 5 * kRawBytes;
-    const uint32_t per = (mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes;
-    acp::mbar_expect_tx(&barRaw[buf], (unit_forget ? 4u : 5u) * per);
-#pragma unroll
-    for (int i = 0; i < 5; ++i)
-      if (!(i == 1 && unit_forget)) seq::fetch_block<T>(mp, i, r + i * kRawBytes, row, hc, nv, &barRaw[buf]);
+  const bool unit_forget = kFused && (mp.flags & seq::kUnitForget) != 0;
+  const bool sigmoid_gate = kFused && (mp.flags & seq::kSigmoidGate) != 0;
+  const float q_scale = kFused ? mp.q_scale : 1.f;
+  auto valid_steps = [&](const ItemWalk &w, int64_t ci) {
+    if (ci >= total) return 0;
+    const int64_t left = T_ - (int64_t)w.c * kC;
+    return (int)(left < kC ? left : kC);
   };
-
-  // start state of a chunk (the caller's state for the first chunk of a row, else the checkpoint
-  // written by the carry): one 16-byte asynchronous copy per thread into the padded landing zone
-  auto issue_state = [&](int64_t ci) {   // every thread
-    const Item w = split_item(ci, nc, mp.heads);
-    const int64_t b = w.bh, c = w.c;
-    const T *s0p = (c == 0) ? state + (size_t)b * kDim * kDim : ckpt + ((size_t)b * nc + (c - 1)) * kDim * kDim;
-    cp_async16(sm + oS0L + (tid >> 3) * kS0Ld + (tid & 7) * 16, s0p + (tid >> 3) * kDim + (tid & 7) * 8);
+  auto issue_raw = [&](const ItemWalk *w, int64_t ci) {     // thread 0 only: one copy per tensor and chunk
+    uint32_t bytes = 0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int nv = valid_steps(w[e], ci + e);
+      if (nv > 0) bytes += (unit_forget ? 4u : 5u) * ((mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
+    }
+    acp::mbar_expect_tx(&barRaw, bytes);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int nv = valid_steps(w[e], ci + e);
+      if (nv <= 0) continue;
+      int b, hc;
+      w[e].row(mp.heads, &b, &hc);
+      const int row = (int)(b * T_ + w[e].c * kC);
+#pragma unroll
+      for (int i = 0; i < 5; ++i)
+        if (!(i == 1 && unit_forget)) seq::fetch_block<T>(mp, i, sm + oRaw + (e * 5 + i) * kRawBytes, row, hc, nv, &barRaw);
+    }
+  };
+  // start states of the pair (the caller's state for the first chunk of a row, else the checkpoint written
+  // by the carry): one 16-byte asynchronous copy per thread and chunk into the padded landing zones
+  auto issue_state = [&](const ItemWalk *w, int64_t ci) {   // every thread
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      if (ci + e >= total) continue;
+      const T *s0p = (w[e].c == 0) ? state + (size_t)w[e].bh * kDim * kDim : ckpt + (size_t)(ci + e - 1) * kDim * kDim;
+      cp_async16(sm + oS0L + e * kDim * kS0Ld + (tid >> 3) * kS0Ld + (tid & 7) * 16, s0p + (tid >> 3) * kDim + (tid & 7) * 8);
+    }
     cp_async_commit();
   };
 
   if (tid == 0) {
-    umma::mbar_init(&barRaw[0], 1);
-    umma::mbar_init(&barRaw[1], 1);
-    umma::mbar_init(&barP, 1);
-    umma::mbar_init(&barO, 1);
+    umma::mbar_init(&barRaw, 1);
+    umma::mbar_init(&barP, 2);       // one commit per chunk
+    umma::mbar_init(&barO, 4);       // O1 and O2 of both chunks
     umma::mbar_fence_init();
     s_fail = 0;
+    s_bad2[0][0] = s_bad2[0][1] = s_bad2[1][0] = s_bad2[1][1] = 0;
   }
-  if (warp == 0) umma::tmem_alloc(&tmem_slot, 64);
-  if (unit_forget) {      // the d-side gate block of both buffers is the constant 1 and never loaded
-    seq::fill_block(reinterpret_cast<T *>(sm + oRaw + kRawBytes), 1.f, tid, kThreadsF);
-    seq::fill_block(reinterpret_cast<T *>(sm + oRaw + 6 * kRawBytes), 1.f, tid, kThreadsF);
-  }
+  if (warp == 0) umma::tmem_alloc(&tmem_slot, kTmemColsF);
   sync_all();
   dependency_wait();
   const uint32_t tb = __shfl_sync(0xffffffffu, tmem_slot, 0);
   const uint32_t tl = umma::tmem_addr(tb, 32 * q4, 0);
-  uint32_t n_issued[2] = {0u, 0u}, n_landed[2] = {0u, 0u};      // thread 0: bulk-copy rounds per buffer
-  if ((int64_t)blockIdx.x < total) {
+  ItemWalk wn[2] = {ItemWalk(2 * blockIdx.x, 2 * gridDim.x, nc), ItemWalk(2 * blockIdx.x + 1, 2 * gridDim.x, nc)};
+  bool raw_pending = false;      // thread 0
+  if (2 * (int64_t)blockIdx.x < total) {
     if (tid == 0) {
-      issue_raw(blockIdx.x, 0);
-      ++n_issued[0];
+      issue_raw(wn, 2 * (int64_t)blockIdx.x);
+      raw_pending = true;
     }
-    issue_state(blockIdx.x);
+    issue_state(wn, 2 * (int64_t)blockIdx.x);
   }
   const uint32_t aT = umma::smem_u32(sm + oT);
-  const uint64_t dT0 = desc_sw128(aT), dT1 = desc_sw128(aT + kTile), dT2 = desc_sw128(aT + 2 * kTile);
-  const uint64_t dT3 = desc_sw128(aT + 3 * kTile), dT4 = desc_sw128(aT + 4 * kTile);
+  // tile column offset of the own feature: row r of the swizzled tile adds r * 128 and XORs r % 8 into bits 4-6
+  unsigned char *const tq_col = sm + oT + h * 2 * kTile + (feat >> 5) * kColBlock + ((feat & 3) << 2) + t0 * 128;
+  const int tswz = ((feat >> 2) & 7) << 4;
+  // P tile: row 16 q4 + fl, columns t0 ..
+  const int p_row = 16 * q4 + fl;
+  unsigned char *const prow = sm + oT + (h * 2 + 1) * kTile + (t0 >> 5) * kColBlock + p_row * 128;
+  const int psw = (((t0 >> 2) & 7) ^ (p_row & 7)) << 4;
+  const T *raw = reinterpret_cast<const T *>(sm + oRaw + h * 5 * kRawBytes) + t0 * kDim + feat;
+  auto rawv = [&](int blk, int j) { return Elem<T>::ld(raw + blk * kC * kDim + j * kDim); };
 
   uint32_t it = 0;
-  for (int64_t ci = blockIdx.x; ci < total; ci += gridDim.x, ++it) {
-    const int buf = it & 1;
-    const Item wi = split_item(ci, nc, mp.heads);
-    const int64_t b = wi.bh, c = wi.c, t0c = c * kC;      // b: problem row (batch item x head)
-    const int nvalid = (int)((T_ - t0c < kC) ? T_ - t0c : kC);
-    T *raw = reinterpret_cast<T *>(sm + oRaw + buf * 5 * kRawBytes);
-    const bool by_row = (mp.flags & seq::kOutByRow) != 0;
-    T *orow = out.p + ((by_row ? wi.bh : wi.b) * T_ + t0c) * out.ld + out.col + (by_row ? 0 : wi.h * kDim);
+  for (int64_t ci = 2 * (int64_t)blockIdx.x; ci < total; ci += 2 * (int64_t)gridDim.x, ++it) {
+    const ItemWalk w0 = wn[0], w1 = wn[1];
+    wn[0].step();
+    wn[1].step();
+    const int nv0 = valid_steps(w0, ci), nv1 = valid_steps(w1, ci + 1);
+    const int nvalid = h ? nv1 : nv0;
+    const bool partial = nv0 < kC || nv1 < kC;      // steps beyond the valid ones become identity steps
+    int *s_bad = s_bad2[it & 1];
 
-    if (tid == 0) {
-      s_bad = 0;
-      if (ci + gridDim.x < total) {      // the other buffer was released at the end of the previous chunk
-        issue_raw(ci + gridDim.x, buf ^ 1);
-        ++n_issued[buf ^ 1];
+    cp_async_wait_all();       // this thread's share of the start states (requested one pair ahead)
+    if (!acp::mbar_wait(&barRaw, it & 1u)) s_fail = 1;
+    if (tid == 0) raw_pending = false;
+
+    // ---- gates of the own feature and quarter on both sides, products of the quarters ----
+    float gk[16], gd[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      gk[j] = rawv(4, j);
+      if (kFused && sigmoid_gate) gk[j] = seq::sigmoid_gate<T>(gk[j]);
+      gd[j] = kFused && unit_forget ? 1.f : rawv(1, j);
+    }
+    if (partial) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        gk[j] = t0 + j < nvalid ? gk[j] : 1.f;
+        gd[j] = t0 + j < nvalid ? gd[j] : 1.f;
       }
     }
-    cp_async_wait_all();       // this thread's share of this chunk's start state (requested one chunk ahead)
-    if (acp::mbar_wait(&barRaw[buf], (it >> 1) & 1u)) {
-      if (tid == 0) ++n_landed[buf];
-    } else {
-      s_fail = 1;
-    }
-    __syncthreads();
-    if (s_fail) break;
-    if ((mp.flags & seq::kSigmoidGate) || mp.q_scale != 1.f) {      // fused layer: activations applied here
-      if (mp.flags & seq::kSigmoidGate) seq::sigmoid_gate_block(raw + 4 * kC * kDim, tid, kThreadsF);
-      if (mp.q_scale != 1.f) seq::scale_block(raw + 2 * kC * kDim, mp.q_scale, tid, kThreadsF);
-      __syncthreads();
-    }
-    if (nvalid < kC) {      // partial chunk: identity steps beyond the valid ones
-      pad_raw_tail<T>(raw, 5, (1u << 1) | (1u << 4), nvalid, tid, kThreadsF);
-      __syncthreads();
-    }
-
-    // ---- stage 1: gate products of the four quarters, then the ratios to the anchor ----
-    float g[16];
-    qtot[(gs * 4 + tq) * kDim + feat] = load_gates16<T>(raw + (gs ? 1 : 4) * kC * kDim + feat, tq, g);
-    __syncthreads();
-    {
-      const float *qt = qtot + gs * 4 * kDim + feat;
-      const float carry = tq == 0 ? qt[kDim] : tq == 3 ? qt[2 * kDim] : 1.f;
-      float pm[16];
-      if (!ratios16(tq, g, carry, pm)) s_bad = 1;
-      if (gs == 0) {
+    float mn = kRangeHi;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) pmk[(16 * tq + j) * kDim + feat] = pm[j];
+    for (int j = 0; j < 16; ++j) mn = fminf(mn, fminf(fabsf(gk[j]), fabsf(gd[j])));
+    if (!(mn >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        gk[j] = sanitize_gate(gk[j]);
+        gd[j] = sanitize_gate(gd[j]);
+      }
+    }
+    float pk = gk[0], pd = gd[0];
+#pragma unroll
+    for (int j = 1; j < 16; ++j) { pk *= gk[j]; pd *= gd[j]; }
+    qtot[tq * kDim + feat] = pk;
+    qtot[(4 + tq) * kDim + feat] = pd;
+    __syncthreads();           // also: the start states of both chunks have landed
+    if (s_fail) break;
+
+    // ---- operands ----
+    float lo, hi;
+    {   // k side: q pm_g and k / pm_g as [step][feature] tiles
+      float s = tq == 0 ? qtot[kDim + feat] : tq == 3 ? qtot[2 * kDim + feat] : 1.f;
+      float mw[16], vw[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        mw[j] = rawv(2, j);
+        vw[j] = rawv(3, j);
+      }
+      if (kFused && q_scale != 1.f) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) mw[j] = seq::round_to<T>(mw[j] * q_scale);
+      }
+      if (partial) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          mw[j] = t0 + j < nvalid ? mw[j] : 0.f;
+          vw[j] = t0 + j < nvalid ? vw[j] : 0.f;
+        }
+      }
+      lo = hi = fabsf(s);
+      if (tq < 2) {
+#pragma unroll
+        for (int j = 15; j >= 0; --j) {
+          mw[j] = bias_tf32(mw[j] * rcp_fast(s));
+          vw[j] = bias_tf32(vw[j] * s);
+          s *= gk[j];
+          lo = fminf(lo, fabsf(s));
+          hi = fmaxf(hi, fabsf(s));
+        }
       } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) pmA[(16 * tq + j) * kPmLd + feat] = pm[j];
-#pragma unroll
-        for (int j = 0; j < 16; j += 4)
-          *reinterpret_cast<float4 *>(pmF + feat * kPmLd + 16 * tq + j) = make_float4(pm[j], pm[j + 1], pm[j + 2], pm[j + 3]);
-      }
-    }
-    __syncthreads();
-
-    // ---- stage 2: operand tiles ----
-    {   // k side, time-major: this thread = four features, steps t and t + 32
-      const int f4 = (tid & 15) * 4;
-      const float4 g_ref = mul4(*reinterpret_cast<const float4 *>(qtot + f4),
-                                *reinterpret_cast<const float4 *>(qtot + kDim + f4));
-      const T *r_q = raw + 2 * kC * kDim + f4, *r_k = raw + 3 * kC * kDim + f4;
-      unsigned char *t0p = sm + oT;
-#pragma unroll
-      for (int i2 = 0; i2 < 2; ++i2) {
-        const int t = (tid >> 4) + 32 * i2;
-        const float4 pv = *reinterpret_cast<const float4 *>(pmk + t * kDim + f4);
-        const float4 qm = mul4(Vec4<T>::ld(r_q + t * kDim), pv);
-        const float4 km = mul4(Vec4<T>::ld(r_k + t * kDim), rcp4(pv));
-        const int o = toff(t, f4);
-        *reinterpret_cast<float4 *>(t0p + o) = bias4(qm);
-        *reinterpret_cast<float4 *>(t0p + kTile + o) = bias4(km);
-        *reinterpret_cast<float4 *>(t0p + 2 * kTile + o) = bias4(mul4(qm, g_ref));
-      }
-    }
-    {   // d side, feature-major: this thread = features 2 * lane, 2 * lane + 1, steps 4 * warp .. + 3
-      const int f0 = 2 * lane, t = 4 * warp;
-      const T *r_x = raw + t * kDim + f0;
-      float2 x2[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) x2[j] = Vec2<T>::ld(r_x + j * kDim);
-      const float4 i0 = rcp4(*reinterpret_cast<const float4 *>(pmF + f0 * kPmLd + t));
-      const float4 i1 = rcp4(*reinterpret_cast<const float4 *>(pmF + (f0 + 1) * kPmLd + t));
-      unsigned char *tX = sm + oT + 3 * kTile;
-      *reinterpret_cast<float4 *>(tX + toff(f0, t)) = bias4(mul4(make_float4(x2[0].x, x2[1].x, x2[2].x, x2[3].x), i0));
-      *reinterpret_cast<float4 *>(tX + toff(f0 + 1, t)) = bias4(mul4(make_float4(x2[0].y, x2[1].y, x2[2].y, x2[3].y), i1));
-    }
-    // ---- state tile S0' = A_REF .* S0 ----
-    {
-      const float a_ref = qtot[4 * kDim + sr] * qtot[5 * kDim + sr];
-      const uint4 u = *reinterpret_cast<const uint4 *>(sm + oS0L + sr * kS0Ld + sc0 * 2);
-      const T *e = reinterpret_cast<const T *>(&u);
-      const float4 s_lo = make_float4(Elem<T>::ld(e), Elem<T>::ld(e + 1), Elem<T>::ld(e + 2), Elem<T>::ld(e + 3));
-      const float4 s_hi = make_float4(Elem<T>::ld(e + 4), Elem<T>::ld(e + 5), Elem<T>::ld(e + 6), Elem<T>::ld(e + 7));
-      unsigned char *tS = sm + oT + 4 * kTile;
-      *reinterpret_cast<float4 *>(tS + toff(sr, sc0)) =
-          make_float4(bias_tf32(s_lo.x * a_ref), bias_tf32(s_lo.y * a_ref), bias_tf32(s_lo.z * a_ref),
-                      bias_tf32(s_lo.w * a_ref));
-      *reinterpret_cast<float4 *>(tS + toff(sr, sc0 + 4)) =
-          make_float4(bias_tf32(s_hi.x * a_ref), bias_tf32(s_hi.y * a_ref), bias_tf32(s_hi.z * a_ref),
-                      bias_tf32(s_hi.w * a_ref));
-    }
-    umma::fence_async_smem();
-    sync_all();       // tiles complete, raw buffer and start state consumed
-    if (ci + gridDim.x < total) issue_state(ci + gridDim.x);
-
-    // A product is a chain of eight dependent instructions; the tensor core executes in issue
-    // order, so one lane issues the independent chains interleaved and they overlap in the pipeline.
-    if (warp == 0) {
-      const uint32_t d0 = tb, d1 = umma::tmem_addr(tb, 16, 0);
-      constexpr uint32_t idesc = umma::make_idesc_tf32(64, 32, false, false);
-      constexpr uint64_t n1 = (uint64_t)(32 * 128 >> 4);     // B rows 32..63
-      if (elect_one()) {
-        // P first and on its own barrier: the state term runs while P is masked and stored
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t o = (uint64_t)(((ks >> 2) * kColBlock + (ks & 3) * 32) >> 4);
-          umma::mma_tf32(d0 + cP, dT0 + o, dT1 + o, idesc, ks > 0);             // P = Qmid Kmid^T
-          umma::mma_tf32(d1 + cP, dT0 + o, dT1 + n1 + o, idesc, ks > 0);
+        for (int j = 0; j < 16; ++j) {
+          s *= gk[j];
+          lo = fminf(lo, fabsf(s));
+          hi = fmaxf(hi, fabsf(s));
+          mw[j] = bias_tf32(mw[j] * s);
+          vw[j] = bias_tf32(vw[j] * rcp_fast(s));
         }
-        umma::mma_commit(&barP);
+      }
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t o = (uint64_t)(((ks >> 2) * kColBlock + (ks & 3) * 32) >> 4);
-          umma::mma_tf32(d0 + cO, dT2 + o, dT4 + o, idesc, ks > 0);             // O^ = Qstart S0'^T
-          umma::mma_tf32(d1 + cO, dT2 + o, dT4 + n1 + o, idesc, ks > 0);
+      for (int j = 0; j < 16; ++j) {
+        unsigned char *p = tq_col + (tswz ^ ((j & 7) << 4)) + j * 128;
+        *reinterpret_cast<float *>(p) = mw[j];
+        *reinterpret_cast<float *>(p + kTile) = vw[j];
+      }
+    }
+    float up;                  // A_REF of the own feature; gd[j] becomes pm_a[j]
+    {   // d side: x / pm_a into tensor memory
+      const float q0 = qtot[4 * kDim + feat], q1 = qtot[5 * kDim + feat];
+      up = q0 * q1;
+      float s = tq == 0 ? q1 : tq == 3 ? qtot[6 * kDim + feat] : 1.f;
+      float vw[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) vw[j] = rawv(0, j);
+      if (partial) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) vw[j] = t0 + j < nvalid ? vw[j] : 0.f;
+      }
+      lo = fminf(lo, fabsf(s));
+      hi = fmaxf(hi, fabsf(s));
+      if (tq < 2) {
+#pragma unroll
+        for (int j = 15; j >= 0; --j) {
+          const float a = gd[j];
+          gd[j] = rcp_fast(s);
+          vw[j] = bias_tf32(vw[j] * s);
+          s *= a;
+          lo = fminf(lo, fabsf(s));
+          hi = fmaxf(hi, fabsf(s));
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          s *= gd[j];
+          lo = fminf(lo, fabsf(s));
+          hi = fmaxf(hi, fabsf(s));
+          gd[j] = s;
+          vw[j] = bias_tf32(vw[j] * rcp_fast(s));
+        }
+      }
+      umma::tmem_st16(tl + cX + t0, vw);
+    }
+    if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad[h] = 1;      // also NaN
+    {   // state: row d = own feature, columns k = t0 .. t0 + 15, scaled by G_REF
+      float sv[16];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint4 u = *reinterpret_cast<const uint4 *>(sm + oS0L + h * kDim * kS0Ld + feat * kS0Ld + t0 * 2 + 16 * i);
+        const T *e = reinterpret_cast<const T *>(&u);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sv[8 * i + j] = Elem<T>::ld(e + j);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 a = *reinterpret_cast<const float4 *>(qtot + t0 + 4 * i);
+        const float4 b = *reinterpret_cast<const float4 *>(qtot + kDim + t0 + 4 * i);
+        sv[4 * i] = bias_tf32(sv[4 * i] * (a.x * b.x));
+        sv[4 * i + 1] = bias_tf32(sv[4 * i + 1] * (a.y * b.y));
+        sv[4 * i + 2] = bias_tf32(sv[4 * i + 2] * (a.z * b.z));
+        sv[4 * i + 3] = bias_tf32(sv[4 * i + 3] * (a.w * b.w));
+      }
+      umma::tmem_st16(tl + cS2 + t0, sv);
+    }
+    umma::tmem_st_wait();
+    umma::fence_async_smem();
+    sync_all();       // operands complete, raw blocks and start states consumed
+
+    // P of both chunks first and on their own barrier (warps 0, 1), then O1 (warps 2, 3): chains of eight dependent
+    // instructions from several warps interleave in the tensor core
+    if (warp < 4) {
+      const int e = warp & 1;
+      const uint32_t ls = umma::tmem_addr(tb, 16 * e, 0);
+      const uint64_t dq = desc_sw128(aT + e * 2 * kTile), dk = desc_sw128(aT + (e * 2 + 1) * kTile);
+      if (elect_one()) {
+        if (warp < 2) {
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) umma::mma_tf32(ls + cP, dq + kstep(ks), dk + kstep(ks), kIdesc64, ks > 0);
+          umma::mma_commit(&barP);
+        } else {
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) mma_tf32_ts(ls + cO1, ls + cS2 + 8 * ks, dq + kstep(ks), kIdesc64, ks > 0);
+          umma::mma_commit(&barO);
         }
       }
       __syncwarp();
-      if (tid == 0 && s_bad) atomicExch(rowflag + b, 1);      // the scan kernel redoes this batch row
     }
-    // ---- P: mask, round, store as the [t][s] operand (over Qmid, which only the P product reads) ----
+    if (ci + 2 * (int64_t)gridDim.x < total) {
+      if (tid == 0) {
+        issue_raw(wn, ci + 2 * (int64_t)gridDim.x);
+        raw_pending = true;
+      }
+      issue_state(wn, ci + 2 * (int64_t)gridDim.x);
+    }
+    if (tid == 0) {
+      if (s_bad[0]) atomicExch(rowflag + w0.bh, 1);      // the scan kernel redoes these batch rows
+      if (s_bad[1] && nv1 > 0) atomicExch(rowflag + w1.bh, 1);
+      s_bad2[(it & 1) ^ 1][0] = s_bad2[(it & 1) ^ 1][1] = 0;
+    }
+
+    // ---- P: mask, round, store as the [t][s] operand (over k / pm_g, which only the P product reads) ----
     if (!umma::mbar_wait(&barP, it & 1u)) s_fail = 1;
     umma::fence_after_sync();
     {
-      const int t = 16 * q4 + fl, s0 = 32 * h + 8 * part;
-      float v[8];
-      umma::tmem_ld8(tl + cP + 8 * part, v);
-      umma::tmem_ld_wait();
+      float v[16];
+      if (tq <= q4) {        // above the diagonal there is nothing to read
+        umma::tmem_ld16(tl + cP + t0, v);
+        umma::tmem_ld_wait();
+      }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = (s0 + j <= t) ? bias_tf32(v[j]) : 0.f;
-      unsigned char *tP = sm + oT;
-      *reinterpret_cast<float4 *>(tP + toff(t, s0)) = make_float4(v[0], v[1], v[2], v[3]);
-      *reinterpret_cast<float4 *>(tP + toff(t, s0 + 4)) = make_float4(v[4], v[5], v[6], v[7]);
+      for (int j = 0; j < 16; ++j) v[j] = t0 + j <= p_row ? bias_tf32(v[j]) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4 *>(prow + (psw ^ (j << 4))) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     }
     umma::fence_async_smem();
     sync_all();
     if (s_fail) break;
-    if (warp == 0) {     // the same lane as above: O^ += P Xmid follows O^ = ... in issue order
-      const uint32_t d0 = tb, d1 = umma::tmem_addr(tb, 16, 0);
-      constexpr uint32_t idesc = umma::make_idesc_tf32(64, 32, false, false);
-      constexpr uint64_t n1 = (uint64_t)(32 * 128 >> 4);
+    if (warp == 4 || warp == 5) {      // O2
+      const int e = warp & 1;
+      const uint32_t ls = umma::tmem_addr(tb, 16 * e, 0);
+      const uint64_t dp = desc_sw128(aT + (e * 2 + 1) * kTile);
       if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t o = (uint64_t)(((ks >> 2) * kColBlock + (ks & 3) * 32) >> 4);
-          umma::mma_tf32(d0 + cO, dT0 + o, dT3 + o, idesc, true);
-          umma::mma_tf32(d1 + cO, dT0 + o, dT3 + n1 + o, idesc, true);
-        }
+        for (int ks = 0; ks < 8; ++ks) mma_tf32_ts(ls + cO2, ls + cX + 8 * ks, dp + kstep(ks), kIdesc64, ks > 0);
         umma::mma_commit(&barO);
       }
       __syncwarp();
     }
-    {
-      const int t = 16 * q4 + fl, d0 = 32 * h + 8 * part;
-      const float4 p0 = *reinterpret_cast<const float4 *>(pmA + t * kPmLd + d0);
-      const float4 p1 = *reinterpret_cast<const float4 *>(pmA + t * kPmLd + d0 + 4);
-      if (!umma::mbar_wait(&barO, it & 1u)) s_fail = 1;
-      umma::fence_after_sync();
-      float v[8];
-      umma::tmem_ld8(tl + cO + 8 * part, v);
-      umma::tmem_ld_wait();
-      if (t < nvalid) {
-        __align__(16) T o[8];
-        o[0] = (T)(v[0] * p0.x); o[1] = (T)(v[1] * p0.y); o[2] = (T)(v[2] * p0.z); o[3] = (T)(v[3] * p0.w);
-        o[4] = (T)(v[4] * p1.x); o[5] = (T)(v[5] * p1.y); o[6] = (T)(v[6] * p1.z); o[7] = (T)(v[7] * p1.w);
-        *reinterpret_cast<uint4 *>(orow + (size_t)t * out.ld + d0) = *reinterpret_cast<const uint4 *>(o);
-      }
+    // first row and column window of the own chunk in the output array; 16 features of one step are 32 contiguous bytes
+    int b = h ? w1.bh : w0.bh, hcol = 0;
+    if (!(mp.flags & seq::kOutByRow)) {
+      int hh;
+      (h ? w1 : w0).row(mp.heads, &b, &hh);
+      hcol = hh * kDim;
     }
-    // No barrier here: the next chunk writes nothing before the barrier at its start (which every
-    // thread reaches only after this read-out), and that barrier also spreads s_fail.
+    T *po = out.p + ((size_t)b * T_ + (size_t)(h ? w1.c : w0.c) * kC + t0) * out.ld + out.col + hcol + feat;
+    if (!umma::mbar_wait(&barO, it & 1u)) s_fail = 1;
+    umma::fence_after_sync();
+    float o1[16], o2[16];
+    umma::tmem_ld16(tl + cO1 + t0, o1);
+    umma::tmem_ld16(tl + cO2 + t0, o2);
+    umma::tmem_ld_wait();
+    const int64_t ld = kFused ? out.ld : kDim;
+    if (!partial) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) po[j * ld] = (T)(gd[j] * fmaf(up, o1[j], o2[j]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (t0 + j < nvalid) po[j * ld] = (T)(gd[j] * fmaf(up, o1[j], o2[j]));
+    }
+    __syncwarp();
+    // No barrier here: what the next pair writes before its first barrier (products of the quarters) nobody still
+    // reads, and its tiles and tensor-memory operands are written after that barrier.
     umma::fence_before_sync();
   }
   cp_async_wait_all();
-  __syncthreads();      // s_fail of the last chunk is visible
-  if (tid == 0) {
-    if (s_fail) atomicExch(status, 1);
-    // bounded: let copies that are still in flight land before the CTA leaves
-    for (int bb = 0; bb < 2; ++bb)
-      if (n_issued[bb] > n_landed[bb]) acp::mbar_wait(&barRaw[bb], n_landed[bb] & 1u);
+  __syncthreads();      // s_fail of the last pair is visible
+  if (tid == 0 && s_fail) {
+    atomicExch(status, 1);
+    if (raw_pending) acp::mbar_wait(&barRaw, it & 1u);      // bounded: let copies that are still in flight land
   }
   sync_all();
-  if (warp == 0) umma::tmem_dealloc(tb, 64);
+  if (warp == 0) umma::tmem_dealloc(tb, kTmemColsF);
 }
 
 }  // namespace
@@ -334,16 +413,22 @@ int lfw_c64_forward_out(const seq::Maps &mp, const void *state, const void *ckpt
   rc = lfw_chunk_sm_count(&n_sm);
   if (rc != T2FW_OK) return rc;
   const int64_t nc = ceil_div64(T_, kC), total = BH * nc;
-  const unsigned grid = (unsigned)(total < n_sm ? total : n_sm);
-#define T2FW_LAUNCH(TT)                                                                              \
+  const int64_t pairs = (total + 1) / 2;
+  const unsigned grid = (unsigned)(pairs < n_sm ? pairs : n_sm);
+#define T2FW_LAUNCH(TT, FF)                                                                              \
   do {                                                                                               \
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(lfw_c64_fwd_kernel<TT>,                                     \
+    T2FW_CHECK_CUDA(cudaFuncSetAttribute(lfw_c64_fwd_kernel<TT, FF>,                                     \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF));      \
-    T2FW_CHECK_CUDA(launch_dependent(lfw_c64_fwd_kernel<TT>, dim3(grid), dim3(kThreadsF), kSmemF, st, mp,       \
+    T2FW_CHECK_CUDA(launch_dependent(lfw_c64_fwd_kernel<TT, FF>, dim3(grid), dim3(kThreadsF), kSmemF, st, mp,       \
                                      (const TT *)state, (const TT *)ckpt, seq::Out<TT>{(TT *)out, out_ld, out_col}, \
                                      rowflag, status, T_, nc, total));                               \
   } while (0)
-  if (dtype == T2FW_F16) T2FW_LAUNCH(__half); else T2FW_LAUNCH(__nv_bfloat16);
+  const bool fused = (mp.flags & (seq::kUnitForget | seq::kSigmoidGate)) != 0 || mp.q_scale != 1.f;
+  if (dtype == T2FW_F16) {
+    if (fused) T2FW_LAUNCH(__half, true); else T2FW_LAUNCH(__half, false);
+  } else {
+    if (fused) T2FW_LAUNCH(__nv_bfloat16, true); else T2FW_LAUNCH(__nv_bfloat16, false);
+  }
 #undef T2FW_LAUNCH
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;

@@ -12,13 +12,15 @@
 // vectors.  A chunk whose products exceed 2^100 is flagged (its batch row is redone by the scan
 // kernels); products that underflow lose nothing.
 //
-// Persistent CTAs of 16 warps, two per SM.  The four raw 8 KB input blocks of a chunk arrive by
-// bulk asynchronous copy into one of two buffers.  Thread (side, feature, 16-step quarter) forms
-// the product of its quarter, then walks its steps with a running product that starts from the
-// quarters between it and the anchoring end of the chunk.  The d-side values become the A operand
-// in tensor memory (row = feature, stored in both lane sets), the k-side values a K-major
-// shared-memory tile; one lane issues the sixteen MMAs (two interleaved 32-column halves); the fp32
-// result leaves with 32-byte stores.
+// Persistent CTAs of 16 warps, two per SM, each on TWO chunks at a time: chunk 0 of the pair in one lane
+// set of tensor memory, chunk 1 in the other (an M = 64 operand or accumulator takes half of the lanes), so
+// nothing is stored twice.  Thread (chunk, feature, 16-step quarter) walks the gates of its feature on both
+// sides with a running product that starts from the quarters between it and the anchoring end of the chunk:
+// the d-side values become the A operand in tensor memory (row = feature), the k-side values a feature-major
+// shared-memory tile; eight MMAs per chunk; the fp32 result leaves with 16-byte stores.
+//
+// What bounds it: the latency of its phases (two CTAs per SM hide part of it) and shared-memory loads.
+// Config B*H = 96, T = 1024 (1536 chunks): LOC_US against the version with one chunk per iteration.
 #include <mutex>
 
 #include "lfw_c64.cuh"
@@ -33,205 +35,227 @@ namespace {
 
 constexpr int kThreadsL = 512;
 constexpr int kCtasPerSmL = 2;
-// shared-memory map (bytes from the 1024-byte aligned base)
-constexpr int oTk = 0;                             // k-side tile [k][t]
-constexpr int oQtL = oTk + kTile;                  // quarter products [2 sides][4][64]
-constexpr int oRawL = oQtL + 2 * 4 * kDim * 4;     // [2 buffers] val_d, gate_d, val_k, gate_k
+// shared-memory map (bytes from the 1024-byte aligned base), everything once per chunk of the pair
+constexpr int oTk = 0;                             // [chunk] k-side tile [k][t]
+constexpr int oQtL = oTk + 2 * kTile;              // [chunk][side][4][64] products of the quarters
+constexpr int oRawL = oQtL + 2 * 2 * 4 * kDim * 4; // [chunk] val_d, gate_d, val_k, gate_k
 constexpr int kSmemL = oRawL + 2 * 4 * kRawBytes + 1024;
 static_assert(oRawL % 128 == 0, "bulk-copy destination alignment");
 static_assert(kCtasPerSmL * (kSmemL + 1024) <= 227 * 1024, "two CTAs per SM");
 
-constexpr int cA = 0, cD = 64;                     // tensor-memory columns
+constexpr int cA = 0, cD = 64;                     // tensor-memory columns, one lane set per chunk
 constexpr int kTmemColsL = 128;
 
 // kSuffix = true : value * (product of the gates AFTER the step, to the chunk end)   [forward]
 // kSuffix = false: value * (product of the gates up to and including the step)       [backward]
-template <typename T, bool kSuffix>
+template <typename T, bool kSuffix, bool kFused>
 __global__ void __launch_bounds__(kThreadsL, kCtasPerSmL)
 lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M, float *__restrict__ Ac,
                      float *__restrict__ Gc, int *__restrict__ flags, int *__restrict__ status, int64_t T_,
                      int64_t nc, int64_t total) {
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);
-  __shared__ __align__(8) uint64_t barRaw[2], barM;
+  __shared__ __align__(8) uint64_t barRaw, barM;
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_fail, s_bad;
+  __shared__ int s_fail, s_bad2[2][2];
 
   const int tid = threadIdx.x, warp = uniform_warp_idx(), lane = tid & 31;
-  // warps 0-7: d side, tensor-memory rows: lane quarter q4, column part, lane set h, row fl;
-  //            thread = feature 16 * q4 + fl, quarter 2 * h + part of the chunk
-  // warps 8-15: k side: thread = feature, quarter
-  const bool dside = warp < 8;
-  const int q4 = warp & 3, part = (warp >> 2) & 1, h = lane >> 4, fl = lane & 15;
-  const int feat = dside ? 16 * q4 + fl : ((warp - 8) & 1) * 32 + lane;
-  const int tq = dside ? 2 * h + part : (warp - 8) >> 1;
-  float *qtot = reinterpret_cast<float *>(sm + oQtL);
+  // lane quarter of tensor memory, 16-step quarter of the chunk, chunk of the pair, row in the quarter
+  const int q4 = warp & 3, tq = warp >> 2, h = lane >> 4, fl = lane & 15;
+  const int feat = 16 * ((q4 + h) & 3) + fl;       // own feature, both sides
+  const int t0 = 16 * tq;
+  float *qtot = reinterpret_cast<float *>(sm + oQtL) + h * 2 * 4 * kDim + feat;      // own chunk and feature
 
   // tensors: 0 val_d, 1 gate_d, 2 val_k, 3 gate_k
-  const bool unit_forget = (mp.flags & seq::kUnitForget) != 0;
-  auto issue_raw = [&](int64_t ci, int buf) {     // thread 0 only: one copy per tensor
-    const Item w = split_item(ci, nc, mp.heads);
-    const int row = (int)(w.b * T_ + w.c * kC), hc = w.h;
-    const int nv = (int)((T_ - (int64_t)w.c * kC < kC) ? T_ - (int64_t)w.c * kC : kC);
-    unsigned char *r = sm + oRawL + buf * 4 * kRawBytes;
-    const uint32_t per = (mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes;
-    acp::mbar_expect_tx(&barRaw[buf], (unit_forget ? 3u : 4u) * per);
+  const bool unit_forget = kFused && (mp.flags & seq::kUnitForget) != 0;
+  const bool sigmoid_gate = kFused && (mp.flags & seq::kSigmoidGate) != 0;
+  const float k_scale = kFused ? mp.q_scale : 1.f;
+  auto valid_steps = [&](const ItemWalk &w, int64_t ci) {
+    if (ci >= total) return 0;
+    const int64_t left = T_ - (int64_t)w.c * kC;
+    return (int)(left < kC ? left : kC);
+  };
+  auto issue_raw = [&](const ItemWalk *w, int64_t ci) {     // thread 0 only: one copy per tensor and chunk
+    uint32_t bytes = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (!(i == 1 && unit_forget)) seq::fetch_block<T>(mp, i, r + i * kRawBytes, row, hc, nv, &barRaw[buf]);
+    for (int e = 0; e < 2; ++e) {
+      const int nv = valid_steps(w[e], ci + e);
+      if (nv > 0) bytes += (unit_forget ? 3u : 4u) * ((mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
+    }
+    acp::mbar_expect_tx(&barRaw, bytes);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int nv = valid_steps(w[e], ci + e);
+      if (nv <= 0) continue;
+      int b, hc;
+      w[e].row(mp.heads, &b, &hc);
+      const int row = (int)(b * T_ + w[e].c * kC);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (!(i == 1 && unit_forget)) seq::fetch_block<T>(mp, i, sm + oRawL + (e * 4 + i) * kRawBytes, row, hc, nv, &barRaw);
+    }
   };
 
   if (tid == 0) {
-    umma::mbar_init(&barRaw[0], 1);
-    umma::mbar_init(&barRaw[1], 1);
-    umma::mbar_init(&barM, 1);
+    umma::mbar_init(&barRaw, 1);
+    umma::mbar_init(&barM, 2);       // one commit per chunk
     umma::mbar_fence_init();
     s_fail = 0;
+    s_bad2[0][0] = s_bad2[0][1] = s_bad2[1][0] = s_bad2[1][1] = 0;
   }
   if (warp == 0) umma::tmem_alloc(&tmem_slot, kTmemColsL);
-  if (unit_forget) {      // the d-side gate block of both buffers is the constant 1 and never loaded
-    seq::fill_block(reinterpret_cast<T *>(sm + oRawL + kRawBytes), 1.f, tid, kThreadsL);
-    seq::fill_block(reinterpret_cast<T *>(sm + oRawL + 5 * kRawBytes), 1.f, tid, kThreadsL);
-  }
   sync_all();
   dependency_wait();
   const uint32_t tb = __shfl_sync(0xffffffffu, tmem_slot, 0);
   const uint32_t tl = umma::tmem_addr(tb, 32 * q4, 0);
-  uint32_t n_issued[2] = {0u, 0u}, n_landed[2] = {0u, 0u};      // thread 0: bulk-copy rounds per buffer
-  if (tid == 0 && (int64_t)blockIdx.x < total) {
-    issue_raw(blockIdx.x, 0);
-    ++n_issued[0];
+  ItemWalk wn[2] = {ItemWalk(2 * blockIdx.x, 2 * gridDim.x, nc), ItemWalk(2 * blockIdx.x + 1, 2 * gridDim.x, nc)};
+  bool raw_pending = false;      // thread 0
+  if (2 * (int64_t)blockIdx.x < total && tid == 0) {
+    issue_raw(wn, 2 * (int64_t)blockIdx.x);
+    raw_pending = true;
   }
-  const uint64_t dTk = desc_sw128(umma::smem_u32(sm + oTk));
+  const T *raw = reinterpret_cast<const T *>(sm + oRawL + h * 4 * kRawBytes) + t0 * kDim + feat;
+  auto rawv = [&](int blk, int j) { return Elem<T>::ld(raw + blk * kC * kDim + j * kDim); };
+  // k-side tile: row = own feature, 16-byte pieces of steps t0 ..
+  unsigned char *const krow = sm + oTk + h * kTile + (t0 >> 5) * kColBlock + feat * 128;
+  const int ksw = (((t0 >> 2) & 7) ^ (feat & 7)) << 4;
 
   uint32_t it = 0;
-  for (int64_t ci = blockIdx.x; ci < total; ci += gridDim.x, ++it) {
-    const int buf = it & 1;
-    const int64_t c = (int64_t)((uint32_t)ci % (uint32_t)nc), t0c = c * kC;
-    const int nvalid = (int)((T_ - t0c < kC) ? T_ - t0c : kC);
-    T *raw = reinterpret_cast<T *>(sm + oRawL + buf * 4 * kRawBytes);
-    if (tid == 0) {
-      s_bad = 0;
-      if (ci + gridDim.x < total) {      // the other buffer was released at the end of the previous chunk
-        issue_raw(ci + gridDim.x, buf ^ 1);
-        ++n_issued[buf ^ 1];
+  for (int64_t ci = 2 * (int64_t)blockIdx.x; ci < total; ci += 2 * (int64_t)gridDim.x, ++it) {
+    const int nv0 = valid_steps(wn[0], ci), nv1 = valid_steps(wn[1], ci + 1);
+    wn[0].step();
+    wn[1].step();
+    const int nvalid = h ? nv1 : nv0;
+    const bool partial = nv0 < kC || nv1 < kC;      // steps beyond the valid ones become identity steps
+    int *s_bad = s_bad2[it & 1];
+
+    if (!acp::mbar_wait(&barRaw, it & 1u)) s_fail = 1;
+    if (tid == 0) raw_pending = false;
+
+    // gates of one side, own feature and quarter
+    auto gates = [&](int blk, bool kside, float (&g)[16]) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        if (kFused && !kside && unit_forget) g[j] = 1.f;
+        else g[j] = rawv(blk, j);
+        if (kFused && kside && sigmoid_gate) g[j] = seq::sigmoid_gate<T>(g[j]);
       }
-    }
-    if (acp::mbar_wait(&barRaw[buf], (it >> 1) & 1u)) {
-      if (tid == 0) ++n_landed[buf];
-    } else {
-      s_fail = 1;
-    }
-    __syncthreads();
-    if (s_fail) break;
-    if ((mp.flags & seq::kSigmoidGate) || mp.q_scale != 1.f) {      // fused layer: activations applied here
-      if (mp.flags & seq::kSigmoidGate) seq::sigmoid_gate_block(raw + 3 * kC * kDim, tid, kThreadsL);
-      if (mp.q_scale != 1.f) seq::scale_block(raw + 2 * kC * kDim, mp.q_scale, tid, kThreadsL);
-      __syncthreads();
-    }
-    if (nvalid < kC) {      // partial chunk: identity steps beyond the valid ones
-      pad_raw_tail<T>(raw, 4, (1u << 1) | (1u << 3), nvalid, tid, kThreadsL);
-      __syncthreads();
-    }
-
-    // ---- products of the four quarters ----
-    const T *gcol = raw + (dside ? 1 : 3) * kC * kDim + feat, *vcol = raw + (dside ? 0 : 2) * kC * kDim + feat;
-    float g[16];
-    qtot[((dside ? 0 : 4) + tq) * kDim + feat] = load_gates16<T>(gcol, tq, g);
-    __syncthreads();
-
-    // ---- running products from the anchoring end, scaled values ----
-    float w[16];
-    {
-      const float *qt = qtot + (dside ? 0 : 4) * kDim + feat;
+      if (partial) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) g[j] = t0 + j < nvalid ? g[j] : 1.f;
+      }
+      float mn = kRangeHi;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) mn = fminf(mn, fabsf(g[j]));
+      if (!(mn >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+#pragma unroll
+        for (int j = 0; j < 16; ++j) g[j] = sanitize_gate(g[j]);
+      }
+    };
+    auto product = [](const float (&g)[16]) {
+      float p0 = g[0], p1 = g[1];
+#pragma unroll
+      for (int j = 2; j < 16; j += 2) { p0 *= g[j]; p1 *= g[j + 1]; }
+      return p0 * p1;
+    };
+    // values of one side times the running product from the anchoring end; the chunk's total goes to `tot`
+    auto walk = [&](int blk, bool kside, const float (&g)[16], const float *qt, float *tot, float (&w)[16]) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) w[j] = rawv(blk, j);
+      if (kFused && kside && k_scale != 1.f) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) w[j] = seq::round_to<T>(w[j] * k_scale);
+      }
+      if (partial) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) w[j] = t0 + j < nvalid ? w[j] : 0.f;
+      }
       float s = 1.f, hi = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (kSuffix ? i > tq : i < tq) s *= qt[i * kDim];
       if (kSuffix) {
 #pragma unroll
-        for (int i = 3; i > 0; --i)
-          if (i > tq) s *= qt[i * kDim];
-#pragma unroll
         for (int j = 15; j >= 0; --j) {
-          w[j] = bias_tf32(Elem<T>::ld(vcol + (16 * tq + j) * kDim) * s);
+          w[j] = bias_tf32(w[j] * s);
           s *= g[j];
           hi = fmaxf(hi, fabsf(s));
         }
       } else {
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
-          if (i < tq) s *= qt[i * kDim];
-#pragma unroll
         for (int j = 0; j < 16; ++j) {
           s *= g[j];
           hi = fmaxf(hi, fabsf(s));
-          w[j] = bias_tf32(Elem<T>::ld(vcol + (16 * tq + j) * kDim) * s);
+          w[j] = bias_tf32(w[j] * s);
         }
       }
-      if (!(hi <= kRangeHi)) s_bad = 1;     // also catches NaN
-      // total decay of the chunk for this feature
-      if (tq == (kSuffix ? 0 : 3)) (dside ? Ac : Gc)[(size_t)ci * kDim + feat] = s;
-    }
-    if (dside) {
-      // A operand [d][t] in both lane sets: the lower half warp holds quarter `part`, the upper
-      // half warp quarter 2 + part of the same rows; one store names one column range per warp
-      float lo[16], hi2[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float p = __shfl_xor_sync(0xffffffffu, w[j], 16);
-        lo[j] = h ? p : w[j];
-        hi2[j] = h ? w[j] : p;
-      }
-      umma::tmem_st16(tl + cA + 16 * part, lo);
-      umma::tmem_st16(tl + cA + 32 + 16 * part, hi2);
-      umma::tmem_st_wait();
-    } else {
-      unsigned char *tk = sm + oTk;
-#pragma unroll
-      for (int j = 0; j < 16; j += 4)
-        *reinterpret_cast<float4 *>(tk + toff(feat, 16 * tq + j)) = make_float4(w[j], w[j + 1], w[j + 2], w[j + 3]);
-    }
-    umma::fence_async_smem();
-    sync_all();       // operands complete, raw buffer consumed
+      if (!(hi <= kRangeHi)) s_bad[h] = 1;     // also catches NaN
+      if (tq == (kSuffix ? 0 : 3) && nvalid > 0) tot[(size_t)(ci + h) * kDim + feat] = s;
+    };
 
-    if (warp == 0) {
-      const uint32_t d0 = tb, d1 = umma::tmem_addr(tb, 16, 0);
-      constexpr uint32_t idesc = umma::make_idesc_tf32(64, 32, false, false);
-      constexpr uint64_t n1 = (uint64_t)(32 * 128 >> 4);     // k rows 32..63
+    float gk[16], gd[16];
+    gates(3, true, gk);
+    qtot[(4 + tq) * kDim] = product(gk);
+    gates(1, false, gd);
+    qtot[tq * kDim] = product(gd);
+    umma::named_barrier(1 + q4, 128);      // the four warps that hold the quarters of the same features
+    {
+      float w[16];
+      walk(2, true, gk, qtot + 4 * kDim, Gc, w);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4 *>(krow + (ksw ^ (j << 4))) = make_float4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+      walk(0, false, gd, qtot, Ac, w);
+      umma::tmem_st16(tl + cA + t0, w);
+    }
+    umma::tmem_st_wait();
+    umma::fence_async_smem();
+    sync_all();       // operands complete, raw blocks consumed
+    if (s_fail) break;
+
+    if (warp < 2) {
+      const uint32_t ls = umma::tmem_addr(tb, 16 * warp, 0);
+      const uint64_t dk = desc_sw128(umma::smem_u32(sm + oTk) + warp * kTile);
       if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint64_t o = (uint64_t)(((ks >> 2) * kColBlock + (ks & 3) * 32) >> 4);
-          mma_tf32_ts(d0 + cD, d0 + cA + 8 * ks, dTk + o, idesc, ks > 0);
-          mma_tf32_ts(d1 + cD, d1 + cA + 8 * ks, dTk + n1 + o, idesc, ks > 0);
-        }
+        for (int ks = 0; ks < 8; ++ks) mma_tf32_ts(ls + cD, ls + cA + 8 * ks, dk + kstep(ks), kIdesc64, ks > 0);
         umma::mma_commit(&barM);
       }
       __syncwarp();
-      if (tid == 0) flags[ci] = s_bad;
+    }
+    if (tid == 0) {
+      if (ci + 2 * (int64_t)gridDim.x < total) {
+        issue_raw(wn, ci + 2 * (int64_t)gridDim.x);
+        raw_pending = true;
+      }
+      flags[ci] = s_bad[0];
+      if (nv1 > 0) flags[ci + 1] = s_bad[1];
+      s_bad2[(it & 1) ^ 1][0] = s_bad2[(it & 1) ^ 1][1] = 0;
     }
     if (!umma::mbar_wait(&barM, it & 1u)) {
       s_fail = 1;
-      flags[ci] = 1;      // results unusable: let the scan kernels redo the row
+      if (nvalid > 0) flags[ci + h] = 1;      // results unusable: let the scan kernels redo the row
     }
     umma::fence_after_sync();
     {
-      // thread (lane quarter, column part, lane set, row): row d, columns 32 * h + 8 * (warp >> 2) .. + 7
-      const int d = 16 * q4 + fl, k0 = 32 * h + 8 * (warp >> 2);
-      float v[8];
-      umma::tmem_ld8(tl + cD + 8 * (warp >> 2), v);
+      float v[16];      // row d = own feature, columns k = t0 .. t0 + 15
+      umma::tmem_ld16(tl + cD + t0, v);
       umma::tmem_ld_wait();
-      float *dst = M + ((size_t)ci * kDim + d) * kDim + k0;
-      *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-      *reinterpret_cast<float4 *>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+      if (nvalid > 0) {
+        float *dst = M + ((size_t)(ci + h) * kDim + feat) * kDim + t0;
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4 *>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+      }
+      __syncwarp();
     }
-    // No barrier here: the next chunk writes nothing before the barrier at its start, which every
-    // thread reaches only after this read-out; that barrier also spreads s_fail.
+    // No barrier here: what the next pair writes before its full barrier (products of the quarters, own rows of the
+    // operands) is read by nobody any more once this thread's wait for the MMAs is over.
     umma::fence_before_sync();
   }
-  __syncthreads();      // s_fail of the last chunk is visible
-  if (tid == 0) {
-    if (s_fail) atomicExch(status, 1);
-    for (int bb = 0; bb < 2; ++bb)     // bounded: let copies that are still in flight land
-      if (n_issued[bb] > n_landed[bb]) acp::mbar_wait(&barRaw[bb], n_landed[bb] & 1u);
+  __syncthreads();      // s_fail of the last pair is visible
+  if (tid == 0 && s_fail) {
+    atomicExch(status, 1);
+    if (raw_pending) acp::mbar_wait(&barRaw, it & 1u);      // bounded: let copies that are still in flight land
   }
   sync_all();
   if (warp == 0) umma::tmem_dealloc(tb, kTmemColsL);
@@ -297,19 +321,26 @@ int lfw_chunk_local_umma(bool backward, const seq::Maps &mp, float *M, float *Ac
   rc = lfw_chunk_sm_count(&sms);
   if (rc != T2FW_OK) return rc;
   const int64_t max_ctas = (int64_t)sms * kCtasPerSmL;
-  const unsigned grid = (unsigned)(total < max_ctas ? total : max_ctas);
-#define T2FW_LAUNCH(TT, SUF)                                                                          \
+  const int64_t pairs = (total + 1) / 2;
+  const unsigned grid = (unsigned)(pairs < max_ctas ? pairs : max_ctas);
+#define T2FW_LAUNCH(TT, SUF, FF)                                                                          \
   do {                                                                                                \
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(lfw_c64_local_kernel<TT, SUF>,                               \
+    T2FW_CHECK_CUDA(cudaFuncSetAttribute(lfw_c64_local_kernel<TT, SUF, FF>,                               \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemL));       \
-    T2FW_CHECK_CUDA(launch_dependent(lfw_c64_local_kernel<TT, SUF>, dim3(grid), dim3(kThreadsL), kSmemL, st, mp, M, \
+    T2FW_CHECK_CUDA(launch_dependent(lfw_c64_local_kernel<TT, SUF, FF>, dim3(grid), dim3(kThreadsL), kSmemL, st, mp, M, \
                                      Ac, Gc, flags, status, T_, nc, total));                         \
   } while (0)
+  const bool fused = (mp.flags & (seq::kUnitForget | seq::kSigmoidGate)) != 0 || mp.q_scale != 1.f;
+#define T2FW_FUSED(TT, SUF)                                                   \
+  do {                                                                        \
+    if (fused) T2FW_LAUNCH(TT, SUF, true); else T2FW_LAUNCH(TT, SUF, false);  \
+  } while (0)
   if (dtype == T2FW_F16) {
-    if (backward) T2FW_LAUNCH(__half, false); else T2FW_LAUNCH(__half, true);
+    if (backward) T2FW_FUSED(__half, false); else T2FW_FUSED(__half, true);
   } else {
-    if (backward) T2FW_LAUNCH(__nv_bfloat16, false); else T2FW_LAUNCH(__nv_bfloat16, true);
+    if (backward) T2FW_FUSED(__nv_bfloat16, false); else T2FW_FUSED(__nv_bfloat16, true);
   }
+#undef T2FW_FUSED
 #undef T2FW_LAUNCH
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;
