@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -39,6 +40,20 @@ void count_launch(int n = 1);
   do {                                                                               \
     ::t2fw::count_launch(n);                                                         \
     T2FW_CHECK_CUDA(cudaGetLastError());                                             \
+  } while (0)
+
+// Opt a kernel in to `bytes` of dynamic shared memory, once per device: the attribute belongs to the device's
+// context, and setting it anew costs a fifth of a launch.  (Two threads may both set it: the value is the same.)
+#define T2FW_ALLOW_SMEM(kernel, bytes)                                                                          \
+  do {                                                                                                          \
+    static std::atomic<unsigned long long> _done{0};                                                            \
+    int _dev = 0;                                                                                               \
+    T2FW_CHECK_CUDA(cudaGetDevice(&_dev));                                                                      \
+    const unsigned long long _bit = 1ull << (_dev & 63);                                                        \
+    if (!(_done.load(std::memory_order_relaxed) & _bit)) {                                                      \
+      T2FW_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))); \
+      _done.fetch_or(_bit, std::memory_order_relaxed);                                                          \
+    }                                                                                                           \
   } while (0)
 
 // ---- programmatic dependent launch -------------------------------------------------------

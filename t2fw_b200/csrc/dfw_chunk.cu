@@ -680,8 +680,8 @@ static int dfw_chunk_forward_typed(const void *q, const void *k, const void *v, 
                                    cudaStream_t st) {
   const int64_t nc = ceil_div64(T_, kC);
   float *W = static_cast<float *>(scratch), *U = W + wu_floats(B, nc);
-  T2FW_CHECK_CUDA(cudaFuncSetAttribute(dfw_chunk_prep_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(3 * kPrepTile)));
+  auto *const kern1 = &dfw_chunk_prep_kernel<T, false>;
+  T2FW_ALLOW_SMEM(kern1, 3 * kPrepTile);
   dfw_chunk_prep_kernel<T, false><<<(unsigned)(B * nc), 128, 3 * kPrepTile, st>>>(
       (const T *)q, (const T *)k, (const T *)v, W, U, T_, nc);
   if (dfw_umma_enabled()) {
@@ -689,8 +689,8 @@ static int dfw_chunk_forward_typed(const void *q, const void *k, const void *v, 
                                           std::is_same<T, __half>::value ? T2FW_F16 : T2FW_BF16, st);
     if (rc != T2FW_ERR_UNSUPPORTED) return rc;
   }
-  T2FW_CHECK_CUDA(cudaFuncSetAttribute(dfw_chunk_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(7 * kTileVBytes)));
+  auto *const kern2 = &dfw_chunk_fwd_kernel<T>;
+  T2FW_ALLOW_SMEM(kern2, 7 * kTileVBytes);
   dfw_chunk_fwd_kernel<T><<<(unsigned)B, kSeqThreads, 7 * kTileVBytes, st>>>(
       (const T *)q, (const T *)k, (const T *)state, W, U, (T *)out, (T *)final_state, (float *)delta, T_, nc);
   T2FW_CHECK_LAUNCH(2);
@@ -711,8 +711,8 @@ static int dfw_chunk_backward_typed(const void *go, const void *gs, const void *
                                     void *ds, int64_t B, int64_t T_, void *scratch, cudaStream_t st) {
   const int64_t nc = ceil_div64(T_, kC);
   float *Wb = static_cast<float *>(scratch), *Ub = Wb + wu_floats(B, nc);
-  T2FW_CHECK_CUDA(cudaFuncSetAttribute(dfw_chunk_prep_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(4 * kPrepTile)));
+  auto *const kern3 = &dfw_chunk_prep_kernel<T, true>;
+  T2FW_ALLOW_SMEM(kern3, 4 * kPrepTile);
   dfw_chunk_prep_kernel<T, true><<<(unsigned)(B * nc), 128, 4 * kPrepTile, st>>>(
       (const T *)q, (const T *)k, (const T *)go, Wb, Ub, T_, nc);
   float *Sc = Ub + u_floats(B, nc), *Rc = Sc + wu_floats(B, nc), *Ec = Rc + wu_floats(B, nc);
@@ -722,8 +722,8 @@ static int dfw_chunk_backward_typed(const void *go, const void *gs, const void *
                                     std::is_same<T, __half>::value ? T2FW_F16 : T2FW_BF16, st);
   if (seq_rc != T2FW_OK && seq_rc != T2FW_ERR_UNSUPPORTED) return seq_rc;
   if (seq_rc == T2FW_ERR_UNSUPPORTED) {
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(dfw_chunk_bwd_seq_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(7 * kTileVBytes)));
+    auto *const kern4 = &dfw_chunk_bwd_seq_kernel<T>;
+  T2FW_ALLOW_SMEM(kern4, 7 * kTileVBytes);
     dfw_chunk_bwd_seq_kernel<T><<<(unsigned)B, kSeqThreads, 7 * kTileVBytes, st>>>(
         (const T *)go, (const T *)gs, (const T *)q, (const T *)k, (const float *)delta, (const T *)final_state,
         Wb, Ub, Sc, Rc, Ec, (T *)dv, (T *)ds, T_, nc);
@@ -734,8 +734,8 @@ static int dfw_chunk_backward_typed(const void *go, const void *gs, const void *
                                     std::is_same<T, __half>::value ? T2FW_F16 : T2FW_BF16, st);
   if (par_rc != T2FW_OK && par_rc != T2FW_ERR_UNSUPPORTED) return par_rc;
   if (par_rc == T2FW_ERR_UNSUPPORTED) {
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(dfw_chunk_bwd_par_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(10 * kTileVBytes)));
+    auto *const kern5 = &dfw_chunk_bwd_par_kernel<T>;
+  T2FW_ALLOW_SMEM(kern5, 10 * kTileVBytes);
     dfw_chunk_bwd_par_kernel<T><<<(unsigned)(B * nc), kSeqThreads, 10 * kTileVBytes, st>>>(
         (const T *)go, (const T *)q, (const T *)k, (const float *)delta, Sc, Rc, Ec, (T *)dq, (T *)dk, T_, nc);
   }

@@ -790,8 +790,8 @@ int dfw_chunk_forward_umma(const void *q, const void *k, const void *state, cons
   const int64_t nc = ceil_div64(T_, kC);
 #define T2FW_LAUNCH(TT)                                                                                  \
   do {                                                                                                   \
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(dfw_chunk_fwd_umma_kernel<TT>,                                  \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemU));          \
+    auto *const kern1 = &dfw_chunk_fwd_umma_kernel<TT>; \
+    T2FW_ALLOW_SMEM(kern1, kSmemU);          \
     dfw_chunk_fwd_umma_kernel<TT><<<(unsigned)B, kTh, kSmemU, st>>>(                                     \
         (const TT *)q, (const TT *)k, (const TT *)state, W, U, (TT *)out, (TT *)final_state, (float *)delta, \
         status, T_, nc);                                                                                 \
@@ -816,8 +816,8 @@ int dfw_chunk_bwd_seq_umma(const void *go, const void *gs, const void *q, const 
   const int64_t nc = ceil_div64(T_, kC);
 #define T2FW_LAUNCH(TT)                                                                                  \
   do {                                                                                                   \
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(dfw_chunk_bwd_seq_umma_kernel<TT>,                              \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemB));          \
+    auto *const kern2 = &dfw_chunk_bwd_seq_umma_kernel<TT>; \
+    T2FW_ALLOW_SMEM(kern2, kSmemB);          \
     dfw_chunk_bwd_seq_umma_kernel<TT><<<(unsigned)B, kTh, kSmemB, st>>>(                                 \
         (const TT *)go, (const TT *)gs, (const TT *)q, (const TT *)k, (const float *)delta,              \
         (const TT *)final_state, Wb, Ub, ScT, RcT, Ec, (TT *)dv, (TT *)ds, status, T_, nc);              \
@@ -850,8 +850,8 @@ int dfw_chunk_bwd_par_umma(const void *go, const void *q, const void *k, const v
   const unsigned grid = (unsigned)(total < n_sm ? total : n_sm);     // one persistent CTA per SM
 #define T2FW_LAUNCH(TT)                                                                                  \
   do {                                                                                                   \
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(dfw_chunk_bwd_par_umma_kernel<TT>,                              \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemP));          \
+    auto *const kern3 = &dfw_chunk_bwd_par_umma_kernel<TT>; \
+    T2FW_ALLOW_SMEM(kern3, kSmemP);          \
     dfw_chunk_bwd_par_umma_kernel<TT><<<grid, kTh, kSmemP, st>>>(                                        \
         (const TT *)go, (const TT *)q, (const TT *)k, (const float *)delta, ScT, RcT, Ec, (TT *)dq,      \
         (TT *)dk, status, T_, nc, total);                                                                \

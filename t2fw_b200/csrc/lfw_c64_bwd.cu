@@ -637,7 +637,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         for (int j = 0; j < 16; ++j) {
           float dg = (H[j] + base + sb[j]) * pm[j];
           if (kFused && sigmoid_gate && h == 0) {      // d gate / d pre-activation, from the pre-activation itself in fp32
-            const float e = __expf(-Elem<T>::ld(pre + j * kDim)), sg = rcp_fast(1.f + e);
+            const float e = seq::exp_neg(Elem<T>::ld(pre + j * kDim)), sg = seq::rcp1p(e);
             dg *= sg > seq::kGateFloor ? sg * sg * e : 0.f;      // s (1 - s) = s^2 e^{-g}
           }
           if (full || j < n_own) p_gt[j * ld_gt] = (T)dg;
@@ -675,8 +675,8 @@ int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ck
 #define T2FW_OUT(TT, i) seq::Out<TT>{(TT *)outs[i], out_ld[i], out_col[i]}
 #define T2FW_LAUNCH(TT, FF)                                                                           \
   do {                                                                                                \
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(lfw_c64_bwd_kernel<TT, FF>,                                  \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemB));       \
+    auto *const kern1 = &lfw_c64_bwd_kernel<TT, FF>; \
+    T2FW_ALLOW_SMEM(kern1, kSmemB);       \
     T2FW_CHECK_CUDA(launch_dependent(lfw_c64_bwd_kernel<TT, FF>, dim3(grid), dim3(kThreadsB), kSmemB, st, mp,   \
                                      (const TT *)state, (const TT *)ckpt, Rend, T2FW_OUT(TT, 0), T2FW_OUT(TT, 1), \
                                      T2FW_OUT(TT, 2), T2FW_OUT(TT, 3), T2FW_OUT(TT, 4), rowflag, status, T_, nc,  \

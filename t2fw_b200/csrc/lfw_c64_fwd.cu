@@ -61,7 +61,7 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
                    int64_t nc, int64_t total) {
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);   // swizzle atoms are 1024-byte aligned
-  __shared__ __align__(8) uint64_t barRaw, barP, barO;
+  __shared__ __align__(8) uint64_t barG, barV, barP, barO;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_fail, s_bad2[2][2];
 
@@ -81,14 +81,18 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     const int64_t left = T_ - (int64_t)w.c * kC;
     return (int)(left < kC ? left : kC);
   };
-  auto issue_raw = [&](const ItemWalk *w, int64_t ci) {     // thread 0 only: one copy per tensor and chunk
+  // Two groups with a barrier each: the gate blocks (f, fk) are free again after the products of the quarters, the value
+  // blocks (x, q, k) only once the operands are built, so the next pair's gates are requested that much earlier.
+  auto issue_raw = [&](const ItemWalk *w, int64_t ci, bool gates) {     // thread 0 only: one copy per tensor and chunk
+    const uint32_t n = gates ? (unit_forget ? 1u : 2u) : 3u;
+    uint64_t *bar = gates ? &barG : &barV;
     uint32_t bytes = 0;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int nv = valid_steps(w[e], ci + e);
-      if (nv > 0) bytes += (unit_forget ? 4u : 5u) * ((mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
+      if (nv > 0) bytes += n * ((mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
     }
-    acp::mbar_expect_tx(&barRaw, bytes);
+    acp::mbar_expect_tx(bar, bytes);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int nv = valid_steps(w[e], ci + e);
@@ -98,7 +102,8 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       const int row = (int)(b * T_ + w[e].c * kC);
 #pragma unroll
       for (int i = 0; i < 5; ++i)
-        if (!(i == 1 && unit_forget)) seq::fetch_block<T>(mp, i, sm + oRaw + (e * 5 + i) * kRawBytes, row, hc, nv, &barRaw);
+        if ((i == 1 || i == 4) == gates && !(i == 1 && unit_forget))
+          seq::fetch_block<T>(mp, i, sm + oRaw + (e * 5 + i) * kRawBytes, row, hc, nv, bar);
     }
   };
   // start states of the pair (the caller's state for the first chunk of a row, else the checkpoint written
@@ -114,7 +119,8 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   };
 
   if (tid == 0) {
-    umma::mbar_init(&barRaw, 1);
+    umma::mbar_init(&barG, 1);
+    umma::mbar_init(&barV, 1);
     umma::mbar_init(&barP, 2);       // one commit per chunk
     umma::mbar_init(&barO, 4);       // O1 and O2 of both chunks
     umma::mbar_fence_init();
@@ -127,11 +133,12 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   const uint32_t tb = __shfl_sync(0xffffffffu, tmem_slot, 0);
   const uint32_t tl = umma::tmem_addr(tb, 32 * q4, 0);
   ItemWalk wn[2] = {ItemWalk(2 * blockIdx.x, 2 * gridDim.x, nc), ItemWalk(2 * blockIdx.x + 1, 2 * gridDim.x, nc)};
-  bool raw_pending = false;      // thread 0
+  uint32_t n_issued[2] = {0u, 0u}, n_landed[2] = {0u, 0u};      // thread 0: bulk-copy rounds of the gates and of the values
   if (2 * (int64_t)blockIdx.x < total) {
     if (tid == 0) {
-      issue_raw(wn, 2 * (int64_t)blockIdx.x);
-      raw_pending = true;
+      issue_raw(wn, 2 * (int64_t)blockIdx.x, true);
+      issue_raw(wn, 2 * (int64_t)blockIdx.x, false);
+      n_issued[0] = n_issued[1] = 1u;
     }
     issue_state(wn, 2 * (int64_t)blockIdx.x);
   }
@@ -157,8 +164,8 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     int *s_bad = s_bad2[it & 1];
 
     cp_async_wait_all();       // this thread's share of the start states (requested one pair ahead)
-    if (!acp::mbar_wait(&barRaw, it & 1u)) s_fail = 1;
-    if (tid == 0) raw_pending = false;
+    if (acp::mbar_wait(&barG, it & 1u)) ++n_landed[0];
+    else s_fail = 1;
 
     // ---- gates of the own feature and quarter on both sides, products of the quarters ----
     float gk[16], gd[16];
@@ -192,6 +199,12 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     qtot[(4 + tq) * kDim + feat] = pd;
     __syncthreads();           // also: the start states of both chunks have landed
     if (s_fail) break;
+    if (tid == 0 && ci + 2 * (int64_t)gridDim.x < total) {
+      issue_raw(wn, ci + 2 * (int64_t)gridDim.x, true);
+      ++n_issued[0];
+    }
+    if (acp::mbar_wait(&barV, it & 1u)) ++n_landed[1];
+    else s_fail = 1;
 
     // ---- operands ----
     float lo, hi;
@@ -323,8 +336,8 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     }
     if (ci + 2 * (int64_t)gridDim.x < total) {
       if (tid == 0) {
-        issue_raw(wn, ci + 2 * (int64_t)gridDim.x);
-        raw_pending = true;
+        issue_raw(wn, ci + 2 * (int64_t)gridDim.x, false);
+        ++n_issued[1];
       }
       issue_state(wn, ci + 2 * (int64_t)gridDim.x);
     }
@@ -338,13 +351,22 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     if (!umma::mbar_wait(&barP, it & 1u)) s_fail = 1;
     umma::fence_after_sync();
     {
+      // a warp holds 16 x 16 values: on the diagonal it masks, below it nothing is masked, above it all is zero
       float v[16];
-      if (tq <= q4) {        // above the diagonal there is nothing to read
+      if (tq <= q4) {
         umma::tmem_ld16(tl + cP + t0, v);
         umma::tmem_ld_wait();
-      }
+        if (tq == q4) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = t0 + j <= p_row ? bias_tf32(v[j]) : 0.f;
+          for (int j = 0; j < 16; ++j) v[j] = j <= fl ? bias_tf32(v[j]) : 0.f;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = bias_tf32(v[j]);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = 0.f;
+      }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
         *reinterpret_cast<float4 *>(prow + (psw ^ (j << 4))) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
@@ -395,7 +417,9 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   __syncthreads();      // s_fail of the last pair is visible
   if (tid == 0 && s_fail) {
     atomicExch(status, 1);
-    if (raw_pending) acp::mbar_wait(&barRaw, it & 1u);      // bounded: let copies that are still in flight land
+    // bounded: let copies that are still in flight land before the CTA leaves
+    if (n_issued[0] > n_landed[0]) acp::mbar_wait(&barG, n_landed[0] & 1u);
+    if (n_issued[1] > n_landed[1]) acp::mbar_wait(&barV, n_landed[1] & 1u);
   }
   sync_all();
   if (warp == 0) umma::tmem_dealloc(tb, kTmemColsF);
@@ -417,8 +441,8 @@ int lfw_c64_forward_out(const seq::Maps &mp, const void *state, const void *ckpt
   const unsigned grid = (unsigned)(pairs < n_sm ? pairs : n_sm);
 #define T2FW_LAUNCH(TT, FF)                                                                              \
   do {                                                                                               \
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(lfw_c64_fwd_kernel<TT, FF>,                                     \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF));      \
+    auto *const kern1 = &lfw_c64_fwd_kernel<TT, FF>; \
+    T2FW_ALLOW_SMEM(kern1, kSmemF);      \
     T2FW_CHECK_CUDA(launch_dependent(lfw_c64_fwd_kernel<TT, FF>, dim3(grid), dim3(kThreadsF), kSmemF, st, mp,       \
                                      (const TT *)state, (const TT *)ckpt, seq::Out<TT>{(TT *)out, out_ld, out_col}, \
                                      rowflag, status, T_, nc, total));                               \

@@ -238,18 +238,26 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
     }
     umma::fence_after_sync();
     {
-      float v[16];      // row d = own feature, columns k = t0 .. t0 + 15
+      // Row d = own feature, columns k = t0 .. t0 + 15.  Stored straight from here, the lanes of a warp would write 32
+      // different lines with every instruction; so the rows of a quarter pass through the k-side tile (consumed), its
+      // 16-byte pieces XOR-ed with the row, and leave as whole rows.
+      float v[16];
       umma::tmem_ld16(tl + cD + t0, v);
       umma::tmem_ld_wait();
-      if (nvalid > 0) {
-        float *dst = M + ((size_t)(ci + h) * kDim + feat) * kDim + t0;
+      unsigned char *stg = sm + oTk + h * kTile + feat * 256;
 #pragma unroll
-        for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4 *>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float4 *>(stg + (((4 * tq + j) ^ (feat & 7)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      umma::named_barrier(1 + q4, 128);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {      // two rows per instruction: rows 8 (tq & 1) .. of this quarter's 16 in chunk tq >> 1
+        const int e = tq >> 1, r = 16 * ((q4 + e) & 3) + 8 * (tq & 1) + 2 * i + h;
+        const float4 o = *reinterpret_cast<const float4 *>(sm + oTk + e * kTile + r * 256 + ((fl ^ (r & 7)) << 4));
+        if (e == 0 || nv1 > 0) *reinterpret_cast<float4 *>(M + ((size_t)(ci + e) * kDim + r) * kDim + 4 * fl) = o;
       }
-      __syncwarp();
     }
-    // No barrier here: what the next pair writes before its full barrier (products of the quarters, own rows of the
-    // operands) is read by nobody any more once this thread's wait for the MMAs is over.
+    // No full barrier here: before the next one the next pair writes only products of quarters, which nobody reads any
+    // more, and, after the quarter's own barrier, the operand rows of its features, which only this quarter's warps used.
     umma::fence_before_sync();
   }
   __syncthreads();      // s_fail of the last pair is visible
@@ -325,8 +333,8 @@ int lfw_chunk_local_umma(bool backward, const seq::Maps &mp, float *M, float *Ac
   const unsigned grid = (unsigned)(pairs < max_ctas ? pairs : max_ctas);
 #define T2FW_LAUNCH(TT, SUF, FF)                                                                          \
   do {                                                                                                \
-    T2FW_CHECK_CUDA(cudaFuncSetAttribute(lfw_c64_local_kernel<TT, SUF, FF>,                               \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemL));       \
+    auto *const kern1 = &lfw_c64_local_kernel<TT, SUF, FF>; \
+    T2FW_ALLOW_SMEM(kern1, kSmemL);       \
     T2FW_CHECK_CUDA(launch_dependent(lfw_c64_local_kernel<TT, SUF, FF>, dim3(grid), dim3(kThreadsL), kSmemL, st, mp, M, \
                                      Ac, Gc, flags, status, T_, nc, total));                         \
   } while (0)

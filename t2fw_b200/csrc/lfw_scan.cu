@@ -11,85 +11,141 @@
 // is produced inside the kernels; no [B,T,D,K] tensor exists.  Only every C-th state is
 // stored; the backward pass recomputes the others from those checkpoints.
 //
-// The backward runs the same kernel twice with the two axes exchanged:
+// The backward runs the same code twice with the two axes exchanged, side by side:
 //   row orientation    (own = d, lanes = k): d_x = R k, d_f = (R.*S_prev) fk, d_state
 //   column orientation (own = k, lanes = d): d_k = R^T x, d_f_key = (R.*S_prev)^T f, d_q = S^T dO
 // so every reduction is a warp reduction and the result is deterministic.
-#include "common.cuh"
+//
+// A chain of T steps bounds these kernels.  The steps' vectors come from shared memory, fetched a group ahead
+// (scan.cuh); the sums of a step share their shuffles; the two orientations run side by side; the backward
+// walks a checkpoint's steps forward once to leave the state at each segment start and then segment by segment
+// (128 forward steps per 64 instead of 160).  fp32, 16 rows of 129 steps, 96 x 48: forward 95 -> SCAN_FWD us,
+// backward 366 -> SCAN_BWD us.
+//
+// These kernels also redo the batch rows that the chunk kernels flagged (gate products outside the range of
+// the factored form): CTAs walk over all work items and skip the rows without a flag, and the launch is a
+// dependent one, so an all-clear costs about a microsecond.
+#include "scan.cuh"
 
 namespace t2fw {
 
 namespace {
 
 constexpr int kWarpsPerCta = 4;
+constexpr int kThreads = kWarpsPerCta * 32;
+
+template <typename T>
+struct FwdArgs {
+  const T *x, *f, *q, *k, *fk, *state;
+  T *out, *ckpt;
+  int64_t B, T_;
+  int D, K;
+  int64_t C, nslots;
+  int G;                  // steps per group
+  int64_t items;          // work items: (batch row, block of state rows)
+  const int *rowflag;     // if not null, only batch rows with a non-zero flag are processed
+};
+
+// One buffer: fk, k, q [G][K], x, f [G][kWarpsPerCta * OWN], each part 16-byte aligned
+template <typename T>
+__host__ __device__ inline int fwd_part(int G, int n) { return (int)((((size_t)G * n * sizeof(T)) + 15) / 16 * 16); }
 
 template <typename T, int NL, int OWN>
-__global__ void __launch_bounds__(kWarpsPerCta * 32)
-lfw_scan_fwd_kernel(const T *__restrict__ x, const T *__restrict__ f, const T *__restrict__ q,
-                    const T *__restrict__ k, const T *__restrict__ fk,
-                    const T *__restrict__ state, T *__restrict__ out, T *__restrict__ ckpt,
-                    int64_t B, int64_t T_, int64_t D, int64_t K, int64_t C, int64_t nslots,
-                    const int *__restrict__ rowflag) {
+__global__ void __launch_bounds__(kThreads) lfw_scan_fwd_kernel(const FwdArgs<T> a) {
   using A = typename Elem<T>::acc;
-  const int lane = threadIdx.x & 31;
-  const int64_t groups = (D + OWN - 1) / OWN;
-  const int64_t warp = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
-  if (warp >= B * groups) return;
-  const int64_t b = warp / groups;
-  const int64_t r0 = (warp % groups) * OWN;
-  if (rowflag != nullptr && rowflag[b] == 0) return;  // only rows the caller marked
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int RC = kWarpsPerCta * OWN;      // state rows of the CTA
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int kp = fwd_part<T>(a.G, a.K), dp = fwd_part<T>(a.G, RC), buf_bytes = 3 * kp + 2 * dp;
+  const int blocks_d = (a.D + RC - 1) / RC;
+  dependency_wait();
+  for (int64_t item = blockIdx.x; item < a.items; item += gridDim.x) {
+    const int64_t b = item / blocks_d;
+    if (a.rowflag != nullptr && a.rowflag[b] == 0) continue;      // the same for the whole CTA
+    const int rb = (int)(item - b * blocks_d) * RC, nrows = a.D - rb < RC ? a.D - rb : RC;
+    const int r0 = rb + warp * OWN;
 
-  A S[OWN][NL];
-#pragma unroll
-  for (int o = 0; o < OWN; ++o)
-#pragma unroll
-    for (int j = 0; j < NL; ++j) {
-      const int64_t row = r0 + o, c = lane + 32 * j;
-      S[o][j] = (row < D && c < K) ? Elem<T>::ld(state + (b * D + row) * K + c) : A(0);
-    }
+    auto fetch = [&](int64_t t0, int which) {
+      const int n = (int)(a.T_ - t0 < a.G ? a.T_ - t0 : a.G);
+      unsigned char *p = smem_raw + which * buf_bytes;
+      const int64_t ko = (b * a.T_ + t0) * a.K, od = (b * a.T_ + t0) * a.D + rb;
+      scan::stage(reinterpret_cast<T *>(p), a.fk + ko, n * a.K, tid, kThreads);
+      scan::stage(reinterpret_cast<T *>(p + kp), a.k + ko, n * a.K, tid, kThreads);
+      scan::stage(reinterpret_cast<T *>(p + 2 * kp), a.q + ko, n * a.K, tid, kThreads);
+      scan::stage_rows(reinterpret_cast<T *>(p + 3 * kp), a.x + od, n, nrows, a.D, tid, kThreads);
+      scan::stage_rows(reinterpret_cast<T *>(p + 3 * kp + dp), a.f + od, n, nrows, a.D, tid, kThreads);
+      scan::commit();
+    };
+    fetch(0, 0);
 
-  for (int64_t t = 0; t < T_; ++t) {
-    const int64_t bk = (b * T_ + t) * K, bd = (b * T_ + t) * D;
-    A gl[NL], kl[NL], ql[NL];
+    A S[OWN][NL];
 #pragma unroll
-    for (int j = 0; j < NL; ++j) {
-      const int64_t c = lane + 32 * j;
-      const bool in = c < K;
-      gl[j] = in ? Elem<T>::ld(fk + bk + c) : A(0);
-      kl[j] = in ? Elem<T>::ld(k + bk + c) : A(0);
-      ql[j] = in ? Elem<T>::ld(q + bk + c) : A(0);
-    }
-#pragma unroll
-    for (int o = 0; o < OWN; ++o) {
-      const int64_t row = r0 + o;
-      const bool in = row < D;
-      const A xo = in ? Elem<T>::ld(x + bd + row) : A(0);
-      const A ao = in ? Elem<T>::ld(f + bd + row) : A(0);
-      A acc = A(0);
+    for (int o = 0; o < OWN; ++o)
 #pragma unroll
       for (int j = 0; j < NL; ++j) {
-        S[o][j] = S[o][j] * (ao * gl[j]) + xo * kl[j];
-        acc += S[o][j] * ql[j];
+        const int row = r0 + o, c = lane + 32 * j;
+        S[o][j] = (row < a.D && c < a.K) ? Elem<T>::ld(a.state + (b * a.D + row) * a.K + c) : A(0);
       }
-      acc = warp_sum(acc);
-      if (lane == 0 && in) Elem<T>::st(out + bd + row, acc);
-    }
-    if ((t + 1) % C == 0 || t == T_ - 1) {
-      const int64_t slot = t / C;
-#pragma unroll
-      for (int o = 0; o < OWN; ++o)
+
+    int which = 0;
+    int64_t ck_next = a.C < a.T_ ? a.C : a.T_, slot = 0;      // step count at the next checkpoint
+    for (int64_t t0 = 0; t0 < a.T_; t0 += a.G, which ^= 1) {
+      if (t0 + a.G < a.T_) fetch(t0 + a.G, which ^ 1);
+      else scan::commit();
+      scan::wait<1>();
+      __syncthreads();
+      const int n = (int)(a.T_ - t0 < a.G ? a.T_ - t0 : a.G);
+      const unsigned char *p = smem_raw + which * buf_bytes;
+      const T *sg = reinterpret_cast<const T *>(p), *sk = reinterpret_cast<const T *>(p + kp);
+      const T *sq = reinterpret_cast<const T *>(p + 2 * kp);
+      const T *sx = reinterpret_cast<const T *>(p + 3 * kp), *sf = reinterpret_cast<const T *>(p + 3 * kp + dp);
+#pragma unroll(NL <= 4 ? 2 : 1)
+      for (int t = 0; t < n; ++t) {
+        A gl[NL], kl[NL], ql[NL];
 #pragma unroll
         for (int j = 0; j < NL; ++j) {
-          const int64_t row = r0 + o, c = lane + 32 * j;
-          if (row < D && c < K)
-            Elem<T>::st(ckpt + ((b * nslots + slot) * D + row) * K + c, S[o][j]);
+          const int c = lane + 32 * j;
+          const bool in = c < a.K;
+          gl[j] = in ? Elem<T>::ld(sg + t * a.K + c) : A(0);
+          kl[j] = in ? Elem<T>::ld(sk + t * a.K + c) : A(0);
+          ql[j] = in ? Elem<T>::ld(sq + t * a.K + c) : A(0);
         }
+        A acc[OWN];
+#pragma unroll
+        for (int o = 0; o < OWN; ++o) {
+          const int rl = warp * OWN + o;
+          const bool in = rl < nrows;
+          const A xo = in ? Elem<T>::ld(sx + t * nrows + rl) : A(0);
+          const A ao = in ? Elem<T>::ld(sf + t * nrows + rl) : A(0);
+          acc[o] = A(0);
+#pragma unroll
+          for (int j = 0; j < NL; ++j) {
+            S[o][j] = S[o][j] * (ao * gl[j]) + xo * kl[j];
+            acc[o] += S[o][j] * ql[j];
+          }
+        }
+        int o;
+        if (scan::lane_sums<OWN>(acc, lane, &o) && r0 + o < a.D)
+          Elem<T>::st(a.out + (b * a.T_ + t0 + t) * a.D + r0 + o, acc[0]);
+        if (t0 + t + 1 == ck_next) {
+#pragma unroll
+          for (int oo = 0; oo < OWN; ++oo)
+#pragma unroll
+            for (int j = 0; j < NL; ++j) {
+              const int row = r0 + oo, c = lane + 32 * j;
+              if (row < a.D && c < a.K) Elem<T>::st(a.ckpt + ((b * a.nslots + slot) * a.D + row) * a.K + c, S[oo][j]);
+            }
+          ++slot;
+          ck_next = ck_next + a.C < a.T_ ? ck_next + a.C : a.T_;
+        }
+      }
+      __syncthreads();
     }
   }
 }
 
-// Arguments of the orientation-agnostic backward kernel.  "own" is the axis whose lines a warp
-// owns, "lane" the axis the lanes spread over.
+// Arguments of one orientation of the backward.  "own" is the axis whose lines a warp owns, "lane" the axis
+// the lanes spread over.
 template <typename T>
 struct LineArgs {
   const T *xo, *go, *po;  // own-axis vectors  [B,T,NO]: (x, f, dO) or (k, fk, q)
@@ -97,33 +153,98 @@ struct LineArgs {
   T *d_xo;                // sum over lanes of R * xl             -> d_x  or d_k
   T *d_go;                // sum over lanes of R * S_prev * gl    -> d_f  or d_f_key
   T *d_po;                // sum over lanes of S_t * pl           -> d_q  (column orientation only)
-  const T *state0, *ckpt, *grad_state;
-  T *d_state;             // written by the row orientation only (may be null)
-  int64_t B, T_, NO, NLn; // batch, time, own extent, lane extent
+  T *d_state;             // row orientation only
+  int NO, NLn;            // own extent, lane extent
   int64_t so, sl;         // strides of the own / lane axis inside one [D,K] state
-  int64_t C, nslots;      // checkpoint interval and slot count
-  int seg;                // steps of state history kept in shared memory at once
-  const int *rowflag;     // if not null, only batch rows with a non-zero flag are processed
+  int64_t items;          // work items: (batch row, block of own lines)
 };
 
+template <typename T>
+struct BwdArgs {
+  LineArgs<T> col, row;
+  const T *state0, *ckpt, *grad_state;
+  int64_t B, T_, C, nslots;
+  int seg, mids;          // steps per segment; segment starts whose states are kept besides the chunk's
+  const int *rowflag;
+};
+
+// Which segment a warp is at.  A checkpoint interval of ns segments is first walked forward over all but the last
+// (target -1), leaving the state at every ms-th segment start; then segments are taken from the last to the
+// first, each reached from the nearest start that was kept (ms = 1 unless the interval is very long).
+struct SegWalk {
+  int64_t c;              // checkpoint interval
+  int ns, ms, cur, target;
+  int64_t T_, C;
+  int seg, mids;
+  __device__ __forceinline__ void open() {      // interval c
+    const int64_t n = T_ - c * C < C ? T_ - c * C : C;
+    ns = (int)((n + seg - 1) / seg);
+    ms = (ns + mids) / (mids + 1);
+    cur = 0;
+    target = ns > 1 ? -1 : 0;
+  }
+  __device__ __forceinline__ void step() {
+    if (target < 0) {
+      if (cur < ns - 2) { ++cur; return; }
+      target = ns - 1;
+      cur = target / ms * ms;
+    } else if (cur < target) {
+      ++cur;
+    } else if (--target >= 0) {
+      cur = target / ms * ms;
+    } else if (--c >= 0) {
+      open();
+    }
+  }
+  __device__ __forceinline__ int64_t first() const { return c * C + (int64_t)cur * seg; }
+  __device__ __forceinline__ int count() const {
+    const int64_t end = (c + 1) * C < T_ ? (c + 1) * C : T_, left = end - first();
+    return (int)(left < seg ? left : seg);
+  }
+};
+
+// shared memory: two buffers of xl, gl, pl [seg][NLn] and xo, go, po [seg][RC] (storage type), then per warp the
+// states of a segment's steps and the kept segment starts (accumulation type)
+template <typename T>
+__host__ __device__ inline int bwd_part(int seg, int n) { return (int)((((size_t)seg * n * sizeof(T)) + 15) / 16 * 16); }
+
 template <typename T, int NL, int OWN, bool WITH_SP>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) lfw_line_bwd_kernel(const LineArgs<T> a) {
+__device__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> &ln, int64_t item, int vec_ext, unsigned char *smem) {
   using A = typename Elem<T>::acc;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31;
-  const int wic = threadIdx.x >> 5;
-  A *hist = reinterpret_cast<A *>(smem_raw) + (size_t)wic * a.seg * OWN * NL * 32;
+  constexpr int RC = kWarpsPerCta * OWN;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int lp = bwd_part<T>(a.seg, vec_ext), op = bwd_part<T>(a.seg, RC), buf_bytes = 3 * lp + 3 * op;
+  A *hist = reinterpret_cast<A *>(smem + 2 * buf_bytes) + (size_t)warp * (a.seg + a.mids) * OWN * NL * 32;
+  A *mid = hist + (size_t)a.seg * OWN * NL * 32;
 
-  const int64_t groups = (a.NO + OWN - 1) / OWN;
-  const int64_t warp = (int64_t)blockIdx.x * kWarpsPerCta + wic;
-  if (warp >= a.B * groups) return;
-  const int64_t b = warp / groups;
-  const int64_t o0 = (warp % groups) * OWN;
-  const int64_t DK = a.NO * a.NLn;
-  if (a.rowflag != nullptr && a.rowflag[b] == 0) return;
+  const int blocks = (ln.NO + RC - 1) / RC;
+  const int64_t b = item / blocks;
+  const int ob = (int)(item - b * blocks) * RC, nown = ln.NO - ob < RC ? ln.NO - ob : RC;
+  const int o0 = ob + warp * OWN;
+  const int64_t DK = (int64_t)ln.NO * ln.NLn;
 
-  auto state_off = [&](int o, int j) { return (o0 + o) * a.so + (int64_t)(lane + 32 * j) * a.sl; };
-  auto valid = [&](int o, int j) { return (o0 + o) < a.NO && (lane + 32 * j) < a.NLn; };
+  auto state_off = [&](int o, int j) { return (o0 + o) * ln.so + (int64_t)(lane + 32 * j) * ln.sl; };
+  auto valid = [&](int o, int j) { return (o0 + o) < ln.NO && (lane + 32 * j) < ln.NLn; };
+
+  SegWalk w;
+  w.T_ = a.T_; w.C = a.C; w.seg = a.seg; w.mids = a.mids;
+  w.c = (a.T_ + a.C - 1) / a.C - 1;
+  w.open();
+  auto fetch = [&](const SegWalk &s, int which) {
+    const int n = s.count();
+    const int64_t lo = (b * a.T_ + s.first()) * ln.NLn, oo = (b * a.T_ + s.first()) * ln.NO + ob;
+    unsigned char *p = smem + which * buf_bytes;
+    scan::stage(reinterpret_cast<T *>(p), ln.xl + lo, n * ln.NLn, tid, kThreads);
+    scan::stage(reinterpret_cast<T *>(p + lp), ln.gl + lo, n * ln.NLn, tid, kThreads);
+    scan::stage_rows(reinterpret_cast<T *>(p + 3 * lp), ln.xo + oo, n, nown, ln.NO, tid, kThreads);
+    scan::stage_rows(reinterpret_cast<T *>(p + 3 * lp + op), ln.go + oo, n, nown, ln.NO, tid, kThreads);
+    if (s.cur == s.target) {      // upstream vectors: only where the gradients are formed
+      scan::stage(reinterpret_cast<T *>(p + 2 * lp), ln.pl + lo, n * ln.NLn, tid, kThreads);
+      scan::stage_rows(reinterpret_cast<T *>(p + 3 * lp + 2 * op), ln.po + oo, n, nown, ln.NO, tid, kThreads);
+    }
+    scan::commit();
+  };
+  fetch(w, 0);
 
   A R[OWN][NL], S[OWN][NL];
 #pragma unroll
@@ -132,71 +253,84 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) lfw_line_bwd_kernel(const L
     for (int j = 0; j < NL; ++j)
       R[o][j] = valid(o, j) ? Elem<T>::ld(a.grad_state + b * DK + state_off(o, j)) : A(0);
 
-  // one forward step of the recurrence on the register tile
-  auto fwd_step = [&](int64_t t) {
-    const int64_t bo = (b * a.T_ + t) * a.NO, bl = (b * a.T_ + t) * a.NLn;
-    A gl[NL], xl[NL];
-#pragma unroll
-    for (int j = 0; j < NL; ++j) {
-      const int64_t c = lane + 32 * j;
-      const bool in = c < a.NLn;
-      gl[j] = in ? Elem<T>::ld(a.gl + bl + c) : A(0);
-      xl[j] = in ? Elem<T>::ld(a.xl + bl + c) : A(0);
-    }
-#pragma unroll
-    for (int o = 0; o < OWN; ++o) {
-      const bool in = (o0 + o) < a.NO;
-      const A xo = in ? Elem<T>::ld(a.xo + bo + o0 + o) : A(0);
-      const A go = in ? Elem<T>::ld(a.go + bo + o0 + o) : A(0);
-#pragma unroll
-      for (int j = 0; j < NL; ++j) S[o][j] = S[o][j] * (go * gl[j]) + xo * xl[j];
-    }
-  };
+  int which = 0;
+  while (w.c >= 0) {
+    SegWalk nx = w;
+    nx.step();
+    if (nx.c >= 0) fetch(nx, which ^ 1);
+    else scan::commit();
 
-  const int64_t nchunks = (a.T_ + a.C - 1) / a.C;
-  for (int64_t c = nchunks - 1; c >= 0; --c) {
-    const int64_t t0 = c * a.C;
-    const int64_t t1 = (t0 + a.C < a.T_) ? t0 + a.C : a.T_;
-    const int64_t nseg = (t1 - t0 + a.seg - 1) / a.seg;
-    const T *src = (c == 0) ? a.state0 + b * DK : a.ckpt + (b * a.nslots + (c - 1)) * DK;
-    for (int64_t sg = nseg - 1; sg >= 0; --sg) {
-      const int64_t s0 = t0 + sg * a.seg;
-      const int64_t s1 = (s0 + a.seg < t1) ? s0 + a.seg : t1;
+    if (w.cur == 0) {      // the interval's own checkpoint
+      const T *src = (w.c == 0) ? a.state0 + b * DK : a.ckpt + (b * a.nslots + (w.c - 1)) * DK;
 #pragma unroll
       for (int o = 0; o < OWN; ++o)
 #pragma unroll
-        for (int j = 0; j < NL; ++j)
-          S[o][j] = valid(o, j) ? Elem<T>::ld(src + state_off(o, j)) : A(0);
-      for (int64_t t = t0; t < s0; ++t) fwd_step(t);
-      for (int64_t t = s0; t < s1; ++t) {
+        for (int j = 0; j < NL; ++j) S[o][j] = valid(o, j) ? Elem<T>::ld(src + state_off(o, j)) : A(0);
+    } else if (w.target >= 0 && w.cur % w.ms == 0) {      // a kept segment start
+      const A *m = mid + (size_t)(w.cur / w.ms - 1) * OWN * NL * 32;
 #pragma unroll
-        for (int o = 0; o < OWN; ++o)
+      for (int o = 0; o < OWN; ++o)
 #pragma unroll
-          for (int j = 0; j < NL; ++j)
-            hist[(((t - s0) * OWN + o) * NL + j) * 32 + lane] = S[o][j];
-        fwd_step(t);
+        for (int j = 0; j < NL; ++j) S[o][j] = m[(o * NL + j) * 32 + lane];
+    }
+    scan::wait<1>();
+    __syncthreads();
+
+    const int n = w.count();
+    const unsigned char *p = smem + which * buf_bytes;
+    const T *s_xl = reinterpret_cast<const T *>(p), *s_gl = reinterpret_cast<const T *>(p + lp);
+    const T *s_pl = reinterpret_cast<const T *>(p + 2 * lp);
+    const T *s_xo = reinterpret_cast<const T *>(p + 3 * lp) + warp * OWN, *s_go = reinterpret_cast<const T *>(p + 3 * lp + op) + warp * OWN;
+    const T *s_po = reinterpret_cast<const T *>(p + 3 * lp + 2 * op) + warp * OWN;
+    const bool last = w.cur == w.target;
+    auto vec = [&](const T *v, int t, A (&o)[NL]) {
+#pragma unroll
+      for (int j = 0; j < NL; ++j) {
+        const int c = lane + 32 * j;
+        o[j] = c < ln.NLn ? Elem<T>::ld(v + t * ln.NLn + c) : A(0);
       }
-      // S now holds the state after step s1-1; walk back to s0.
-      for (int64_t t = s1 - 1; t >= s0; --t) {
-        const int64_t bo = (b * a.T_ + t) * a.NO, bl = (b * a.T_ + t) * a.NLn;
-        A gl[NL], xl[NL], pl[NL];
+    };
+    auto own = [&](const T *v, int t, int o) { return o0 + o < ln.NO ? Elem<T>::ld(v + t * nown + o) : A(0); };
+
+#pragma unroll(NL <= 4 ? 2 : 1)
+    for (int t = 0; t < n; ++t) {      // forward over the segment
+      A gl[NL], xl[NL];
+      vec(s_gl, t, gl);
+      vec(s_xl, t, xl);
+#pragma unroll
+      for (int o = 0; o < OWN; ++o) {
+        const A xo = own(s_xo, t, o), go = own(s_go, t, o);
 #pragma unroll
         for (int j = 0; j < NL; ++j) {
-          const int64_t cc = lane + 32 * j;
-          const bool in = cc < a.NLn;
-          gl[j] = in ? Elem<T>::ld(a.gl + bl + cc) : A(0);
-          xl[j] = in ? Elem<T>::ld(a.xl + bl + cc) : A(0);
-          pl[j] = in ? Elem<T>::ld(a.pl + bl + cc) : A(0);
+          if (last) hist[((t * OWN + o) * NL + j) * 32 + lane] = S[o][j];
+          S[o][j] = S[o][j] * (go * gl[j]) + xo * xl[j];
         }
+      }
+    }
+    if (w.target < 0 && (w.cur + 1) % w.ms == 0) {
+      A *m = mid + (size_t)((w.cur + 1) / w.ms - 1) * OWN * NL * 32;
+#pragma unroll
+      for (int o = 0; o < OWN; ++o)
+#pragma unroll
+        for (int j = 0; j < NL; ++j) m[(o * NL + j) * 32 + lane] = S[o][j];
+    }
+    if (last) {
+      const int64_t ob_t = (b * a.T_ + w.first()) * ln.NO + o0;
+#pragma unroll(NL <= 4 ? 2 : 1)
+      for (int t = n - 1; t >= 0; --t) {      // S is the state after step t
+        A gl[NL], xl[NL], pl[NL];
+        vec(s_gl, t, gl);
+        vec(s_xl, t, xl);
+        vec(s_pl, t, pl);
+        constexpr int kSums = WITH_SP ? 4 : 2;
+        A v[kSums * OWN];
 #pragma unroll
         for (int o = 0; o < OWN; ++o) {
-          const bool in = (o0 + o) < a.NO;
-          const A go = in ? Elem<T>::ld(a.go + bo + o0 + o) : A(0);
-          const A po = in ? Elem<T>::ld(a.po + bo + o0 + o) : A(0);
+          const A go = own(s_go, t, o), po = own(s_po, t, o);
           A ax = A(0), ag = A(0), ap = A(0);
 #pragma unroll
           for (int j = 0; j < NL; ++j) {
-            const A sp = hist[(((t - s0) * OWN + o) * NL + j) * 32 + lane];
+            const A sp = hist[((t * OWN + o) * NL + j) * 32 + lane];
             const A r = R[o][j] + po * pl[j];   // gradient w.r.t. S_t
             ax += r * xl[j];
             ag += (r * sp) * gl[j];
@@ -204,91 +338,148 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) lfw_line_bwd_kernel(const L
             R[o][j] = r * (go * gl[j]);         // what flows on to S_{t-1}
             S[o][j] = sp;
           }
-          ax = warp_sum(ax);
-          ag = warp_sum(ag);
-          if (WITH_SP) ap = warp_sum(ap);
-          if (lane == 0 && in) {
-            Elem<T>::st(a.d_xo + bo + o0 + o, ax);
-            Elem<T>::st(a.d_go + bo + o0 + o, ag);
-            if (WITH_SP) Elem<T>::st(a.d_po + bo + o0 + o, ap);
+          v[kSums * o] = ax;
+          v[kSums * o + 1] = ag;
+          if (WITH_SP) {
+            v[kSums * o + 2] = ap;
+            v[kSums * o + 3] = A(0);
           }
+        }
+        int i;
+        const bool mine = scan::lane_sums<kSums * OWN>(v, lane, &i);
+        const int o = i / kSums, kind = i % kSums;
+        if (mine && kind < 3 && o0 + o < ln.NO) {
+          T *dst = kind == 0 ? ln.d_xo : kind == 1 ? ln.d_go : ln.d_po;
+          Elem<T>::st(dst + ob_t + (int64_t)t * ln.NO + o, v[0]);
         }
       }
     }
+    __syncthreads();
+    w = nx;
+    which ^= 1;
   }
-  if (a.d_state != nullptr) {
+  if (!WITH_SP) {
 #pragma unroll
     for (int o = 0; o < OWN; ++o)
 #pragma unroll
       for (int j = 0; j < NL; ++j)
-        if (valid(o, j)) Elem<T>::st(a.d_state + b * DK + state_off(o, j), R[o][j]);
+        if (valid(o, j)) Elem<T>::st(ln.d_state + b * DK + state_off(o, j), R[o][j]);
   }
+}
+
+// kBoth: both orientations in one launch (redoing flagged rows).  Otherwise two launches, columns first, then
+// rows: the row launch may start as soon as every CTA of the column launch has (which is after everything before
+// it has completed), runs beside it, and ends only after it, so that what follows may rely on both.
+enum Part { kBoth = 0, kColumns = 1, kRows = 2 };
+
+template <typename T, int NL, int OWN>
+__global__ void __launch_bounds__(kThreads) lfw_line_bwd_kernel(const BwdArgs<T> a, const int part) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int RC = kWarpsPerCta * OWN;
+  const int ext = a.col.NLn > a.row.NLn ? a.col.NLn : a.row.NLn;
+  if (part != kRows) dependency_wait();
+  const int64_t first_row = part == kRows ? 0 : a.col.items, n = first_row + (part == kColumns ? 0 : a.row.items);
+  for (int64_t item = blockIdx.x; item < n; item += gridDim.x) {
+    const bool col = item < first_row;
+    const int64_t i = col ? item : item - first_row;
+    const int64_t b = i / (((col ? a.col.NO : a.row.NO) + RC - 1) / RC);
+    if (a.rowflag != nullptr && a.rowflag[b] == 0) continue;
+    if (col) line_bwd<T, NL, OWN, true>(a, a.col, i, ext, smem_raw);
+    else line_bwd<T, NL, OWN, false>(a, a.row, i, ext, smem_raw);
+  }
+  if (part == kRows) dependency_wait();
 }
 
 int pick_nl(int64_t extent) {
   const int64_t need = (extent + 31) / 32;
-  for (int nl : {1, 2, 4, 8, 16})
+  for (int nl : {1, 2, 3, 4, 8, 16})
     if (need <= nl) return nl;
   return 0;
 }
 
-template <typename T, int NL>
-int launch_fwd(const void *x, const void *f, const void *q, const void *k, const void *fk,
-               const void *state, void *out, void *ckpt, int64_t B, int64_t T_, int64_t D,
-               int64_t K, int64_t C, cudaStream_t st, const int *rowflag) {
-  constexpr int OWN = 4;
-  const int64_t warps = B * ceil_div64(D, OWN);
-  const int64_t grid = ceil_div64(warps, kWarpsPerCta);
-  lfw_scan_fwd_kernel<T, NL, OWN><<<(unsigned)grid, kWarpsPerCta * 32, 0, st>>>(
-      (const T *)x, (const T *)f, (const T *)q, (const T *)k, (const T *)fk, (const T *)state,
-      (T *)out, (T *)ckpt, B, T_, D, K, C, ceil_div64(T_, C), rowflag);
+// CTAs of a launch: one per work item; the walk over flagged rows only is cut to a few waves
+unsigned grid_for(int64_t items, const int *rowflag) {
+  const int64_t most = rowflag != nullptr ? 148 * 4 : (int64_t)1 << 30;
+  return (unsigned)(items < most ? items : most);
+}
+
+template <typename T, int NL, int OWN>
+int launch_fwd(FwdArgs<T> a, cudaStream_t st) {
+  constexpr int RC = kWarpsPerCta * OWN;
+  a.items = a.B * ((a.D + RC - 1) / RC);
+  for (a.G = 32; a.G > 1 && 2 * (3 * fwd_part<T>(a.G, a.K) + 2 * fwd_part<T>(a.G, RC)) > 64 * 1024;) a.G /= 2;
+  const size_t smem = 2 * (size_t)(3 * fwd_part<T>(a.G, a.K) + 2 * fwd_part<T>(a.G, RC));
+  auto *const kernel = &lfw_scan_fwd_kernel<T, NL, OWN>;
+  T2FW_ALLOW_SMEM(kernel, 64 * 1024);
+  T2FW_CHECK_CUDA(launch_dependent(kernel, dim3(grid_for(a.items, a.rowflag)), dim3(kThreads), smem, st, a));
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;
 }
 
-template <typename T, int NL, bool WITH_SP>
-int launch_line(LineArgs<T> a, cudaStream_t st) {
-  constexpr int OWN = 2;
-  using A = typename Elem<T>::acc;
-  const size_t per_step = (size_t)kWarpsPerCta * OWN * NL * 32 * sizeof(A);
-  int seg = (int)(49152 / per_step);
-  if (seg > 16) seg = 16;
-  if (seg < 1) seg = 1;
-  a.seg = seg;
-  const int64_t warps = a.B * ceil_div64(a.NO, OWN);
-  const int64_t grid = ceil_div64(warps, kWarpsPerCta);
-  lfw_line_bwd_kernel<T, NL, OWN, WITH_SP>
-      <<<(unsigned)grid, kWarpsPerCta * 32, per_step * seg, st>>>(a);
-  T2FW_CHECK_LAUNCH(1);
-  return T2FW_OK;
+// Rows per warp: four share the key-side loads and most of the shuffles; one while four would leave the chip
+// with less than 16 warps per SM (the chain of steps is then what counts, and more CTAs shorten each step).
+template <typename T, int NL>
+int launch_fwd_rows(const FwdArgs<T> &a, cudaStream_t st) {
+  if (a.B * ((a.D + 3) / 4) >= 148 * 16 || a.rowflag != nullptr) return launch_fwd<T, NL, 4>(a, st);
+  return launch_fwd<T, NL, 1>(a, st);
 }
 
 template <typename T>
 int fwd_typed(const void *x, const void *f, const void *q, const void *k, const void *fk,
               const void *state, void *out, void *ckpt, int64_t B, int64_t T_, int64_t D,
               int64_t K, int64_t C, cudaStream_t st, const int *rowflag) {
+  FwdArgs<T> a{};
+  a.x = (const T *)x; a.f = (const T *)f; a.q = (const T *)q; a.k = (const T *)k; a.fk = (const T *)fk;
+  a.state = (const T *)state; a.out = (T *)out; a.ckpt = (T *)ckpt;
+  a.B = B; a.T_ = T_; a.D = (int)D; a.K = (int)K; a.C = C; a.nslots = ceil_div64(T_, C); a.rowflag = rowflag;
   switch (pick_nl(K)) {
-    case 1: return launch_fwd<T, 1>(x, f, q, k, fk, state, out, ckpt, B, T_, D, K, C, st, rowflag);
-    case 2: return launch_fwd<T, 2>(x, f, q, k, fk, state, out, ckpt, B, T_, D, K, C, st, rowflag);
-    case 4: return launch_fwd<T, 4>(x, f, q, k, fk, state, out, ckpt, B, T_, D, K, C, st, rowflag);
-    case 8: return launch_fwd<T, 8>(x, f, q, k, fk, state, out, ckpt, B, T_, D, K, C, st, rowflag);
-    case 16: return launch_fwd<T, 16>(x, f, q, k, fk, state, out, ckpt, B, T_, D, K, C, st, rowflag);
+    case 1: return launch_fwd_rows<T, 1>(a, st);
+    case 2: return launch_fwd_rows<T, 2>(a, st);
+    case 3: return launch_fwd_rows<T, 3>(a, st);
+    case 4: return launch_fwd_rows<T, 4>(a, st);
+    case 8: return launch_fwd_rows<T, 8>(a, st);
+    case 16: return launch_fwd_rows<T, 16>(a, st);
   }
   set_error("lfw forward: K=%lld exceeds the supported maximum of 512", (long long)K);
   return T2FW_ERR_UNSUPPORTED;
 }
 
-template <typename T, bool WITH_SP>
-int line_typed(const LineArgs<T> &a, cudaStream_t st) {
-  switch (pick_nl(a.NLn)) {
-    case 1: return launch_line<T, 1, WITH_SP>(a, st);
-    case 2: return launch_line<T, 2, WITH_SP>(a, st);
-    case 4: return launch_line<T, 4, WITH_SP>(a, st);
-    case 8: return launch_line<T, 8, WITH_SP>(a, st);
-    case 16: return launch_line<T, 16, WITH_SP>(a, st);
+template <typename T, int NL>
+int launch_bwd(BwdArgs<T> a, cudaStream_t st) {
+  using A = typename Elem<T>::acc;
+  constexpr int OWN = NL * sizeof(A) <= 32 ? 2 : 1, RC = kWarpsPerCta * OWN;
+  const int ext = a.col.NLn > a.row.NLn ? a.col.NLn : a.row.NLn;
+  a.col.items = a.B * ((a.col.NO + RC - 1) / RC);
+  a.row.items = a.B * ((a.row.NO + RC - 1) / RC);
+  auto bytes = [&](int seg, int mids) {
+    return 2 * (size_t)(3 * bwd_part<T>(seg, ext) + 3 * bwd_part<T>(seg, RC)) +
+           (size_t)kWarpsPerCta * (seg + mids) * OWN * NL * 32 * sizeof(A);
+  };
+  // Segments of 16 steps with up to seven kept starts where two CTAs still fit an SM; less history for wide states.
+  constexpr size_t kMost = 224 * 1024;
+  a.seg = 16;
+  a.mids = 7;
+  while (a.seg > 4 && bytes(a.seg, a.mids) > 112 * 1024) a.seg /= 2;
+  while (bytes(a.seg, a.mids) > kMost && (a.seg > 1 || a.mids > 1)) {
+    if (a.mids > a.seg) a.mids /= 2;
+    else a.seg /= 2;
   }
-  set_error("lfw backward: extent %lld exceeds the supported maximum of 512", (long long)a.NLn);
-  return T2FW_ERR_UNSUPPORTED;
+  const size_t smem = bytes(a.seg, a.mids);
+  if (smem > kMost) {
+    set_error("lfw backward: %zu bytes of shared memory needed", smem);
+    return T2FW_ERR_UNSUPPORTED;
+  }
+  auto *const kernel = &lfw_line_bwd_kernel<T, NL, OWN>;
+  T2FW_ALLOW_SMEM(kernel, (int)kMost);
+  if (a.rowflag != nullptr) {
+    T2FW_CHECK_CUDA(launch_dependent(kernel, dim3(grid_for(a.col.items + a.row.items, a.rowflag)), dim3(kThreads), smem, st, a, (int)kBoth));
+    T2FW_CHECK_LAUNCH(1);
+    return T2FW_OK;
+  }
+  T2FW_CHECK_CUDA(launch_dependent(kernel, dim3((unsigned)a.col.items), dim3(kThreads), smem, st, a, (int)kColumns));
+  T2FW_CHECK_CUDA(launch_dependent(kernel, dim3((unsigned)a.row.items), dim3(kThreads), smem, st, a, (int)kRows));
+  T2FW_CHECK_LAUNCH(2);
+  return T2FW_OK;
 }
 
 template <typename T>
@@ -296,26 +487,28 @@ int bwd_typed(const void *go, const void *gs, const void *x, const void *f, cons
               const void *k, const void *fk, const void *state, const void *ckpt, void *dx,
               void *df, void *dq, void *dk, void *dfk, void *ds, int64_t B, int64_t T_, int64_t D,
               int64_t K, int64_t C, cudaStream_t st, const int *rowflag) {
-  LineArgs<T> row{};
+  BwdArgs<T> a{};
+  a.state0 = (const T *)state; a.ckpt = (const T *)ckpt; a.grad_state = (const T *)gs;
+  a.B = B; a.T_ = T_; a.C = C < T_ ? C : T_; a.nslots = ceil_div64(T_, C); a.rowflag = rowflag;
+  LineArgs<T> &row = a.row, &col = a.col;
   row.xo = (const T *)x; row.go = (const T *)f; row.po = (const T *)go;
   row.xl = (const T *)k; row.gl = (const T *)fk; row.pl = (const T *)q;
-  row.d_xo = (T *)dx; row.d_go = (T *)df; row.d_po = nullptr;
-  row.state0 = (const T *)state; row.ckpt = (const T *)ckpt; row.grad_state = (const T *)gs;
-  row.d_state = (T *)ds;
-  row.B = B; row.T_ = T_; row.NO = D; row.NLn = K; row.so = K; row.sl = 1;
-  row.C = C; row.nslots = ceil_div64(T_, C); row.rowflag = rowflag;
-  int rc = line_typed<T, false>(row, st);
-  if (rc != T2FW_OK) return rc;
-
-  LineArgs<T> col{};
+  row.d_xo = (T *)dx; row.d_go = (T *)df; row.d_po = nullptr; row.d_state = (T *)ds;
+  row.NO = (int)D; row.NLn = (int)K; row.so = K; row.sl = 1;
   col.xo = (const T *)k; col.go = (const T *)fk; col.po = (const T *)q;
   col.xl = (const T *)x; col.gl = (const T *)f; col.pl = (const T *)go;
-  col.d_xo = (T *)dk; col.d_go = (T *)dfk; col.d_po = (T *)dq;
-  col.state0 = (const T *)state; col.ckpt = (const T *)ckpt; col.grad_state = (const T *)gs;
-  col.d_state = nullptr;
-  col.B = B; col.T_ = T_; col.NO = K; col.NLn = D; col.so = 1; col.sl = K;
-  col.C = C; col.nslots = ceil_div64(T_, C); col.rowflag = rowflag;
-  return line_typed<T, true>(col, st);
+  col.d_xo = (T *)dk; col.d_go = (T *)dfk; col.d_po = (T *)dq; col.d_state = nullptr;
+  col.NO = (int)K; col.NLn = (int)D; col.so = 1; col.sl = K;
+  switch (pick_nl(D > K ? D : K)) {
+    case 1: return launch_bwd<T, 1>(a, st);
+    case 2: return launch_bwd<T, 2>(a, st);
+    case 3: return launch_bwd<T, 3>(a, st);
+    case 4: return launch_bwd<T, 4>(a, st);
+    case 8: return launch_bwd<T, 8>(a, st);
+    case 16: return launch_bwd<T, 16>(a, st);
+  }
+  set_error("lfw backward: D=%lld, K=%lld exceed the supported maximum of 512", (long long)D, (long long)K);
+  return T2FW_ERR_UNSUPPORTED;
 }
 
 }  // namespace

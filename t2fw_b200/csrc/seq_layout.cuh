@@ -58,35 +58,29 @@ __device__ __forceinline__ void load_block(void *dst, const CUtensorMap *map, in
       : "memory");
 }
 
-// ---- in-place transforms of a raw [64][64] block in shared memory (all threads of the CTA) ------
-template <typename T>
-__device__ __forceinline__ void fill_block(T *blk, float v, int tid, int nthreads) {
-  const T tv = (T)v;
-  for (int i = tid; i < 64 * 64; i += nthreads) blk[i] = tv;
-}
+// ---- activations of the fused layer: gate = max(sigmoid(g), 1/8), rounded to the storage type (what a separate
+//      elementwise pass followed by the plain operator would have fed the kernels) ------------------------
 template <typename T>
 __device__ __forceinline__ float round_to(float v) {
   const T r = (T)v;
   return Elem<T>::ld(&r);
 }
+// e^-g and 1 / v as single hardware approximations (about 2 ulp; the library forms add range handling that these
+// arguments do not need: an overflow gives gate 0, which the floor lifts, and denormals count as zero)
+__device__ __forceinline__ float exp_neg(float g) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(g * -1.4426950408889634f));
+  return r;
+}
+__device__ __forceinline__ float rcp1p(float e) {      // 1 / (1 + e)
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return r;
+}
 template <typename T>
 __device__ __forceinline__ float sigmoid_gate(float g) {
-  return round_to<T>(fmaxf(__fdividef(1.f, 1.f + __expf(-g)), kGateFloor));
+  return round_to<T>(fmaxf(rcp1p(exp_neg(g)), kGateFloor));
 }
-// gate = max(sigmoid(g), 1/8), rounded to the storage type (what a separate elementwise pass
-// followed by the plain operator would have fed the kernel)
-template <typename T>
-__device__ __forceinline__ void sigmoid_gate_block(T *blk, int tid, int nthreads) {
-  for (int i = tid; i < 64 * 64; i += nthreads) {
-    const float g = Elem<T>::ld(blk + i);
-    blk[i] = (T)fmaxf(__fdividef(1.f, 1.f + __expf(-g)), kGateFloor);
-  }
-}
-template <typename T>
-__device__ __forceinline__ void scale_block(T *blk, float s, int tid, int nthreads) {
-  for (int i = tid; i < 64 * 64; i += nthreads) blk[i] = (T)(Elem<T>::ld(blk + i) * s);
-}
-
 // The block of tensor i for the chunk whose first row is `row` (nv valid rows), sub-item h.
 // Dense [rows][64] arrays: one linear bulk copy of the valid rows; otherwise the tiled copy of the
 // whole box.  Returns the bytes that will arrive on the barrier.
