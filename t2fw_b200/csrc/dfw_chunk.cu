@@ -670,6 +670,7 @@ bool dfw_chunk_supported(int64_t D, int64_t M, int dtype) {
 // fp32 [B][n_chunks][64][64] arrays: W and U (forward); Wb, Ub and the per-chunk S0, R_end, E (backward);
 // U and Ub with rows of kLdU floats
 size_t dfw_chunk_scratch_bytes(int64_t B, int64_t T_, bool backward) {
+  if (!backward) return dfw_forward_images_bytes(B, T_);
   const int64_t nc = ceil_div64(T_, kC);
   return align_up(((backward ? 4 : 1) * wu_floats(B, nc) + u_floats(B, nc)) * sizeof(float), 256);
 }
@@ -700,6 +701,7 @@ static int dfw_chunk_forward_typed(const void *q, const void *k, const void *v, 
 int dfw_chunk_forward(const void *q, const void *k, const void *v, const void *state, void *out,
                       void *final_state, void *delta, int64_t B, int64_t T_, int dtype, void *scratch,
                       cudaStream_t st) {
+  return dfw_forward_images(q, k, v, state, out, final_state, delta, B, T_, dtype, scratch, st);
   if (dtype == T2FW_F16)
     return dfw_chunk_forward_typed<__half>(q, k, v, state, out, final_state, delta, B, T_, scratch, st);
   return dfw_chunk_forward_typed<__nv_bfloat16>(q, k, v, state, out, final_state, delta, B, T_, scratch, st);

@@ -1,0 +1,293 @@
+// Warp-level tensor-core fragments of the chunked delta rule (dfw_fwd.cu, dfw_bwd.cu): 64 x 64 matrices, TF32
+// (m16n8k8) and 16-bit (m16n8k16) products with fp32 accumulation.
+//
+// Fragment image.  A 64 x 64 fp32 matrix X[r][c] as 1024 float4: element (rb, cb, lane) at (rb * 8 + cb) * 32 + lane
+// holds, with g = lane / 4 and t = lane % 4,
+//     x, y = X[16 rb + g][8 cb + 2t], [.. + 1]        z, w = X[16 rb + g + 8][8 cb + 2t], [.. + 1]
+// which is how a warp's accumulators of rows 16 rb .. lie in its registers.  The sum over the contraction index
+// does not depend on its order, so with logical index t read as column 2t and t + 4 as column 2t + 1 the same
+// float4 is, without any exchange between lanes,
+//   * the A operand of rows 16 rb .. , contraction columns 8 cb ..:  (x, z, y, w)
+//   * the B operand of two 8-column tiles n = 16 rb + g and n = 16 rb + 8 + g, contraction columns 8 cb ..: (x, y), (z, w)
+// A result therefore feeds the next product from registers, and travels through memory in 512-byte warp accesses.
+//
+// Raw 16-bit blocks [64][64] lie in shared memory as 128-byte rows whose eight 16-byte pieces are XOR-ed with
+// (row % 8): ldmatrix reads them, straight or transposed, without bank conflicts, and its registers hold two
+// consecutive contraction values, i.e. the operands of a 16-bit product as they are and, widened (every 16-bit
+// value is exact in TF32), those of a TF32 product in the order above.
+#pragma once
+
+#include "common.cuh"
+
+namespace t2fw {
+namespace frag {
+
+constexpr int kC = 64;                       // chunk length
+constexpr int kDim = 64;                     // D = M = 64
+constexpr int kImg = kC * kDim;              // floats of an image
+constexpr int kRaw = kC * kDim * 2;          // bytes of a raw block
+constexpr int kThreads = 128;                // four warps
+
+// ---- products ------------------------------------------------------------------------------------
+__device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+template <typename T>
+__device__ __forceinline__ void mma_16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
+template <>
+__device__ __forceinline__ void mma_16<__half>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <>
+__device__ __forceinline__ void mma_16<__nv_bfloat16>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// ---- operand values --------------------------------------------------------------------------------
+// TF32 rounding (nearest, ties away) of a value that only feeds a product: the tensor core drops the low 13 bits
+__device__ __forceinline__ uint32_t op(float v) { return __float_as_uint(v) + 0x1000u; }
+// the rounded value itself
+__device__ __forceinline__ float rnd(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u); }
+// v = hi + lo with both parts TF32 operands: together 22 bits
+__device__ __forceinline__ void split(float v, uint32_t &hi, uint32_t &lo) {
+  const float h = rnd(v);
+  hi = __float_as_uint(h);
+  lo = __float_as_uint(v - h);
+}
+// the two 16-bit values of a register as TF32 operands (exact)
+template <typename T> __device__ __forceinline__ uint32_t lo16(uint32_t u);
+template <typename T> __device__ __forceinline__ uint32_t hi16(uint32_t u);
+template <> __device__ __forceinline__ uint32_t lo16<__half>(uint32_t u) {
+  return __float_as_uint(__low2float(*reinterpret_cast<const __half2 *>(&u)));
+}
+template <> __device__ __forceinline__ uint32_t hi16<__half>(uint32_t u) {
+  return __float_as_uint(__high2float(*reinterpret_cast<const __half2 *>(&u)));
+}
+template <> __device__ __forceinline__ uint32_t lo16<__nv_bfloat16>(uint32_t u) { return u << 16; }
+template <> __device__ __forceinline__ uint32_t hi16<__nv_bfloat16>(uint32_t u) { return u & 0xffff0000u; }
+template <typename T> __device__ __forceinline__ uint32_t pack16(float a, float b);
+template <> __device__ __forceinline__ uint32_t pack16<__half>(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+template <> __device__ __forceinline__ uint32_t pack16<__nv_bfloat16>(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+// ---- raw 16-bit blocks in shared memory -------------------------------------------------------------
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ int raw_off(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
+__device__ __forceinline__ void ldsm(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_t(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// A operand, rows r0 .. r0+15 of the block, contraction columns 16 kk ..
+__device__ __forceinline__ void raw_a(uint32_t (&r)[4], uint32_t base, int r0, int kk, int lane) {
+  ldsm(r, base + raw_off(r0 + (lane & 15), 2 * kk + (lane >> 4)));
+}
+// A operand, rows = block columns m0 .. m0+15, contraction = block rows k0 .. k0+15
+__device__ __forceinline__ void raw_at(uint32_t (&r)[4], uint32_t base, int m0, int k0, int lane) {
+  ldsm_t(r, base + raw_off(k0 + (lane & 7) + ((lane >> 4) & 1) * 8, (m0 >> 3) + ((lane >> 3) & 1)));
+}
+// B operands of two 8-column tiles, columns = block rows n0 .. n0+15, contraction columns 16 kk ..:
+// tile 0: r[0], r[1], tile 1: r[2], r[3] (first and second eight contraction values)
+__device__ __forceinline__ void raw_b(uint32_t (&r)[4], uint32_t base, int n0, int kk, int lane) {
+  ldsm(r, base + raw_off(n0 + (lane & 7) + ((lane >> 4) & 1) * 8, 2 * kk + ((lane >> 3) & 1)));
+}
+// the same with columns = block columns n0 .. n0+15, contraction = block rows k0 .. k0+15
+__device__ __forceinline__ void raw_bt(uint32_t (&r)[4], uint32_t base, int k0, int n0, int lane) {
+  ldsm_t(r, base + raw_off(k0 + (lane & 15), (n0 >> 3) + (lane >> 4)));
+}
+// TF32 product of 16 contraction values with both operands from raw registers / A from raw registers
+template <typename T>
+__device__ __forceinline__ void mma_raw_a(float (&c)[4], const uint32_t (&a)[4], int s, uint32_t b0, uint32_t b1) {
+  mma_tf32(c, lo16<T>(a[2 * s]), lo16<T>(a[2 * s + 1]), hi16<T>(a[2 * s]), hi16<T>(a[2 * s + 1]), b0, b1);
+}
+// A operand from accumulators (rows of the warp, contraction columns = the eight columns of the tile)
+__device__ __forceinline__ void mma_acc_a(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  mma_tf32(c, a[0], a[2], a[1], a[3], b0, b1);
+}
+
+// Block [64][64] of a dense [rows][64] array into shared memory, asynchronously; rows beyond nvalid become zeros.
+template <typename T>
+__device__ __forceinline__ void load_raw(unsigned char *dst, const T *src, int nvalid, int tid) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int i = tid + kThreads * j, r = i >> 3, p = i & 7;
+    unsigned char *d = dst + raw_off(r, p);
+    if (r < nvalid)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d)), "l"(src + (size_t)r * kDim + p * 8) : "memory");
+    else
+      *reinterpret_cast<uint4 *>(d) = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+// an image (or any 16 KB) into shared memory, asynchronously
+__device__ __forceinline__ void load_image(float *dst, const float *src, int tid) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int i = tid + kThreads * j;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + 4 * i)), "l"(src + 4 * i) : "memory");
+  }
+}
+__device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void zero(float (&c)[8][4]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) c[i][0] = c[i][1] = c[i][2] = c[i][3] = 0.f;
+}
+// a warp's rows of an image: accumulators -> memory (optionally rounded and negated), memory -> registers
+template <bool kRound>
+__device__ __forceinline__ void store_rows(float *img, const float (&c)[8][4], int w, int lane, float sign = 1.f) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float4 v = make_float4(sign * c[i][0], sign * c[i][1], sign * c[i][2], sign * c[i][3]);
+    if (kRound) v = make_float4(rnd(v.x), rnd(v.y), rnd(v.z), rnd(v.w));
+    reinterpret_cast<float4 *>(img)[(w * 8 + i) * 32 + lane] = v;
+  }
+}
+__device__ __forceinline__ float4 image_at(const float *img, int rb, int cb, int lane) {
+  return reinterpret_cast<const float4 *>(img)[(rb * 8 + cb) * 32 + lane];
+}
+__device__ __forceinline__ uint32_t bits(float v) { return __float_as_uint(v); }
+
+// c[n tiles] += A B^T over 64 contraction values, A = a warp's rows as accumulator registers (already operands),
+// B = image in shared memory (rows = result columns)
+__device__ __forceinline__ void mma_image(float (&c)[8][4], const uint32_t (&a)[8][4], const float *img, int lane) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int np = 0; np < 4; ++np) {
+      const float4 b = image_at(img, np, j, lane);
+      mma_acc_a(c[2 * np], a[j], bits(b.x), bits(b.y));
+      mma_acc_a(c[2 * np + 1], a[j], bits(b.z), bits(b.w));
+    }
+}
+
+// ---- (I + L)^-1 of a strictly lower triangular 64 x 64 matrix, fp32 -----------------------------------
+// L in Ls [64][kLdL], the inverse to Ts [64][kLdT] (diagonal blocks with their zeros; the blocks above the diagonal are
+// neither written nor meant to be read).  Warp w owns block row w: it inverts its 16 x 16 diagonal block by
+// substitution, one column per lane, and, once all of those are there, its blocks left of it from right to left,
+//     T_ij = -( sum_{j<k<=i} T_ik L_kj ) T_jj ,
+// which needs nothing from the other block rows of T.  The products are three TF32 products each (operands split in
+// two), i.e. fp32-like.  Called by all four warps; ends without a barrier.
+constexpr int kLdL = 68, kLdT = 72;
+__device__ __forceinline__ void mma_split(float (&c)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0, float b1) {
+  uint32_t bh0, bl0, bh1, bl1;
+  split(b0, bh0, bl0);
+  split(b1, bh1, bl1);
+  mma_acc_a(c, ah, bh0, bh1);
+  mma_acc_a(c, al, bh0, bh1);
+  mma_acc_a(c, ah, bl0, bl1);
+}
+__device__ __forceinline__ void unit_lower_inverse(const float *Ls, float *Ts, int w, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  if (lane < 16) {
+    const float *Lb = Ls + (16 * w) * kLdL + 16 * w;
+    float x[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      float a = r == lane ? 1.f : 0.f;
+#pragma unroll
+      for (int k4 = 0; k4 < r; k4 += 4) {
+        const float4 l = *reinterpret_cast<const float4 *>(Lb + r * kLdL + k4);
+        a = fmaf(-l.x, x[k4], a);
+        if (k4 + 1 < r) a = fmaf(-l.y, x[k4 + 1], a);
+        if (k4 + 2 < r) a = fmaf(-l.z, x[k4 + 2], a);
+        if (k4 + 3 < r) a = fmaf(-l.w, x[k4 + 3], a);
+      }
+      x[r] = a;
+      Ts[(16 * w + r) * kLdT + 16 * w + lane] = a;
+    }
+  }
+  __syncthreads();
+  uint32_t th[4][2][4], tl[4][2][4];      // T_{w, w-r}, as A operands (hi, lo), r = 0 the diagonal block
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const float2 u = *reinterpret_cast<const float2 *>(Ts + (16 * w + g) * kLdT + 16 * w + 8 * s + 2 * t);
+    const float2 v = *reinterpret_cast<const float2 *>(Ts + (16 * w + g + 8) * kLdT + 16 * w + 8 * s + 2 * t);
+    split(u.x, th[0][s][0], tl[0][s][0]);
+    split(u.y, th[0][s][1], tl[0][s][1]);
+    split(v.x, th[0][s][2], tl[0][s][2]);
+    split(v.y, th[0][s][3], tl[0][s][3]);
+  }
+#pragma unroll
+  for (int jj = 0; jj < 3; ++jj) {
+    const int j = w - 1 - jj;
+    if (j < 0) break;
+    float m[2][4] = {};
+#pragma unroll
+    for (int r = 0; r <= jj; ++r) {
+      const float *L = Ls + (16 * (w - r)) * kLdL + 16 * j;
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+          mma_split(m[n], th[r][s], tl[r][s], L[(8 * s + 2 * t) * kLdL + 8 * n + g], L[(8 * s + 2 * t + 1) * kLdL + 8 * n + g]);
+    }
+    uint32_t mh[2][4], ml[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) split(-m[n][e], mh[n][e], ml[n][e]);
+    const float *D = Ts + (16 * j) * kLdT + 16 * j;
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      float c[4] = {};
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+        mma_split(c, mh[s], ml[s], D[(8 * s + 2 * t) * kLdT + 8 * n + g], D[(8 * s + 2 * t + 1) * kLdT + 8 * n + g]);
+      *reinterpret_cast<float2 *>(Ts + (16 * w + g) * kLdT + 16 * j + 8 * n + 2 * t) = make_float2(c[0], c[1]);
+      *reinterpret_cast<float2 *>(Ts + (16 * w + g + 8) * kLdT + 16 * j + 8 * n + 2 * t) = make_float2(c[2], c[3]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) split(c[e], th[jj + 1][n][e], tl[jj + 1][n][e]);
+    }
+  }
+}
+
+// strictly lower triangle of X Y^T (both raw blocks), rows 16 w .. of this warp, into Ls [64][kLdL]: exact products
+template <typename T>
+__device__ __forceinline__ void gram_lower(float *Ls, uint32_t x, uint32_t y, int w, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  uint32_t a[4][4];
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) raw_a(a[kk], x, 16 * w, kk, lane);
+#pragma unroll
+  for (int np = 0; np < 4; ++np) {
+    if (np > w) break;
+    float c[2][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      uint32_t b[4];
+      raw_b(b, y, 16 * np, kk, lane);
+      mma_16<T>(c[0], a[kk], b[0], b[1]);
+      mma_16<T>(c[1], a[kk], b[2], b[3]);
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const int col = 16 * np + 8 * n + 2 * t, r0 = 16 * w + g, r1 = r0 + 8;
+      *reinterpret_cast<float2 *>(Ls + r0 * kLdL + col) = make_float2(col < r0 ? c[n][0] : 0.f, col + 1 < r0 ? c[n][1] : 0.f);
+      *reinterpret_cast<float2 *>(Ls + r1 * kLdL + col) = make_float2(col < r1 ? c[n][2] : 0.f, col + 1 < r1 ? c[n][3] : 0.f);
+    }
+  }
+}
+
+}  // namespace frag
+}  // namespace t2fw
