@@ -670,7 +670,7 @@ bool dfw_chunk_supported(int64_t D, int64_t M, int dtype) {
 // fp32 [B][n_chunks][64][64] arrays: W and U (forward); Wb, Ub and the per-chunk S0, R_end, E (backward);
 // U and Ub with rows of kLdU floats
 size_t dfw_chunk_scratch_bytes(int64_t B, int64_t T_, bool backward) {
-  if (!backward) return dfw_forward_images_bytes(B, T_);
+  return backward ? dfw_backward_images_bytes(B, T_) : dfw_forward_images_bytes(B, T_);
   const int64_t nc = ceil_div64(T_, kC);
   return align_up(((backward ? 4 : 1) * wu_floats(B, nc) + u_floats(B, nc)) * sizeof(float), 256);
 }
@@ -748,6 +748,7 @@ static int dfw_chunk_backward_typed(const void *go, const void *gs, const void *
 int dfw_chunk_backward(const void *go, const void *gs, const void *q, const void *k, const void *delta,
                        const void *final_state, void *dq, void *dk, void *dv, void *ds, int64_t B, int64_t T_,
                        int dtype, void *scratch, cudaStream_t st) {
+  return dfw_backward_images(go, gs, q, k, delta, final_state, dq, dk, dv, ds, B, T_, dtype, scratch, st);
   if (dtype == T2FW_F16)
     return dfw_chunk_backward_typed<__half>(go, gs, q, k, delta, final_state, dq, dk, dv, ds, B, T_, scratch, st);
   return dfw_chunk_backward_typed<__nv_bfloat16>(go, gs, q, k, delta, final_state, dq, dk, dv, ds, B, T_, scratch,

@@ -154,24 +154,31 @@ dfw_prep_fwd_kernel(const T *__restrict__ k, const T *__restrict__ v, float *__r
 }
 
 // ---- carry: one CTA per row, warp w = state rows 16 w .. ------------------------------------------------
+// Qc^T and N of a chunk arrive together, two chunks ahead.  Start states replace N: a chunk's N is in shared memory
+// before its start state is written.
 constexpr int kStages = 3;
-constexpr int kSmemCarry = kStages * kImg * 4;
+constexpr int kSmemCarry = kStages * 2 * kImg * 4;
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg, const float *__restrict__ Nimg,
-                     float *__restrict__ Simg, T *__restrict__ final_state, int nc) {
+dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg, float *__restrict__ NSimg,
+                     T *__restrict__ final_state, int nc) {
   extern __shared__ __align__(128) unsigned char sm[];
   float *ring = reinterpret_cast<float *>(sm);
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int64_t b = blockIdx.x;
   const size_t img0 = (size_t)b * nc * kImg;
   dependency_wait();
-#pragma unroll
-  for (int s = 0; s < kStages - 1; ++s) {
-    if (s < nc) load_image(ring + s * kImg, Qimg + img0 + (size_t)s * kImg, tid);
+  auto fetch = [&](int c) {
+    if (c < nc) {
+      float *dst = ring + (c % kStages) * 2 * kImg;
+      load_image(dst, Qimg + img0 + (size_t)c * kImg, tid);
+      load_image(dst + kImg, NSimg + img0 + (size_t)c * kImg, tid);
+    }
     commit();
-  }
+  };
+#pragma unroll
+  for (int c = 0; c < kStages - 1; ++c) fetch(c);
   float S[8][4];
   const T *sp = state + ((size_t)b * kDim + 16 * w + g) * kDim + 2 * t;
 #pragma unroll
@@ -180,28 +187,21 @@ dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg
     S[n][0] = __uint_as_float(lo16<T>(u)); S[n][1] = __uint_as_float(hi16<T>(u));
     S[n][2] = __uint_as_float(lo16<T>(x)); S[n][3] = __uint_as_float(hi16<T>(x));
   }
-  float4 nx[8];      // N of the chunk at work, fetched one chunk ahead
-#pragma unroll
-  for (int n = 0; n < 8; ++n) nx[n] = image_at(Nimg + img0, w, n, lane);
-
   for (int c = 0; c < nc; ++c) {
     wait<kStages - 2>();
-    __syncthreads();             // chunk c's Qc has landed for all; the buffer refilled next is no longer read
-    if (c + kStages - 1 < nc) load_image(ring + (c + kStages - 1) % kStages * kImg, Qimg + img0 + (size_t)(c + kStages - 1) * kImg, tid);
-    commit();
-    store_rows<true>(Simg + img0 + (size_t)c * kImg, S, w, lane);
+    __syncthreads();             // chunk c has landed for all; the buffer refilled next is no longer read
+    fetch(c + kStages - 1);
+    const float *buf = ring + (c % kStages) * 2 * kImg;
+    store_rows<true>(NSimg + img0 + (size_t)c * kImg, S, w, lane);
     uint32_t a[8][4];
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
+      const float4 nx = image_at(buf + kImg, w, n, lane);
 #pragma unroll
       for (int e = 0; e < 4; ++e) a[n][e] = op(S[n][e]);
-      S[n][0] += nx[n].x; S[n][1] += nx[n].y; S[n][2] += nx[n].z; S[n][3] += nx[n].w;
+      S[n][0] += nx.x; S[n][1] += nx.y; S[n][2] += nx.z; S[n][3] += nx.w;
     }
-    if (c + 1 < nc) {
-#pragma unroll
-      for (int n = 0; n < 8; ++n) nx[n] = image_at(Nimg + img0 + (size_t)(c + 1) * kImg, w, n, lane);
-    }
-    mma_image(S, a, ring + c % kStages * kImg, lane);
+    mma_image(S, a, buf, lane);
   }
   T *fp = final_state + ((size_t)b * kDim + 16 * w + g) * kDim + 2 * t;
 #pragma unroll
@@ -336,26 +336,26 @@ int forward_typed(const void *q, const void *k, const void *v, const void *state
     set_error("chunked delta rule: %lld chunks exceed a grid", (long long)n);
     return T2FW_ERR_UNSUPPORTED;
   }
-  float *W = static_cast<float *>(scratch), *U = W + n * kImg, *Qc = U + n * kImg, *N = Qc + n * kImg, *S = N + n * kImg;
+  float *W = static_cast<float *>(scratch), *U = W + n * kImg, *Qc = U + n * kImg, *NS = Qc + n * kImg;
   auto *const prep = &dfw_prep_fwd_kernel<T>;
   T2FW_ALLOW_SMEM(prep, kSmemPrep);
-  T2FW_CHECK_CUDA(launch_dependent(prep, dim3((unsigned)n), dim3(kThreads), kSmemPrep, st, (const T *)k, (const T *)v, W, U, Qc, N, T_, (int)nc));
+  T2FW_CHECK_CUDA(launch_dependent(prep, dim3((unsigned)n), dim3(kThreads), kSmemPrep, st, (const T *)k, (const T *)v, W, U, Qc, NS, T_, (int)nc));
   auto *const carry = &dfw_carry_fwd_kernel<T>;
   T2FW_ALLOW_SMEM(carry, kSmemCarry);
-  T2FW_CHECK_CUDA(launch_dependent(carry, dim3((unsigned)B), dim3(kThreads), kSmemCarry, st, (const T *)state, (const float *)Qc,
-                                   (const float *)N, S, (T *)final_state, (int)nc));
+  T2FW_CHECK_CUDA(launch_dependent(carry, dim3((unsigned)B), dim3(kThreads), kSmemCarry, st, (const T *)state, (const float *)Qc, NS,
+                                   (T *)final_state, (int)nc));
   auto *const outk = &dfw_out_fwd_kernel<T>;
   T2FW_ALLOW_SMEM(outk, kSmemOut);
   T2FW_CHECK_CUDA(launch_dependent(outk, dim3((unsigned)n), dim3(kThreads), kSmemOut, st, (const T *)q, (const T *)k, (const float *)W,
-                                   (const float *)U, (const float *)S, (T *)out, (float *)delta, T_, (int)nc));
+                                   (const float *)U, (const float *)NS, (T *)out, (float *)delta, T_, (int)nc));
   T2FW_CHECK_LAUNCH(3);
   return T2FW_OK;
 }
 
 }  // namespace
 
-// five fp32 images per chunk: W, U^T, Qc^T, N, start state
-size_t dfw_forward_images_bytes(int64_t B, int64_t T_) { return (size_t)B * ceil_div64(T_, kC) * 5 * kImg * sizeof(float); }
+// four fp32 images per chunk: W, U^T, Qc^T, N (then the start state)
+size_t dfw_forward_images_bytes(int64_t B, int64_t T_) { return (size_t)B * ceil_div64(T_, kC) * 4 * kImg * sizeof(float); }
 
 int dfw_forward_images(const void *q, const void *k, const void *v, const void *state, void *out, void *final_state, void *delta,
                        int64_t B, int64_t T_, int dtype, void *scratch, cudaStream_t st) {
