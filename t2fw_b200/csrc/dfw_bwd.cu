@@ -27,7 +27,7 @@ using namespace frag;
 namespace {
 
 // ---- prep: grid = B * nc, four warps -----------------------------------------------------------------
-constexpr int oK = 0, oQ = kRaw, oG = 2 * kRaw, oT = 3 * kRaw, oL = oT + kC * kLdT * 4;
+constexpr int oK = 0, oQ = kRaw, oG = 2 * kRaw, oT = 3 * kRaw, oL = oT + kC * kLdL * 4;
 constexpr int kSmemPrep = oL + kC * kLdL * 4;
 
 template <typename T>
@@ -44,41 +44,42 @@ dfw_prep_bwd_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *
   const size_t base = ((size_t)b * T_ + t0) * kDim, img = (size_t)blockIdx.x * kImg;
   dependency_wait();
   load_raw(sm + oK, k + base, nvalid, tid);
-  commit();
   load_raw(sm + oQ, q + base, nvalid, tid);
   load_raw(sm + oG, go + base, nvalid, tid);
   commit();
-  wait<1>();
+  wait<0>();
   __syncthreads();
   gram_lower<T>(Ls, aK, aK, w, lane);
   __syncwarp();
-  unit_lower_inverse(Ls, Ts, w, lane);
-  wait<0>();
-  __syncthreads();
-
-  // C = strict_upper(K Q^T), rows t = 16 w .., as an image over L
+  unit_lower_inverse<kLdL>(Ls, Ts, w, lane);
+  // C = strict_upper(K Q^T), rows t = 16 w ..: the warps with the least to do in the inverse have the most blocks here
   float *Cs = Ls;
   {
+    float c[4][2][4] = {};
     uint32_t a[4][4];
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) raw_a(a[kk], aK, 16 * w, kk, lane);
 #pragma unroll
     for (int np = 0; np < 4; ++np) {
       if (np < w) continue;
-      float c[2][4] = {};
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
         uint32_t r[4];
         raw_b(r, aQ, 16 * np, kk, lane);
-        mma_16<T>(c[0], a[kk], r[0], r[1]);
-        mma_16<T>(c[1], a[kk], r[2], r[3]);
+        mma_16<T>(c[np][0], a[kk], r[0], r[1]);
+        mma_16<T>(c[np][1], a[kk], r[2], r[3]);
       }
+    }
+    __syncthreads();             // L is no longer read: C over it, as an image
+#pragma unroll
+    for (int np = 0; np < 4; ++np) {
+      if (np < w) continue;
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         const int col = 16 * np + 8 * n + 2 * t, r0 = 16 * w + g, r1 = r0 + 8;
         reinterpret_cast<float4 *>(Cs)[(w * 8 + 2 * np + n) * 32 + lane] =
-            make_float4(col > r0 ? rnd(c[n][0]) : 0.f, col + 1 > r0 ? rnd(c[n][1]) : 0.f, col > r1 ? rnd(c[n][2]) : 0.f,
-                        col + 1 > r1 ? rnd(c[n][3]) : 0.f);
+            make_float4(col > r0 ? rnd(c[np][n][0]) : 0.f, col + 1 > r0 ? rnd(c[np][n][1]) : 0.f, col > r1 ? rnd(c[np][n][2]) : 0.f,
+                        col + 1 > r1 ? rnd(c[np][n][3]) : 0.f);
       }
     }
   }
@@ -109,8 +110,8 @@ dfw_prep_bwd_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
         if (n > (j | 1)) continue;      // blocks of T above the diagonal
-        const float *p = Ts + (8 * j + 2 * t) * kLdT + 8 * n + g;
-        mma_split(u[n], ah, al, p[0], p[kLdT]);
+        const float *p = Ts + (8 * j + 2 * t) * kLdL + 8 * n + g;
+        mma_split(u[n], ah, al, p[0], p[kLdL]);
       }
     }
     float *up = Ub + img + 16 * w + g;      // [t][d]: eight lanes = 32 contiguous bytes of a step
@@ -158,11 +159,11 @@ dfw_prep_bwd_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *
       uint32_t ah[2][4], al[2][4];
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const float *p = Ts + (16 * kk + 8 * s + 2 * t) * kLdT + 16 * w + g;
+        const float *p = Ts + (16 * kk + 8 * s + 2 * t) * kLdL + 16 * w + g;
         split(p[0], ah[s][0], al[s][0]);
-        split(p[kLdT], ah[s][1], al[s][1]);
+        split(p[kLdL], ah[s][1], al[s][1]);
         split(p[8], ah[s][2], al[s][2]);
-        split(p[kLdT + 8], ah[s][3], al[s][3]);
+        split(p[kLdL + 8], ah[s][3], al[s][3]);
       }
 #pragma unroll
       for (int np = 0; np < 4; ++np) {
@@ -198,31 +199,10 @@ dfw_prep_bwd_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *
     *reinterpret_cast<float2 *>(Ws + (16 * w + g + 8) * kLdL + 8 * n + 2 * t) = make_float2(rnd(wb[n][2]), rnd(wb[n][3]));
   }
   __syncthreads();
-  // Qb^T = -K^T Wb, then (Dl^T K)^T = K^T Dl, rows 16 w ..
-#pragma unroll 1
-  for (int pass = 0; pass < 2; ++pass) {
-    if (pass) {
-      wait<0>();
-      __syncthreads();
-    }
-    const float *Bs = pass ? Ds : Ws;
-    float c[8][4];
-    zero(c);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      uint32_t a[4];
-      raw_at(a, aK, 16 * w, 16 * kk, lane);
-#pragma unroll
-      for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const float *p = Bs + (16 * kk + 8 * s + 2 * t) * kLdL + 8 * n + g;
-          mma_raw_a<T>(c[n], a, s, op(p[0]), op(p[kLdL]));      // (Wb is rounded already: the increment is dropped again)
-        }
-    }
-    if (pass) store_rows<false>(Gimg + img, c, w, lane);
-    else store_rows<true>(Qimg + img, c, w, lane, -1.f);
-  }
+  mma_kt_b<T, false, true>(Qimg + img, aK, Ws, -1.f, w, lane);      // Qb^T = -K^T Wb
+  wait<0>();
+  __syncthreads();
+  mma_kt_b<T, true, false>(Gimg + img, aK, Ds, 1.f, w, lane);       // (Dl^T K)^T = K^T Dl
 }
 
 // ---- carry: one CTA per row, chunks in reverse; warp w = rows 16 w .. of R [d][m] and of S^T [m][d] -------------
@@ -296,28 +276,39 @@ dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state
   wait<0>();
 }
 
-// ---- gradients: grid = B * nc, four warps, warp w = steps 16 w .. --------------------------------------------
+// ---- gradients: grid = B * nc, eight warps ---------------------------------------------------------------------
+// Two groups of four warps, warp w of a group = steps 16 w ..: group 0 forms E and everything that contracts with
+// strictly lower blocks (d_query, part of d_key), group 1 the rest of d_key; equal numbers of products, and half
+// the registers of one group doing both.
+constexpr int kThreadsG = 256;
 constexpr int kLdD = 72;      // row stride of Dl: 8-byte reads along its rows are free of bank conflicts
-constexpr int oKg = 0, oQg = kRaw, oGg = 2 * kRaw, oDg = 3 * kRaw, oRg = oDg + kC * kLdD * 4;      // R [64][kLdL], then E image
-constexpr int kSmemGrad = oRg + kC * kLdL * 4;
+constexpr int oKg = 0, oQg = kRaw, oGg = 2 * kRaw, oDg = 3 * kRaw, oRg = oDg + kC * kLdD * 4;      // R, then E image
+constexpr int oSg = oRg + kImg * 4;                                                               // S0^T image, then group 0's d_key
+constexpr int oEg = oSg + kImg * 4, kSmemGrad = oEg + kRaw;                                       // d_value on its way out
+// R is read along rows (8 bytes of eight consecutive rows at a time) and along columns (4 bytes of every other row): its
+// 16-byte pieces are XOR-ed with twice a number that differs between any four rows a wavefront of either kind touches.
+__device__ __forceinline__ int r_off(int d, int m) {
+  return d * kDim + ((((m >> 2) ^ (2 * ((d & 3) ^ ((d >> 2) & 1)))) << 2) | (m & 3));
+}
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreadsG, 2)
 dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__restrict__ k, const float *__restrict__ delta,
                 const float *__restrict__ Wimg, const float *__restrict__ Ub, const float *__restrict__ Rrow,
                 const float *__restrict__ STimg, T *__restrict__ dq, T *__restrict__ dk, T *__restrict__ dv, int64_t T_, int nc) {
   extern __shared__ __align__(128) unsigned char sm[];
-  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int tid = threadIdx.x, w = (tid >> 5) & 3, group = tid >> 7, lane = tid & 31, g = lane >> 2, t = lane & 3;
   float *Ds = reinterpret_cast<float *>(sm + oDg), *Rs = reinterpret_cast<float *>(sm + oRg), *Es = Rs;
+  float *Ss = reinterpret_cast<float *>(sm + oSg);
   const uint32_t aK = smem_u32(sm + oKg), aQ = smem_u32(sm + oQg), aG = smem_u32(sm + oGg);
   const int64_t b = blockIdx.x / (uint32_t)nc, t0 = (int64_t)(blockIdx.x - (uint32_t)b * nc) * kC;
   const int nvalid = (int)(T_ - t0 < kC ? T_ - t0 : kC);
   const size_t base = ((size_t)b * T_ + t0) * kDim, img = (size_t)blockIdx.x * kImg;
   dependency_wait();
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int i = tid + kThreads * j, r = i >> 4, p = i & 15;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(Rs + r * kLdL + 4 * p)), "l"(Rrow + img + r * kDim + 4 * p) : "memory");
+  for (int j = 0; j < 4; ++j) {
+    const int i = tid + kThreadsG * j, r = i >> 4, p = i & 15;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(Rs + r_off(r, 4 * p))), "l"(Rrow + img + r * kDim + 4 * p) : "memory");
     float *d = Ds + r * kLdD + 4 * p;
     if (r < nvalid)
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d)), "l"(delta + base + (size_t)r * kDim + 4 * p) : "memory");
@@ -325,80 +316,63 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
       *reinterpret_cast<float4 *>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   commit();
-  load_raw(sm + oGg, go + base, nvalid, tid);
-  load_raw(sm + oKg, k + base, nvalid, tid);
-  load_raw(sm + oQg, q + base, nvalid, tid);
+  load_raw<T, kThreadsG>(sm + oGg, go + base, nvalid, tid);
+  load_raw<T, kThreadsG>(sm + oKg, k + base, nvalid, tid);
+  load_raw<T, kThreadsG>(sm + oQg, q + base, nvalid, tid);
+  load_image<kThreadsG>(Ss, STimg + img, tid);
   commit();
   const int r0 = 16 * w + g, r1 = r0 + 8;
-  float e[8][4];      // E, rows t
-  uint32_t ea[8][4];  // Wb, then E as an operand
-#pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    const float4 w4 = image_at(Wimg + img, w, n, lane);
-    ea[n][0] = bits(w4.x); ea[n][1] = bits(w4.y); ea[n][2] = bits(w4.z); ea[n][3] = bits(w4.w);
-    const float2 u0 = *reinterpret_cast<const float2 *>(Ub + img + r0 * kDim + 8 * n + 2 * t);
-    const float2 u1 = *reinterpret_cast<const float2 *>(Ub + img + r1 * kDim + 8 * n + 2 * t);
-    e[n][0] = u0.x; e[n][1] = u0.y; e[n][2] = u1.x; e[n][3] = u1.y;
-  }
-  wait<1>();
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < 8; ++j)      // E = Ub + Wb R^T
-#pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      const float2 r2 = *reinterpret_cast<const float2 *>(Rs + (8 * n + g) * kLdL + 8 * j + 2 * t);
-      mma_acc_a(e[n], ea[j], bits(r2.x), bits(r2.y));
-    }
-  uint32_t da[8][4];      // Dl, own rows
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float2 x = *reinterpret_cast<const float2 *>(Ds + r0 * kLdD + 8 * j + 2 * t);
-    const float2 y = *reinterpret_cast<const float2 *>(Ds + r1 * kLdD + 8 * j + 2 * t);
-    da[j][0] = op(x.x); da[j][1] = op(x.y); da[j][2] = op(y.x); da[j][3] = op(y.y);
-  }
+  uint32_t ea[8][4];      // -E as an operand, own rows
   float ck[8][4];         // d_key
   zero(ck);
-#pragma unroll
-  for (int j = 0; j < 8; ++j)      // Dl R
+
+  if (group == 0) {
+    float e[8][4];      // E = Ub + Wb R^T
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
-      const float *p = Rs + (8 * j + 2 * t) * kLdL + 8 * n + g;
-      mma_acc_a(ck[n], da[j], bits(p[0]), bits(p[kLdL]));
+      const float4 w4 = image_at(Wimg + img, w, n, lane);
+      ea[n][0] = bits(w4.x); ea[n][1] = bits(w4.y); ea[n][2] = bits(w4.z); ea[n][3] = bits(w4.w);
+      const float2 u0 = *reinterpret_cast<const float2 *>(Ub + img + r0 * kDim + 8 * n + 2 * t);
+      const float2 u1 = *reinterpret_cast<const float2 *>(Ub + img + r1 * kDim + 8 * n + 2 * t);
+      e[n][0] = u0.x; e[n][1] = u0.y; e[n][2] = u1.x; e[n][3] = u1.y;
     }
-  wait<0>();
-  __syncthreads();             // R has been read; raw blocks are there
+    wait<1>();
+    __syncthreads();             // R and Dl are there
 #pragma unroll
-  for (int n = 0; n < 8; ++n) {
+    for (int j = 0; j < 8; ++j)
 #pragma unroll
-    for (int x = 0; x < 4; ++x) ea[n][x] = op(e[n][x]);
-    reinterpret_cast<uint4 *>(Es)[(w * 8 + n) * 32 + lane] = make_uint4(ea[n][0], ea[n][1], ea[n][2], ea[n][3]);
-    // d_value: rows r0, r1, two columns per lane
-    if (r0 < nvalid) *reinterpret_cast<uint32_t *>(dv + base + (size_t)r0 * kDim + 8 * n + 2 * t) = pack16<T>(e[n][0], e[n][1]);
-    if (r1 < nvalid) *reinterpret_cast<uint32_t *>(dv + base + (size_t)r1 * kDim + 8 * n + 2 * t) = pack16<T>(e[n][2], e[n][3]);
+      for (int n = 0; n < 8; ++n) {
+        const float2 r2 = *reinterpret_cast<const float2 *>(Rs + r_off(8 * n + g, 8 * j + 2 * t));
+        mma_acc_a(e[n], ea[j], bits(r2.x), bits(r2.y));
+      }
+    wait<0>();
+    __syncthreads();             // R has been read by both groups; raw blocks and S0^T are there
 #pragma unroll
-    for (int x = 0; x < 4; ++x) ea[n][x] ^= 0x80000000u;      // from here on -E
-  }
-  __syncthreads();
-
-  uint32_t ga[4][4];      // dO, own rows
+    for (int n = 0; n < 8; ++n) {
 #pragma unroll
-  for (int kk = 0; kk < 4; ++kk) raw_a(ga[kk], aG, 16 * w, kk, lane);
-  float cq[8][4];         // d_query
-  zero(cq);
-#pragma unroll
-  for (int j = 0; j < 8; ++j)      // dO S0 and -E S0
-#pragma unroll
-    for (int np = 0; np < 4; ++np) {
-      const float4 s4 = image_at(STimg + img, np, j, lane);
-      mma_raw_a<T>(cq[2 * np], ga[j >> 1], j & 1, bits(s4.x), bits(s4.y));
-      mma_raw_a<T>(cq[2 * np + 1], ga[j >> 1], j & 1, bits(s4.z), bits(s4.w));
-      mma_acc_a(ck[2 * np], ea[j], bits(s4.x), bits(s4.y));
-      mma_acc_a(ck[2 * np + 1], ea[j], bits(s4.z), bits(s4.w));
+      for (int x = 0; x < 4; ++x) ea[n][x] = op(-e[n][x]);
+      reinterpret_cast<uint4 *>(Es)[(w * 8 + n) * 32 + lane] = make_uint4(ea[n][0], ea[n][1], ea[n][2], ea[n][3]);
+      *reinterpret_cast<uint32_t *>(sm + oEg + raw_off(r0, n) + 4 * t) = pack16<T>(e[n][0], e[n][1]);
+      *reinterpret_cast<uint32_t *>(sm + oEg + raw_off(r1, n) + 4 * t) = pack16<T>(e[n][2], e[n][3]);
     }
+    __syncthreads();             // (-E) image complete
+    rows_out<T>(dv + base, sm + oEg, w, nvalid, lane);
+    uint32_t ga[4][4];      // dO, own rows
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) raw_a(ga[kk], aG, 16 * w, kk, lane);
+    float cq[8][4];         // d_query = dO S0 ..
+    zero(cq);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int np = 0; np < 4; ++np) {
+        const float4 s4 = image_at(Ss, np, j, lane);
+        mma_raw_a<T>(cq[2 * np], ga[j >> 1], j & 1, bits(s4.x), bits(s4.y));
+        mma_raw_a<T>(cq[2 * np + 1], ga[j >> 1], j & 1, bits(s4.z), bits(s4.w));
+      }
 #pragma unroll 1
-  for (int ip = 0; ip < 4; ++ip) {      // 16 steps s at a time: below the diagonal, on it (both parts), above it
-    const int s0 = 16 * ip;
-    if (ip <= w) {      // strict_lower(dO Dl^T) K to d_query, strict_lower(-E Dl^T) K to d_key
+    for (int ip = 0; ip <= w; ++ip) {      // .. + strict_lower(dO Dl^T) K;  d_key: strict_lower(-E Dl^T) K; 16 steps at a time
+      const int s0 = 16 * ip;
       float x[2][4] = {}, y[2][4] = {};
 #pragma unroll
       for (int j = 0; j < 8; ++j)
@@ -432,7 +406,49 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
           }
       }
     }
-    if (ip >= w) {      // strict_upper(Dl dO^T) Q and strict_upper(-Dl E^T) K to d_key
+    __syncthreads();             // S0^T, Q and K have been read
+    store_rows<false>(Ss, ck, w, lane);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      *reinterpret_cast<uint32_t *>(sm + oQg + raw_off(r0, n) + 4 * t) = pack16<T>(cq[n][0], cq[n][1]);
+      *reinterpret_cast<uint32_t *>(sm + oQg + raw_off(r1, n) + 4 * t) = pack16<T>(cq[n][2], cq[n][3]);
+    }
+    __syncthreads();             // group 0's part of d_key is there
+  } else {
+    wait<1>();
+    __syncthreads();
+    uint32_t da[8][4];      // Dl, own rows
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float2 x = *reinterpret_cast<const float2 *>(Ds + r0 * kLdD + 8 * j + 2 * t);
+      const float2 y = *reinterpret_cast<const float2 *>(Ds + r1 * kLdD + 8 * j + 2 * t);
+      da[j][0] = op(x.x); da[j][1] = op(x.y); da[j][2] = op(y.x); da[j][3] = op(y.y);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)      // Dl R
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        mma_acc_a(ck[n], da[j], bits(Rs[r_off(8 * j + 2 * t, 8 * n + g)]), bits(Rs[r_off(8 * j + 2 * t + 1, 8 * n + g)]));
+      }
+    wait<0>();
+    __syncthreads();
+    __syncthreads();             // (-E) image complete
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float4 e4 = image_at(Es, w, j, lane);
+      ea[j][0] = bits(e4.x); ea[j][1] = bits(e4.y); ea[j][2] = bits(e4.z); ea[j][3] = bits(e4.w);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)      // -E S0
+#pragma unroll
+      for (int np = 0; np < 4; ++np) {
+        const float4 s4 = image_at(Ss, np, j, lane);
+        mma_acc_a(ck[2 * np], ea[j], bits(s4.x), bits(s4.y));
+        mma_acc_a(ck[2 * np + 1], ea[j], bits(s4.z), bits(s4.w));
+      }
+#pragma unroll 1
+    for (int ip = w; ip < 4; ++ip) {      // strict_upper(Dl dO^T) Q and strict_upper(-Dl E^T) K
+      const int s0 = 16 * ip;
       float x[2][4] = {}, y[2][4] = {};
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
@@ -457,7 +473,7 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
         for (int i = 0; i < 4; ++i) {
           const bool in = s0 + 8 * n + 2 * t + (i & 1) > (i < 2 ? r0 : r1);
           xa[n][i] = in ? op(x[n][i]) : 0u;
-          ya[n][i] = in ? op(-y[n][i]) : 0u;
+          ya[n][i] = in ? op(y[n][i]) : 0u;
         }
 #pragma unroll
       for (int np = 0; np < 4; ++np) {
@@ -473,24 +489,18 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
           }
       }
     }
-  }
-  __syncthreads();             // Q and K have been read: this warp's rows of them carry its results out in whole rows
+    __syncthreads();
+    __syncthreads();
 #pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    *reinterpret_cast<uint32_t *>(sm + oQg + raw_off(r0, n) + 4 * t) = pack16<T>(cq[n][0], cq[n][1]);
-    *reinterpret_cast<uint32_t *>(sm + oQg + raw_off(r1, n) + 4 * t) = pack16<T>(cq[n][2], cq[n][3]);
-    *reinterpret_cast<uint32_t *>(sm + oKg + raw_off(r0, n) + 4 * t) = pack16<T>(ck[n][0], ck[n][1]);
-    *reinterpret_cast<uint32_t *>(sm + oKg + raw_off(r1, n) + 4 * t) = pack16<T>(ck[n][2], ck[n][3]);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = 16 * w + 4 * i + (lane >> 3), p = lane & 7;
-    if (r < nvalid) {
-      *reinterpret_cast<uint4 *>(dq + base + (size_t)r * kDim + 8 * p) = *reinterpret_cast<const uint4 *>(sm + oQg + raw_off(r, p));
-      *reinterpret_cast<uint4 *>(dk + base + (size_t)r * kDim + 8 * p) = *reinterpret_cast<const uint4 *>(sm + oKg + raw_off(r, p));
+    for (int n = 0; n < 8; ++n) {
+      const float4 c4 = image_at(Ss, w, n, lane);
+      *reinterpret_cast<uint32_t *>(sm + oKg + raw_off(r0, n) + 4 * t) = pack16<T>(ck[n][0] + c4.x, ck[n][1] + c4.y);
+      *reinterpret_cast<uint32_t *>(sm + oKg + raw_off(r1, n) + 4 * t) = pack16<T>(ck[n][2] + c4.z, ck[n][3] + c4.w);
     }
   }
+  __syncwarp();
+  // this warp's own rows of Q (group 0: d_query) or K (group 1: d_key), now results
+  rows_out<T>((group ? dk : dq) + base, sm + (group ? oKg : oQg), w, nvalid, lane);
 }
 
 template <typename T>
@@ -512,7 +522,7 @@ int backward_typed(const void *go, const void *gs, const void *q, const void *k,
                                    (const float *)Qb, NR, GS, (T *)ds, (int)nc));
   auto *const grad = &dfw_grad_kernel<T>;
   T2FW_ALLOW_SMEM(grad, kSmemGrad);
-  T2FW_CHECK_CUDA(launch_dependent(grad, dim3((unsigned)n), dim3(kThreads), kSmemGrad, st, (const T *)go, (const T *)q, (const T *)k,
+  T2FW_CHECK_CUDA(launch_dependent(grad, dim3((unsigned)n), dim3(kThreadsG), kSmemGrad, st, (const T *)go, (const T *)q, (const T *)k,
                                    (const float *)delta, (const float *)W, (const float *)U, (const float *)NR, (const float *)GS, (T *)dq,
                                    (T *)dk, (T *)dv, T_, (int)nc));
   T2FW_CHECK_LAUNCH(3);
@@ -521,11 +531,8 @@ int backward_typed(const void *go, const void *gs, const void *q, const void *k,
 
 }  // namespace
 
-// five fp32 images per chunk: Wb, Ub, Qb^T, Nb (then R_end), (Dl^T K)^T (then S0^T)
-size_t dfw_backward_images_bytes(int64_t B, int64_t T_) { return (size_t)B * ceil_div64(T_, kC) * 5 * kImg * sizeof(float); }
-
-int dfw_backward_images(const void *go, const void *gs, const void *q, const void *k, const void *delta, const void *final_state,
-                        void *dq, void *dk, void *dv, void *ds, int64_t B, int64_t T_, int dtype, void *scratch, cudaStream_t st) {
+int dfw_chunk_backward(const void *go, const void *gs, const void *q, const void *k, const void *delta, const void *final_state,
+                       void *dq, void *dk, void *dv, void *ds, int64_t B, int64_t T_, int dtype, void *scratch, cudaStream_t st) {
   if (dtype == T2FW_F16) return backward_typed<__half>(go, gs, q, k, delta, final_state, dq, dk, dv, ds, B, T_, scratch, st);
   return backward_typed<__nv_bfloat16>(go, gs, q, k, delta, final_state, dq, dk, dv, ds, B, T_, scratch, st);
 }

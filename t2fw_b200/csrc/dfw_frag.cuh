@@ -27,6 +27,7 @@ constexpr int kDim = 64;                     // D = M = 64
 constexpr int kImg = kC * kDim;              // floats of an image
 constexpr int kRaw = kC * kDim * 2;          // bytes of a raw block
 constexpr int kThreads = 128;                // four warps
+constexpr int kLdL = 68;                     // row stride (floats) of matrices that are read along columns (conflict-free)
 
 // ---- products ------------------------------------------------------------------------------------
 __device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
@@ -124,11 +125,11 @@ __device__ __forceinline__ void mma_acc_a(float (&c)[4], const uint32_t (&a)[4],
 }
 
 // Block [64][64] of a dense [rows][64] array into shared memory, asynchronously; rows beyond nvalid become zeros.
-template <typename T>
+template <typename T, int kN = kThreads>
 __device__ __forceinline__ void load_raw(unsigned char *dst, const T *src, int nvalid, int tid) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int i = tid + kThreads * j, r = i >> 3, p = i & 7;
+  for (int j = 0; j < 512 / kN; ++j) {
+    const int i = tid + kN * j, r = i >> 3, p = i & 7;
     unsigned char *d = dst + raw_off(r, p);
     if (r < nvalid)
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d)), "l"(src + (size_t)r * kDim + p * 8) : "memory");
@@ -136,11 +137,21 @@ __device__ __forceinline__ void load_raw(unsigned char *dst, const T *src, int n
       *reinterpret_cast<uint4 *>(d) = make_uint4(0u, 0u, 0u, 0u);
   }
 }
+// this warp's rows 16 w .. of a raw-format block in shared memory to a dense [rows][64] array, in whole rows
+template <typename T>
+__device__ __forceinline__ void rows_out(T *dst, const unsigned char *src, int w, int nvalid, int lane) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = 16 * w + 4 * i + (lane >> 3), p = lane & 7;
+    if (r < nvalid) *reinterpret_cast<uint4 *>(dst + (size_t)r * kDim + 8 * p) = *reinterpret_cast<const uint4 *>(src + raw_off(r, p));
+  }
+}
 // an image (or any 16 KB) into shared memory, asynchronously
+template <int kN = kThreads>
 __device__ __forceinline__ void load_image(float *dst, const float *src, int tid) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int i = tid + kThreads * j;
+  for (int j = 0; j < 1024 / kN; ++j) {
+    const int i = tid + kN * j;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + 4 * i)), "l"(src + 4 * i) : "memory");
   }
 }
@@ -181,14 +192,50 @@ __device__ __forceinline__ void mma_image(float (&c)[8][4], const uint32_t (&a)[
     }
 }
 
+// K^T B with the raw block K [t][m] and B [t][n] in shared memory (row stride kLdL): this warp's 32 x 32 part of the
+// result, rows 32 (w / 2) .., columns 32 (w % 2) .. (a square part halves the reads of B, which cost most), to an image
+template <typename T, bool kRoundB, bool kRoundOut>
+__device__ __forceinline__ void mma_kt_b(float *img, uint32_t k, const float *B, float sign, int w, int lane) {
+  const int g = lane >> 2, t = lane & 3, rb = 2 * (w >> 1), cb = 4 * (w & 1);
+  float c[2][4][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) c[i][n][0] = c[i][n][1] = c[i][n][2] = c[i][n][3] = 0.f;
+#pragma unroll
+  for (int kk = 0; kk < 4; ++kk) {
+    uint32_t a[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) raw_at(a[i], k, 16 * (rb + i), 16 * kk, lane);
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const float *p = B + (16 * kk + 8 * s + 2 * t) * kLdL + 8 * (cb + n) + g;
+        const uint32_t b0 = kRoundB ? op(p[0]) : bits(p[0]), b1 = kRoundB ? op(p[kLdL]) : bits(p[kLdL]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) mma_raw_a<T>(c[i][n], a[i], s, b0, b1);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      float4 v = make_float4(sign * c[i][n][0], sign * c[i][n][1], sign * c[i][n][2], sign * c[i][n][3]);
+      if (kRoundOut) v = make_float4(rnd(v.x), rnd(v.y), rnd(v.z), rnd(v.w));
+      reinterpret_cast<float4 *>(img)[((rb + i) * 8 + cb + n) * 32 + lane] = v;
+    }
+}
+
 // ---- (I + L)^-1 of a strictly lower triangular 64 x 64 matrix, fp32 -----------------------------------
-// L in Ls [64][kLdL], the inverse to Ts [64][kLdT] (diagonal blocks with their zeros; the blocks above the diagonal are
+// L in Ls [64][kLdL], the inverse to Ts [64][kLd] (diagonal blocks with their zeros; the blocks above the diagonal are
 // neither written nor meant to be read).  Warp w owns block row w: it inverts its 16 x 16 diagonal block by
 // substitution, one column per lane, and, once all of those are there, its blocks left of it from right to left,
 //     T_ij = -( sum_{j<k<=i} T_ik L_kj ) T_jj ,
 // which needs nothing from the other block rows of T.  The products are three TF32 products each (operands split in
 // two), i.e. fp32-like.  Called by all four warps; ends without a barrier.
-constexpr int kLdL = 68, kLdT = 72;
+constexpr int kLdT = 72;      // stride of T where it is read along rows (8-byte reads, conflict-free)
+// kLd: row stride of Ts
 __device__ __forceinline__ void mma_split(float (&c)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], float b0, float b1) {
   uint32_t bh0, bl0, bh1, bl1;
   split(b0, bh0, bl0);
@@ -197,6 +244,7 @@ __device__ __forceinline__ void mma_split(float (&c)[4], const uint32_t (&ah)[4]
   mma_acc_a(c, al, bh0, bh1);
   mma_acc_a(c, ah, bl0, bl1);
 }
+template <int kLd>
 __device__ __forceinline__ void unit_lower_inverse(const float *Ls, float *Ts, int w, int lane) {
   const int g = lane >> 2, t = lane & 3;
   if (lane < 16) {
@@ -214,15 +262,15 @@ __device__ __forceinline__ void unit_lower_inverse(const float *Ls, float *Ts, i
         if (k4 + 3 < r) a = fmaf(-l.w, x[k4 + 3], a);
       }
       x[r] = a;
-      Ts[(16 * w + r) * kLdT + 16 * w + lane] = a;
+      Ts[(16 * w + r) * kLd + 16 * w + lane] = a;
     }
   }
   __syncthreads();
   uint32_t th[4][2][4], tl[4][2][4];      // T_{w, w-r}, as A operands (hi, lo), r = 0 the diagonal block
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
-    const float2 u = *reinterpret_cast<const float2 *>(Ts + (16 * w + g) * kLdT + 16 * w + 8 * s + 2 * t);
-    const float2 v = *reinterpret_cast<const float2 *>(Ts + (16 * w + g + 8) * kLdT + 16 * w + 8 * s + 2 * t);
+    const float2 u = *reinterpret_cast<const float2 *>(Ts + (16 * w + g) * kLd + 16 * w + 8 * s + 2 * t);
+    const float2 v = *reinterpret_cast<const float2 *>(Ts + (16 * w + g + 8) * kLd + 16 * w + 8 * s + 2 * t);
     split(u.x, th[0][s][0], tl[0][s][0]);
     split(u.y, th[0][s][1], tl[0][s][1]);
     split(v.x, th[0][s][2], tl[0][s][2]);
@@ -247,15 +295,15 @@ __device__ __forceinline__ void unit_lower_inverse(const float *Ls, float *Ts, i
     for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) split(-m[n][e], mh[n][e], ml[n][e]);
-    const float *D = Ts + (16 * j) * kLdT + 16 * j;
+    const float *D = Ts + (16 * j) * kLd + 16 * j;
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       float c[4] = {};
 #pragma unroll
       for (int s = 0; s < 2; ++s)
-        mma_split(c, mh[s], ml[s], D[(8 * s + 2 * t) * kLdT + 8 * n + g], D[(8 * s + 2 * t + 1) * kLdT + 8 * n + g]);
-      *reinterpret_cast<float2 *>(Ts + (16 * w + g) * kLdT + 16 * j + 8 * n + 2 * t) = make_float2(c[0], c[1]);
-      *reinterpret_cast<float2 *>(Ts + (16 * w + g + 8) * kLdT + 16 * j + 8 * n + 2 * t) = make_float2(c[2], c[3]);
+        mma_split(c, mh[s], ml[s], D[(8 * s + 2 * t) * kLd + 8 * n + g], D[(8 * s + 2 * t + 1) * kLd + 8 * n + g]);
+      *reinterpret_cast<float2 *>(Ts + (16 * w + g) * kLd + 16 * j + 8 * n + 2 * t) = make_float2(c[0], c[1]);
+      *reinterpret_cast<float2 *>(Ts + (16 * w + g + 8) * kLd + 16 * j + 8 * n + 2 * t) = make_float2(c[2], c[3]);
 #pragma unroll
       for (int e = 0; e < 4; ++e) split(c[e], th[jj + 1][n][e], tl[jj + 1][n][e]);
     }

@@ -50,7 +50,7 @@ dfw_prep_fwd_kernel(const T *__restrict__ k, const T *__restrict__ v, float *__r
   __syncthreads();
   gram_lower<T>(Ls, aK, aK, w, lane);
   __syncwarp();
-  unit_lower_inverse(Ls, Ts, w, lane);
+  unit_lower_inverse<kLdT>(Ls, Ts, w, lane);
   __syncthreads();
 
   {   // W = T K, rows 16 w ..: to memory and, rounded, over L for the product below
@@ -133,24 +133,7 @@ dfw_prep_fwd_kernel(const T *__restrict__ k, const T *__restrict__ v, float *__r
     store_rows<false>(Nimg + img, d, w, lane);
   }
   __syncthreads();
-  {   // Qc^T = -K^T W, rows 16 w ..
-    const float *Ws = Ls;
-    float c[8][4];
-    zero(c);
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      uint32_t a[4];
-      raw_at(a, aK, 16 * w, 16 * kk, lane);
-#pragma unroll
-      for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const float *p = Ws + (16 * kk + 8 * s + 2 * t) * kLdL + 8 * n + g;
-          mma_raw_a<T>(c[n], a, s, bits(p[0]), bits(p[kLdL]));
-        }
-    }
-    store_rows<true>(Qimg + img, c, w, lane, -1.f);
-  }
+  mma_kt_b<T, false, true>(Qimg + img, aK, Ls, -1.f, w, lane);      // Qc^T = -K^T W
 }
 
 // ---- carry: one CTA per row, warp w = state rows 16 w .. ------------------------------------------------
@@ -321,11 +304,7 @@ dfw_out_fwd_kernel(const T *__restrict__ q, const T *__restrict__ k, const float
     *reinterpret_cast<uint32_t *>(sm + oQo + raw_off(16 * w + g + 8, n) + 4 * t) = pack16<T>(c[n][2], c[n][3]);
   }
   __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = 16 * w + 4 * i + (lane >> 3), p = lane & 7;
-    if (r < nvalid) *reinterpret_cast<uint4 *>(out + base + (size_t)r * kDim + 8 * p) = *reinterpret_cast<const uint4 *>(sm + oQo + raw_off(r, p));
-  }
+  rows_out<T>(out + base, sm + oQo, w, nvalid, lane);
 }
 
 template <typename T>
@@ -354,11 +333,18 @@ int forward_typed(const void *q, const void *k, const void *v, const void *state
 
 }  // namespace
 
-// four fp32 images per chunk: W, U^T, Qc^T, N (then the start state)
-size_t dfw_forward_images_bytes(int64_t B, int64_t T_) { return (size_t)B * ceil_div64(T_, kC) * 4 * kImg * sizeof(float); }
+bool dfw_chunk_supported(int64_t D, int64_t M, int dtype) {
+  return D == kDim && M == kDim && (dtype == T2FW_F16 || dtype == T2FW_BF16);
+}
 
-int dfw_forward_images(const void *q, const void *k, const void *v, const void *state, void *out, void *final_state, void *delta,
-                       int64_t B, int64_t T_, int dtype, void *scratch, cudaStream_t st) {
+// fp32 images per chunk: W, U^T, Qc^T, N (then the start state); backward: Wb, Ub, Qb^T, Nb (then R_end), (Dl^T K)^T
+// (then S0^T)
+size_t dfw_chunk_scratch_bytes(int64_t B, int64_t T_, bool backward) {
+  return align_up((size_t)B * ceil_div64(T_, kC) * (backward ? 5 : 4) * kImg * sizeof(float), 256);
+}
+
+int dfw_chunk_forward(const void *q, const void *k, const void *v, const void *state, void *out, void *final_state, void *delta,
+                      int64_t B, int64_t T_, int dtype, void *scratch, cudaStream_t st) {
   if (dtype == T2FW_F16) return forward_typed<__half>(q, k, v, state, out, final_state, delta, B, T_, scratch, st);
   return forward_typed<__nv_bfloat16>(q, k, v, state, out, final_state, delta, B, T_, scratch, st);
 }
