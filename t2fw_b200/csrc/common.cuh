@@ -151,30 +151,17 @@ int lfw_chunk_backward(const void *go, const void *gs, const void *x, const void
                        void *df, void *dq, void *dk, void *dfk, void *ds, int64_t B, int64_t T,
                        int dtype, int64_t ckpt_every, void *scratch, cudaStream_t st,
                        const int **rowflag_out);
-// the same for a batch of D x K states cut into (D/64) x (K/64) blocks: sequence inputs dense
-// [B*T][D] / [B*T][K] read in place; states, checkpoints and all results per block
-// ([B * nd * nk][..][64][64] and [B * nd * nk][T][64], block (i, j) of item b at b * nd * nk + i * nk + j)
-int lfw_chunk_forward_grid(const void *x, const void *f, const void *q, const void *k, const void *fk,
-                           const void *state_blocks, void *out_blocks, void *ckpt_blocks, int64_t B, int64_t T,
-                           int nd, int nk, int dtype, int64_t ckpt_every, void *scratch, cudaStream_t st,
-                           const int **rowflag_out);
-int lfw_chunk_backward_grid(const void *go, const void *gs_blocks, const void *x, const void *f, const void *q,
-                            const void *k, const void *fk, const void *state_blocks, const void *ckpt_blocks,
-                            void *dx, void *df, void *dq, void *dk, void *dfk, void *ds_blocks, int64_t B, int64_t T,
-                            int nd, int nk, int dtype, int64_t ckpt_every, void *scratch, cudaStream_t st,
-                            const int **rowflag_out);
-// state shapes that are grids of 64 x 64 blocks (D, K multiples of 64, up to 256)
-bool lfw_blocked_supported(int64_t D, int64_t K, int dtype, int64_t ckpt_every);
-size_t lfw_blocked_forward_scratch_bytes(int64_t B, int64_t T, int64_t D, int64_t K, int64_t ckpt_every);
-size_t lfw_blocked_backward_scratch_bytes(int64_t B, int64_t T, int64_t D, int64_t K, int64_t ckpt_every);
-int lfw_blocked_forward(const void *x, const void *f, const void *q, const void *k, const void *fk,
-                        const void *state, void *out, void *ckpt, int64_t B, int64_t T, int64_t D,
-                        int64_t K, int dtype, int64_t ckpt_every, void *scratch, cudaStream_t st);
-int lfw_blocked_backward(const void *go, const void *gs, const void *x, const void *f, const void *q,
-                         const void *k, const void *fk, const void *state, const void *ckpt, void *dx,
-                         void *df, void *dq, void *dk, void *dfk, void *ds, int64_t B, int64_t T,
-                         int64_t D, int64_t K, int dtype, int64_t ckpt_every, void *scratch,
-                         cudaStream_t st);
+// the same for D x K states, D and K multiples of 64 up to 256 (a grid of 64 x 64 blocks); all arrays dense, the row
+// flags are per batch item
+bool lfw_grid_supported(int64_t D, int64_t K, int dtype, int64_t ckpt_every);
+size_t lfw_grid_scratch_bytes(int64_t B, int64_t T, int64_t D, int64_t K, int64_t ckpt_every);
+int lfw_grid_forward(const void *x, const void *f, const void *q, const void *k, const void *fk, const void *state, void *out,
+                     void *ckpt, int64_t B, int64_t T, int64_t D, int64_t K, int dtype, int64_t ckpt_every, void *scratch,
+                     cudaStream_t st, const int **rowflag_out);
+int lfw_grid_backward(const void *go, const void *gs, const void *x, const void *f, const void *q, const void *k, const void *fk,
+                      const void *state, const void *ckpt, void *dx, void *df, void *dq, void *dk, void *dfk, void *ds, int64_t B,
+                      int64_t T, int64_t D, int64_t K, int dtype, int64_t ckpt_every, void *scratch, cudaStream_t st,
+                      const int **rowflag_out);
 // what a sequence segment does to the state / state gradient (D = K = 64, 16-bit): see lfw_c64_host.cu
 size_t lfw_segment_summary_scratch_bytes(int64_t B, int64_t T);
 int lfw_segment_summary(bool backward, const void *val_d, const void *gate_d, const void *val_k, const void *gate_k,

@@ -130,29 +130,46 @@ __device__ __forceinline__ bool elect_one() {
 // warp index as a value the compiler knows to be the same in all lanes
 __device__ __forceinline__ int uniform_warp_idx() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
-// Chunk indices first, first + stride, ... of a persistent CTA as (problem row, chunk), stepped without divisions.
+// The work items of a persistent CTA: chunks first, first + stride, .. of the rows (problem rows; batch items when the
+// state is a grid of blocks), and for each of them its nsub blocks in order - one CTA walks all blocks of a chunk, so
+// that a thread meets its own results again when it sums over them.  Stepped without divisions.
 struct ItemWalk {
-  int bh, c;             // problem row, chunk
-  int step_bh, step_c, nc;
-  __device__ __forceinline__ ItemWalk(uint32_t first, uint32_t stride, int64_t nc_) {
+  int row, c, sub;       // row, chunk, block
+  int64_t unit;          // row * nc + c
+  int step_row, step_c, nc, nsub;
+  uint32_t stride;
+  __device__ __forceinline__ ItemWalk(uint32_t first, uint32_t stride_, int64_t nc_, int nsub_) {
     nc = (int)nc_;
-    bh = (int)(first / (uint32_t)nc);
-    c = (int)first - bh * nc;
-    step_bh = (int)(stride / (uint32_t)nc);
-    step_c = (int)stride - step_bh * nc;
+    nsub = nsub_;
+    stride = stride_;
+    unit = first;
+    sub = 0;
+    row = (int)(first / (uint32_t)nc);
+    c = (int)first - row * nc;
+    step_row = (int)(stride / (uint32_t)nc);
+    step_c = (int)stride - step_row * nc;
   }
   __device__ __forceinline__ void step() {
-    bh += step_bh;
+    if (++sub < nsub) return;
+    sub = 0;
+    unit += stride;
+    row += step_row;
     c += step_c;
     if (c >= nc) {
       c -= nc;
-      ++bh;
+      ++row;
     }
   }
-  // batch item and head of the problem row
-  __device__ __forceinline__ void row(int heads, int *b, int *h) const {
-    *b = heads == 1 ? bh : (int)((uint32_t)bh / (uint32_t)heads);
-    *h = heads == 1 ? 0 : bh - *b * heads;
+  // problem row, and the batch item and head (or block) that the tensors' windows are named by
+  __device__ __forceinline__ int bh() const { return nsub == 1 ? row : row * nsub + sub; }
+  __device__ __forceinline__ void item(int heads, int *b, int *h) const {
+    if (nsub != 1 || heads == 1) {
+      *b = row;
+      *h = sub;
+      return;
+    }
+    *b = (int)((uint32_t)row / (uint32_t)heads);
+    *h = row - *b * heads;
   }
 };
 

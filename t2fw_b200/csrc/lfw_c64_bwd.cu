@@ -83,13 +83,14 @@ constexpr int cS2 = 0, cR2 = 64, cVw = 128, cMw = 192;
 constexpr int cZ = 256, cT2 = 256, cTQ1 = 320, cTQ2 = 384, cT7 = 448;
 constexpr int kTmemCols = 512;
 
-// kFused = false: the plain operator (no activation flags, query scale 1), decided at compile time.
-template <typename T, bool kFused>
+// kMode: 0 the plain operator, 1 the fused layer, 2 a grid of blocks (gradients summed over the blocks of the other axis)
+template <typename T, int kMode>
 __global__ void __launch_bounds__(kThreadsB, 1)
 lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ state, const T *__restrict__ ckpt,
                    const float *__restrict__ Rend, const seq::Out<T> dx, const seq::Out<T> df, const seq::Out<T> dq,
                    const seq::Out<T> dk, const seq::Out<T> dfk, int *__restrict__ rowflag, int *__restrict__ status,
                    int64_t T_, int64_t nc, int64_t total) {
+  constexpr bool kFused = kMode == 1, kGrid = kMode == 2;
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);
   __shared__ __align__(8) uint64_t barRaw, barG, barZ, barM1, barM2;
@@ -119,7 +120,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   const float q_scale = kFused ? mp.q_scale : 1.f;
   auto issue_raw = [&](const ItemWalk &w) {     // thread 0 only: one copy per tensor
     int b, hc;
-    w.row(mp.heads, &b, &hc);
+    w.item(mp.heads, &b, &hc);
     const int row = (int)(b * T_ + w.c * kC);
     const int nv = (int)((T_ - (int64_t)w.c * kC < kC) ? T_ - (int64_t)w.c * kC : kC);
     const uint32_t per = (mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes;
@@ -132,17 +133,17 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   // The epilogue reads them, after the raw blocks have been handed to the next chunk.
   auto issue_preact = [&](const ItemWalk &w) {
     int b, hc;
-    w.row(mp.heads, &b, &hc);
+    w.item(mp.heads, &b, &hc);
     const int nv = (int)((T_ - (int64_t)w.c * kC < kC) ? T_ - (int64_t)w.c * kC : kC);
     acp::mbar_expect_tx(&barG, (mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
     seq::fetch_block<T>(mp, 4, sm + oRaw + kRawBytes, (int)(b * T_ + w.c * kC), hc, nv, &barG);
   };
   // start state (16-bit, 8 KB) and end state gradient (fp32, 16 KB) of a chunk into the padded
   // landing zones: three 16-byte asynchronous copies per thread
-  auto issue_state = [&](const ItemWalk &w, int64_t ci) {   // every thread
-    const T *s0p = (w.c == 0) ? state + (size_t)w.bh * kDim * kDim : ckpt + (size_t)(ci - 1) * kDim * kDim;
-    const float *rp = Rend + (size_t)ci * kDim * kDim;
-    cp_async16(sm + oS0L + (tid >> 3) * kS0Ld + (tid & 7) * 16, s0p + (tid >> 3) * kDim + (tid & 7) * 8);
+  auto issue_state = [&](const ItemWalk &w) {   // every thread
+    const T *s0p = (w.c == 0) ? state + seq::state_off(mp, w.row, w.sub, 0, 1) : ckpt + seq::state_off(mp, w.row, w.sub, w.c - 1, nc);
+    const float *rp = Rend + ((size_t)w.bh() * nc + w.c) * kDim * kDim;
+    cp_async16(sm + oS0L + (tid >> 3) * kS0Ld + (tid & 7) * 16, s0p + (size_t)(tid >> 3) * mp.state_ld + (tid & 7) * 8);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int c16 = tid + i * kThreadsB;
@@ -170,13 +171,13 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   const uint32_t tb = __shfl_sync(0xffffffffu, tmem_slot, 0);
   const uint32_t tl = umma::tmem_addr(tb, 32 * q4, 0);
   bool raw_pending = false, pre_pending = false;      // thread 0
-  ItemWalk wi(blockIdx.x, gridDim.x, nc), wn = wi;           // this chunk and the next one
-  if ((int64_t)blockIdx.x < total) {
+  ItemWalk wi(blockIdx.x, gridDim.x, nc, kGrid ? mp.nsub : 1), wn = wi;           // this chunk and the next one
+  if (wi.unit < total) {
     if (tid == 0) {
       issue_raw(wi);
       raw_pending = true;
     }
-    issue_state(wi, blockIdx.x);
+    issue_state(wi);
   }
   const uint32_t aT = umma::smem_u32(sm);
   // tile column offset of the own feature: row r of the swizzled tile adds r * 128 and XORs r % 8 into bits 4-6
@@ -194,22 +195,19 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   const T *vcol = raw + (h ? 0 : 3) * kC * kDim + t0 * kDim + feat;
 
   uint32_t it = 0;
-  for (int64_t ci = blockIdx.x; ci < total; ci += gridDim.x, ++it) {
+  for (; wn.unit < total; ++it) {
     wi = wn;
     wn.step();
     const int64_t t0c = (int64_t)wi.c * kC;
     const int nvalid = (int)((T_ - t0c < kC) ? T_ - t0c : kC);
-    // first row and column window of the chunk in the output arrays
-    const bool by_row = (mp.flags & seq::kOutByRow) != 0;
-    int64_t row0 = wi.bh;
-    int hcol = 0;
-    if (!by_row) {
-      int b, hh;
-      wi.row(mp.heads, &b, &hh);
-      row0 = b;
-      hcol = hh * kDim;
-    }
-    row0 = row0 * T_ + t0c;
+    // first row and column windows of the chunk in the output arrays
+    int ob, oh;
+    wi.item(mp.heads, &ob, &oh);
+    const int64_t row0 = (int64_t)ob * T_ + t0c;
+    // grid: block (i, j) holds d-side window i and k-side window j; `add`: not the first block of the sum over the other axis
+    const int gi = kGrid ? oh / mp.nk : 0, gj = kGrid ? oh - gi * mp.nk : 0;
+    const int hcol = (kGrid ? (h ? gi : gj) : oh) * kDim;
+    const bool add = kGrid && (h ? gj : gi) != 0;
     int &fix_n = fix_n2[it & 1], &s_bad = s_bad2[it & 1];
 
     if (!acp::mbar_wait(&barRaw, it & 1u)) s_fail = 1;
@@ -429,15 +427,15 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       }
       __syncwarp();
     }
-    if (ci + gridDim.x < total) {      // the next chunk's inputs and state blocks
+    if (wn.unit < total) {      // the next chunk's inputs and state blocks
       if (tid == 0) {
         issue_raw(wn);
         raw_pending = true;
       }
-      issue_state(wn, ci + gridDim.x);
+      issue_state(wn);
     }
     if (tid == 0) {
-      if (s_bad) atomicExch(rowflag + wi.bh, 1);      // the scan kernels redo this batch row
+      if (s_bad) atomicExch(rowflag + wi.row, 1);      // the scan kernels redo this row
       s_bad2[(it & 1) ^ 1] = 0;
       fix_n2[(it & 1) ^ 1] = 0;
     }
@@ -546,10 +544,10 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       }
       tot_a = run * up;
     }
-    // element pointers of step t0; one row pitch further per step.  The plain operator and the block-grid form
-    // write dense [rows][64] arrays.
+    // element pointers of step t0; one row pitch further per step.  The plain operator writes
+    // dense [rows][64] arrays.
     const seq::Out<T> &o_dv = h ? dx : dk, &o_gt = h ? df : dfk;
-    const int64_t ld_mu = kFused ? dq.ld : kDim, ld_dv = kFused ? o_dv.ld : kDim, ld_gt = kFused ? o_gt.ld : kDim;
+    const int64_t ld_mu = kMode ? dq.ld : kDim, ld_dv = kMode ? o_dv.ld : kDim, ld_gt = kMode ? o_gt.ld : kDim;
     T *p_mu = dq.p + (size_t)(row0 + t0) * dq.ld + dq.col + hcol + feat;
     T *p_dv = o_dv.p + (size_t)(row0 + t0) * o_dv.ld + o_dv.col + hcol + feat;
     const int n_own = nvalid - t0;      // valid own steps (may be negative)
@@ -574,6 +572,19 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
           sb[8 * half + j] = run_b;
         }
       }
+      // grid: this thread's own sums over the blocks before, as stored.  All loads of a batch before the first use or
+      // store, none behind a branch of its own: each would be a round trip to L2.
+      T old_mu[8] = {}, old_dv[8] = {};
+      if (kGrid && add && n_own > 0) {
+        const T *pm_old = h == 0 ? p_mu : p_dv;      // (the d side has no such result: any valid address)
+        const int64_t ld_old = h == 0 ? ld_mu : ld_dv;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int jj = 8 * half + j < n_own ? 8 * half + j : 0;
+          old_mu[j] = pm_old[jj * ld_old];
+          old_dv[j] = p_dv[jj * ld_dv];
+        }
+      }
       float tq1[8], t7[8];
       umma::tmem_ld8(tl + cTQ1 + t0 + 8 * half, tq1);
       umma::tmem_ld8(tl + cT7 + t0 + 8 * half, t7);
@@ -585,10 +596,16 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         const float dmu = pm[jj] * fmaf(up, tq1[j], tq2[j]), ddv = ip * fmaf(after, t7[j], t2[j]);
         pm[jj] = (jj > 0 ? pm[jj > 0 ? jj - 1 : 0] : pm_prev) * ip;      // from here on: 1 / gate of the step
         if (full || jj < n_own) {
-          if (h == 0) p_mu[jj * ld_mu] = (T)(kFused ? dmu * q_scale : dmu);
-          p_dv[jj * ld_dv] = (T)ddv;
+          if (h == 0) p_mu[jj * ld_mu] = (T)(kFused ? dmu * q_scale : kGrid ? dmu + Elem<T>::ld(&old_mu[j]) : dmu);
+          p_dv[jj * ld_dv] = (T)(kGrid ? ddv + Elem<T>::ld(&old_dv[j]) : ddv);
         }
       }
+    }
+    T *p_gt = o_gt.p == nullptr ? nullptr : o_gt.p + (size_t)(row0 + t0) * o_gt.ld + o_gt.col + hcol + feat;
+    T old_gt[16] = {};
+    if (kGrid && add && n_own > 0) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) old_gt[j] = p_gt[(j < n_own ? j : 0) * ld_gt];
     }
     {
       const int o = h * kDim + feat;
@@ -631,7 +648,6 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         if (tid == 0) pre_pending = false;
       }
       if (o_gt.p != nullptr) {
-        T *p_gt = o_gt.p + (size_t)(row0 + t0) * o_gt.ld + o_gt.col + hcol + feat;
         const T *pre = raw + kC * kDim + t0 * kDim + feat;     // fused layer: pre-activations
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -640,7 +656,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
             const float e = seq::exp_neg(Elem<T>::ld(pre + j * kDim)), sg = seq::rcp1p(e);
             dg *= sg > seq::kGateFloor ? sg * sg * e : 0.f;      // s (1 - s) = s^2 e^{-g}
           }
-          if (full || j < n_own) p_gt[j * ld_gt] = (T)dg;
+          if (full || j < n_own) p_gt[j * ld_gt] = (T)(kGrid ? dg + Elem<T>::ld(&old_gt[j]) : dg);
         }
       }
       __syncwarp();
@@ -670,7 +686,7 @@ int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ck
   int n_sm = 0;
   rc = lfw_chunk_sm_count(&n_sm);
   if (rc != T2FW_OK) return rc;
-  const int64_t nc = ceil_div64(T_, kC), total = BH * nc;
+  const int64_t nc = ceil_div64(T_, kC), total = BH / mp.nsub * nc;
   const unsigned grid = (unsigned)(total < n_sm ? total : n_sm);
 #define T2FW_OUT(TT, i) seq::Out<TT>{(TT *)outs[i], out_ld[i], out_col[i]}
 #define T2FW_LAUNCH(TT, FF)                                                                           \
@@ -683,11 +699,12 @@ int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ck
                                      total));                                                         \
   } while (0)
   const bool fused = (mp.flags & (seq::kUnitForget | seq::kSigmoidGate)) != 0 || mp.q_scale != 1.f;
-  if (dtype == T2FW_F16) {
-    if (fused) T2FW_LAUNCH(__half, true); else T2FW_LAUNCH(__half, false);
-  } else {
-    if (fused) T2FW_LAUNCH(__nv_bfloat16, true); else T2FW_LAUNCH(__nv_bfloat16, false);
-  }
+#define T2FW_MODES(TT)                                                                              \
+  do {                                                                                              \
+    if (mp.nsub > 1) T2FW_LAUNCH(TT, 2); else if (fused) T2FW_LAUNCH(TT, 1); else T2FW_LAUNCH(TT, 0); \
+  } while (0)
+  if (dtype == T2FW_F16) T2FW_MODES(__half); else T2FW_MODES(__nv_bfloat16);
+#undef T2FW_MODES
 #undef T2FW_LAUNCH
 #undef T2FW_OUT
   T2FW_CHECK_LAUNCH(1);

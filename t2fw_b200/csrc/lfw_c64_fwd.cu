@@ -54,11 +54,13 @@ static_assert(kSmemF + 256 <= 227 * 1024, "shared memory limit");
 constexpr int cS2 = 0, cX = 64, cP = 128, cO1 = 192, cO2 = 256;
 constexpr int kTmemColsF = 512;
 
-template <typename T, bool kFused>
+// kMode: 0 the plain operator, 1 the fused layer, 2 a grid of blocks (outputs summed over the blocks of a row)
+template <typename T, int kMode>
 __global__ void __launch_bounds__(kThreadsF, 1)
 lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ state, const T *__restrict__ ckpt,
                    const seq::Out<T> out, int *__restrict__ rowflag, int *__restrict__ status, int64_t T_,
                    int64_t nc, int64_t total) {
+  constexpr bool kFused = kMode == 1, kGrid = kMode == 2;
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);   // swizzle atoms are 1024-byte aligned
   __shared__ __align__(8) uint64_t barG, barV, barP, barO;
@@ -76,29 +78,29 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   const bool unit_forget = kFused && (mp.flags & seq::kUnitForget) != 0;
   const bool sigmoid_gate = kFused && (mp.flags & seq::kSigmoidGate) != 0;
   const float q_scale = kFused ? mp.q_scale : 1.f;
-  auto valid_steps = [&](const ItemWalk &w, int64_t ci) {
-    if (ci >= total) return 0;
+  auto valid_steps = [&](const ItemWalk &w) {
+    if (w.unit >= total) return 0;
     const int64_t left = T_ - (int64_t)w.c * kC;
     return (int)(left < kC ? left : kC);
   };
   // Two groups with a barrier each: the gate blocks (f, fk) are free again after the products of the quarters, the value
   // blocks (x, q, k) only once the operands are built, so the next pair's gates are requested that much earlier.
-  auto issue_raw = [&](const ItemWalk *w, int64_t ci, bool gates) {     // thread 0 only: one copy per tensor and chunk
+  auto issue_raw = [&](const ItemWalk *w, bool gates) {     // thread 0 only: one copy per tensor and chunk
     const uint32_t n = gates ? (unit_forget ? 1u : 2u) : 3u;
     uint64_t *bar = gates ? &barG : &barV;
     uint32_t bytes = 0;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int nv = valid_steps(w[e], ci + e);
+      const int nv = valid_steps(w[e]);
       if (nv > 0) bytes += n * ((mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
     }
     acp::mbar_expect_tx(bar, bytes);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int nv = valid_steps(w[e], ci + e);
+      const int nv = valid_steps(w[e]);
       if (nv <= 0) continue;
       int b, hc;
-      w[e].row(mp.heads, &b, &hc);
+      w[e].item(mp.heads, &b, &hc);
       const int row = (int)(b * T_ + w[e].c * kC);
 #pragma unroll
       for (int i = 0; i < 5; ++i)
@@ -108,12 +110,13 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   };
   // start states of the pair (the caller's state for the first chunk of a row, else the checkpoint written
   // by the carry): one 16-byte asynchronous copy per thread and chunk into the padded landing zones
-  auto issue_state = [&](const ItemWalk *w, int64_t ci) {   // every thread
+  auto issue_state = [&](const ItemWalk *w) {   // every thread
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      if (ci + e >= total) continue;
-      const T *s0p = (w[e].c == 0) ? state + (size_t)w[e].bh * kDim * kDim : ckpt + (size_t)(ci + e - 1) * kDim * kDim;
-      cp_async16(sm + oS0L + e * kDim * kS0Ld + (tid >> 3) * kS0Ld + (tid & 7) * 16, s0p + (tid >> 3) * kDim + (tid & 7) * 8);
+      if (w[e].unit >= total) continue;
+      const T *s0p = (w[e].c == 0) ? state + seq::state_off(mp, w[e].row, w[e].sub, 0, 1)
+                                   : ckpt + seq::state_off(mp, w[e].row, w[e].sub, w[e].c - 1, nc);
+      cp_async16(sm + oS0L + e * kDim * kS0Ld + (tid >> 3) * kS0Ld + (tid & 7) * 16, s0p + (size_t)(tid >> 3) * mp.state_ld + (tid & 7) * 8);
     }
     cp_async_commit();
   };
@@ -132,15 +135,16 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   dependency_wait();
   const uint32_t tb = __shfl_sync(0xffffffffu, tmem_slot, 0);
   const uint32_t tl = umma::tmem_addr(tb, 32 * q4, 0);
-  ItemWalk wn[2] = {ItemWalk(2 * blockIdx.x, 2 * gridDim.x, nc), ItemWalk(2 * blockIdx.x + 1, 2 * gridDim.x, nc)};
+  const int nsub = kGrid ? mp.nsub : 1;
+  ItemWalk wn[2] = {ItemWalk(2 * blockIdx.x, 2 * gridDim.x, nc, nsub), ItemWalk(2 * blockIdx.x + 1, 2 * gridDim.x, nc, nsub)};
   uint32_t n_issued[2] = {0u, 0u}, n_landed[2] = {0u, 0u};      // thread 0: bulk-copy rounds of the gates and of the values
   if (2 * (int64_t)blockIdx.x < total) {
     if (tid == 0) {
-      issue_raw(wn, 2 * (int64_t)blockIdx.x, true);
-      issue_raw(wn, 2 * (int64_t)blockIdx.x, false);
+      issue_raw(wn, true);
+      issue_raw(wn, false);
       n_issued[0] = n_issued[1] = 1u;
     }
-    issue_state(wn, 2 * (int64_t)blockIdx.x);
+    issue_state(wn);
   }
   const uint32_t aT = umma::smem_u32(sm + oT);
   // tile column offset of the own feature: row r of the swizzled tile adds r * 128 and XORs r % 8 into bits 4-6
@@ -154,11 +158,11 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   auto rawv = [&](int blk, int j) { return Elem<T>::ld(raw + blk * kC * kDim + j * kDim); };
 
   uint32_t it = 0;
-  for (int64_t ci = 2 * (int64_t)blockIdx.x; ci < total; ci += 2 * (int64_t)gridDim.x, ++it) {
+  for (; wn[0].unit < total; ++it) {
     const ItemWalk w0 = wn[0], w1 = wn[1];
     wn[0].step();
     wn[1].step();
-    const int nv0 = valid_steps(w0, ci), nv1 = valid_steps(w1, ci + 1);
+    const int nv0 = valid_steps(w0), nv1 = valid_steps(w1);
     const int nvalid = h ? nv1 : nv0;
     const bool partial = nv0 < kC || nv1 < kC;      // steps beyond the valid ones become identity steps
     int *s_bad = s_bad2[it & 1];
@@ -199,8 +203,8 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     qtot[(4 + tq) * kDim + feat] = pd;
     __syncthreads();           // also: the start states of both chunks have landed
     if (s_fail) break;
-    if (tid == 0 && ci + 2 * (int64_t)gridDim.x < total) {
-      issue_raw(wn, ci + 2 * (int64_t)gridDim.x, true);
+    if (tid == 0 && wn[0].unit < total) {
+      issue_raw(wn, true);
       ++n_issued[0];
     }
     if (acp::mbar_wait(&barV, it & 1u)) ++n_landed[1];
@@ -334,16 +338,16 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       }
       __syncwarp();
     }
-    if (ci + 2 * (int64_t)gridDim.x < total) {
+    if (wn[0].unit < total) {
       if (tid == 0) {
-        issue_raw(wn, ci + 2 * (int64_t)gridDim.x, false);
+        issue_raw(wn, false);
         ++n_issued[1];
       }
-      issue_state(wn, ci + 2 * (int64_t)gridDim.x);
+      issue_state(wn);
     }
     if (tid == 0) {
-      if (s_bad[0]) atomicExch(rowflag + w0.bh, 1);      // the scan kernel redoes these batch rows
-      if (s_bad[1] && nv1 > 0) atomicExch(rowflag + w1.bh, 1);
+      if (s_bad[0]) atomicExch(rowflag + w0.row, 1);      // the scan kernel redoes these rows
+      if (s_bad[1] && nv1 > 0) atomicExch(rowflag + w1.row, 1);
       s_bad2[(it & 1) ^ 1][0] = s_bad2[(it & 1) ^ 1][1] = 0;
     }
 
@@ -386,12 +390,10 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       __syncwarp();
     }
     // first row and column window of the own chunk in the output array; 16 features of one step are 32 contiguous bytes
-    int b = h ? w1.bh : w0.bh, hcol = 0;
-    if (!(mp.flags & seq::kOutByRow)) {
-      int hh;
-      (h ? w1 : w0).row(mp.heads, &b, &hh);
-      hcol = hh * kDim;
-    }
+    int b, hcol;
+    (h ? w1 : w0).item(mp.heads, &b, &hcol);
+    const bool add = kGrid && hcol % mp.nk != 0;      // not the first block of its row of blocks
+    hcol = (kGrid ? hcol / mp.nk : hcol) * kDim;
     T *po = out.p + ((size_t)b * T_ + (size_t)(h ? w1.c : w0.c) * kC + t0) * out.ld + out.col + hcol + feat;
     if (!umma::mbar_wait(&barO, it & 1u)) s_fail = 1;
     umma::fence_after_sync();
@@ -399,8 +401,17 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     umma::tmem_ld16(tl + cO1 + t0, o1);
     umma::tmem_ld16(tl + cO2 + t0, o2);
     umma::tmem_ld_wait();
-    const int64_t ld = kFused ? out.ld : kDim;
-    if (!partial) {
+    const int64_t ld = kMode ? out.ld : kDim;
+    if (kGrid && add) {      // this thread's own sum over the blocks before
+      T old[16] = {};
+      if (t0 < nvalid) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) old[j] = po[(t0 + j < nvalid ? j : 0) * ld];
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (t0 + j < nvalid) po[j * ld] = (T)fmaf(gd[j], fmaf(up, o1[j], o2[j]), Elem<T>::ld(&old[j]));
+    } else if (!partial) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) po[j * ld] = (T)(gd[j] * fmaf(up, o1[j], o2[j]));
     } else {
@@ -436,7 +447,7 @@ int lfw_c64_forward_out(const seq::Maps &mp, const void *state, const void *ckpt
   int n_sm = 0;
   rc = lfw_chunk_sm_count(&n_sm);
   if (rc != T2FW_OK) return rc;
-  const int64_t nc = ceil_div64(T_, kC), total = BH * nc;
+  const int64_t nc = ceil_div64(T_, kC), total = BH / mp.nsub * nc;
   const int64_t pairs = (total + 1) / 2;
   const unsigned grid = (unsigned)(pairs < n_sm ? pairs : n_sm);
 #define T2FW_LAUNCH(TT, FF)                                                                              \
@@ -448,11 +459,12 @@ int lfw_c64_forward_out(const seq::Maps &mp, const void *state, const void *ckpt
                                      rowflag, status, T_, nc, total));                               \
   } while (0)
   const bool fused = (mp.flags & (seq::kUnitForget | seq::kSigmoidGate)) != 0 || mp.q_scale != 1.f;
-  if (dtype == T2FW_F16) {
-    if (fused) T2FW_LAUNCH(__half, true); else T2FW_LAUNCH(__half, false);
-  } else {
-    if (fused) T2FW_LAUNCH(__nv_bfloat16, true); else T2FW_LAUNCH(__nv_bfloat16, false);
-  }
+#define T2FW_MODES(TT)                                                                              \
+  do {                                                                                              \
+    if (mp.nsub > 1) T2FW_LAUNCH(TT, 2); else if (fused) T2FW_LAUNCH(TT, 1); else T2FW_LAUNCH(TT, 0); \
+  } while (0)
+  if (dtype == T2FW_F16) T2FW_MODES(__half); else T2FW_MODES(__nv_bfloat16);
+#undef T2FW_MODES
 #undef T2FW_LAUNCH
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;

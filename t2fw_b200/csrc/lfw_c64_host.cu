@@ -13,8 +13,15 @@
 //      stored in place of G_c (fp32); what is left after chunk 0 is d_state
 //   3. lfw_c64_bwd_kernel               per (row, chunk): d_x, d_f, d_q, d_k, d_f_key
 // Scratch (floats): M[B][nc][64][64] | Ac[B][nc][64] | Gc[B][nc][64] | flags[B][nc] (int) |
-// rowflag[B] (int).  A flagged batch row (gate products outside the range of the factored form) is
-// recomputed by the scan kernels afterwards.
+// rowflag[B] (int).  A flagged row (gate products outside the range of the factored form) is recomputed by the
+// scan kernels afterwards.
+// States larger than 64 x 64 (D, K multiples of 64): the recurrence never mixes state rows or columns, so a D x K state
+// is a (D/64) x (K/64) grid of independent blocks, problem rows of their own for the kernels (B above counts them);
+// block (i, j) reads the d-side vectors' window i and the k-side vectors' window j in place, states and checkpoints are
+// read and written in place too, and what leaves the state is summed over the other axis' blocks by the output and
+// gradient kernels, whose CTAs walk all blocks of a chunk: a thread adds to what it wrote itself (per-block results and
+// separate summing and re-layout passes took 0.4 of 2.4 ms at B = 16, T = 16384, D = K = 128).  Flags are then per
+// batch item.
 #include "lfw_c64.cuh"
 #include "seq_layout.cuh"
 
@@ -22,8 +29,8 @@ namespace t2fw {
 
 using namespace c64;
 
-int lfw_chunk_local_umma(bool backward, const seq::Maps &mp, float *M, float *Ac, float *Gc, int *flags, int64_t BH,
-                         int64_t T_, int dtype, cudaStream_t st);
+int lfw_chunk_local_umma(bool backward, const seq::Maps &mp, float *M, float *Ac, float *Gc, int *flags, int *rowflag,
+                         int64_t BH, int64_t T_, int dtype, cudaStream_t st);
 int lfw_c64_forward_out(const seq::Maps &mp, const void *state, const void *ckpt, void *out, int64_t out_ld,
                         int out_col, int *rowflag, int64_t BH, int64_t T_, int dtype, cudaStream_t st);
 int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ckpt, const float *Rend,
@@ -93,6 +100,12 @@ template <> struct Quad<__nv_bfloat16> {
   }
 };
 
+// States of the call: one 64 x 64 block per problem row (nsub = 1), or a grid of nsub blocks per item
+struct Grid2D {
+  int nsub, nk;
+  int item, ld;          // elements of a state, row stride
+};
+
 // One thread per (row, d, four consecutive k); a block covers 16 state rows of one batch row.  The
 // recurrence over the chunks is a dependent chain, so the loads of up to 16 chunks are all issued
 // before the chain starts (one round of memory latency per 16 chunks); the decay vectors of those
@@ -104,7 +117,7 @@ template <typename T, bool kFwd>
 __global__ void __launch_bounds__(kCarryThreads, 3)
 lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const float *__restrict__ Ac,
                      const float *__restrict__ Gc, const int *__restrict__ flags, int *__restrict__ rowflag,
-                     int keep_rowflag, T *__restrict__ out, int64_t B, int64_t nc) {
+                     T *__restrict__ out, const Grid2D gr, int64_t nc) {
   __shared__ float a_s[kBatch][kCarryRows];
   __shared__ __align__(16) float g_s[kBatch][kDim];
   const int tid = threadIdx.x;
@@ -112,47 +125,53 @@ lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const fl
   const int64_t b = blockIdx.x / (kDim / kCarryRows);
   const int d0 = (int)(blockIdx.x % (kDim / kCarryRows)) * kCarryRows;
   const int dl = tid / (kDim / 4), d = d0 + dl, k0 = (tid % (kDim / 4)) * 4;
+  // where this block of the states lies: item, offset inside one state, row stride
+  const int item = gr.nsub == 1 ? (int)b : (int)b / gr.nsub, sub = (int)b - item * gr.nsub;
+  const int in_state = (sub / gr.nk * kDim + d) * gr.ld + sub % gr.nk * kDim + k0, whole = gr.item;
   // init may be null: the carry then starts from zero (the summary of a sequence segment)
-  float4 S = init != nullptr ? Quad<T>::ld(init + ((size_t)b * kDim + d) * kDim + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 S = init != nullptr ? Quad<T>::ld(init + (size_t)item * whole + in_state) : make_float4(0.f, 0.f, 0.f, 0.f);
   int any = 0;
-  for (int64_t c0 = 0; c0 < nc; c0 += kBatch) {
+  const int n = (int)nc;
+  T *op = out + (size_t)item * (kFwd ? nc : 1) * whole + in_state;      // forward: the block's next checkpoint
+  // this thread's four values of the first chunk of the walk; one chunk further along it per step
+  float *mp = M + (((size_t)b * nc + (kFwd ? 0 : nc - 1)) * kDim + d) * kDim + k0;
+  constexpr int kNext = (kFwd ? 1 : -1) * kDim * kDim;
+  const float *ac = Ac + (size_t)b * nc * kDim + d0, *gc = Gc + (size_t)b * nc * kDim;
+  for (int c0 = 0; c0 < n; c0 += kBatch) {
     float4 l[kBatch];
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      int64_t c = c0 + j < nc ? c0 + j : nc - 1;
-      if (!kFwd) c = nc - 1 - c;
-      l[j] = *reinterpret_cast<const float4 *>(M + (((size_t)b * nc + c) * kDim + d) * kDim + k0);
-    }
+    for (int j = 0; j < kBatch; ++j)
+      l[j] = *reinterpret_cast<const float4 *>(mp + (c0 + j < n ? j : 0) * kNext);
     __syncthreads();      // the previous batch's decay vectors are no longer read
     for (int i = tid; i < kBatch * (kCarryRows + kDim); i += kCarryThreads) {
       const int j = i / (kCarryRows + kDim), r = i % (kCarryRows + kDim);
-      int64_t c = c0 + j < nc ? c0 + j : nc - 1;
-      if (!kFwd) c = nc - 1 - c;
-      const size_t bc = (size_t)b * nc + c;
-      if (r < kCarryRows) a_s[j][r] = Ac[bc * kDim + d0 + r];
-      else g_s[j][r - kCarryRows] = Gc[bc * kDim + r - kCarryRows];
+      int c = c0 + j < n ? c0 + j : n - 1;
+      if (!kFwd) c = n - 1 - c;
+      if (r < kCarryRows) a_s[j][r] = ac[c * kDim + r];
+      else g_s[j][r - kCarryRows] = gc[c * kDim + r - kCarryRows];
     }
-    if (tid == 0 && d0 == 0)
-      for (int j = 0; j < kBatch && c0 + j < nc; ++j) any |= flags[(size_t)b * nc + c0 + j];
+    if (d0 == 0 && tid < kBatch && c0 + tid < n) any |= flags[(size_t)b * nc + c0 + tid];
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
-      if (c0 + j < nc) {
-        const int64_t c = kFwd ? c0 + j : nc - 1 - (c0 + j);
-        const size_t off = (((size_t)b * nc + c) * kDim + d) * kDim + k0;
-        if (!kFwd) *reinterpret_cast<float4 *>(M + off) = S;
+      if (c0 + j < n) {
+        if (!kFwd) *reinterpret_cast<float4 *>(mp) = S;
         const float a = a_s[j][dl];
         const float4 g = *reinterpret_cast<const float4 *>(&g_s[j][k0]);
         S.x = a * g.x * S.x + l[j].x;
         S.y = a * g.y * S.y + l[j].y;
         S.z = a * g.z * S.z + l[j].z;
         S.w = a * g.w * S.w + l[j].w;
-        if (kFwd) Quad<T>::st(out + off, S);
+        if (kFwd) {
+          Quad<T>::st(op, S);
+          op += whole;
+        }
+        mp += kNext;
       }
     }
   }
-  if (!kFwd) Quad<T>::st(out + ((size_t)b * kDim + d) * kDim + k0, S);
-  if (tid == 0 && d0 == 0) rowflag[b] = keep_rowflag ? (rowflag[b] | any) : any;
+  if (!kFwd) Quad<T>::st(op, S);
+  if (any) atomicExch(rowflag + item, 1);
 }
 
 // Checkpoint interval of m chunks: slot j of the caller's checkpoints = state after chunk
@@ -160,8 +179,7 @@ lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const fl
 template <typename T>
 __global__ void __launch_bounds__(256)
 lfw_c64_pick_ckpt_kernel(const T *__restrict__ all, T *__restrict__ ckpt, int64_t B, int64_t nc, int64_t m,
-                         int64_t slots) {
-  constexpr int kVec = kDim * kDim / 8;      // 16-byte pieces of one state
+                         int64_t slots, int64_t kVec) {      // kVec: 16-byte pieces of one state
   const int64_t n = B * slots * kVec;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t v = i % kVec, j = (i / kVec) % slots, b = i / (kVec * slots);
@@ -218,7 +236,11 @@ struct Call {
   int64_t B, T_;        // batch items, steps;  problem rows BH = B * heads
   int heads, flags;
   float q_scale;
+  Grid2D grid{1, 1, kDim * kDim, kDim};
 };
+void set_grid(seq::Maps &mp, const Grid2D &g) {
+  mp.nsub = g.nsub; mp.nk = g.nk; mp.state_item = g.item; mp.state_ld = (int)g.ld;
+}
 
 // The states after every chunk (16-bit) from the caller's state: local kernel + carry.
 template <typename T>
@@ -228,11 +250,12 @@ int chunk_states(const Call &c, const Scratch &s, const void *state, T *ck_all, 
   const Tensor2D loc[4] = {c.x, c.f, c.k, c.fk};
   int rc = build_maps(mp, loc, 4, rows, c.heads, c.flags, 1.f);
   if (rc != T2FW_OK) return rc;
-  rc = lfw_chunk_local_umma(false, mp, s.M, s.Ac, s.Gc, s.flags, BH, c.T_, dtype, st);
+  set_grid(mp, c.grid);
+  rc = lfw_chunk_local_umma(false, mp, s.M, s.Ac, s.Gc, s.flags, s.rowflag, BH, c.T_, dtype, st);
   if (rc != T2FW_OK) return rc;
   T2FW_CHECK_CUDA(launch_dependent(lfw_c64_carry_kernel<T, true>, dim3((unsigned)(BH * (kDim / kCarryRows))),
                                    dim3(kCarryThreads), 0, st, (const T *)state, s.M, (const float *)s.Ac,
-                                   (const float *)s.Gc, (const int *)s.flags, s.rowflag, 0, ck_all, BH, nc));
+                                   (const float *)s.Gc, (const int *)s.flags, s.rowflag, ck_all, c.grid, nc));
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;
 }
@@ -251,12 +274,13 @@ int forward_typed(const Call &c, const void *state, void *out, int64_t out_ld, i
   const Tensor2D all[5] = {c.x, c.f, c.q, c.k, c.fk};
   rc = build_maps(mp, all, 5, rows, c.heads, c.flags, c.q_scale);
   if (rc != T2FW_OK) return rc;
+  set_grid(mp, c.grid);
   rc = lfw_c64_forward_out(mp, state, ck_all, out, out_ld, out_col, s.rowflag, BH, c.T_, dtype, st);
   if (rc != T2FW_OK || m == 1) return rc;
-  const int64_t slots = ceil_div64(c.T_, ckpt_every), n = BH * slots * (kDim * kDim / 8);
+  const int64_t items = BH / c.grid.nsub, slots = ceil_div64(c.T_, ckpt_every), n = items * slots * (c.grid.item / 8);
   const int64_t blocks = ceil_div64(n, 256);
   lfw_c64_pick_ckpt_kernel<T><<<(unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, st>>>(
-      ck_all, (T *)ckpt, BH, nc, m, slots);
+      ck_all, (T *)ckpt, items, nc, m, slots, c.grid.item / 8);
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;
 }
@@ -278,16 +302,18 @@ int backward_typed(const Call &c, const void *gs, const void *state, const void 
   const Tensor2D loc[4] = {c.go, c.f, c.q, c.fk};
   int rc = build_maps(mp, loc, 4, rows, c.heads, c.flags, c.q_scale);
   if (rc != T2FW_OK) return rc;
-  rc = lfw_chunk_local_umma(true, mp, s.M, s.Ac, s.Gc, s.flags, BH, c.T_, dtype, st);
+  set_grid(mp, c.grid);
+  rc = lfw_chunk_local_umma(true, mp, s.M, s.Ac, s.Gc, s.flags, m > 1 ? nullptr : s.rowflag, BH, c.T_, dtype, st);
   if (rc != T2FW_OK) return rc;
   T2FW_CHECK_CUDA(launch_dependent(lfw_c64_carry_kernel<T, false>, dim3((unsigned)(BH * (kDim / kCarryRows))),
                                    dim3(kCarryThreads), 0, st, (const T *)gs, s.M, (const float *)s.Ac,
-                                   (const float *)s.Gc, (const int *)s.flags, s.rowflag, m > 1 ? 1 : 0, (T *)ds, BH,
+                                   (const float *)s.Gc, (const int *)s.flags, s.rowflag, (T *)ds, c.grid,
                                    nc));
   T2FW_CHECK_LAUNCH(1);
   const Tensor2D all[6] = {c.x, c.f, c.q, c.k, c.fk, c.go};
   rc = build_maps(mp, all, 6, rows, c.heads, c.flags, c.q_scale);
   if (rc != T2FW_OK) return rc;
+  set_grid(mp, c.grid);
   return lfw_c64_backward_main(mp, state, ckpt, s.M, outs, out_ld, out_col, s.rowflag, BH, c.T_, dtype, st);
 }
 
@@ -300,16 +326,16 @@ Call plain_call(const void *x, const void *f, const void *q, const void *k, cons
   return c;
 }
 
-// A D x K state cut into (D/64) x (K/64) blocks: sub-item h = i * nk + j of a batch item is block
-// (i, j); the d-side tensors [B*T][D] are read at window i, the k-side tensors [B*T][K] at window j,
-// and every sub-item writes its own [T][64] result arrays (summed over the other index afterwards).
+// A D x K state cut into (D/64) x (K/64) blocks: sub-item h = i * nk + j of a batch item is block (i, j); the d-side
+// tensors [B*T][D] are read at window i, the k-side tensors [B*T][K] at window j.
 Call grid_call(const void *x, const void *f, const void *q, const void *k, const void *fk, const void *go, int64_t B,
                int64_t T_, int nd, int nk) {
   const int64_t D = (int64_t)nd * kDim, K = (int64_t)nk * kDim;
   Call c;
   c.x = {x, D, 0, nk, nd}; c.f = {f, D, 0, nk, nd}; c.go = {go, D, 0, nk, nd};
   c.q = {q, K, 0, 1, nk}; c.k = {k, K, 0, 1, nk}; c.fk = {fk, K, 0, 1, nk};
-  c.B = B; c.T_ = T_; c.heads = nd * nk; c.flags = seq::kOutByRow; c.q_scale = 1.f;
+  c.B = B; c.T_ = T_; c.heads = nd * nk; c.flags = 0; c.q_scale = 1.f;
+  c.grid = {nd * nk, nk, (int)(D * K), (int)K};
   return c;
 }
 
@@ -365,35 +391,38 @@ int lfw_chunk_backward(const void *go, const void *gs, const void *x, const void
   return backward_typed<__nv_bfloat16>(c, gs, state, ckpt, outs, ld, col, ds, dtype, ckpt_every, scratch, st);
 }
 
-// ---- block-grid form: inputs dense [B*T][D] / [B*T][K], states, checkpoints and results per block ----
-int lfw_chunk_forward_grid(const void *x, const void *f, const void *q, const void *k, const void *fk,
-                           const void *state_blocks, void *out_blocks, void *ckpt_blocks, int64_t B, int64_t T_,
-                           int nd, int nk, int dtype, int64_t ckpt_every, void *scratch, cudaStream_t st,
-                           const int **rowflag_out) {
-  const int64_t VB = B * nd * nk;
-  if (rowflag_out) *rowflag_out = carve(scratch, VB, ceil_div64(T_, kC)).rowflag;
-  const Call c = grid_call(x, f, q, k, fk, nullptr, B, T_, nd, nk);
-  if (dtype == T2FW_F16)
-    return forward_typed<__half>(c, state_blocks, out_blocks, kDim, 0, ckpt_blocks, dtype, ckpt_every, scratch, st);
-  return forward_typed<__nv_bfloat16>(c, state_blocks, out_blocks, kDim, 0, ckpt_blocks, dtype, ckpt_every, scratch, st);
+// ---- states that are grids of 64 x 64 blocks; all arrays dense, rowflag per batch item ----------------
+bool lfw_grid_supported(int64_t D, int64_t K, int dtype, int64_t ckpt_every) {
+  return (dtype == T2FW_F16 || dtype == T2FW_BF16) && ckpt_every >= kC && ckpt_every % kC == 0 && D % kDim == 0 && K % kDim == 0 &&
+         D <= 256 && K <= 256 && (D > kDim || K > kDim);
 }
 
-int lfw_chunk_backward_grid(const void *go, const void *gs_blocks, const void *x, const void *f, const void *q,
-                            const void *k, const void *fk, const void *state_blocks, const void *ckpt_blocks,
-                            void *dx, void *df, void *dq, void *dk, void *dfk, void *ds_blocks, int64_t B, int64_t T_,
-                            int nd, int nk, int dtype, int64_t ckpt_every, void *scratch, cudaStream_t st,
-                            const int **rowflag_out) {
-  const int64_t VB = B * nd * nk;
-  if (rowflag_out) *rowflag_out = carve(scratch, VB, ceil_div64(T_, kC)).rowflag;
+size_t lfw_grid_scratch_bytes(int64_t B, int64_t T_, int64_t D, int64_t K, int64_t ckpt_every) {
+  return scratch_bytes(B * (D / kDim) * (K / kDim), ceil_div64(T_, kC), ckpt_every);
+}
+
+int lfw_grid_forward(const void *x, const void *f, const void *q, const void *k, const void *fk, const void *state, void *out,
+                     void *ckpt, int64_t B, int64_t T_, int64_t D, int64_t K, int dtype, int64_t ckpt_every, void *scratch,
+                     cudaStream_t st, const int **rowflag_out) {
+  const int nd = (int)(D / kDim), nk = (int)(K / kDim);
+  *rowflag_out = carve(scratch, B * nd * nk, ceil_div64(T_, kC)).rowflag;
+  const Call c = grid_call(x, f, q, k, fk, nullptr, B, T_, nd, nk);
+  if (dtype == T2FW_F16) return forward_typed<__half>(c, state, out, D, 0, ckpt, dtype, ckpt_every, scratch, st);
+  return forward_typed<__nv_bfloat16>(c, state, out, D, 0, ckpt, dtype, ckpt_every, scratch, st);
+}
+
+int lfw_grid_backward(const void *go, const void *gs, const void *x, const void *f, const void *q, const void *k, const void *fk,
+                      const void *state, const void *ckpt, void *dx, void *df, void *dq, void *dk, void *dfk, void *ds, int64_t B,
+                      int64_t T_, int64_t D, int64_t K, int dtype, int64_t ckpt_every, void *scratch, cudaStream_t st,
+                      const int **rowflag_out) {
+  const int nd = (int)(D / kDim), nk = (int)(K / kDim);
+  *rowflag_out = carve(scratch, B * nd * nk, ceil_div64(T_, kC)).rowflag;
   const Call c = grid_call(x, f, q, k, fk, go, B, T_, nd, nk);
   void *const outs[5] = {dx, df, dq, dk, dfk};
-  const int64_t ld[5] = {kDim, kDim, kDim, kDim, kDim};
+  const int64_t ld[5] = {D, D, K, K, K};
   const int col[5] = {0, 0, 0, 0, 0};
-  if (dtype == T2FW_F16)
-    return backward_typed<__half>(c, gs_blocks, state_blocks, ckpt_blocks, outs, ld, col, ds_blocks, dtype, ckpt_every,
-                                  scratch, st);
-  return backward_typed<__nv_bfloat16>(c, gs_blocks, state_blocks, ckpt_blocks, outs, ld, col, ds_blocks, dtype,
-                                       ckpt_every, scratch, st);
+  if (dtype == T2FW_F16) return backward_typed<__half>(c, gs, state, ckpt, outs, ld, col, ds, dtype, ckpt_every, scratch, st);
+  return backward_typed<__nv_bfloat16>(c, gs, state, ckpt, outs, ld, col, ds, dtype, ckpt_every, scratch, st);
 }
 
 // ---- summary of a sequence segment (for splitting the time axis over devices) ------------------
@@ -424,19 +453,21 @@ int summary_typed(bool backward, const void *val_d, const void *gate_d, const vo
   const Tensor2D loc[4] = {{val_d, kDim, 0}, {gate_d, kDim, 0}, {val_k, kDim, 0}, {gate_k, kDim, 0}};
   int rc = build_maps(mp, loc, 4, rows, 1, 0, 1.f);
   if (rc != T2FW_OK) return rc;
-  rc = lfw_chunk_local_umma(backward, mp, s.M, s.Ac, s.Gc, s.flags, B, T_, dtype, st);
+  const Grid2D one{1, 1, kDim * kDim, kDim};
+  set_grid(mp, one);
+  rc = lfw_chunk_local_umma(backward, mp, s.M, s.Ac, s.Gc, s.flags, s.rowflag, B, T_, dtype, st);
   if (rc != T2FW_OK) return rc;
   const dim3 grid((unsigned)(B * (kDim / kCarryRows)));
   if (backward) {      // the state gradient at the segment start that the segment's own output gradients cause
     T2FW_CHECK_CUDA(launch_dependent(lfw_c64_carry_kernel<T, false>, grid, dim3(kCarryThreads), 0, st, (const T *)nullptr,
-                                     s.M, (const float *)s.Ac, (const float *)s.Gc, (const int *)s.flags, s.rowflag, 0,
-                                     (T *)end_state, B, nc));
+                                     s.M, (const float *)s.Ac, (const float *)s.Gc, (const int *)s.flags, s.rowflag,
+                                     (T *)end_state, one, nc));
   } else {             // the state at the segment end that the segment's own inputs cause
     T2FW_CHECK_CUDA(launch_dependent(lfw_c64_carry_kernel<T, true>, grid, dim3(kCarryThreads), 0, st, (const T *)nullptr,
-                                     s.M, (const float *)s.Ac, (const float *)s.Gc, (const int *)s.flags, s.rowflag, 0,
-                                     (T *)s.ck_all, B, nc));
+                                     s.M, (const float *)s.Ac, (const float *)s.Gc, (const int *)s.flags, s.rowflag,
+                                     (T *)s.ck_all, one, nc));
     lfw_c64_pick_ckpt_kernel<T><<<(unsigned)ceil_div64(B * (kDim * kDim / 8), 256), 256, 0, st>>>(
-        (const T *)s.ck_all, (T *)end_state, B, nc, nc, 1);
+        (const T *)s.ck_all, (T *)end_state, B, nc, nc, 1, (int64_t)(kDim * kDim / 8));
   }
   lfw_c64_decay_totals_kernel<<<(unsigned)ceil_div64(B * 2 * kDim, 128), 128, 0, st>>>(s.Ac, s.Gc, s.rowflag, A_out,
                                                                                      G_out, B, nc);

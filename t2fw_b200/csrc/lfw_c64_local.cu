@@ -51,8 +51,8 @@ constexpr int kTmemColsL = 128;
 template <typename T, bool kSuffix, bool kFused>
 __global__ void __launch_bounds__(kThreadsL, kCtasPerSmL)
 lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M, float *__restrict__ Ac,
-                     float *__restrict__ Gc, int *__restrict__ flags, int *__restrict__ status, int64_t T_,
-                     int64_t nc, int64_t total) {
+                     float *__restrict__ Gc, int *__restrict__ flags, int *__restrict__ rowflag, int items,
+                     int *__restrict__ status, int64_t T_, int64_t nc, int64_t total) {
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);
   __shared__ __align__(8) uint64_t barRaw, barM;
@@ -88,7 +88,7 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
       const int nv = valid_steps(w[e], ci + e);
       if (nv <= 0) continue;
       int b, hc;
-      w[e].row(mp.heads, &b, &hc);
+      w[e].item(mp.heads, &b, &hc);
       const int row = (int)(b * T_ + w[e].c * kC);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -106,9 +106,13 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
   if (warp == 0) umma::tmem_alloc(&tmem_slot, kTmemColsL);
   sync_all();
   dependency_wait();
+  // row flags of the call (null: they are kept), set by the kernels behind this one
+  if (rowflag != nullptr)
+    for (int i = (int)(blockIdx.x * kThreadsL) + tid; i < items; i += (int)(gridDim.x * kThreadsL)) rowflag[i] = 0;
   const uint32_t tb = __shfl_sync(0xffffffffu, tmem_slot, 0);
   const uint32_t tl = umma::tmem_addr(tb, 32 * q4, 0);
-  ItemWalk wn[2] = {ItemWalk(2 * blockIdx.x, 2 * gridDim.x, nc), ItemWalk(2 * blockIdx.x + 1, 2 * gridDim.x, nc)};
+  // (the blocks of a grid are problem rows of their own here)
+  ItemWalk wn[2] = {ItemWalk(2 * blockIdx.x, 2 * gridDim.x, nc, 1), ItemWalk(2 * blockIdx.x + 1, 2 * gridDim.x, nc, 1)};
   bool raw_pending = false;      // thread 0
   if (2 * (int64_t)blockIdx.x < total && tid == 0) {
     issue_raw(wn, 2 * (int64_t)blockIdx.x);
@@ -319,8 +323,8 @@ int lfw_chunk_umma_status() {
 
 // Forward flavour: M = L_c from (x, f) and (k, fk).  Backward flavour: M = G_c from (dO, f), (q, fk).
 // mp describes the four tensors in that order (mp.q_scale applies to the third one).
-int lfw_chunk_local_umma(bool backward, const seq::Maps &mp, float *M, float *Ac, float *Gc, int *flags, int64_t BH,
-                         int64_t T_, int dtype, cudaStream_t st) {
+int lfw_chunk_local_umma(bool backward, const seq::Maps &mp, float *M, float *Ac, float *Gc, int *flags, int *rowflag,
+                         int64_t BH, int64_t T_, int dtype, cudaStream_t st) {
   const int64_t nc = ceil_div64(T_, kC), total = BH * nc;
   int *status = nullptr;
   int rc = lfw_chunk_status_ptr(&status);
@@ -336,7 +340,7 @@ int lfw_chunk_local_umma(bool backward, const seq::Maps &mp, float *M, float *Ac
     auto *const kern1 = &lfw_c64_local_kernel<TT, SUF, FF>; \
     T2FW_ALLOW_SMEM(kern1, kSmemL);       \
     T2FW_CHECK_CUDA(launch_dependent(lfw_c64_local_kernel<TT, SUF, FF>, dim3(grid), dim3(kThreadsL), kSmemL, st, mp, M, \
-                                     Ac, Gc, flags, status, T_, nc, total));                         \
+                                     Ac, Gc, flags, rowflag, (int)(BH / mp.nsub), status, T_, nc, total));                         \
   } while (0)
   const bool fused = (mp.flags & (seq::kUnitForget | seq::kSigmoidGate)) != 0 || mp.q_scale != 1.f;
 #define T2FW_FUSED(TT, SUF)                                                   \

@@ -24,7 +24,6 @@ enum : int {
   kUnitForget = 1,     // the d-side gate is the constant 1: nothing is read for it
   kSigmoidGate = 2,    // the k-side gate tensor holds pre-activations: gate = max(sigmoid(g), 1/8)
   kContiguous = 4,     // every tensor is a dense [rows][64] array: a chunk's block is one linear 8 KB copy
-  kOutByRow = 8,       // outputs are [problem row][T][64] arrays (one per sub-item), not windows of a batch item's row
 };
 constexpr float kGateFloor = 0.125f;   // with gates >= 1/8 no 32-step product leaves the safe range
 
@@ -37,9 +36,19 @@ struct Maps {
   int heads;                     // sub-items per batch item: problem row bh = b * heads + h.  Heads of a
                                  // layer: hdiv = 1, hmod = heads.  A D x K state cut into 64 x 64 blocks:
                                  // h = i * (K/64) + j, d-side tensors hdiv = K/64, hmod = D/64, k-side 1, K/64
+  int nsub, nk;                  // state cut into a grid of 64 x 64 blocks: nsub blocks per batch item (1: no grid), block
+                                 // i * nk + j; results are summed over the blocks of the other axis
+  int64_t state_item;            // elements of one state of a batch item (or problem row without a grid), and the
+  int state_ld;                  //   stride of its rows
   int flags;
   float q_scale;                 // factor on the query tensor (1 for the plain operators)
 };
+
+// element offset of the 64 x 64 block of sub-item `sub` of item `b` (problem row without a grid), state number c of S
+__device__ __forceinline__ size_t state_off(const Maps &mp, int b, int sub, int64_t c, int64_t S) {
+  const int i = mp.nsub == 1 ? 0 : sub / mp.nk, j = mp.nsub == 1 ? 0 : sub - i * mp.nk;
+  return ((size_t)b * S + c) * mp.state_item + (size_t)i * 64 * mp.state_ld + j * 64;
+}
 
 // an output tensor: element (row of the 2-D array, feature) at p[row * ld + col + 64 * h + feature]
 template <typename T>
