@@ -33,9 +33,9 @@
 // sums over time are register-local plus one exchange between the four threads of a feature.  The d side's
 // rows are rotated by 16 features against the k side's so that the two half warps touch different banks.
 //
-// What bounds it: instruction issue (about 1000 instructions per thread and chunk; 53 k -> BWD_INSTR k warp
+// What bounds it: instruction issue (about 1000 instructions per thread and chunk; 53 k -> 25.5 k warp
 // instructions per chunk against the version that ran the two sides one after the other) and the latency of
-// its phases.  Config B*H = 96, T = 1024 (1536 chunks): 151 -> BWD_US us.
+// its phases.  Config B*H = 96, T = 1024 (1536 chunks): 151 -> 101 us per launch with cold caches.
 //
 // One persistent CTA of 16 warps per SM; six raw 8 KB input blocks per chunk by bulk asynchronous copy (the
 // next chunk's are requested once this chunk's operands are built); operand tiles in shared memory (TF32,

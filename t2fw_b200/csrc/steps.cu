@@ -1,5 +1,5 @@
 // Short sequences walked step by step with the state in registers: the decay rule over n steps (a ring of
-// decode steps, or a whole T <= 64 forward call) and the delta rule over a few steps, 16-bit storage.
+// decode steps, or a whole T < 64 forward call) and the delta rule over a few steps, 16-bit storage.
 //
 // Why a kernel of its own: a chain of n decode launches moves the whole state through memory n times and
 // pays a launch each time (512 rows: 3.6 us per step); a chunked call on a short sequence pays three
