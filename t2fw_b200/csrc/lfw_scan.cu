@@ -19,8 +19,9 @@
 // A chain of T steps bounds these kernels.  The steps' vectors come from shared memory, fetched a group ahead
 // (scan.cuh); the sums of a step share their shuffles; the two orientations run side by side; the backward
 // walks a checkpoint's steps forward once to leave the state at each segment start and then segment by segment
-// (128 forward steps per 64 instead of 160).  fp32, 16 rows of 129 steps, 96 x 48: forward 95 -> 31 us,
-// backward 366 -> 84 us.
+// (128 forward steps per 64 instead of 160).  In the forward eight lanes own a row of up to 128 elements, and the
+// sums of eight outputs are formed together, seven exchanges for four rows where a row per warp took 40.  fp32, 16 rows
+// of 129 steps, 96 x 48: forward 95 -> 31 us with a row per warp, -> 16.5; backward 366 -> 84 us.
 //
 // These kernels also redo the batch rows that the chunk kernels flagged (gate products outside the range of
 // the factored form): CTAs walk over all work items and skip the rows without a flag, and the launch is a
@@ -46,16 +47,19 @@ struct FwdArgs {
   const int *rowflag;     // if not null, only batch rows with a non-zero flag are processed
 };
 
-// One buffer: fk, k, q [G][K], x, f [G][kWarpsPerCta * OWN], each part 16-byte aligned
+// One buffer: fk, k, q [G][K], x, f [G][lines of the CTA], each part 16-byte aligned
 template <typename T>
 __host__ __device__ inline int fwd_part(int G, int n) { return (int)((((size_t)G * n * sizeof(T)) + 15) / 16 * 16); }
 
-template <typename T, int NL, int OWN>
-__global__ void __launch_bounds__(kThreads) lfw_scan_fwd_kernel(const FwdArgs<T> a) {
+// Element c of a state row lies in lane c % L of the L lanes that own OWN rows; the first SAFE elements of a lane
+// exist for every row length that takes this NL.
+template <typename T, int L, int NL, int SAFE, int OWN>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 1 : 4) lfw_scan_fwd_kernel(const FwdArgs<T> a) {
   using A = typename Elem<T>::acc;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int RC = kWarpsPerCta * OWN;      // state rows of the CTA
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int RC = kThreads / L * OWN;      // state rows of the CTA
+  constexpr int U = 8 / OWN;                  // steps whose sums are formed together
+  const int tid = threadIdx.x, l = tid % L, rl = tid / L * OWN;
   const int kp = fwd_part<T>(a.G, a.K), dp = fwd_part<T>(a.G, RC), buf_bytes = 3 * kp + 2 * dp;
   const int blocks_d = (a.D + RC - 1) / RC;
   dependency_wait();
@@ -63,7 +67,6 @@ __global__ void __launch_bounds__(kThreads) lfw_scan_fwd_kernel(const FwdArgs<T>
     const int64_t b = item / blocks_d;
     if (a.rowflag != nullptr && a.rowflag[b] == 0) continue;      // the same for the whole CTA
     const int rb = (int)(item - b * blocks_d) * RC, nrows = a.D - rb < RC ? a.D - rb : RC;
-    const int r0 = rb + warp * OWN;
 
     auto fetch = [&](int64_t t0, int which) {
       const int n = (int)(a.T_ - t0 < a.G ? a.T_ - t0 : a.G);
@@ -82,10 +85,8 @@ __global__ void __launch_bounds__(kThreads) lfw_scan_fwd_kernel(const FwdArgs<T>
 #pragma unroll
     for (int o = 0; o < OWN; ++o)
 #pragma unroll
-      for (int j = 0; j < NL; ++j) {
-        const int row = r0 + o, c = lane + 32 * j;
-        S[o][j] = (row < a.D && c < a.K) ? Elem<T>::ld(a.state + (b * a.D + row) * a.K + c) : A(0);
-      }
+      for (int j = 0; j < NL; ++j)
+        S[o][j] = rl + o < nrows && l + L * j < a.K ? Elem<T>::ld(a.state + (b * a.D + rb + rl + o) * a.K + l + L * j) : A(0);
 
     int which = 0;
     int64_t ck_next = a.C < a.T_ ? a.C : a.T_, slot = 0;      // step count at the next checkpoint
@@ -96,45 +97,54 @@ __global__ void __launch_bounds__(kThreads) lfw_scan_fwd_kernel(const FwdArgs<T>
       __syncthreads();
       const int n = (int)(a.T_ - t0 < a.G ? a.T_ - t0 : a.G);
       const unsigned char *p = smem_raw + which * buf_bytes;
-      const T *sg = reinterpret_cast<const T *>(p), *sk = reinterpret_cast<const T *>(p + kp);
-      const T *sq = reinterpret_cast<const T *>(p + 2 * kp);
-      const T *sx = reinterpret_cast<const T *>(p + 3 * kp), *sf = reinterpret_cast<const T *>(p + 3 * kp + dp);
-#pragma unroll(NL <= 4 ? 2 : 1)
-      for (int t = 0; t < n; ++t) {
-        A gl[NL], kl[NL], ql[NL];
-#pragma unroll
-        for (int j = 0; j < NL; ++j) {
-          const int c = lane + 32 * j;
-          const bool in = c < a.K;
-          gl[j] = in ? Elem<T>::ld(sg + t * a.K + c) : A(0);
-          kl[j] = in ? Elem<T>::ld(sk + t * a.K + c) : A(0);
-          ql[j] = in ? Elem<T>::ld(sq + t * a.K + c) : A(0);
-        }
-        A acc[OWN];
+      const T *sg = reinterpret_cast<const T *>(p) + l, *sk = reinterpret_cast<const T *>(p + kp) + l;
+      const T *sq = reinterpret_cast<const T *>(p + 2 * kp) + l;
+      const T *sx = reinterpret_cast<const T *>(p + 3 * kp) + rl, *sf = reinterpret_cast<const T *>(p + 3 * kp + dp) + rl;
+      auto step = [&](int t, A *acc) {
+        A xo[OWN], ao[OWN];
 #pragma unroll
         for (int o = 0; o < OWN; ++o) {
-          const int rl = warp * OWN + o;
-          const bool in = rl < nrows;
-          const A xo = in ? Elem<T>::ld(sx + t * nrows + rl) : A(0);
-          const A ao = in ? Elem<T>::ld(sf + t * nrows + rl) : A(0);
+          const bool in = rl + o < nrows;
+          xo[o] = in ? Elem<T>::ld(sx + t * nrows + o) : A(0);
+          ao[o] = in ? Elem<T>::ld(sf + t * nrows + o) : A(0);
           acc[o] = A(0);
+        }
 #pragma unroll
-          for (int j = 0; j < NL; ++j) {
-            S[o][j] = S[o][j] * (ao * gl[j]) + xo * kl[j];
-            acc[o] += S[o][j] * ql[j];
+        for (int j = 0; j < NL; ++j) {
+          const bool in = j < SAFE || l + L * j < a.K;
+          const A g = in ? Elem<T>::ld(sg + t * a.K + L * j) : A(0), k = in ? Elem<T>::ld(sk + t * a.K + L * j) : A(0);
+          const A q = in ? Elem<T>::ld(sq + t * a.K + L * j) : A(0);
+#pragma unroll
+          for (int o = 0; o < OWN; ++o) {
+            S[o][j] = S[o][j] * (ao[o] * g) + xo[o] * k;
+            acc[o] += S[o][j] * q;
           }
         }
-        int o;
-        if (scan::lane_sums<OWN>(acc, lane, &o) && r0 + o < a.D)
-          Elem<T>::st(a.out + (b * a.T_ + t0 + t) * a.D + r0 + o, acc[0]);
-        if (t0 + t + 1 == ck_next) {
+      };
+      T *out = a.out + (b * a.T_ + t0) * a.D + rb + rl;
+      for (int t = 0; t < n;) {
+        const int te = ck_next - t0 < n ? (int)(ck_next - t0) : n;      // up to the next checkpoint
+        for (; t + U <= te; t += U) {
+          A acc[8];
 #pragma unroll
-          for (int oo = 0; oo < OWN; ++oo)
+          for (int u = 0; u < U; ++u) step(t + u, acc + u * OWN);
+          int i;
+          if (scan::lane_sums<8, L>(acc, l, &i) && rl + i % OWN < nrows)
+            Elem<T>::st(out + (int64_t)(t + i / OWN) * a.D + i % OWN, acc[0]);
+        }
+        for (; t < te; ++t) {
+          A acc[OWN];
+          step(t, acc);
+          int i;
+          if (scan::lane_sums<OWN, L>(acc, l, &i) && rl + i < nrows) Elem<T>::st(out + (int64_t)t * a.D + i, acc[0]);
+        }
+        if (t0 + te == ck_next) {
 #pragma unroll
-            for (int j = 0; j < NL; ++j) {
-              const int row = r0 + oo, c = lane + 32 * j;
-              if (row < a.D && c < a.K) Elem<T>::st(a.ckpt + ((b * a.nslots + slot) * a.D + row) * a.K + c, S[oo][j]);
-            }
+          for (int o = 0; o < OWN; ++o)
+#pragma unroll
+            for (int j = 0; j < NL; ++j)
+              if (rl + o < nrows && l + L * j < a.K)
+                Elem<T>::st(a.ckpt + ((b * a.nslots + slot) * a.D + rb + rl + o) * a.K + l + L * j, S[o][j]);
           ++slot;
           ck_next = ck_next + a.C < a.T_ ? ck_next + a.C : a.T_;
         }
@@ -403,25 +413,25 @@ unsigned grid_for(int64_t items, const int *rowflag) {
   return (unsigned)(items < most ? items : most);
 }
 
-template <typename T, int NL, int OWN>
+template <typename T, int L, int NL, int SAFE, int OWN>
 int launch_fwd(FwdArgs<T> a, cudaStream_t st) {
-  constexpr int RC = kWarpsPerCta * OWN;
+  constexpr int RC = kThreads / L * OWN;
   a.items = a.B * ((a.D + RC - 1) / RC);
-  for (a.G = 32; a.G > 1 && 2 * (3 * fwd_part<T>(a.G, a.K) + 2 * fwd_part<T>(a.G, RC)) > 64 * 1024;) a.G /= 2;
-  const size_t smem = 2 * (size_t)(3 * fwd_part<T>(a.G, a.K) + 2 * fwd_part<T>(a.G, RC));
-  auto *const kernel = &lfw_scan_fwd_kernel<T, NL, OWN>;
-  T2FW_ALLOW_SMEM(kernel, 64 * 1024);
-  T2FW_CHECK_CUDA(launch_dependent(kernel, dim3(grid_for(a.items, a.rowflag)), dim3(kThreads), smem, st, a));
+  auto bytes = [&](int G) { return 2 * (size_t)(3 * fwd_part<T>(G, a.K) + 2 * fwd_part<T>(G, RC)); };
+  for (a.G = 32; a.G > 1 && (a.G / 2 >= a.T_ || bytes(a.G) > 48 * 1024);) a.G /= 2;
+  const size_t smem = bytes(a.G);
+  T2FW_CHECK_CUDA(launch_dependent(&lfw_scan_fwd_kernel<T, L, NL, SAFE, OWN>, dim3(grid_for(a.items, a.rowflag)),
+                                   dim3(kThreads), smem, st, a));
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;
 }
 
-// Rows per warp: four share the key-side loads and most of the shuffles; one while four would leave the chip
-// with less than 16 warps per SM (the chain of steps is then what counts, and more CTAs shorten each step).
-template <typename T, int NL>
+// Rows per group of lanes: MORE share the key-side loads; one while MORE would leave the chip with less than four
+// warps per SM (the chain of steps is then what counts, and more CTAs shorten each step).
+template <typename T, int L, int NL, int SAFE, int MORE>
 int launch_fwd_rows(const FwdArgs<T> &a, cudaStream_t st) {
-  if (a.B * ((a.D + 3) / 4) >= 148 * 16 || a.rowflag != nullptr) return launch_fwd<T, NL, 4>(a, st);
-  return launch_fwd<T, NL, 1>(a, st);
+  if (a.B * a.D * L / (32 * MORE) >= 148 * 4 || a.rowflag != nullptr) return launch_fwd<T, L, NL, SAFE, MORE>(a, st);
+  return launch_fwd<T, L, NL, SAFE, 1>(a, st);
 }
 
 template <typename T>
@@ -432,14 +442,16 @@ int fwd_typed(const void *x, const void *f, const void *q, const void *k, const 
   a.x = (const T *)x; a.f = (const T *)f; a.q = (const T *)q; a.k = (const T *)k; a.fk = (const T *)fk;
   a.state = (const T *)state; a.out = (T *)out; a.ckpt = (T *)ckpt;
   a.B = B; a.T_ = T_; a.D = (int)D; a.K = (int)K; a.C = C; a.nslots = ceil_div64(T_, C); a.rowflag = rowflag;
-  switch (pick_nl(K)) {
-    case 1: return launch_fwd_rows<T, 1>(a, st);
-    case 2: return launch_fwd_rows<T, 2>(a, st);
-    case 3: return launch_fwd_rows<T, 3>(a, st);
-    case 4: return launch_fwd_rows<T, 4>(a, st);
-    case 8: return launch_fwd_rows<T, 8>(a, st);
-    case 16: return launch_fwd_rows<T, 16>(a, st);
-  }
+  // elements per lane: the smallest that holds the row
+  if (K <= 16) return launch_fwd_rows<T, 8, 2, 0, 2>(a, st);
+  if (K <= 32) return launch_fwd_rows<T, 8, 4, 2, 2>(a, st);
+  if (K <= 48) return launch_fwd_rows<T, 8, 6, 4, 2>(a, st);
+  if (K <= 64) return launch_fwd_rows<T, 8, 8, 6, 2>(a, st);
+  if (K <= 80) return launch_fwd_rows<T, 8, 10, 8, 2>(a, st);
+  if (K <= 104) return launch_fwd_rows<T, 8, 13, 10, 2>(a, st);
+  if (K <= 128) return launch_fwd_rows<T, 8, 16, 13, 2>(a, st);
+  if (K <= 256) return launch_fwd_rows<T, 32, 8, 4, 4>(a, st);
+  if (K <= 512) return launch_fwd_rows<T, 32, 16, 8, 4>(a, st);
   set_error("lfw forward: K=%lld exceeds the supported maximum of 512", (long long)K);
   return T2FW_ERR_UNSUPPORTED;
 }

@@ -53,29 +53,31 @@ __device__ __forceinline__ void wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Sums over the 32 lanes of R values (R a power of two): at each distance a lane keeps half of its values and
-// hands over the partner's half, so R sums cost about R + 4 shuffles instead of 5 R.  On return v[0] is the
-// total of value *which in every lane; the lanes for which the function returns true cover each value once.
-template <int R, typename A>
-__device__ __forceinline__ bool lane_sums(A (&v)[R], int lane, int *which) {
-  int idx = 0;
+// Sums of R values (R a power of two) over the L lanes of an aligned group, lane = number within it: at each distance
+// a lane keeps half of its values and hands over the partner's half, so R <= L sums cost about R + log2(L / R)
+// shuffles instead of R log2(L).  On return v[0] is the total of value *which; the lanes for which the function
+// returns true cover each value once.
+template <int R, int L = 32, typename A>
+__device__ __forceinline__ bool lane_sums(A *v, int lane, int *which) {
+  static_assert(R <= L, "one value per lane at most");
+  int idx = 0, live = R;
 #pragma unroll
-  for (int l = 0; l < 5; ++l) {
-    const int o = 16 >> l, live = (R >> l) > 1 ? (R >> l) : 1;
+  for (int o = L / 2; o > 0; o >>= 1) {
     if (live > 1) {
       const bool up = (lane & o) != 0;
+      live >>= 1;
 #pragma unroll
-      for (int i = 0; i < (live >> 1); ++i) {
-        const A send = up ? v[i] : v[i + (live >> 1)], keep = up ? v[i + (live >> 1)] : v[i];
+      for (int i = 0; i < live; ++i) {
+        const A send = up ? v[i] : v[i + live], keep = up ? v[i + live] : v[i];
         v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
-      idx += up ? (live >> 1) : 0;
+      idx += up ? live : 0;
     } else {
       v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
     }
   }
   *which = idx;
-  return (lane & (32 / R - 1)) == 0;
+  return (lane & (L / R - 1)) == 0;
 }
 
 }  // namespace scan
