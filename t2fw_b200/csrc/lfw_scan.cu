@@ -2,7 +2,7 @@
 //
 //   S_t = (f_t fk_t^T) .* S_{t-1} + x_t k_t^T ,  o_t = S_t q_t
 //
-// One warp owns a few lines of the D x K state (rows in the "row" orientation, columns in the
+// A group of lanes owns a line of the D x K state (a row in the "row" orientation, a column in the
 // "column" orientation), the lanes spread along the other axis, and time is walked
 // sequentially with the state in registers in the accumulation type (float, or double for
 // double storage).  Every output of the reference's forward (scan kernel + einsum,
@@ -19,9 +19,10 @@
 // A chain of T steps bounds these kernels.  The steps' vectors come from shared memory, fetched a group ahead
 // (scan.cuh); the sums of a step share their shuffles; the two orientations run side by side; the backward
 // walks a checkpoint's steps forward once to leave the state at each segment start and then segment by segment
-// (128 forward steps per 64 instead of 160).  In the forward eight lanes own a row of up to 128 elements, and the
-// sums of eight outputs are formed together, seven exchanges for four rows where a row per warp took 40.  fp32, 16 rows
-// of 129 steps, 96 x 48: forward 95 -> 31 us with a row per warp, -> 16.5; backward 366 -> 84 us.
+// (128 forward steps per 64 instead of 160).  Eight, 16 or 32 lanes own a line (lanes_for), and eight sums are formed
+// together: seven exchanges for four lines where a line per warp took 40.  fp32, 16 rows of 129 steps, 96 x 48: forward
+// 95 -> 16.5 us, backward 366 -> 70 us (84 with a warp per two lines); 48 x 300, 100 x 100, forward and backward
+// 2475 -> 1136; 8 x 128, 256 x 256 825 -> 476.
 //
 // These kernels also redo the batch rows that the chunk kernels flagged (gate products outside the range of
 // the factored form): CTAs walk over all work items and skip the rows without a flag, and the launch is a
@@ -218,11 +219,11 @@ struct SegWalk {
 template <typename T>
 __host__ __device__ inline int bwd_part(int seg, int n) { return (int)((((size_t)seg * n * sizeof(T)) + 15) / 16 * 16); }
 
-template <typename T, int NL, int OWN, bool WITH_SP>
+template <typename T, int L, int NL, int SAFE, int OWN, bool WITH_SP>
 __device__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> &ln, int64_t item, int vec_ext, unsigned char *smem) {
   using A = typename Elem<T>::acc;
-  constexpr int RC = kWarpsPerCta * OWN;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int RC = kThreads / L * OWN;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = tid % L, rl = tid / L * OWN;
   const int lp = bwd_part<T>(a.seg, vec_ext), op = bwd_part<T>(a.seg, RC), buf_bytes = 3 * lp + 3 * op;
   A *hist = reinterpret_cast<A *>(smem + 2 * buf_bytes) + (size_t)warp * (a.seg + a.mids) * OWN * NL * 32;
   A *mid = hist + (size_t)a.seg * OWN * NL * 32;
@@ -230,11 +231,11 @@ __device__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> &ln, int64_t ite
   const int blocks = (ln.NO + RC - 1) / RC;
   const int64_t b = item / blocks;
   const int ob = (int)(item - b * blocks) * RC, nown = ln.NO - ob < RC ? ln.NO - ob : RC;
-  const int o0 = ob + warp * OWN;
+  const int o0 = ob + rl;
   const int64_t DK = (int64_t)ln.NO * ln.NLn;
 
-  auto state_off = [&](int o, int j) { return (o0 + o) * ln.so + (int64_t)(lane + 32 * j) * ln.sl; };
-  auto valid = [&](int o, int j) { return (o0 + o) < ln.NO && (lane + 32 * j) < ln.NLn; };
+  auto state_off = [&](int o, int j) { return (o0 + o) * ln.so + (int64_t)(l + L * j) * ln.sl; };
+  auto valid = [&](int o, int j) { return (o0 + o) < ln.NO && (l + L * j) < ln.NLn; };
 
   SegWalk w;
   w.T_ = a.T_; w.C = a.C; w.seg = a.seg; w.mids = a.mids;
@@ -288,32 +289,31 @@ __device__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> &ln, int64_t ite
 
     const int n = w.count();
     const unsigned char *p = smem + which * buf_bytes;
-    const T *s_xl = reinterpret_cast<const T *>(p), *s_gl = reinterpret_cast<const T *>(p + lp);
-    const T *s_pl = reinterpret_cast<const T *>(p + 2 * lp);
-    const T *s_xo = reinterpret_cast<const T *>(p + 3 * lp) + warp * OWN, *s_go = reinterpret_cast<const T *>(p + 3 * lp + op) + warp * OWN;
-    const T *s_po = reinterpret_cast<const T *>(p + 3 * lp + 2 * op) + warp * OWN;
+    const T *s_xl = reinterpret_cast<const T *>(p) + l, *s_gl = reinterpret_cast<const T *>(p + lp) + l;
+    const T *s_pl = reinterpret_cast<const T *>(p + 2 * lp) + l;
+    const T *s_xo = reinterpret_cast<const T *>(p + 3 * lp) + rl, *s_go = reinterpret_cast<const T *>(p + 3 * lp + op) + rl;
+    const T *s_po = reinterpret_cast<const T *>(p + 3 * lp + 2 * op) + rl;
     const bool last = w.cur == w.target;
-    auto vec = [&](const T *v, int t, A (&o)[NL]) {
-#pragma unroll
-      for (int j = 0; j < NL; ++j) {
-        const int c = lane + 32 * j;
-        o[j] = c < ln.NLn ? Elem<T>::ld(v + t * ln.NLn + c) : A(0);
-      }
+    auto vec = [&](const T *v, int t, int j) {
+      return (j < SAFE || l + L * j < ln.NLn) ? Elem<T>::ld(v + t * ln.NLn + L * j) : A(0);
     };
     auto own = [&](const T *v, int t, int o) { return o0 + o < ln.NO ? Elem<T>::ld(v + t * nown + o) : A(0); };
 
-#pragma unroll(NL <= 4 ? 2 : 1)
+#pragma unroll(NL <= 8 ? 2 : 1)
     for (int t = 0; t < n; ++t) {      // forward over the segment
-      A gl[NL], xl[NL];
-      vec(s_gl, t, gl);
-      vec(s_xl, t, xl);
+      A xo[OWN], go[OWN];
 #pragma unroll
       for (int o = 0; o < OWN; ++o) {
-        const A xo = own(s_xo, t, o), go = own(s_go, t, o);
+        xo[o] = own(s_xo, t, o);
+        go[o] = own(s_go, t, o);
+      }
 #pragma unroll
-        for (int j = 0; j < NL; ++j) {
+      for (int j = 0; j < NL; ++j) {
+        const A g = vec(s_gl, t, j), x = vec(s_xl, t, j);
+#pragma unroll
+        for (int o = 0; o < OWN; ++o) {
           if (last) hist[((t * OWN + o) * NL + j) * 32 + lane] = S[o][j];
-          S[o][j] = S[o][j] * (go * gl[j]) + xo * xl[j];
+          S[o][j] = S[o][j] * (go[o] * g) + xo[o] * x;
         }
       }
     }
@@ -326,42 +326,49 @@ __device__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> &ln, int64_t ite
     }
     if (last) {
       const int64_t ob_t = (b * a.T_ + w.first()) * ln.NO + o0;
-#pragma unroll(NL <= 4 ? 2 : 1)
-      for (int t = n - 1; t >= 0; --t) {      // S is the state after step t
-        A gl[NL], xl[NL], pl[NL];
-        vec(s_gl, t, gl);
-        vec(s_xl, t, xl);
-        vec(s_pl, t, pl);
-        constexpr int kSums = WITH_SP ? 4 : 2;
-        A v[kSums * OWN];
+      constexpr int kSums = WITH_SP ? 4 : 2, kStep = kSums * OWN, U = 8 / kStep;      // U steps' sums are formed together
+      auto step = [&](int t, A *v) {      // S is the state after step t
+        A go[OWN], po[OWN];
 #pragma unroll
         for (int o = 0; o < OWN; ++o) {
-          const A go = own(s_go, t, o), po = own(s_po, t, o);
-          A ax = A(0), ag = A(0), ap = A(0);
+          go[o] = own(s_go, t, o);
+          po[o] = own(s_po, t, o);
+        }
 #pragma unroll
-          for (int j = 0; j < NL; ++j) {
+        for (int i = 0; i < kStep; ++i) v[i] = A(0);
+#pragma unroll
+        for (int j = 0; j < NL; ++j) {
+          const A g = vec(s_gl, t, j), x = vec(s_xl, t, j), p = vec(s_pl, t, j);
+#pragma unroll
+          for (int o = 0; o < OWN; ++o) {
             const A sp = hist[((t * OWN + o) * NL + j) * 32 + lane];
-            const A r = R[o][j] + po * pl[j];   // gradient w.r.t. S_t
-            ax += r * xl[j];
-            ag += (r * sp) * gl[j];
-            if (WITH_SP) ap += S[o][j] * pl[j];
-            R[o][j] = r * (go * gl[j]);         // what flows on to S_{t-1}
+            const A r = R[o][j] + po[o] * p;    // gradient w.r.t. S_t
+            v[kSums * o] += r * x;
+            v[kSums * o + 1] += (r * sp) * g;
+            if (WITH_SP) v[kSums * o + 2] += S[o][j] * p;
+            R[o][j] = r * (go[o] * g);          // what flows on to S_{t-1}
             S[o][j] = sp;
           }
-          v[kSums * o] = ax;
-          v[kSums * o + 1] = ag;
-          if (WITH_SP) {
-            v[kSums * o + 2] = ap;
-            v[kSums * o + 3] = A(0);
-          }
         }
-        int i;
-        const bool mine = scan::lane_sums<kSums * OWN>(v, lane, &i);
-        const int o = i / kSums, kind = i % kSums;
-        if (mine && kind < 3 && o0 + o < ln.NO) {
+      };
+      auto put = [&](int t, int i, A v) {      // sum i of the steps t, t - 1, ..
+        const int o = i % kStep / kSums, kind = i % kSums;
+        if (kind < 3 && o0 + o < ln.NO) {
           T *dst = kind == 0 ? ln.d_xo : kind == 1 ? ln.d_go : ln.d_po;
-          Elem<T>::st(dst + ob_t + (int64_t)t * ln.NO + o, v[0]);
+          Elem<T>::st(dst + ob_t + (int64_t)(t - i / kStep) * ln.NO + o, v);
         }
+      };
+      int t = n - 1, i;
+      for (; t + 1 >= U; t -= U) {
+        A v[8];
+#pragma unroll
+        for (int u = 0; u < U; ++u) step(t - u, v + u * kStep);
+        if (scan::lane_sums<8, L>(v, l, &i)) put(t, i, v[0]);
+      }
+      for (; t >= 0; --t) {
+        A v[kStep];
+        step(t, v);
+        if (scan::lane_sums<kStep, L>(v, l, &i)) put(t, i, v[0]);
       }
     }
     __syncthreads();
@@ -382,11 +389,11 @@ __device__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> &ln, int64_t ite
 // it has completed), runs beside it, and ends only after it, so that what follows may rely on both.
 enum Part { kBoth = 0, kColumns = 1, kRows = 2 };
 
-template <typename T, int NL, int OWN>
+template <typename T, int L, int NL, int SAFE, int OWN>
 __global__ void __launch_bounds__(kThreads) lfw_line_bwd_kernel(const BwdArgs<T> a, const int part) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int RC = kWarpsPerCta * OWN;
-  const int ext = a.col.NLn > a.row.NLn ? a.col.NLn : a.row.NLn;
+  constexpr int RC = kThreads / L * OWN;
+  const int ext = part == kRows || (part == kBoth && a.row.NLn > a.col.NLn) ? a.row.NLn : a.col.NLn;
   if (part != kRows) dependency_wait();
   const int64_t first_row = part == kRows ? 0 : a.col.items, n = first_row + (part == kColumns ? 0 : a.row.items);
   for (int64_t item = blockIdx.x; item < n; item += gridDim.x) {
@@ -394,18 +401,16 @@ __global__ void __launch_bounds__(kThreads) lfw_line_bwd_kernel(const BwdArgs<T>
     const int64_t i = col ? item : item - first_row;
     const int64_t b = i / (((col ? a.col.NO : a.row.NO) + RC - 1) / RC);
     if (a.rowflag != nullptr && a.rowflag[b] == 0) continue;
-    if (col) line_bwd<T, NL, OWN, true>(a, a.col, i, ext, smem_raw);
-    else line_bwd<T, NL, OWN, false>(a, a.row, i, ext, smem_raw);
+    if (col) line_bwd<T, L, NL, SAFE, OWN, true>(a, a.col, i, ext, smem_raw);
+    else line_bwd<T, L, NL, SAFE, OWN, false>(a, a.row, i, ext, smem_raw);
   }
   if (part == kRows) dependency_wait();
 }
 
-int pick_nl(int64_t extent) {
-  const int64_t need = (extent + 31) / 32;
-  for (int nl : {1, 2, 3, 4, 8, 16})
-    if (need <= nl) return nl;
-  return 0;
-}
+// Lanes per line for lines of up to 128 elements.  Eight cost the fewest instructions, where they still give every
+// scheduler a warp and a half; with fewer lines a step's length is what counts, and the lines are spread over 16 lanes
+// while that fills half of the schedulers, over a warp below.
+int lanes_for(int64_t lines) { return lines >= 148 * 24 ? 8 : lines >= 148 * 4 ? 16 : 32; }
 
 // CTAs of a launch: one per work item; the walk over flagged rows only is cut to a few waves
 unsigned grid_for(int64_t items, const int *rowflag) {
@@ -443,6 +448,20 @@ int fwd_typed(const void *x, const void *f, const void *q, const void *k, const 
   a.state = (const T *)state; a.out = (T *)out; a.ckpt = (T *)ckpt;
   a.B = B; a.T_ = T_; a.D = (int)D; a.K = (int)K; a.C = C; a.nslots = ceil_div64(T_, C); a.rowflag = rowflag;
   // elements per lane: the smallest that holds the row
+  const int lanes = rowflag != nullptr ? 8 : lanes_for(B * D);
+  if (K <= 128 && lanes == 32) {
+    if (K <= 32) return launch_fwd<T, 32, 1, 0, 1>(a, st);
+    if (K <= 64) return launch_fwd<T, 32, 2, 1, 1>(a, st);
+    if (K <= 96) return launch_fwd<T, 32, 3, 2, 1>(a, st);
+    return launch_fwd<T, 32, 4, 3, 1>(a, st);
+  }
+  if (K <= 128 && lanes == 16) {
+    if (K <= 32) return launch_fwd<T, 16, 2, 0, 1>(a, st);
+    if (K <= 48) return launch_fwd<T, 16, 3, 2, 1>(a, st);
+    if (K <= 64) return launch_fwd<T, 16, 4, 3, 1>(a, st);
+    if (K <= 96) return launch_fwd<T, 16, 6, 4, 1>(a, st);
+    return launch_fwd<T, 16, 8, 6, 1>(a, st);
+  }
   if (K <= 16) return launch_fwd_rows<T, 8, 2, 0, 2>(a, st);
   if (K <= 32) return launch_fwd_rows<T, 8, 4, 2, 2>(a, st);
   if (K <= 48) return launch_fwd_rows<T, 8, 6, 4, 2>(a, st);
@@ -456,42 +475,82 @@ int fwd_typed(const void *x, const void *f, const void *q, const void *k, const 
   return T2FW_ERR_UNSUPPORTED;
 }
 
-template <typename T, int NL>
-int launch_bwd(BwdArgs<T> a, cudaStream_t st) {
+template <typename T, int L, int NL, int SAFE>
+int launch_bwd(BwdArgs<T> a, int part, cudaStream_t st) {
   using A = typename Elem<T>::acc;
-  constexpr int OWN = NL * sizeof(A) <= 32 ? 2 : 1, RC = kWarpsPerCta * OWN;
-  const int ext = a.col.NLn > a.row.NLn ? a.col.NLn : a.row.NLn;
+  constexpr int OWN = 1, RC = kThreads / L;
+  const int ext = part == kRows || (part == kBoth && a.row.NLn > a.col.NLn) ? a.row.NLn : a.col.NLn;
   a.col.items = a.B * ((a.col.NO + RC - 1) / RC);
   a.row.items = a.B * ((a.row.NO + RC - 1) / RC);
+  const int64_t items = (part != kRows ? a.col.items : 0) + (part != kColumns ? a.row.items : 0);
   auto bytes = [&](int seg, int mids) {
     return 2 * (size_t)(3 * bwd_part<T>(seg, ext) + 3 * bwd_part<T>(seg, RC)) +
            (size_t)kWarpsPerCta * (seg + mids) * OWN * NL * 32 * sizeof(A);
   };
-  // Segments of 16 steps with up to seven kept starts where two CTAs still fit an SM; less history for wide states.
+  // Segments of 16 steps and as many kept starts as an interval of 64 steps has, where that leaves room for two CTAs per
+  // SM (a launch that does not fill the chip once may take the SM); else less history.
   constexpr size_t kMost = 224 * 1024;
+  const size_t most = items <= 148 && part != kBoth ? kMost : 112 * 1024;
   a.seg = 16;
-  a.mids = 7;
-  while (a.seg > 4 && bytes(a.seg, a.mids) > 112 * 1024) a.seg /= 2;
+  a.mids = 3;
+  while (a.seg > 4 && bytes(a.seg, a.mids) > most) a.seg /= 2;
   while (bytes(a.seg, a.mids) > kMost && (a.seg > 1 || a.mids > 1)) {
     if (a.mids > a.seg) a.mids /= 2;
     else a.seg /= 2;
   }
+  while (a.mids < 7 && bytes(a.seg, a.mids + 4) <= most) a.mids += 4;
   const size_t smem = bytes(a.seg, a.mids);
   if (smem > kMost) {
     set_error("lfw backward: %zu bytes of shared memory needed", smem);
     return T2FW_ERR_UNSUPPORTED;
   }
-  auto *const kernel = &lfw_line_bwd_kernel<T, NL, OWN>;
+  auto *const kernel = &lfw_line_bwd_kernel<T, L, NL, SAFE, OWN>;
   T2FW_ALLOW_SMEM(kernel, (int)kMost);
-  if (a.rowflag != nullptr) {
-    T2FW_CHECK_CUDA(launch_dependent(kernel, dim3(grid_for(a.col.items + a.row.items, a.rowflag)), dim3(kThreads), smem, st, a, (int)kBoth));
-    T2FW_CHECK_LAUNCH(1);
-    return T2FW_OK;
-  }
-  T2FW_CHECK_CUDA(launch_dependent(kernel, dim3((unsigned)a.col.items), dim3(kThreads), smem, st, a, (int)kColumns));
-  T2FW_CHECK_CUDA(launch_dependent(kernel, dim3((unsigned)a.row.items), dim3(kThreads), smem, st, a, (int)kRows));
-  T2FW_CHECK_LAUNCH(2);
+  T2FW_CHECK_CUDA(launch_dependent(kernel, dim3(grid_for(items, a.rowflag)), dim3(kThreads), smem, st, a, part));
+  T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;
+}
+
+// one orientation: elements per lane are the smallest that hold the lines
+template <typename T>
+int launch_part(const BwdArgs<T> &a, int part, cudaStream_t st) {
+  const int n = part == kColumns ? a.col.NLn : a.row.NLn;
+  const int lanes = lanes_for(a.B * (part == kColumns ? a.col.NO : a.row.NO));
+  if (n <= 128 && lanes == 32) {
+    if (n <= 32) return launch_bwd<T, 32, 1, 0>(a, part, st);
+    if (n <= 64) return launch_bwd<T, 32, 2, 1>(a, part, st);
+    if (n <= 96) return launch_bwd<T, 32, 3, 2>(a, part, st);
+    return launch_bwd<T, 32, 4, 3>(a, part, st);
+  }
+  if (n <= 128 && lanes == 16) {
+    if (n <= 32) return launch_bwd<T, 16, 2, 0>(a, part, st);
+    if (n <= 48) return launch_bwd<T, 16, 3, 2>(a, part, st);
+    if (n <= 64) return launch_bwd<T, 16, 4, 3>(a, part, st);
+    if (n <= 96) return launch_bwd<T, 16, 6, 4>(a, part, st);
+    return launch_bwd<T, 16, 8, 6>(a, part, st);
+  }
+  if (n <= 16) return launch_bwd<T, 8, 2, 0>(a, part, st);
+  if (n <= 32) return launch_bwd<T, 8, 4, 2>(a, part, st);
+  if (n <= 48) return launch_bwd<T, 8, 6, 4>(a, part, st);
+  if (n <= 64) return launch_bwd<T, 8, 8, 6>(a, part, st);
+  if (n <= 80) return launch_bwd<T, 8, 10, 8>(a, part, st);
+  if (n <= 104) return launch_bwd<T, 8, 13, 10>(a, part, st);
+  if (n <= 128) return launch_bwd<T, 8, 16, 13>(a, part, st);
+  if (n <= 256) return launch_bwd<T, 32, 8, 4>(a, part, st);
+  return launch_bwd<T, 32, 16, 8>(a, part, st);
+}
+
+// flagged rows, both orientations: only the chunk kernels flag rows, of 16-bit states up to 256 x 256
+template <typename T>
+int launch_flagged(const BwdArgs<T> &a, cudaStream_t st) {
+  const int n = a.col.NLn > a.row.NLn ? a.col.NLn : a.row.NLn;
+  if constexpr (sizeof(T) == 2) {
+    if (n <= 64) return launch_bwd<T, 8, 8, 0>(a, kBoth, st);
+    if (n <= 128) return launch_bwd<T, 8, 16, 0>(a, kBoth, st);
+    if (n <= 256) return launch_bwd<T, 32, 8, 0>(a, kBoth, st);
+  }
+  set_error("lfw backward: no flagged rows at this size or type");
+  return T2FW_ERR_UNSUPPORTED;
 }
 
 template <typename T>
@@ -511,16 +570,9 @@ int bwd_typed(const void *go, const void *gs, const void *x, const void *f, cons
   col.xl = (const T *)x; col.gl = (const T *)f; col.pl = (const T *)go;
   col.d_xo = (T *)dk; col.d_go = (T *)dfk; col.d_po = (T *)dq; col.d_state = nullptr;
   col.NO = (int)K; col.NLn = (int)D; col.so = 1; col.sl = K;
-  switch (pick_nl(D > K ? D : K)) {
-    case 1: return launch_bwd<T, 1>(a, st);
-    case 2: return launch_bwd<T, 2>(a, st);
-    case 3: return launch_bwd<T, 3>(a, st);
-    case 4: return launch_bwd<T, 4>(a, st);
-    case 8: return launch_bwd<T, 8>(a, st);
-    case 16: return launch_bwd<T, 16>(a, st);
-  }
-  set_error("lfw backward: D=%lld, K=%lld exceed the supported maximum of 512", (long long)D, (long long)K);
-  return T2FW_ERR_UNSUPPORTED;
+  if (rowflag != nullptr) return launch_flagged<T>(a, st);
+  const int rc = launch_part<T>(a, kColumns, st);
+  return rc != T2FW_OK ? rc : launch_part<T>(a, kRows, st);
 }
 
 }  // namespace
