@@ -7,8 +7,8 @@
 // the interpreter on the engine's thread.  Here the arguments are unpacked straight from the argument
 // vector, the graph node is a C++ node, and without gradients no node is made at all.
 //
-// A call that is not the plain case (an argument that is no tensor, a tensor subclass, a failed shape or
-// type check, tracing, a function transform) is handed to the Python class, which then raises, or does,
+// A call that is not the plain case (an argument that is no tensor, a tensor subclass, a dual tensor, a failed shape
+// or type check, tracing, a function transform) is handed to the Python class, which then raises, or does,
 // what it always did.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -94,14 +94,15 @@ PyObject *call_fallback(int which, PyObject *const *args, Py_ssize_t n) {
   return PyObject_Vectorcall(g_fallback[which], args, (size_t)n, nullptr);
 }
 
-// plain tensors only: exact type (or nn.Parameter), no Python dispatch, no wrapped function-transform levels
+// plain tensors only: exact type (or nn.Parameter), no Python dispatch, no wrapped function-transform levels, no
+// forward-mode tangent (which an entry point without a jvp would drop: the class raises)
 bool plain_tensor(PyObject *o) {
   if (!THPVariable_Check(o)) return false;
   const Tensor &t = THPVariable_Unpack(o);
   if (!THPVariable_CheckExact(o) && !(ParameterClass != nullptr && (PyObject *)Py_TYPE(o) == ParameterClass)) return false;
   const auto ks = t.key_set();
   return t.defined() && t.is_cuda() && !ks.has(c10::DispatchKey::Python) && !ks.has(c10::DispatchKey::FuncTorchGradWrapper) &&
-         !ks.has(c10::DispatchKey::FuncTorchBatched);
+         !ks.has(c10::DispatchKey::FuncTorchBatched) && !t._fw_grad(/*level=*/0).defined();
 }
 
 bool plain_mode() {
