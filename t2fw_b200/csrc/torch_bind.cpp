@@ -12,8 +12,11 @@
 // what it always did.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <torch/csrc/utils/pybind.h>
 #include <ATen/core/PythonFallbackKernel.h>
 #include <ATen/FuncTorchTLS.h>
@@ -39,6 +42,24 @@ Tensor last_slot(const Tensor &ckpt, bool tracked) {
   return t;
 }
 
+// Gradients formed in grad mode (create_graph) from tensors that require gradients: there is no second derivative, so
+// they hang on a node that raises when one runs into it.  Left as they are they would be constants, and that derivative
+// silently zero.  The node's edges lead to those tensors, so that a search for a path to one of them finds it.
+variable_list no_second_derivative(variable_list grads, const variable_list &upstream, const variable_list &saved) {
+  if (!at::GradMode::is_enabled()) return grads;
+  auto needs = [](const variable_list &l) {
+    for (const Tensor &t : l)
+      if (t.requires_grad()) return true;
+    return false;
+  };
+  if (!needs(upstream) && !needs(saved)) return grads;
+  std::shared_ptr<torch::autograd::Node> node(new torch::autograd::NotImplemented("the backward of t2fw's recurrences"),
+                                              torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(upstream, saved));
+  for (const Tensor &g : grads) torch::autograd::set_history(g, node);      // fresh tensors of this call
+  return grads;
+}
+
 // `state` of a T > 1 call may be the strided last slot of another call's checkpoints: the operators ask for
 // contiguous tensors and say so themselves.
 struct LfwNode : torch::autograd::Function<LfwNode> {
@@ -50,8 +71,8 @@ struct LfwNode : torch::autograd::Function<LfwNode> {
   }
   static variable_list backward(AutogradContext *ctx, variable_list g) {
     const auto v = ctx->get_saved_variables();
-    return t2fw_ops::lfw_backward(g[0].contiguous(), g[1].contiguous(), v[0], v[1], v[2], v[3], v[4], v[0], v[5],
-                                  v[6]);
+    return no_second_derivative(t2fw_ops::lfw_backward(g[0].contiguous(), g[1].contiguous(), v[0], v[1], v[2], v[3], v[4],
+                                                       v[0], v[5], v[6]), g, v);
   }
 };
 
@@ -64,7 +85,7 @@ struct DfwNode : torch::autograd::Function<DfwNode> {
   }
   static variable_list backward(AutogradContext *ctx, variable_list g) {
     const auto v = ctx->get_saved_variables();
-    return t2fw_ops::dfw_backward(g[0].contiguous(), g[1].contiguous(), v[0], v[1], v[2], v[3]);
+    return no_second_derivative(t2fw_ops::dfw_backward(g[0].contiguous(), g[1].contiguous(), v[0], v[1], v[2], v[3]), g, v);
   }
 };
 
@@ -77,8 +98,8 @@ struct FusedNode : torch::autograd::Function<FusedNode> {
   }
   static variable_list backward(AutogradContext *ctx, variable_list g) {
     const auto v = ctx->get_saved_variables();
-    auto r = t2fw_ops::lfw_fused_backward(g[0].contiguous(), g[1].contiguous(), v[0], v[1], v[2],
-                                          ctx->saved_data["n_head"].toInt());
+    auto r = no_second_derivative(t2fw_ops::lfw_fused_backward(g[0].contiguous(), g[1].contiguous(), v[0], v[1], v[2],
+                                                               ctx->saved_data["n_head"].toInt()), g, v);
     return {r[0], r[1], Tensor()};
   }
 };
@@ -251,6 +272,26 @@ PyObject *py_decode_ring(PyObject *, PyObject *const *args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// no_second_derivative(gradients, upstream and saved tensors) -> gradients: for the Python classes
+PyObject *py_no_second_derivative(PyObject *, PyObject *const *args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  variable_list l[2];
+  for (int i = 0; i < 2; ++i) {
+    TORCH_CHECK(n == 2 && (PyTuple_Check(args[i]) || PyList_Check(args[i])), "no_second_derivative(gradients, tensors)");
+    for (Py_ssize_t j = 0; j < PySequence_Fast_GET_SIZE(args[i]); ++j) {
+      PyObject *o = PySequence_Fast_GET_ITEM(args[i], j);
+      TORCH_CHECK(THPVariable_Check(o), "no_second_derivative: tensors expected");
+      l[i].push_back(THPVariable_Unpack(o));
+    }
+  }
+  const variable_list r = no_second_derivative(l[0], l[1], {});
+  THPObjectPtr tup(PyTuple_New((Py_ssize_t)r.size()));
+  if (!tup) throw python_error();
+  for (size_t j = 0; j < r.size(); ++j) PyTuple_SET_ITEM(tup.get(), (Py_ssize_t)j, THPVariable_Wrap(r[j]));
+  return tup.release();
+  END_HANDLE_TH_ERRORS
+}
+
 // set_fallback(which, callable): 0 LFWFunction, 1 DFWFunction, 2 LFWFusedFunction
 PyObject *py_set_fallback(PyObject *, PyObject *const *args, Py_ssize_t n) {
   const long w = n == 2 ? PyLong_AsLong(args[0]) : -1;
@@ -270,6 +311,7 @@ PyMethodDef g_methods[] = {
     T2FW_METHOD("fused_apply", py_fused_apply, "apply(qkvg, state, n_head) -> (outputs, next_state)"),
     T2FW_METHOD("decode_step", py_decode_step, "decode_step(x, f, query, key, f_key, state_in, state_out, outputs)"),
     T2FW_METHOD("decode_ring", py_decode_ring, "decode_ring(x, f, query, key, f_key, state, outputs) -> bool"),
+    T2FW_METHOD("no_second_derivative", py_no_second_derivative, "no_second_derivative(gradients, tensors) -> gradients"),
     T2FW_METHOD("set_fallback", py_set_fallback, "set_fallback(which, callable)"),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "t2fw_torch_ops", "Autograd entry points of t2fw_b200.", -1, g_methods,

@@ -32,12 +32,12 @@ class DFWFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_output, grad_state):
-        query, key, delta_value, final_state = ctx.saved_tensors
+        query, key, delta_value, final_state = saved = ctx.saved_tensors
         assert grad_state.dtype == query.dtype
         assert grad_output.dtype == query.dtype
         grads = torch.ops.dfw.backward(grad_output.contiguous(), grad_state.contiguous(),
                                        query, key, delta_value, final_state)
-        return tuple(grads)
+        return _ops.no_second_derivative(grads, (grad_output, grad_state, *saved))
 
 
 _lib.bind_apply(DFWFunction, _lib.DFW, _ops.dfw_apply)

@@ -35,10 +35,10 @@ class LFWFusedFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_output, grad_state):
-        qkvg, state, ckpt = ctx.saved_tensors
-        d_qkvg, d_state = torch.ops.lfw.fused_backward(grad_output.contiguous(), grad_state.contiguous(), qkvg,
-                                                       state, ckpt, ctx.n_head)
-        return d_qkvg, d_state, None
+        qkvg, state, ckpt = saved = ctx.saved_tensors
+        grads = torch.ops.lfw.fused_backward(grad_output.contiguous(), grad_state.contiguous(), qkvg,
+                                             state, ckpt, ctx.n_head)
+        return (*_ops.no_second_derivative(grads, (grad_output, grad_state, *saved)), None)
 
 
 _lib.bind_apply(LFWFusedFunction, _lib.FUSED, _ops.fused_apply)

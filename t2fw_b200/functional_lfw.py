@@ -36,13 +36,13 @@ class LFWFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_output, grad_state):
-        value, forget, query, key, f_key, outputs, state, ckpt_states = ctx.saved_tensors
+        value, forget, query, key, f_key, outputs, state, ckpt_states = saved = ctx.saved_tensors
         assert grad_state.dtype == value.dtype
         assert grad_output.dtype == value.dtype
         grads = torch.ops.lfw.backward(grad_output.contiguous(), grad_state.contiguous(),
                                        value, forget, query, key, f_key, outputs, state,
                                        ckpt_states)
-        return tuple(grads)
+        return _ops.no_second_derivative(grads, (grad_output, grad_state, *saved))
 
 
 _lib.bind_apply(LFWFunction, _lib.LFW, _ops.lfw_apply)

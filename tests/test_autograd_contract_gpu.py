@@ -1,4 +1,5 @@
-"""What the native entry points refuse, as the torch.autograd.Function classes behind them do."""
+"""What the native entry points refuse, as the torch.autograd.Function classes behind them do: forward-mode tangents, and
+second derivatives (a backward under create_graph runs, a derivative through its gradients raises)."""
 import pytest
 import torch
 
@@ -39,3 +40,24 @@ def test_forward_mode_is_refused(cuda, which, grad):
             with pytest.raises(NotImplementedError, match="jvp"):
                 fn.apply(*args, *rest)
         fn.apply(*ins, *rest)      # outside the level the same tensors are plain again
+
+
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("which", ["lfw", "dfw", "fused"])
+def test_second_derivative_raises(cuda, which, native):
+    fn, ins, rest, up = _call(which, cuda)
+    if not native:      # a subclass takes torch.autograd.Function.apply and torch.ops
+        fn = type("Sub", (fn,), {})
+    leaves = [t.clone().requires_grad_(True) for t in ins]
+    first = torch.autograd.grad(fn.apply(*leaves, *rest), leaves, up)
+    # constant upstream gradients: the dependence on the inputs is through the saved tensors alone
+    again = torch.autograd.grad(fn.apply(*leaves, *rest), leaves, up, create_graph=True)
+    for a, b in zip(first, again):
+        assert torch.equal(a, b) and b.requires_grad
+    with pytest.raises(RuntimeError, match="not implemented"):
+        torch.autograd.grad(again[0].float().sum() + leaves[0].float().square().sum(), leaves[0])
+    # and through the upstream gradients
+    up = [t.clone().requires_grad_(True) for t in up]
+    again = torch.autograd.grad(fn.apply(*leaves, *rest), leaves, up, create_graph=True)
+    with pytest.raises(RuntimeError, match="not implemented"):
+        torch.autograd.grad(again[-1].float().sum(), up[0])

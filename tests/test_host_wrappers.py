@@ -56,6 +56,22 @@ def test_dfw_contract():
         DFWFunction.apply(q, k, v, s)
 
 
+def test_gradients_refuse_a_second_derivative():
+    """Gradients formed in grad mode raise when differentiated, also where only a saved tensor required gradients."""
+    from t2fw_b200._lib import load_ops
+
+    mark = load_ops().no_second_derivative
+    x, up = torch.randn(3, requires_grad=True), torch.randn(3)
+    r, _ = mark([torch.ones(3), torch.zeros(3)], (up, x))
+    assert torch.equal(r, torch.ones(3))
+    for derive in (lambda y: y.backward(), lambda y: torch.autograd.grad(y, x)):
+        with pytest.raises(RuntimeError, match="not implemented"):
+            derive(r.sum() + x.square().sum())
+    with torch.no_grad():
+        assert not mark([torch.ones(3)], (up, x))[0].requires_grad
+    assert not mark([torch.ones(3)], (up,))[0].requires_grad
+
+
 def test_numa_binding_reads_the_topology(tmp_path):
     """bind_host_to_gpu_node's sysfs logic on a fake tree: node lookup, CPU list parsing, the
     intersection with the allowed set, and the reasons it gives when it cannot bind."""
