@@ -280,8 +280,10 @@ dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state
 // ---- gradients: grid = B * nc, eight warps ---------------------------------------------------------------------
 // Two groups of four warps, warp w of a group = steps 16 w ..: group 0 forms E and everything that contracts with
 // strictly lower blocks (d_query, part of d_key), group 1 the rest of d_key; equal numbers of products, and half
-// the registers of one group doing both.
+// the registers of one group doing both.  The groups meet at a named barrier: each of the five meetings is in both
+// branches, where __syncthreads() would be undefined.
 constexpr int kThreadsG = 256;
+__device__ __forceinline__ void meet() { asm volatile("bar.sync 1, %0;" ::"n"(kThreadsG) : "memory"); }
 constexpr int kLdD = 72;      // row stride of Dl: 8-byte reads along its rows are free of bank conflicts
 constexpr int oKg = 0, oQg = kRaw, oGg = 2 * kRaw, oDg = 3 * kRaw, oRg = oDg + kC * kLdD * 4;      // R, then E image
 constexpr int oSg = oRg + kImg * 4;                                                               // S0^T image, then group 0's d_key
@@ -338,7 +340,7 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
       e[n][0] = u0.x; e[n][1] = u0.y; e[n][2] = u1.x; e[n][3] = u1.y;
     }
     wait<1>();
-    __syncthreads();             // R and Dl are there
+    meet();             // R and Dl are there
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
@@ -347,7 +349,7 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
         mma_acc_a(e[n], ea[j], bits(r2.x), bits(r2.y));
       }
     wait<0>();
-    __syncthreads();             // R has been read by both groups; raw blocks and S0^T are there
+    meet();             // R has been read by both groups; raw blocks and S0^T are there
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
 #pragma unroll
@@ -356,7 +358,7 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
       *reinterpret_cast<uint32_t *>(sm + oEg + raw_off(r0, n) + 4 * t) = pack16<T>(e[n][0], e[n][1]);
       *reinterpret_cast<uint32_t *>(sm + oEg + raw_off(r1, n) + 4 * t) = pack16<T>(e[n][2], e[n][3]);
     }
-    __syncthreads();             // (-E) image complete
+    meet();             // (-E) image complete
     rows_out<T>(dv + base, sm + oEg, w, nvalid, lane);
     uint32_t ga[4][4];      // dO, own rows
 #pragma unroll
@@ -407,17 +409,17 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
           }
       }
     }
-    __syncthreads();             // S0^T, Q and K have been read
+    meet();             // S0^T, Q and K have been read
     store_rows<false>(Ss, ck, w, lane);
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       *reinterpret_cast<uint32_t *>(sm + oQg + raw_off(r0, n) + 4 * t) = pack16<T>(cq[n][0], cq[n][1]);
       *reinterpret_cast<uint32_t *>(sm + oQg + raw_off(r1, n) + 4 * t) = pack16<T>(cq[n][2], cq[n][3]);
     }
-    __syncthreads();             // group 0's part of d_key is there
+    meet();             // group 0's part of d_key is there
   } else {
     wait<1>();
-    __syncthreads();
+    meet();
     uint32_t da[8][4];      // Dl, own rows
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -432,8 +434,8 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
         mma_acc_a(ck[n], da[j], bits(Rs[r_off(8 * j + 2 * t, 8 * n + g)]), bits(Rs[r_off(8 * j + 2 * t + 1, 8 * n + g)]));
       }
     wait<0>();
-    __syncthreads();
-    __syncthreads();             // (-E) image complete
+    meet();
+    meet();             // (-E) image complete
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float4 e4 = image_at(Es, w, j, lane);
@@ -490,8 +492,8 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
           }
       }
     }
-    __syncthreads();
-    __syncthreads();
+    meet();
+    meet();
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       const float4 c4 = image_at(Ss, w, n, lane);

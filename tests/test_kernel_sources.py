@@ -1,0 +1,46 @@
+"""Rules of the programming model that a GPU run cannot show to be broken, checked in the kernels' sources."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "t2fw_b200", "csrc")
+SOURCES = sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
+
+# a condition on one of these differs between the threads of a block
+PER_THREAD = re.compile(r"\b(threadIdx|tid|lane|warp|group|w)\b")
+
+
+def _text(path):
+    with open(path) as f:
+        return re.sub(r"//[^\n]*|/\*.*?\*/", "", f.read(), flags=re.S)
+
+
+def _block(text, start):
+    """The text between the brace at `start` and its partner, and where that ends."""
+    depth = 0
+    for i in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[start:i + 1], i + 1
+    raise AssertionError("unbalanced braces")
+
+
+def _branches(text):
+    """(condition, text of the branch) of every braced if, its else branches under the same condition."""
+    for m in re.finditer(r"\bif (?:constexpr )?\(([^{};]*)\) \{", text):
+        body, end = _block(text, m.end() - 1)
+        yield m.group(1), body
+        e = re.match(r"\s*else \{", text[end:])
+        if e:
+            yield m.group(1), _block(text, end + e.end() - 1)[0]
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_block_barriers_are_reached_by_the_whole_block(path):
+    """__syncthreads() under a condition that differs within the block is undefined, also where every thread meets some
+    __syncthreads(); groups of warps on different paths meet at named barriers."""
+    for cond, body in _branches(_text(path)):
+        if PER_THREAD.search(cond):
+            assert not re.search(r"__syncthreads\(|\bsync_all\(", body), "if (%s)" % cond
