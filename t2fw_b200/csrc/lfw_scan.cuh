@@ -20,9 +20,11 @@
 // (scan.cuh); the sums of a step share their shuffles; the two orientations run side by side; the backward
 // walks a checkpoint's steps forward once to leave the state at each segment start and then segment by segment
 // (128 forward steps per 64 instead of 160).  Eight, 16 or 32 lanes own a line (lanes_for), and eight sums are formed
-// together: seven exchanges for four lines where a line per warp took 40.  fp32, 16 rows of 129 steps, 96 x 48: forward
-// 95 -> 16.5 us, backward 366 -> 70 us (84 with a warp per two lines); 48 x 300, 100 x 100, forward and backward
-// 2475 -> 1136; 8 x 128, 256 x 256 825 -> 476.
+// together: seven exchanges for four lines where a line per warp took 40.
+//
+// The two orientations of the backward are one launch: kernels of their own would run one after the other (16 x 129, 96 x 48,
+// fp32: 107 us against 72), or the second would read its inputs on the word of the first that they are there, for which
+// there is no rule.
 //
 // These kernels also redo the batch rows that the chunk kernels flagged (gate products outside the range of
 // the factored form): CTAs walk over all work items and skip the rows without a flag, and the launch is a
@@ -31,6 +33,8 @@
 // The kernels are templates; lfw_scan_{f16,bf16,f32,f64}.cu instantiate them for one storage type each (compiled side
 // by side), lfw_scan.cu picks the type.
 #pragma once
+
+#include <initializer_list>
 
 #include "scan.cuh"
 
@@ -52,6 +56,7 @@ namespace {
 
 constexpr int kWarpsPerCta = 4;
 constexpr int kThreads = kWarpsPerCta * 32;
+constexpr size_t kSmemMost = 224 * 1024;      // backward: dynamic shared memory of a CTA
 
 template <typename T>
 struct FwdArgs {
@@ -184,7 +189,8 @@ struct LineArgs {
   T *d_state;             // row orientation only
   int NO, NLn;            // own extent, lane extent
   int64_t so, sl;         // strides of the own / lane axis inside one [D,K] state
-  int64_t items;          // work items: (batch row, block of own lines)
+  int64_t items;          // work items: (batch row, block of own lines); 0: not in this launch
+  int seg, mids;          // steps per segment; segment starts whose states are kept besides the chunk's
 };
 
 template <typename T>
@@ -192,7 +198,6 @@ struct BwdArgs {
   LineArgs<T> col, row;
   const T *state0, *ckpt, *grad_state;
   int64_t B, T_, C, nslots;
-  int seg, mids;          // steps per segment; segment starts whose states are kept besides the chunk's
   const int *rowflag;
 };
 
@@ -236,70 +241,67 @@ struct SegWalk {
 template <typename T>
 __host__ __device__ inline int bwd_part(int seg, int n) { return (int)((((size_t)seg * n * sizeof(T)) + 15) / 16 * 16); }
 
-template <typename T, int L, int NL, int SAFE, int OWN, bool WITH_SP>
-__device__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> &ln, int64_t item, int vec_ext, unsigned char *smem) {
+// One block of own lines of batch row b
+template <typename T, int L, int NL, int SAFE, bool WITH_SP>
+__device__ __forceinline__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> &ln, int64_t b, int block, unsigned char *smem) {
   using A = typename Elem<T>::acc;
-  constexpr int RC = kThreads / L * OWN;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = tid % L, rl = tid / L * OWN;
-  const int lp = bwd_part<T>(a.seg, vec_ext), op = bwd_part<T>(a.seg, RC), buf_bytes = 3 * lp + 3 * op;
-  A *hist = reinterpret_cast<A *>(smem + 2 * buf_bytes) + (size_t)warp * (a.seg + a.mids) * OWN * NL * 32;
-  A *mid = hist + (size_t)a.seg * OWN * NL * 32;
+  constexpr int RC = kThreads / L;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = tid % L, rl = tid / L;
+  const int lp = bwd_part<T>(ln.seg, ln.NLn), op = bwd_part<T>(ln.seg, RC), buf_bytes = 3 * lp + 3 * op;
+  A *hist = reinterpret_cast<A *>(smem + 2 * buf_bytes) + (size_t)warp * (ln.seg + ln.mids) * NL * 32;
+  A *mid = hist + (size_t)ln.seg * NL * 32;
 
-  const int blocks = (ln.NO + RC - 1) / RC;
-  const int64_t b = item / blocks;
-  const int ob = (int)(item - b * blocks) * RC, nown = ln.NO - ob < RC ? ln.NO - ob : RC;
+  const int ob = block * RC, nown = ln.NO - ob < RC ? ln.NO - ob : RC;
   const int o0 = ob + rl;
+  const bool mine = o0 < ln.NO;
   const int64_t DK = (int64_t)ln.NO * ln.NLn;
 
-  auto state_off = [&](int o, int j) { return (o0 + o) * ln.so + (int64_t)(l + L * j) * ln.sl; };
-  auto valid = [&](int o, int j) { return (o0 + o) < ln.NO && (l + L * j) < ln.NLn; };
+  auto state_off = [&](int j) { return o0 * ln.so + (int64_t)(l + L * j) * ln.sl; };
+  auto valid = [&](int j) { return mine && (l + L * j) < ln.NLn; };
 
   SegWalk w;
-  w.T_ = a.T_; w.C = a.C; w.seg = a.seg; w.mids = a.mids;
+  w.T_ = a.T_; w.C = a.C; w.seg = ln.seg; w.mids = ln.mids;
   w.c = (a.T_ + a.C - 1) / a.C - 1;
   w.open();
   auto fetch = [&](const SegWalk &s, int which) {
     const int n = s.count();
     const int64_t lo = (b * a.T_ + s.first()) * ln.NLn, oo = (b * a.T_ + s.first()) * ln.NO + ob;
     unsigned char *p = smem + which * buf_bytes;
-    scan::stage(reinterpret_cast<T *>(p), ln.xl + lo, n * ln.NLn, tid, kThreads);
-    scan::stage(reinterpret_cast<T *>(p + lp), ln.gl + lo, n * ln.NLn, tid, kThreads);
-    scan::stage_rows(reinterpret_cast<T *>(p + 3 * lp), ln.xo + oo, n, nown, ln.NO, tid, kThreads);
-    scan::stage_rows(reinterpret_cast<T *>(p + 3 * lp + op), ln.go + oo, n, nown, ln.NO, tid, kThreads);
+    scan::stage<T, true>(reinterpret_cast<T *>(p), ln.xl + lo, n * ln.NLn, tid, kThreads);
+    scan::stage<T, true>(reinterpret_cast<T *>(p + lp), ln.gl + lo, n * ln.NLn, tid, kThreads);
+    scan::stage_rows<T, true>(reinterpret_cast<T *>(p + 3 * lp), ln.xo + oo, n, nown, ln.NO, tid, kThreads);
+    scan::stage_rows<T, true>(reinterpret_cast<T *>(p + 3 * lp + op), ln.go + oo, n, nown, ln.NO, tid, kThreads);
     if (s.cur == s.target) {      // upstream vectors: only where the gradients are formed
-      scan::stage(reinterpret_cast<T *>(p + 2 * lp), ln.pl + lo, n * ln.NLn, tid, kThreads);
-      scan::stage_rows(reinterpret_cast<T *>(p + 3 * lp + 2 * op), ln.po + oo, n, nown, ln.NO, tid, kThreads);
+      scan::stage<T, true>(reinterpret_cast<T *>(p + 2 * lp), ln.pl + lo, n * ln.NLn, tid, kThreads);
+      scan::stage_rows<T, true>(reinterpret_cast<T *>(p + 3 * lp + 2 * op), ln.po + oo, n, nown, ln.NO, tid, kThreads);
     }
     scan::commit();
   };
-  fetch(w, 0);
-
-  A R[OWN][NL], S[OWN][NL];
+  A R[NL], S[NL];
 #pragma unroll
-  for (int o = 0; o < OWN; ++o)
-#pragma unroll
-    for (int j = 0; j < NL; ++j)
-      R[o][j] = valid(o, j) ? Elem<T>::ld(a.grad_state + b * DK + state_off(o, j)) : A(0);
+  for (int j = 0; j < NL; ++j)
+    R[j] = valid(j) ? Elem<T>::ld(a.grad_state + b * DK + state_off(j)) : A(0);
 
-  int which = 0;
-  while (w.c >= 0) {
-    SegWalk nx = w;
-    nx.step();
+  SegWalk nx = w;
+  int which = 1;
+#pragma unroll 1
+  for (bool first = true; first || w.c >= 0; first = false) {      // the first trip only fetches
     if (nx.c >= 0) fetch(nx, which ^ 1);
     else scan::commit();
+    if (first) {
+      nx.step();
+      which = 0;
+      continue;
+    }
 
     if (w.cur == 0) {      // the interval's own checkpoint
       const T *src = (w.c == 0) ? a.state0 + b * DK : a.ckpt + (b * a.nslots + (w.c - 1)) * DK;
 #pragma unroll
-      for (int o = 0; o < OWN; ++o)
-#pragma unroll
-        for (int j = 0; j < NL; ++j) S[o][j] = valid(o, j) ? Elem<T>::ld(src + state_off(o, j)) : A(0);
+      for (int j = 0; j < NL; ++j) S[j] = valid(j) ? Elem<T>::ld(src + state_off(j)) : A(0);
     } else if (w.target >= 0 && w.cur % w.ms == 0) {      // a kept segment start
-      const A *m = mid + (size_t)(w.cur / w.ms - 1) * OWN * NL * 32;
+      const A *m = mid + (size_t)(w.cur / w.ms - 1) * NL * 32;
 #pragma unroll
-      for (int o = 0; o < OWN; ++o)
-#pragma unroll
-        for (int j = 0; j < NL; ++j) S[o][j] = m[(o * NL + j) * 32 + lane];
+      for (int j = 0; j < NL; ++j) S[j] = m[j * 32 + lane];
     }
     scan::wait<1>();
     __syncthreads();
@@ -314,119 +316,94 @@ __device__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> &ln, int64_t ite
     auto vec = [&](const T *v, int t, int j) {
       return (j < SAFE || l + L * j < ln.NLn) ? Elem<T>::ld(v + t * ln.NLn + L * j) : A(0);
     };
-    auto own = [&](const T *v, int t, int o) { return o0 + o < ln.NO ? Elem<T>::ld(v + t * nown + o) : A(0); };
+    auto own = [&](const T *v, int t) { return mine ? Elem<T>::ld(v + t * nown) : A(0); };
 
 #pragma unroll(NL <= 8 ? 2 : 1)
     for (int t = 0; t < n; ++t) {      // forward over the segment
-      A xo[OWN], go[OWN];
-#pragma unroll
-      for (int o = 0; o < OWN; ++o) {
-        xo[o] = own(s_xo, t, o);
-        go[o] = own(s_go, t, o);
-      }
+      const A xo = own(s_xo, t), go = own(s_go, t);
 #pragma unroll
       for (int j = 0; j < NL; ++j) {
         const A g = vec(s_gl, t, j), x = vec(s_xl, t, j);
-#pragma unroll
-        for (int o = 0; o < OWN; ++o) {
-          if (last) hist[((t * OWN + o) * NL + j) * 32 + lane] = S[o][j];
-          S[o][j] = S[o][j] * (go[o] * g) + xo[o] * x;
-        }
+        if (last) hist[(t * NL + j) * 32 + lane] = S[j];
+        S[j] = S[j] * (go * g) + xo * x;
       }
     }
     if (w.target < 0 && (w.cur + 1) % w.ms == 0) {
-      A *m = mid + (size_t)((w.cur + 1) / w.ms - 1) * OWN * NL * 32;
+      A *m = mid + (size_t)((w.cur + 1) / w.ms - 1) * NL * 32;
 #pragma unroll
-      for (int o = 0; o < OWN; ++o)
-#pragma unroll
-        for (int j = 0; j < NL; ++j) m[(o * NL + j) * 32 + lane] = S[o][j];
+      for (int j = 0; j < NL; ++j) m[j * 32 + lane] = S[j];
     }
     if (last) {
       const int64_t ob_t = (b * a.T_ + w.first()) * ln.NO + o0;
-      constexpr int kSums = WITH_SP ? 4 : 2, kStep = kSums * OWN, U = 8 / kStep;      // U steps' sums are formed together
+      constexpr int kSums = WITH_SP ? 4 : 2, U = 8 / kSums;      // U steps' sums are formed together
       auto step = [&](int t, A *v) {      // S is the state after step t
-        A go[OWN], po[OWN];
+        const A go = own(s_go, t), po = own(s_po, t);
 #pragma unroll
-        for (int o = 0; o < OWN; ++o) {
-          go[o] = own(s_go, t, o);
-          po[o] = own(s_po, t, o);
-        }
-#pragma unroll
-        for (int i = 0; i < kStep; ++i) v[i] = A(0);
+        for (int i = 0; i < kSums; ++i) v[i] = A(0);
 #pragma unroll
         for (int j = 0; j < NL; ++j) {
           const A g = vec(s_gl, t, j), x = vec(s_xl, t, j), p = vec(s_pl, t, j);
-#pragma unroll
-          for (int o = 0; o < OWN; ++o) {
-            const A sp = hist[((t * OWN + o) * NL + j) * 32 + lane];
-            const A r = R[o][j] + po[o] * p;    // gradient w.r.t. S_t
-            v[kSums * o] += r * x;
-            v[kSums * o + 1] += (r * sp) * g;
-            if (WITH_SP) v[kSums * o + 2] += S[o][j] * p;
-            R[o][j] = r * (go[o] * g);          // what flows on to S_{t-1}
-            S[o][j] = sp;
-          }
+          const A sp = hist[(t * NL + j) * 32 + lane];
+          const A r = R[j] + po * p;    // gradient w.r.t. S_t
+          v[0] += r * x;
+          v[1] += (r * sp) * g;
+          if (WITH_SP) v[2] += S[j] * p;
+          R[j] = r * (go * g);          // what flows on to S_{t-1}
+          S[j] = sp;
         }
       };
       auto put = [&](int t, int i, A v) {      // sum i of the steps t, t - 1, ..
-        const int o = i % kStep / kSums, kind = i % kSums;
-        if (kind < 3 && o0 + o < ln.NO) {
+        const int kind = i % kSums;
+        if (kind < 3 && mine) {
           T *dst = kind == 0 ? ln.d_xo : kind == 1 ? ln.d_go : ln.d_po;
-          Elem<T>::st(dst + ob_t + (int64_t)(t - i / kStep) * ln.NO + o, v);
+          Elem<T>::st(dst + ob_t + (int64_t)(t - i / kSums) * ln.NO, v);
         }
       };
       int t = n - 1, i;
       for (; t + 1 >= U; t -= U) {
         A v[8];
 #pragma unroll
-        for (int u = 0; u < U; ++u) step(t - u, v + u * kStep);
+        for (int u = 0; u < U; ++u) step(t - u, v + u * kSums);
         if (scan::lane_sums<8, L>(v, l, &i)) put(t, i, v[0]);
       }
       for (; t >= 0; --t) {
-        A v[kStep];
+        A v[kSums];
         step(t, v);
-        if (scan::lane_sums<kStep, L>(v, l, &i)) put(t, i, v[0]);
+        if (scan::lane_sums<kSums, L>(v, l, &i)) put(t, i, v[0]);
       }
     }
     __syncthreads();
     w = nx;
+    nx.step();
     which ^= 1;
   }
   if (!WITH_SP) {
 #pragma unroll
-    for (int o = 0; o < OWN; ++o)
-#pragma unroll
-      for (int j = 0; j < NL; ++j)
-        if (valid(o, j)) Elem<T>::st(ln.d_state + b * DK + state_off(o, j), R[o][j]);
+    for (int j = 0; j < NL; ++j)
+      if (valid(j)) Elem<T>::st(ln.d_state + b * DK + state_off(j), R[j]);
   }
 }
 
-// kBoth: both orientations in one launch (redoing flagged rows).  Otherwise two launches, columns first, then
-// rows: the row launch may start as soon as every CTA of the column launch has (which is after everything before
-// it has completed), runs beside it, and ends only after it, so that what follows may rely on both.
-enum Part { kBoth = 0, kColumns = 1, kRows = 2 };
-
-template <typename T, int L, int NL, int SAFE, int OWN>
-__global__ void __launch_bounds__(kThreads) lfw_line_bwd_kernel(const BwdArgs<T> a, const int part) {
+// Both orientations side by side, the columns' items first.  LC, NC, SC: lanes, elements per lane (NL) and elements that
+// exist for every line (SAFE) of the columns; LR, NR, SR: of the rows.
+template <typename T, int LC, int NC, int SC, int LR, int NR, int SR>
+__global__ void __launch_bounds__(kThreads) lfw_line_bwd_kernel(const BwdArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int RC = kThreads / L * OWN;
-  const int ext = part == kRows || (part == kBoth && a.row.NLn > a.col.NLn) ? a.row.NLn : a.col.NLn;
-  if (part != kRows) dependency_wait();
-  const int64_t first_row = part == kRows ? 0 : a.col.items, n = first_row + (part == kColumns ? 0 : a.row.items);
-  for (int64_t item = blockIdx.x; item < n; item += gridDim.x) {
-    const bool col = item < first_row;
-    const int64_t i = col ? item : item - first_row;
-    const int64_t b = i / (((col ? a.col.NO : a.row.NO) + RC - 1) / RC);
-    if (a.rowflag != nullptr && a.rowflag[b] == 0) continue;
-    if (col) line_bwd<T, L, NL, SAFE, OWN, true>(a, a.col, i, ext, smem_raw);
-    else line_bwd<T, L, NL, SAFE, OWN, false>(a, a.row, i, ext, smem_raw);
+  dependency_wait();
+  for (int64_t item = blockIdx.x; item < a.col.items + a.row.items; item += gridDim.x) {
+    const bool col = item < a.col.items;
+    const int64_t i = col ? item : item - a.col.items;
+    const int blocks = col ? (a.col.NO + kThreads / LC - 1) / (kThreads / LC) : (a.row.NO + kThreads / LR - 1) / (kThreads / LR);
+    const int64_t b = i / blocks;
+    if (a.rowflag != nullptr && a.rowflag[b] == 0) continue;      // the same for the whole CTA
+    if (col) line_bwd<T, LC, NC, SC, true>(a, a.col, b, (int)(i - b * blocks), smem_raw);
+    else line_bwd<T, LR, NR, SR, false>(a, a.row, b, (int)(i - b * blocks), smem_raw);
   }
-  if (part == kRows) dependency_wait();
 }
 
-// Lanes per line for lines of up to 128 elements.  Eight cost the fewest instructions, where they still give every
-// scheduler a warp and a half; with fewer lines a step's length is what counts, and the lines are spread over 16 lanes
-// while that fills half of the schedulers, over a warp below.
+// Lanes per line for lines of up to 128 elements (backward: by the mean of the two orientations' lines).  Eight cost the
+// fewest instructions, where they still give every scheduler a warp and a half; with fewer lines a step's length is what
+// counts, and the lines are spread over 16 lanes while that fills half of the schedulers, over a warp below.
 int lanes_for(int64_t lines) { return lines >= 148 * 24 ? 8 : lines >= 148 * 4 ? 16 : 32; }
 
 // CTAs of a launch: one per work item; the walk over flagged rows only is cut to a few waves
@@ -466,112 +443,130 @@ int fwd_typed(const void *x, const void *f, const void *q, const void *k, const 
   a.x = (const T *)x; a.f = (const T *)f; a.q = (const T *)q; a.k = (const T *)k; a.fk = (const T *)fk;
   a.state = (const T *)state; a.out = (T *)out; a.ckpt = (T *)ckpt;
   a.B = B; a.T_ = T_; a.D = (int)D; a.K = (int)K; a.C = C; a.nslots = ceil_div64(T_, C); a.rowflag = rowflag;
-  // elements per lane: the smallest that holds the row
-  const int lanes = rowflag != nullptr ? 8 : lanes_for(B * D);
-  if (K <= 128 && lanes == 32) {
-    if (K <= 32) return launch_fwd<T, 32, 1, 0, 1>(a, st);
-    if (K <= 64) return launch_fwd<T, 32, 2, 1, 1>(a, st);
-    if (K <= 96) return launch_fwd<T, 32, 3, 2, 1>(a, st);
-    return launch_fwd<T, 32, 4, 3, 1>(a, st);
+  // elements per lane: the smallest that holds the row (double: in four sizes)
+  if constexpr (sizeof(T) == 8) {
+    if (K <= 64) return launch_fwd<T, 32, 2, 0, 1>(a, st);
+    if (K <= 128) return launch_fwd<T, 32, 4, 0, 1>(a, st);
+    if (K <= 256) return launch_fwd<T, 32, 8, 0, 1>(a, st);
+    if (K <= 512) return launch_fwd<T, 32, 16, 0, 1>(a, st);
+  } else {
+    const int lanes = rowflag != nullptr ? 8 : lanes_for(B * D);
+    if (K <= 128 && lanes == 32) {
+      if (K <= 32) return launch_fwd<T, 32, 1, 0, 1>(a, st);
+      if (K <= 64) return launch_fwd<T, 32, 2, 1, 1>(a, st);
+      if (K <= 96) return launch_fwd<T, 32, 3, 2, 1>(a, st);
+      return launch_fwd<T, 32, 4, 3, 1>(a, st);
+    }
+    if (K <= 128 && lanes == 16) {
+      if (K <= 32) return launch_fwd<T, 16, 2, 0, 1>(a, st);
+      if (K <= 48) return launch_fwd<T, 16, 3, 2, 1>(a, st);
+      if (K <= 64) return launch_fwd<T, 16, 4, 3, 1>(a, st);
+      if (K <= 96) return launch_fwd<T, 16, 6, 4, 1>(a, st);
+      return launch_fwd<T, 16, 8, 6, 1>(a, st);
+    }
+    if (K <= 16) return launch_fwd_rows<T, 8, 2, 0, 2>(a, st);
+    if (K <= 32) return launch_fwd_rows<T, 8, 4, 2, 2>(a, st);
+    if (K <= 48) return launch_fwd_rows<T, 8, 6, 4, 2>(a, st);
+    if (K <= 64) return launch_fwd_rows<T, 8, 8, 6, 2>(a, st);
+    if (K <= 80) return launch_fwd_rows<T, 8, 10, 8, 2>(a, st);
+    if (K <= 104) return launch_fwd_rows<T, 8, 13, 10, 2>(a, st);
+    if (K <= 128) return launch_fwd_rows<T, 8, 16, 13, 2>(a, st);
+    if (K <= 256) return launch_fwd_rows<T, 32, 8, 4, 4>(a, st);
+    if (K <= 512) return launch_fwd_rows<T, 32, 16, 8, 4>(a, st);
   }
-  if (K <= 128 && lanes == 16) {
-    if (K <= 32) return launch_fwd<T, 16, 2, 0, 1>(a, st);
-    if (K <= 48) return launch_fwd<T, 16, 3, 2, 1>(a, st);
-    if (K <= 64) return launch_fwd<T, 16, 4, 3, 1>(a, st);
-    if (K <= 96) return launch_fwd<T, 16, 6, 4, 1>(a, st);
-    return launch_fwd<T, 16, 8, 6, 1>(a, st);
-  }
-  if (K <= 16) return launch_fwd_rows<T, 8, 2, 0, 2>(a, st);
-  if (K <= 32) return launch_fwd_rows<T, 8, 4, 2, 2>(a, st);
-  if (K <= 48) return launch_fwd_rows<T, 8, 6, 4, 2>(a, st);
-  if (K <= 64) return launch_fwd_rows<T, 8, 8, 6, 2>(a, st);
-  if (K <= 80) return launch_fwd_rows<T, 8, 10, 8, 2>(a, st);
-  if (K <= 104) return launch_fwd_rows<T, 8, 13, 10, 2>(a, st);
-  if (K <= 128) return launch_fwd_rows<T, 8, 16, 13, 2>(a, st);
-  if (K <= 256) return launch_fwd_rows<T, 32, 8, 4, 4>(a, st);
-  if (K <= 512) return launch_fwd_rows<T, 32, 16, 8, 4>(a, st);
   set_error("lfw forward: K=%lld exceeds the supported maximum of 512", (long long)K);
   return T2FW_ERR_UNSUPPORTED;
 }
 
 namespace {
 
-template <typename T, int L, int NL, int SAFE>
-int launch_bwd(BwdArgs<T> a, int part, cudaStream_t st) {
+template <typename T, int LC, int NC, int SC, int LR, int NR, int SR>
+int launch_lines(BwdArgs<T> a, cudaStream_t st) {
   using A = typename Elem<T>::acc;
-  constexpr int OWN = 1, RC = kThreads / L;
-  const int ext = part == kRows || (part == kBoth && a.row.NLn > a.col.NLn) ? a.row.NLn : a.col.NLn;
-  a.col.items = a.B * ((a.col.NO + RC - 1) / RC);
-  a.row.items = a.B * ((a.row.NO + RC - 1) / RC);
-  const int64_t items = (part != kRows ? a.col.items : 0) + (part != kColumns ? a.row.items : 0);
-  auto bytes = [&](int seg, int mids) {
-    return 2 * (size_t)(3 * bwd_part<T>(seg, ext) + 3 * bwd_part<T>(seg, RC)) +
-           (size_t)kWarpsPerCta * (seg + mids) * OWN * NL * 32 * sizeof(A);
-  };
+  if (a.col.items) a.col.items = a.B * ceil_div64(a.col.NO, kThreads / LC);
+  if (a.row.items) a.row.items = a.B * ceil_div64(a.row.NO, kThreads / LR);
+  const int64_t items = a.col.items + a.row.items;
   // Segments of 16 steps and as many kept starts as an interval of 64 steps has, where that leaves room for two CTAs per
   // SM (a launch that does not fill the chip once may take the SM); else less history.
-  constexpr size_t kMost = 224 * 1024;
-  const size_t most = items <= 148 && part != kBoth ? kMost : 112 * 1024;
-  a.seg = 16;
-  a.mids = 3;
-  while (a.seg > 4 && bytes(a.seg, a.mids) > most) a.seg /= 2;
-  while (bytes(a.seg, a.mids) > kMost && (a.seg > 1 || a.mids > 1)) {
-    if (a.mids > a.seg) a.mids /= 2;
-    else a.seg /= 2;
+  const size_t most = items <= 148 && a.rowflag == nullptr ? kSmemMost : 112 * 1024;
+  size_t smem = 0;
+  for (int which = 0; which < 2; ++which) {
+    LineArgs<T> &ln = which ? a.row : a.col;
+    auto bytes = [&](int seg, int mids) {
+      return 2 * (size_t)(3 * bwd_part<T>(seg, ln.NLn) + 3 * bwd_part<T>(seg, kThreads / (which ? LR : LC))) +
+             (size_t)kWarpsPerCta * (seg + mids) * (which ? NR : NC) * 32 * sizeof(A);
+    };
+    int seg = 16, mids = 3;
+    while (seg > 4 && bytes(seg, mids) > most) seg /= 2;
+    while (bytes(seg, mids) > kSmemMost && (seg > 1 || mids > 1)) {
+      if (mids > seg) mids /= 2;
+      else seg /= 2;
+    }
+    while (mids < 7 && bytes(seg, mids + 4) <= most) mids += 4;
+    ln.seg = seg;
+    ln.mids = mids;
+    if (ln.items && bytes(seg, mids) > smem) smem = bytes(seg, mids);
   }
-  while (a.mids < 7 && bytes(a.seg, a.mids + 4) <= most) a.mids += 4;
-  const size_t smem = bytes(a.seg, a.mids);
-  if (smem > kMost) {
+  if (smem > kSmemMost) {
     set_error("lfw backward: %zu bytes of shared memory needed", smem);
     return T2FW_ERR_UNSUPPORTED;
   }
-  auto *const kernel = &lfw_line_bwd_kernel<T, L, NL, SAFE, OWN>;
-  T2FW_ALLOW_SMEM(kernel, (int)kMost);
-  T2FW_CHECK_CUDA(launch_dependent(kernel, dim3(grid_for(items, a.rowflag)), dim3(kThreads), smem, st, a, part));
+  auto *const kernel = &lfw_line_bwd_kernel<T, LC, NC, SC, LR, NR, SR>;
+  T2FW_ALLOW_SMEM(kernel, (int)kSmemMost);
+  T2FW_CHECK_CUDA(launch_dependent(kernel, dim3(grid_for(items, a.rowflag)), dim3(kThreads), smem, st, a));
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;
 }
 
-// one orientation: elements per lane are the smallest that hold the lines
-template <typename T>
-int launch_part(const BwdArgs<T> &a, int part, cudaStream_t st) {
-  const int n = part == kColumns ? a.col.NLn : a.row.NLn;
-  const int lanes = lanes_for(a.B * (part == kColumns ? a.col.NO : a.row.NO));
-  if (n <= 128 && lanes == 32) {
-    if (n <= 32) return launch_bwd<T, 32, 1, 0>(a, part, st);
-    if (n <= 64) return launch_bwd<T, 32, 2, 1>(a, part, st);
-    if (n <= 96) return launch_bwd<T, 32, 3, 2>(a, part, st);
-    return launch_bwd<T, 32, 4, 3>(a, part, st);
+// A rung serves the longer orientation's lines; `m` is the length of the other's.  Nearly as long: the same rung, without
+// conditions on the elements that exist.  Up to half as long: half of the lanes with the same elements per lane (of eight
+// lanes half of the elements).  Between: the same rung with conditions.  fp32, 16 x 129, 96 x 48: 72 us (with conditions
+// 80); 48 x 300, 100 x 50: 506 (728); 16 x 129, 96 x 64: 130.
+template <typename T, int L, int NL, int SAFE>
+int launch_rung(const BwdArgs<T> &a, int m, cudaStream_t st) {
+  if constexpr (SAFE > 0) {
+    constexpr int LH = L > 8 ? L / 2 : 8, NH = L > 8 ? NL : (NL + 1) / 2;
+    if (m > L * SAFE) return launch_lines<T, L, NL, SAFE, L, NL, SAFE>(a, st);
+    if (m <= LH * NH)
+      return a.col.NLn > a.row.NLn ? launch_lines<T, L, NL, SAFE, LH, NH, 0>(a, st) : launch_lines<T, LH, NH, 0, L, NL, SAFE>(a, st);
   }
-  if (n <= 128 && lanes == 16) {
-    if (n <= 32) return launch_bwd<T, 16, 2, 0>(a, part, st);
-    if (n <= 48) return launch_bwd<T, 16, 3, 2>(a, part, st);
-    if (n <= 64) return launch_bwd<T, 16, 4, 3>(a, part, st);
-    if (n <= 96) return launch_bwd<T, 16, 6, 4>(a, part, st);
-    return launch_bwd<T, 16, 8, 6>(a, part, st);
-  }
-  if (n <= 16) return launch_bwd<T, 8, 2, 0>(a, part, st);
-  if (n <= 32) return launch_bwd<T, 8, 4, 2>(a, part, st);
-  if (n <= 48) return launch_bwd<T, 8, 6, 4>(a, part, st);
-  if (n <= 64) return launch_bwd<T, 8, 8, 6>(a, part, st);
-  if (n <= 80) return launch_bwd<T, 8, 10, 8>(a, part, st);
-  if (n <= 104) return launch_bwd<T, 8, 13, 10>(a, part, st);
-  if (n <= 128) return launch_bwd<T, 8, 16, 13>(a, part, st);
-  if (n <= 256) return launch_bwd<T, 32, 8, 4>(a, part, st);
-  return launch_bwd<T, 32, 16, 8>(a, part, st);
+  // (ten and more conditions per lane are kept in no registers: sixteen lanes, where six elements hold the lines; 48 x 200,
+  // 60 x 90: 475 -> 415 us)
+  if constexpr (L == 8 && NL > 8)
+    if (a.col.NLn <= 96 && a.row.NLn <= 96) return launch_lines<T, 16, 6, 0, 16, 6, 0>(a, st);
+  return launch_lines<T, L, NL, 0, L, NL, 0>(a, st);
 }
 
-// flagged rows, both orientations: only the chunk kernels flag rows, of 16-bit states up to 256 x 256
+// One launch of the orientations asked for.  Rungs: the smallest that holds the lines, for the number of lanes.
 template <typename T>
-int launch_flagged(const BwdArgs<T> &a, cudaStream_t st) {
-  const int n = a.col.NLn > a.row.NLn ? a.col.NLn : a.row.NLn;
-  if constexpr (sizeof(T) == 2) {
-    if (n <= 64) return launch_bwd<T, 8, 8, 0>(a, kBoth, st);
-    if (n <= 128) return launch_bwd<T, 8, 16, 0>(a, kBoth, st);
-    if (n <= 256) return launch_bwd<T, 32, 8, 0>(a, kBoth, st);
+int launch_bwd(BwdArgs<T> a, bool columns, bool rows, cudaStream_t st) {
+  a.col.items = columns;
+  a.row.items = rows;
+  const int nc = columns ? a.col.NLn : a.row.NLn, nr = rows ? a.row.NLn : a.col.NLn;
+  const int n = nc > nr ? nc : nr, m = nc < nr ? nc : nr;
+  if constexpr (sizeof(T) == 8) {
+    if (n <= 64) return launch_rung<T, 32, 2, 0>(a, m, st);
+    if (n <= 128) return launch_rung<T, 32, 4, 0>(a, m, st);
+    return n <= 256 ? launch_rung<T, 32, 8, 0>(a, m, st) : launch_rung<T, 32, 16, 0>(a, m, st);
+  } else {
+    if (n > 256) return launch_rung<T, 32, 16, 8>(a, m, st);
+    if (n > 128) return launch_rung<T, 32, 8, 4>(a, m, st);
+    const int lanes = a.rowflag != nullptr ? 8 : lanes_for(a.B * (a.col.NO + a.row.NO) / 2);
+    if (lanes == 32)
+      return n <= 32 ? launch_rung<T, 32, 1, 0>(a, m, st) : n <= 64 ? launch_rung<T, 32, 2, 1>(a, m, st)
+             : n <= 96 ? launch_rung<T, 32, 3, 2>(a, m, st) : launch_rung<T, 32, 4, 3>(a, m, st);
+    if (lanes >= 16) {
+      if (n <= 32) return launch_rung<T, 16, 2, 0>(a, m, st);
+      if (n <= 48) return launch_rung<T, 16, 3, 2>(a, m, st);
+      if (n <= 64) return launch_rung<T, 16, 4, 3>(a, m, st);
+      return n <= 96 ? launch_rung<T, 16, 6, 4>(a, m, st) : launch_rung<T, 16, 8, 6>(a, m, st);
+    }
+    if (n <= 16) return launch_rung<T, 8, 2, 0>(a, m, st);
+    if (n <= 32) return launch_rung<T, 8, 4, 2>(a, m, st);
+    if (n <= 64) return launch_rung<T, 8, 8, 4>(a, m, st);
+    if (n <= 80) return launch_rung<T, 8, 10, 8>(a, m, st);
+    return n <= 104 ? launch_rung<T, 8, 13, 10>(a, m, st) : launch_rung<T, 8, 16, 13>(a, m, st);
   }
-  set_error("lfw backward: no flagged rows at this size or type");
-  return T2FW_ERR_UNSUPPORTED;
 }
 
 }  // namespace
@@ -593,9 +588,13 @@ int bwd_typed(const void *go, const void *gs, const void *x, const void *f, cons
   col.xl = (const T *)x; col.gl = (const T *)f; col.pl = (const T *)go;
   col.d_xo = (T *)dk; col.d_go = (T *)dfk; col.d_po = (T *)dq; col.d_state = nullptr;
   col.NO = (int)K; col.NLn = (int)D; col.so = 1; col.sl = K;
-  if (rowflag != nullptr) return launch_flagged<T>(a, st);
-  const int rc = launch_part<T>(a, kColumns, st);
-  return rc != T2FW_OK ? rc : launch_part<T>(a, kRows, st);
+  // Arrays that do not start on 16 bytes (views into larger buffers, a rare call) keep a launch per orientation, one after
+  // the other.
+  uintptr_t at = 0;
+  for (const void *p : {go, gs, x, f, q, k, fk, state, ckpt}) at |= reinterpret_cast<uintptr_t>(p);
+  if (rowflag != nullptr || at % 16 == 0) return launch_bwd<T>(a, true, true, st);
+  const int rc = launch_bwd<T>(a, true, false, st);
+  return rc != T2FW_OK ? rc : launch_bwd<T>(a, false, true, st);
 }
 
 #define T2FW_LFW_SCAN_TYPE(T)                                                                                             \

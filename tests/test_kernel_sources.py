@@ -44,3 +44,22 @@ def test_block_barriers_are_reached_by_the_whole_block(path):
     for cond, body in _branches(_text(path)):
         if PER_THREAD.search(cond):
             assert not re.search(r"__syncthreads\(|\bsync_all\(", body), "if (%s)" % cond
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_dependent_launches_wait_first(path):
+    """A kernel that may start before the one ahead of it has ended (launch_dependent) sees that one's writes, and those of
+    every kernel before it, after its own griddepcontrol.wait only: it waits once and without a condition, in the outermost
+    block."""
+    text = _text(path)
+    if "griddepcontrol.wait" in text:      # the definition
+        return
+    for m in re.finditer(r"__global__[^;{]*?\b(\w+_kernel)\([^;{]*\{", text):
+        body, _ = _block(text, m.end() - 1)
+        launched = re.search(r"launch_dependent\(\s*&?\s*%s\b|\*const \w+ = &%s\b" % (m.group(1), m.group(1)), text)
+        if not launched:
+            continue
+        assert body.count("dependency_wait()") == 1, m.group(1)
+        before = body[:body.index("dependency_wait()")]
+        assert before.count("{") - before.count("}") == 1, m.group(1) + ": not in the outermost block"
+        assert re.search(r"[;{}]\s*$", before), m.group(1) + ": under a condition"
