@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 2 : 4) dfw_bwd_cols
     const int n = (int)(a.T_ - t0 < a.G ? a.T_ - t0 : a.G);
     unsigned char *p = smem_raw + which * buf_bytes;
     const int64_t od = (b * a.T_ + t0) * a.D, om = (b * a.T_ + t0) * a.M + mb;
-    scan::stage<A, scan::kRolled<T>>(reinterpret_cast<A *>(p), a.delta + od, n * a.D, tid, kThreads);
-    scan::stage<A, scan::kRolled<T>>(reinterpret_cast<A *>(p + ap), static_cast<const A *>(a.dv_acc) + od, n * a.D, tid, kThreads);
+    scan::stage(reinterpret_cast<A *>(p), a.delta + od, n * a.D, tid, kThreads);
+    scan::stage(reinterpret_cast<A *>(p + ap), static_cast<const A *>(a.dv_acc) + od, n * a.D, tid, kThreads);
     scan::stage(reinterpret_cast<T *>(p + 2 * ap), a.go + od, n * a.D, tid, kThreads);
     scan::stage_rows(reinterpret_cast<T *>(p + 2 * ap + dp), a.k + om, n, ncols, a.M, tid, kThreads);
     scan::stage_rows(reinterpret_cast<T *>(p + 2 * ap + dp + op), a.q + om, n, ncols, a.M, tid, kThreads);

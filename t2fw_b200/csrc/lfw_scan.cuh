@@ -23,7 +23,7 @@
 // together: seven exchanges for four lines where a line per warp took 40.
 //
 // The two orientations of the backward are one launch: kernels of their own would run one after the other (16 x 129, 96 x 48,
-// fp32: 107 us against 72), or the second would read its inputs on the word of the first that they are there, for which
+// fp32: 107 us against 69.5), or the second would read its inputs on the word of the first that they are there, for which
 // there is no rule.
 //
 // These kernels also redo the batch rows that the chunk kernels flagged (gate products outside the range of
@@ -267,13 +267,13 @@ __device__ __forceinline__ void line_bwd(const BwdArgs<T> &a, const LineArgs<T> 
     const int n = s.count();
     const int64_t lo = (b * a.T_ + s.first()) * ln.NLn, oo = (b * a.T_ + s.first()) * ln.NO + ob;
     unsigned char *p = smem + which * buf_bytes;
-    scan::stage<T, true>(reinterpret_cast<T *>(p), ln.xl + lo, n * ln.NLn, tid, kThreads);
-    scan::stage<T, true>(reinterpret_cast<T *>(p + lp), ln.gl + lo, n * ln.NLn, tid, kThreads);
-    scan::stage_rows<T, true>(reinterpret_cast<T *>(p + 3 * lp), ln.xo + oo, n, nown, ln.NO, tid, kThreads);
-    scan::stage_rows<T, true>(reinterpret_cast<T *>(p + 3 * lp + op), ln.go + oo, n, nown, ln.NO, tid, kThreads);
+    scan::stage_rolled(reinterpret_cast<T *>(p), ln.xl + lo, n * ln.NLn, tid, kThreads);
+    scan::stage_rolled(reinterpret_cast<T *>(p + lp), ln.gl + lo, n * ln.NLn, tid, kThreads);
+    scan::stage_rows_rolled(reinterpret_cast<T *>(p + 3 * lp), ln.xo + oo, n, nown, ln.NO, tid, kThreads);
+    scan::stage_rows_rolled(reinterpret_cast<T *>(p + 3 * lp + op), ln.go + oo, n, nown, ln.NO, tid, kThreads);
     if (s.cur == s.target) {      // upstream vectors: only where the gradients are formed
-      scan::stage<T, true>(reinterpret_cast<T *>(p + 2 * lp), ln.pl + lo, n * ln.NLn, tid, kThreads);
-      scan::stage_rows<T, true>(reinterpret_cast<T *>(p + 3 * lp + 2 * op), ln.po + oo, n, nown, ln.NO, tid, kThreads);
+      scan::stage_rolled(reinterpret_cast<T *>(p + 2 * lp), ln.pl + lo, n * ln.NLn, tid, kThreads);
+      scan::stage_rows_rolled(reinterpret_cast<T *>(p + 3 * lp + 2 * op), ln.po + oo, n, nown, ln.NO, tid, kThreads);
     }
     scan::commit();
   };
@@ -520,8 +520,8 @@ int launch_lines(BwdArgs<T> a, cudaStream_t st) {
 
 // A rung serves the longer orientation's lines; `m` is the length of the other's.  Nearly as long: the same rung, without
 // conditions on the elements that exist.  Up to half as long: half of the lanes with the same elements per lane (of eight
-// lanes half of the elements).  Between: the same rung with conditions.  fp32, 16 x 129, 96 x 48: 72 us (with conditions
-// 80); 48 x 300, 100 x 50: 506 (728); 16 x 129, 96 x 64: 130.
+// lanes half of the elements).  Between: the same rung with conditions.  fp32, 16 x 129, 96 x 48: 69.5 us (with
+// conditions 80); 48 x 300, 100 x 50: 473 (728); 16 x 129, 96 x 64: 123.
 template <typename T, int L, int NL, int SAFE>
 int launch_rung(const BwdArgs<T> &a, int m, cudaStream_t st) {
   if constexpr (SAFE > 0) {

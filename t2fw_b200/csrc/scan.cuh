@@ -12,59 +12,78 @@
 namespace t2fw {
 namespace scan {
 
-// Copying loops are kept rolled for 32-bit types (forward 16 x 129, 96 x 48: 15.5 -> 14.6 us) and in the decay rule's
-// backward, whose fetch is part of a long loop body (48 x 300, 100 x 100, fp16: 1012 us unrolled by four, 897 rolled);
-// elsewhere the compiler unrolls the 16-bit ones as it likes (delta-rule backward 48 x 300, 100 x 100: 405 rolled, 375 so).
-template <typename T>
-constexpr bool kRolled = sizeof(T) >= 4;
-
-template <bool ROLLED, typename F>
-__device__ __forceinline__ void each(int first, int n, int step, F f) {
-  if constexpr (ROLLED) {
-#pragma unroll 1
-    for (int i = first; i < n; i += step) f(i);
-  } else {
-    for (int i = first; i < n; i += step) f(i);
-  }
-}
-
 // Asynchronous copy of n elements (contiguous in global and in shared memory) by the whole CTA.  Copies need
 // 4-byte alignment; a 16-bit array at an odd element offset is copied through registers instead (and is then
 // in place after the next barrier like everything else).  dst is 16-byte aligned.
-template <typename T, bool ROLLED = kRolled<T>>
+template <typename T>
 __device__ __forceinline__ void stage(T *dst, const T *src, int n, int tid, int nthreads) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   const int bytes = n * (int)sizeof(T);
   const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-  auto element = [&](int i) { dst[i] = src[i]; };
   if ((a & 15u) == 0) {
     const int n16 = bytes >> 4;
-    each<ROLLED>(tid, n16, nthreads, [&](int i) {
+    for (int i = tid; i < n16; i += nthreads)
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * i), "l"(reinterpret_cast<const char *>(src) + 16 * i) : "memory");
-    });
-    each<ROLLED>((n16 << 4) / (int)sizeof(T) + tid, n, nthreads, element);
+    for (int i = (n16 << 4) / (int)sizeof(T) + tid; i < n; i += nthreads) dst[i] = src[i];
   } else if (sizeof(T) >= 4 || (a & 3u) == 0) {
     const int n4 = bytes >> 2;
-    each<ROLLED>(tid, n4, nthreads, [&](int i) {
+    for (int i = tid; i < n4; i += nthreads)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * i), "l"(reinterpret_cast<const char *>(src) + 4 * i) : "memory");
-    });
-    each<ROLLED>((n4 << 2) / (int)sizeof(T) + tid, n, nthreads, element);
+    for (int i = (n4 << 2) / (int)sizeof(T) + tid; i < n; i += nthreads) dst[i] = src[i];
   } else {
 #pragma unroll 8
     for (int i = tid; i < n; i += nthreads) dst[i] = src[i];
   }
 }
 // n rows of w elements that lie ld elements apart in global memory
-template <typename T, bool ROLLED = kRolled<T>>
+template <typename T>
 __device__ __forceinline__ void stage_rows(T *dst, const T *src, int n, int w, int ld, int tid, int nthreads) {
-  each<ROLLED>(tid, n * w, nthreads, [&](int i) {
+  for (int i = tid; i < n * w; i += nthreads) {
     const int r = i / w, c = i - r * w;
     if constexpr (sizeof(T) >= 4)
       asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + i)),
                    "l"(src + (size_t)r * ld + c), "n"(sizeof(T) >= 4 ? sizeof(T) : 4) : "memory");
     else
       dst[i] = src[(size_t)r * ld + c];
-  });
+  }
+}
+// The same with loops that are not unrolled, for the decay rule's backward, whose fetch is part of a long loop body
+// (48 x 300, 100 x 100, fp16: 1012 us unrolled by four, 896 rolled; fp32, 16 x 129, 96 x 48: 72 and 69.5).
+template <typename T>
+__device__ __forceinline__ void stage_rolled(T *dst, const T *src, int n, int tid, int nthreads) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  const int bytes = n * (int)sizeof(T);
+  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
+  if ((a & 15u) == 0) {
+    const int n16 = bytes >> 4;
+#pragma unroll 1
+    for (int i = tid; i < n16; i += nthreads)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * i), "l"(reinterpret_cast<const char *>(src) + 16 * i) : "memory");
+#pragma unroll 1
+    for (int i = (n16 << 4) / (int)sizeof(T) + tid; i < n; i += nthreads) dst[i] = src[i];
+  } else if (sizeof(T) >= 4 || (a & 3u) == 0) {
+    const int n4 = bytes >> 2;
+#pragma unroll 1
+    for (int i = tid; i < n4; i += nthreads)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * i), "l"(reinterpret_cast<const char *>(src) + 4 * i) : "memory");
+#pragma unroll 1
+    for (int i = (n4 << 2) / (int)sizeof(T) + tid; i < n; i += nthreads) dst[i] = src[i];
+  } else {
+#pragma unroll 4
+    for (int i = tid; i < n; i += nthreads) dst[i] = src[i];
+  }
+}
+template <typename T>
+__device__ __forceinline__ void stage_rows_rolled(T *dst, const T *src, int n, int w, int ld, int tid, int nthreads) {
+#pragma unroll 1
+  for (int i = tid; i < n * w; i += nthreads) {
+    const int r = i / w, c = i - r * w;
+    if constexpr (sizeof(T) >= 4)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + i)),
+                   "l"(src + (size_t)r * ld + c), "n"(sizeof(T) >= 4 ? sizeof(T) : 4) : "memory");
+    else
+      dst[i] = src[(size_t)r * ld + c];
+  }
 }
 __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
