@@ -17,6 +17,7 @@
 // spread over more CTAs by giving each thread fewer rows (R = 4, 2, 1).
 // Replaces t2fw/csrc/lfw_kernel.cu:18-59 with the einsum of t2fw/csrc/lfw.cpp:45, and
 // t2fw/csrc/dfw_kernel.cu:105-196, for these sizes.
+#include "seq_layout.cuh"
 #include "steps.cuh"
 
 namespace t2fw {
@@ -26,7 +27,6 @@ using namespace steps;
 namespace {
 
 constexpr int kThreadsS = 128;
-constexpr float kFusedGateFloor = 0.125f;      // as in the chunk kernels (seq_layout.cuh)
 constexpr int kGroup = 8;      // steps whose vectors are fetched together
 
 template <typename T>
@@ -110,7 +110,7 @@ steps_kernel(const StepArgs<T> a) {
     if constexpr (kFused) {
       for (int i = tid; i < nt * K; i += kThreadsS) {
         T *g = &buf[which][(i / K) * kStep + i % K], *q = g + 2 * K;
-        *g = (T)fmaxf(__fdividef(1.f, 1.f + __expf(-Elem<T>::ld(g))), kFusedGateFloor);
+        Elem<T>::st(g, seq::sigmoid_gate<T>(Elem<T>::ld(g)));      // the backward's gate, bit for bit
         *q = (T)(Elem<T>::ld(q) * a.q_scale);
       }
       __syncthreads();

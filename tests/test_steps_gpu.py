@@ -53,3 +53,23 @@ def test_short_fused_layer_equals_plain_operator(cuda, B, T, H):
     state = torch.randn(B * H, 64, 64, generator=g).half().to(cuda)
     for a, b in zip(LFWFusedFunction.apply(qkvg, state, H), unfused_reference(qkvg, state, H)):
         assert max_rel_err(a, b) <= 1e-3      # torch's sigmoid may round a gate the other way
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_gates_are_the_chunk_kernels_gates(cuda, dtype):
+    """The fused layer's gate of every finite pre-activation, from a call of one step and from one of a whole chunk (what
+    the backward of either uses): a state of ones and nothing else leaves the gate as the next state."""
+    from t2fw_b200.functional_fused import LFWFusedFunction
+
+    pre = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(dtype)
+    pre = torch.where(torch.isfinite(pre), pre, torch.zeros_like(pre)).reshape(1024, 1, 64).to(cuda)
+    state = torch.zeros(1024, 64, 64, dtype=dtype, device=cuda)
+    state[:, 0] = 1
+    got = []
+    for T in (1, 64):
+        qkvg = torch.zeros(1024, T, 256, dtype=dtype, device=cuda)
+        qkvg[:, :, 192:] = 30      # gate 1
+        qkvg[:, :1, 192:] = pre
+        got.append(LFWFusedFunction.apply(qkvg, state, 1)[1][:, 0])
+    torch.cuda.synchronize()
+    assert (got[0] >= 0.125).all() and (got[0] <= 1).all() and torch.equal(got[0], got[1])
