@@ -26,6 +26,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-Xptxas", "-v",
+    "-Xfatbin=-compress-all",      # with -lineinfo kernels are left uncompressed otherwise: 47 MB instead of 34
 ]
 
 
