@@ -123,7 +123,8 @@ bool plain_tensor(PyObject *o) {
   if (!THPVariable_CheckExact(o) && !(ParameterClass != nullptr && (PyObject *)Py_TYPE(o) == ParameterClass)) return false;
   const auto ks = t.key_set();
   return t.defined() && t.is_cuda() && !ks.has(c10::DispatchKey::Python) && !ks.has(c10::DispatchKey::FuncTorchGradWrapper) &&
-         !ks.has(c10::DispatchKey::FuncTorchBatched) && !t._fw_grad(/*level=*/0).defined();
+         !ks.has(c10::DispatchKey::FuncTorchBatched) &&
+         (t.unsafeGetTensorImpl()->autograd_meta() == nullptr || !t._fw_grad(/*level=*/0).defined());
 }
 
 bool plain_mode() {
