@@ -8,11 +8,10 @@
 // so that no product over more than 32 steps is ever formed or inverted, and only one-sided.
 // "mid" operands carry these ratios (q * pm_g, k / pm_g, dO * pm_a, x / pm_a); their pair products
 // P = tril((q pm_g)(k / pm_g)^T), Z = tril((dO pm_a)(x / pm_a)^T) are the exact in-chunk decays.
-// Terms that involve the state at the chunk start use operands anchored at the chunk START
-// (q * G_t, dO * A_t) and terms that involve the state gradient at the chunk end use operands
-// anchored at the chunk END (k * G_63/G_s, x * A_63/A_s): those products only ever decay, so an
-// underflow there loses nothing that the exact result would keep.  The 64 x 64 state blocks are
-// scaled on ONE side only (by the anchor products of the side whose gradients are formed).
+// The same operands serve the terms through the state at the chunk start and through the state
+// gradient at the chunk end: the 64 x 64 state block carries the anchor product of the side that is
+// contracted away, and the result is scaled by that of its own side.  (The chunk-local kernel alone
+// anchors its operands at the chunk's end or start, lfw_c64_local.cu.)
 // A batch row whose one-sided 32-step products leave [2^-100, 2^100] is flagged and recomputed by
 // the sequential scan kernels.
 //
@@ -31,7 +30,6 @@ namespace c64 {
 
 constexpr int kC = 64;                 // chunk length = checkpoint interval
 constexpr int kDim = 64;               // D = K = 64
-constexpr int kRef = 31;               // anchor: after step 31
 constexpr int kTile = 64 * 64 * 4;     // bytes of one operand tile
 constexpr int kColBlock = 64 * 128;    // bytes of one 32-column block of a tile
 constexpr int kRawBytes = kC * kDim * 2;
@@ -44,11 +42,6 @@ constexpr float kTinyState = 9.094947e-13f;     // 2^-40: smallest gate magnitud
 constexpr float kTinyGate = 1.220703125e-4f;    // 2^-13
 constexpr float kRangeLo = 7.888609e-31f;       // 2^-100
 constexpr float kRangeHi = 1.267651e+30f;       // 2^100
-
-// byte offset of element (r, c) of a tile
-__device__ __forceinline__ int toff(int r, int c) {
-  return (c >> 5) * kColBlock + r * 128 + ((((c >> 2) & 7) ^ (r & 7)) << 4) + ((c & 3) << 2);
-}
 
 // Round to TF32 (10 mantissa bits), nearest with ties away from zero - what cvt.rna.tf32.f32 does -
 // as two integer instructions: the conversion instruction runs on the quarter-rate pipe and there
@@ -96,14 +89,6 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, ui
       "}\n" ::"r"(d_tmem),
       "r"(a_tmem), "l"(desc_b), "r"(idesc), "r"(acc), "r"(zero)
       : "memory");
-}
-
-__device__ __forceinline__ void tmem_st8(uint32_t addr, const float (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(addr),
-               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-               "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
-               "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
-               : "memory");
 }
 
 // 16-byte asynchronous copy global -> shared (no register, no scoreboard)

@@ -19,6 +19,11 @@ namespace {
 
 constexpr int kM = 64;
 
+// byte offset of element (r, c) of a 64 x 64 operand tile of the chunk kernels (lfw_c64.cuh)
+__device__ __forceinline__ int toff(int r, int c) {
+  return (c >> 5) * c64::kColBlock + r * 128 + ((((c >> 2) & 7) ^ (r & 7)) << 4) + ((c & 3) << 2);
+}
+
 __global__ void __launch_bounds__(128)
 umma_selftest_kernel(const float *__restrict__ A1, const float *__restrict__ B1,
                      const float *__restrict__ A2, const float *__restrict__ B2,
@@ -191,7 +196,7 @@ umma_ts_selftest_kernel(const float *__restrict__ A, const float *__restrict__ B
   }
   if (warp == 0) tmem_alloc(&tmem_slot, 128);
   for (int idx = threadIdx.x; idx < 64 * 64; idx += blockDim.x)
-    *reinterpret_cast<float *>(tB + c64::toff(idx / 64, idx % 64)) = B[idx];
+    *reinterpret_cast<float *>(tB + toff(idx / 64, idx % 64)) = B[idx];
   fence_async_smem();
   fence_before_sync();
   __syncthreads();
