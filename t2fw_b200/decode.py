@@ -33,7 +33,8 @@ class LFWDecodeLoop:
     `ring` (even) input slots x, f [ring,B,1,D] and query, key, f_key [ring,B,1,K] are filled by the
     caller; `run_ring()` advances the state by `ring` steps (slot 0 first) and leaves the outputs of
     every step in `outputs` [ring,B,1,D].  Shapes outside the one-kernel trip run eagerly in the first
-    call, which captures the graph that later calls replay.  `state` is the current state (a view of one of the two internal buffers)."""
+    call, which captures the graph that later calls replay.  `state` is the current state: the first of two internal buffers, which the one-kernel trip
+    advances in place and a trip of single steps returns to."""
 
     def __init__(self, state, ring=2):
         if ring < 2 or ring % 2:

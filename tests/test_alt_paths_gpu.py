@@ -1,6 +1,6 @@
 """The kernel families that environment switches select instead of the default ones stay
 parity-green: each case runs in a child process (the switches are read once per process) and
-checks one delta-rule and one decay-rule problem against the oracle."""
+checks one delta-rule and one decay-rule problem and a decode step against the oracle."""
 import os
 import subprocess
 import sys
@@ -40,13 +40,18 @@ o_grads = fw_oracle.lfw_backward(go2, gs2, x, f, qq, kk, fk, st)
 assert max_rel_err(out2, o_out) <= OUT_TOL[dt] and max_rel_err(ckpt[:, -1], o_fin) <= OUT_TOL[dt]
 for g, r in zip(grads2, o_grads):
     assert max_rel_err(g, r) <= GRAD_TOL[dt]
+# a decode step
+x1, f1, q1, k1, fk1 = (t[:, :1].contiguous() for t in (x, f, qq, kk, fk))
+out1, ckpt1 = cabi.lfw_forward(x1, f1, q1, k1, fk1, st)
+s_out, s_fin = fw_oracle.lfw_forward(x1, f1, q1, k1, fk1, st)
+assert max_rel_err(out1, s_out) <= OUT_TOL[dt] and max_rel_err(ckpt1[:, -1], s_fin) <= OUT_TOL[dt]
 from t2fw_b200._lib import load_core
 assert load_core().t2fw_device_status() == 0
 print("ok")
 """
 
 
-@pytest.mark.parametrize("switch", ["T2FW_DISABLE_DFW_UMMA", "T2FW_DISABLE_DFW_CHUNK", "T2FW_DISABLE_CHUNK", "T2FW_DISABLE_PDL"])
+@pytest.mark.parametrize("switch", ["T2FW_DISABLE_DECODE_BULK", "T2FW_DISABLE_DFW_CHUNK", "T2FW_DISABLE_CHUNK", "T2FW_DISABLE_PDL"])
 def test_switched_path_matches_oracle(cuda, switch):
     env = dict(os.environ)
     env[switch] = "1"
