@@ -24,7 +24,8 @@ a step is one forward + backward over the whole batch.  Prints ONE JSON line on 
   value_api . the same step through LFWFunction.apply + autograd with device-resident tensors,
               eager and replayed from a CUDA graph
   extra.decode  the T=1 decode step (B*H=4096) measured in the same run: us/step over 1000 chained
-              steps through the allocation-free decode loop (graph replay), GB/s and fraction
+              steps through the allocation-free decode loop (one launch per ring of 10 steps, the
+              state in registers over the ring), GB/s and fraction of a trip's own bytes
   cpu_baseline  the reference's own TorchScript CPU path (oracle/_ref, placed there by
               oracle/make_ref.py; kind "reference") or, where that is absent, its restatement
               oracle/torch_port.py (kind "port"), on this machine's host cores, on a bounded sample
@@ -801,7 +802,7 @@ def run_ours(args):
         loop.f_key.copy_(torch.sigmoid(torch.randn(ring, Bd, 1, Kd, generator=gd)).to(dtype))
         if args.gates != "raw_f1":
             loop.f.copy_(torch.sigmoid(torch.randn(ring, Bd, 1, Dd, generator=gd)).to(dtype))
-        loop.run_ring()                 # eager trip, then capture
+        loop.run_ring()
         loop.run_ring()
         torch.cuda.synchronize()
         d0, d1 = ev(), ev()
@@ -811,18 +812,19 @@ def run_ours(args):
         d1.record()
         torch.cuda.synchronize()
         us = d0.elapsed_time(d1) * 1e3 / (trips * ring)
-        dbytes = 2 * (2 * Bd * Dd * Kd) + 2 * Bd * (2 * Dd + 3 * Kd) + 2 * Bd * Dd
+        # a trip reads and writes the state once and every step's vectors and outputs
+        dbytes = 2 * (2 * Bd * Dd * Kd) / ring + 2 * Bd * (2 * Dd + 3 * Kd) + 2 * Bd * Dd
         peak_d, kind_d = measured_hbm_peak()
         extra = {"decode": {
             "us_per_step": us, "steps": trips * ring, "tokens_per_s": Bd / (us * 1e-6),
             "achieved_gbs": dbytes / (us * 1e-6) / 1e9, "frac": dbytes / (us * 1e-6) / 1e9 / peak_d,
             "peak": peak_d, "peak_kind": kind_d + " copy bandwidth", "algorithmic_bytes_per_step": dbytes,
             "workload": "decode: B*H=%d, T=1, D=K=64, fp16 I/O, fp32 state arithmetic; %d chained steps, fresh "
-                        "inputs from a ring of %d slots (f_key = sigmoid(N(0,1))); the state is chained through two 67 MB "
-                        "buffers, so part of a step's output is still in the 126 MB L2 when the next step reads it "
-                        "(--workload decode times the step with nothing in L2)"
+                        "inputs from a ring of %d slots (f_key = sigmoid(N(0,1))); a kernel keeps the state in registers "
+                        "over the ring's steps, so the 67 MB state moves once per ring, not per step "
+                        "(--workload decode times single steps with nothing in L2)"
                         % (Bd, trips * ring, ring),
-            "api": "t2fw_b200.decode.LFWDecodeLoop (torch.ops.lfw.decode_step, one CUDA-graph replay per %d steps)" % ring,
+            "api": "t2fw_b200.decode.LFWDecodeLoop.run_ring (one kernel launch per %d steps)" % ring,
             "finite": bool(torch.isfinite(loop.state).all().item())}}
         del loop
 
