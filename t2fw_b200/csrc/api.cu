@@ -133,9 +133,10 @@ static bool aligned16(std::initializer_list<const void *> ps) {
 // rule's step waits for a row sum, so its one-chunk kernels catch up at about 48 steps (16.4 us both at 96 rows).
 constexpr int64_t kLfwStepsMax = 63;
 constexpr int64_t kDfwStepsMax = 48;
-// Largest state (elements) for which a single decode step takes the step kernel: while state and vectors come from
-// L2 its many small CTAs start faster (96 rows of 128 x 128: 2.6 us against 5.2), beyond that the bulk-copy ring
-// streams better (4096 rows of 64 x 64 from HBM: 14.1 us against 16.0).
+// Largest state (elements) for which a single decode step takes the step kernel: its many small CTAs start faster, the
+// bulk-copy ring streams better.  Step kernel against ring, 64 x 64, nothing in L2, us: 512 rows (2 Mi elements) 4.0 / 4.1,
+// 1536 7.5 / 8.0, 2048 (8 Mi) 9.6 / 9.4, 2560 11.1 / 10.2, 3072 13.1 / 12.0, 4096 (16 Mi) 16.7 / 14.1.  At other sizes, where
+// there is no ring, against the register-streaming kernel: 128 x 128, 128 rows 4.0 / 6.5, 512 (8 Mi) 9.7 / 13.5, 1024 16.7 / 23.1.
 constexpr int64_t kOneStepMaxElems = 8ll << 20;
 
 static int check_common(int64_t B, int64_t T, int64_t D, int64_t K, int dtype) {

@@ -16,9 +16,10 @@
 // Fragment images and operand precision as in dfw_fwd.cu: products among K, Q and dO are exact, Wb and Ub come from T
 // (and the right-hand side) split in two, everything else is TF32 with fp32 accumulation.
 //
-// Bound by the tensor pipe (prep ~520, gradients ~580 products per warp, 2.1 cycles per SM each) and by shared-memory
-// reads of operands that contract along rows.  B*H = 96, T = 1024, fp16, whole backward: 188 -> 165 us
-// with cold caches (prep 60, carry 27, gradients 78).
+// What bounds it is latency at few warps, no pipe.  B*H = 96, T = 1024, fp16, cold caches: prep 60 us, tensor pipe 50 %,
+// issue slots 35 %, 11 warps per SM; carry 28 us, 4 warps on each of 96 SMs, tensor 19 %; gradients 78 us, tensor 40 %,
+// issue slots 30 %, 15 warps per SM that wait most for the other group at the five meetings, then for global memory
+// (252 bytes of spills per thread among it).  Whole backward 188 -> 165 us.
 #include "dfw_frag.cuh"
 
 namespace t2fw {

@@ -18,9 +18,11 @@
 // Why mma.sync: with operands in fragment order a warp needs no barrier, no tile conversion and no round trip
 // through tensor memory between products, and small CTAs overlap one another's latencies; the tcgen05 form of this
 // path converted every operand to tiles and walked the whole chunk sequentially per row, 7.2 k cycles each on at
-// most one SM per row.  Bound now: the tensor pipe (prep ~330, out ~200 products per warp at 2.1 cycles per SM) and
-// L2 traffic of the images.  B*H = 96, T = 1024, fp16, whole forward: 108 -> 91 us (prep 39,
-// carry 19, out 33 with cold caches); 48 rows of 1333 steps, bf16, the whole call 110 -> 61 us.
+// most one SM per row.  What bounds it now is latency at few warps, no pipe: with
+// cold caches (B*H = 96, T = 1024, fp16) prep 39 us, tensor pipe 52 %, issue slots 39 %, 14 warps per SM that wait for
+// fixed latencies, the tensor pipe and barriers; carry 19 us, 4 warps on each of 96 SMs, tensor 29 %, waiting for the
+// images and for its own chain; out 33 us, tensor 32 %, DRAM 42 %, waiting for the images.  Whole forward 108 -> 91 us;
+// 48 rows of 1333 steps, bf16, the whole call 110 -> 61 us.
 #include "dfw_frag.cuh"
 
 namespace t2fw {

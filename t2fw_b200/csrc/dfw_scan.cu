@@ -16,7 +16,9 @@
 // A chain of T steps bounds these kernels: in a step the products of a line are summed, the sum goes round the
 // lanes and the line is updated with it.  L = 8 up to 128 elements (four lines per warp): three exchanges per sum
 // instead of five, each of them for four lines, against eight to sixteen products per lane in two chains; longer
-// lines take all 32 lanes.  The steps' vectors come from shared memory, fetched a group of steps ahead (scan.cuh).
+// lines take all 32 lanes.  Sixteen lanes would gain an eighth for few lines and lose half for many, and are left out (64 x 64,
+// 150 steps, fp32, us at 8 / 16 / 32 lanes; forward: 192 lines 28.0 / 24.6 / 24.8, 1792 28.2 / 28.4 / 48.8, 3584
+// 35.8 / 53.6 / 64.4; backward: 192 61 / 54 / 57, 1792 62 / 66 / 76, 4480 78 / 123 / 140).  The steps' vectors come from shared memory, fetched a group of steps ahead (scan.cuh).
 // Whole call, fp32: 16 rows of 129 steps 96 x 48, forward and backward 278 -> 92 us; 48 rows of 300 steps 100 x 100
 // 876 -> 480; forward alone, 40 rows of 200 steps 64 x 64, 139 -> 47.
 #include "scan.cuh"

@@ -33,9 +33,10 @@
 // sums over time are register-local plus one exchange between the four threads of a feature.  The d side's
 // rows are rotated by 16 features against the k side's so that the two half warps touch different banks.
 //
-// What bounds it: instruction issue (about 1000 instructions per thread and chunk; 53 k -> 25.5 k warp
-// instructions per chunk against the version that ran the two sides one after the other) and the latency of
-// its phases.  Config B*H = 96, T = 1024 (1536 chunks): 151 -> 101 us per launch with cold caches.
+// What bounds it: the latency of its phases at one CTA of 16 warps per SM.  Issue slots are 45 % busy (25.5 k warp
+// instructions per chunk; 53 k in the version that ran the two sides one after the other), the tensor pipe 18 %, DRAM 18 %; a
+// warp waits for barriers, fixed latencies, shared memory and instructions about equally.  B*H = 96, T = 1024 (1536 chunks):
+// 151 -> 99 us per launch with cold caches.
 //
 // One persistent CTA of 16 warps per SM; six raw 8 KB input blocks per chunk by bulk asynchronous copy (the
 // next chunk's are requested once this chunk's operands are built); operand tiles in shared memory (TF32,
@@ -495,7 +496,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         // sum_{s >= t} Mw[s] sum_{i < t} Z[s][i] Vw[i]: lanes over i, independent loads over s
         float acc = 0.f;
         for (int i = lane; i < t; i += 32) {
-          const unsigned char *zcol = zt + (i >> 5) * kColBlock + ((i & 3) << 2);      // toff(s, i) without the s terms
+          const unsigned char *zcol = zt + (i >> 5) * kColBlock + ((i & 3) << 2);      // tile offset of (s, i) without the s terms
           const int ic = (i >> 2) & 7;
           float a0 = 0.f, a1 = 0.f;      // two chains: the sums are latency-bound
           int s = t;

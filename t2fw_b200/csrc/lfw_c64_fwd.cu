@@ -21,8 +21,8 @@
 // and steps back, so that the ratios never leave its registers.  Odd chunk lanes are rotated by 16 features
 // so that the half warps touch different banks.
 //
-// What bounds it: instruction issue and the latency of its phases (shared-memory loads, two barriers, the two
-// product rounds); against the one-chunk version with ratio tables in shared memory, config B*H = 96,
+// What bounds it: the latency of its phases at one CTA of 16 warps per SM (issue slots 39 % busy, tensor pipe 14 %, DRAM
+// 25 %; a warp waits for loads, instructions, fixed latencies and shared memory about equally); against the one-chunk version with ratio tables in shared memory, config B*H = 96,
 // T = 1024 (1536 chunks): 12.7 k -> 8.6 k warp instructions per chunk, 57 -> 39 us per launch with cold caches.
 //
 // One persistent CTA of 16 warps per SM.  The raw 8 KB input blocks of the next pair are requested as soon as

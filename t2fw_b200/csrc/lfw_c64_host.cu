@@ -4,12 +4,12 @@
 // Forward (replaces t2fw/csrc/lfw_kernel.cu:18-59 and the output einsum t2fw/csrc/lfw.cpp:45):
 //   1. lfw_c64_local_kernel<.., true>   per (row, chunk): L_c, the chunk's own contribution to the
 //      state at its end, and the chunk's total decay vectors
-//   2. lfw_c64_carry_fwd_kernel         elementwise over chunks: S_{c+1} = (Ac Gc^T) .* S_c + L_c, written
+//   2. lfw_c64_carry_kernel<.., true>   elementwise over chunks: S_{c+1} = (Ac Gc^T) .* S_c + L_c, written
 //      as the 16-bit checkpoints (slot c = state after chunk c; the last slot is the next state)
 //   3. lfw_c64_fwd_kernel               per (row, chunk): the outputs from the chunk's start state
 // Backward (replaces t2fw/csrc/lfw_kernel.cu:61-102 and t2fw/csrc/lfw.cpp:84-93):
 //   1. lfw_c64_local_kernel<.., false>  G_c, the chunk's own contribution to the state gradient at its start
-//   2. lfw_c64_carry_bwd_kernel         from the last chunk down: R_end(c-1) = (Ac Gc^T) .* R_end(c) + G_c,
+//   2. lfw_c64_carry_kernel<.., false>  from the last chunk down: R_end(c-1) = (Ac Gc^T) .* R_end(c) + G_c,
 //      stored in place of G_c (fp32); what is left after chunk 0 is d_state
 //   3. lfw_c64_bwd_kernel               per (row, chunk): d_x, d_f, d_q, d_k, d_f_key
 // Scratch (floats): M[B][nc][64][64] | Ac[B][nc][64] | Gc[B][nc][64] | flags[B][nc] (int) |

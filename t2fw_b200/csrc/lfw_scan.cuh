@@ -28,7 +28,7 @@
 //
 // These kernels also redo the batch rows that the chunk kernels flagged (gate products outside the range of
 // the factored form): CTAs walk over all work items and skip the rows without a flag, and the launch is a
-// dependent one, so an all-clear costs about a microsecond.
+// dependent one.  An all-clear costs 4.9 us forward and 5.7 us backward with cold caches (96 x 1024, one flag per row).
 //
 // The kernels are templates; lfw_scan_{f16,bf16,f32,f64}.cu instantiate them for one storage type each (compiled side
 // by side), lfw_scan.cu picks the type.
@@ -403,7 +403,11 @@ __global__ void __launch_bounds__(kThreads) lfw_line_bwd_kernel(const BwdArgs<T>
 
 // Lanes per line for lines of up to 128 elements (backward: by the mean of the two orientations' lines).  Eight cost the
 // fewest instructions, where they still give every scheduler a warp and a half; with fewer lines a step's length is what
-// counts, and the lines are spread over 16 lanes while that fills half of the schedulers, over a warp below.
+// counts, and the lines are spread over 16 lanes while that fills half of the schedulers, over a warp below.  Rows of 150
+// steps, fp32, us at 8 / 16 / 32 lanes.  64 x 64, forward: 192 lines 23.7 / 18.9 / 17.1, 576 24.1 / 19.0 / 17.3, 896
+// 24.1 / 19.2 / 19.8, 2688 32.1 / 32.4 / 41.9, 3584 32.3 / 32.6 / 45.6, 6400 41.6 / 50.7 / 69.8; backward: 192 75 / 59 / 51, 896
+// 79 / 77 / 77, 2688 165 / 137 / 180, 3584 177 / 186 / 238, 6400 269 / 275 / 382.  100 x 100 turns earlier (2400 lines, forward
+// 41.7 / 49.0 / 49.6, backward 296 / 312 / 301).
 int lanes_for(int64_t lines) { return lines >= 148 * 24 ? 8 : lines >= 148 * 4 ? 16 : 32; }
 
 // CTAs of a launch: one per work item; the walk over flagged rows only is cut to a few waves
