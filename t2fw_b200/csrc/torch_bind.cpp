@@ -214,9 +214,9 @@ PyObject *py_fused_apply(PyObject *, PyObject *const *args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n == 3 && plain_mode() && plain_tensor(args[0]) && plain_tensor(args[1]) && PyLong_CheckExact(args[2])) {
     const Tensor &qkvg = THPVariable_Unpack(args[0]), &state = THPVariable_Unpack(args[1]);
-    const long h = PyLong_AsLong(args[2]);
-    if (h == -1 && PyErr_Occurred()) throw python_error();
-    if (h > 0 && qkvg.dim() == 3 && qkvg.size(2) == 4 * h * 64 && state.dim() == 3 && state.size(0) == qkvg.size(0) * h &&
+    int overflow = 0;      // then the number is -1, which the class refuses
+    const long h = PyLong_AsLongAndOverflow(args[2], &overflow);
+    if (h > 0 && qkvg.dim() == 3 && h <= qkvg.size(2) && qkvg.size(2) == 4 * h * 64 && state.dim() == 3 && state.size(0) == qkvg.size(0) * h &&
         state.size(1) == 64 && state.size(2) == 64 && qkvg.scalar_type() == state.scalar_type() &&
         qkvg.is_contiguous() && state.is_contiguous()) {
       const Tensor *all[2] = {&qkvg, &state};

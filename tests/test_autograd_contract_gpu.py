@@ -61,3 +61,11 @@ def test_second_derivative_raises(cuda, which, native):
     again = torch.autograd.grad(fn.apply(*leaves, *rest), leaves, up, create_graph=True)
     with pytest.raises(RuntimeError, match="not implemented"):
         torch.autograd.grad(again[-1].float().sum(), up[0])
+
+
+@pytest.mark.parametrize("n_head", [0, -1, 3, 1 << 70, (1 << 56) + 2])
+def test_impossible_head_counts_are_refused_alike(cuda, n_head):
+    """The class's assertion, also for numbers that a C integer, or their product with the row length, does not hold."""
+    fn, ins, _, _ = _call("fused", cuda)
+    with pytest.raises(AssertionError):
+        fn.apply(*ins, n_head)
