@@ -1,4 +1,4 @@
-// Pieces of the shape- and dtype-general scan kernels (lfw_scan.cu, dfw_scan.cu): staging of a few steps'
+// Pieces of the shape- and dtype-general scan kernels (lfw_scan.cuh, dfw_scan.cu): staging of a few steps'
 // vectors in shared memory, and sums over a warp for several values at once.
 //
 // A scan step is a few dozen instructions on a state held in registers; read straight from global memory its
