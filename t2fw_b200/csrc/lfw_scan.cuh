@@ -524,8 +524,11 @@ int launch_lines(BwdArgs<T> a, cudaStream_t st) {
 
 // A rung serves the longer orientation's lines; `m` is the length of the other's.  Nearly as long: the same rung, without
 // conditions on the elements that exist.  Up to half as long: half of the lanes with the same elements per lane (of eight
-// lanes half of the elements).  Between: the same rung with conditions.  fp32, 16 x 129, 96 x 48: 69.5 us (with
-// conditions 80); 48 x 300, 100 x 50: 473 (728); 16 x 129, 96 x 64: 123.
+// lanes half of the elements).  Between: the same rung with conditions, or kInTurn where those would be ten and more per lane,
+// which no registers keep: the lines are many there and two launches cost less.  fp32, 16 x 129, 96 x 48: 69.5 us (with
+// conditions 80); 48 x 300, 100 x 50: 473 (728); 16 x 129, 96 x 64: 123.  In turn: 48 x 200, 60 x 90 303 (414 with conditions),
+// 48 x 300, 100 x 60 725 (723), fp16 783 (860).
+constexpr int kInTurn = -1;      // not a status
 template <typename T, int L, int NL, int SAFE>
 int launch_rung(const BwdArgs<T> &a, int m, cudaStream_t st) {
   if constexpr (SAFE > 0) {
@@ -534,14 +537,12 @@ int launch_rung(const BwdArgs<T> &a, int m, cudaStream_t st) {
     if (m <= LH * NH)
       return a.col.NLn > a.row.NLn ? launch_lines<T, L, NL, SAFE, LH, NH, 0>(a, st) : launch_lines<T, LH, NH, 0, L, NL, SAFE>(a, st);
   }
-  // (ten and more conditions per lane are kept in no registers: sixteen lanes, where six elements hold the lines; 48 x 200,
-  // 60 x 90: 475 -> 415 us)
-  if constexpr (L == 8 && NL > 8)
-    if (a.col.NLn <= 96 && a.row.NLn <= 96) return launch_lines<T, 16, 6, 0, 16, 6, 0>(a, st);
-  return launch_lines<T, L, NL, 0, L, NL, 0>(a, st);
+  if constexpr (L == 8 && NL > 8) return kInTurn;
+  else return launch_lines<T, L, NL, 0, L, NL, 0>(a, st);
 }
 
-// One launch of the orientations asked for.  Rungs: the smallest that holds the lines, for the number of lanes.
+// The orientations asked for, in one launch wherever a kernel has their pair of lengths.  Rungs: the smallest that holds the
+// lines, for the number of lanes.
 template <typename T>
 int launch_bwd(BwdArgs<T> a, bool columns, bool rows, cudaStream_t st) {
   a.col.items = columns;
@@ -555,7 +556,7 @@ int launch_bwd(BwdArgs<T> a, bool columns, bool rows, cudaStream_t st) {
   } else {
     if (n > 256) return launch_rung<T, 32, 16, 8>(a, m, st);
     if (n > 128) return launch_rung<T, 32, 8, 4>(a, m, st);
-    const int lanes = a.rowflag != nullptr ? 8 : lanes_for(a.B * (a.col.NO + a.row.NO) / 2);
+    const int lanes = a.rowflag != nullptr ? 8 : lanes_for(a.B * ((columns ? a.col.NO : a.row.NO) + (rows ? a.row.NO : a.col.NO)) / 2);
     if (lanes == 32)
       return n <= 32 ? launch_rung<T, 32, 1, 0>(a, m, st) : n <= 64 ? launch_rung<T, 32, 2, 1>(a, m, st)
              : n <= 96 ? launch_rung<T, 32, 3, 2>(a, m, st) : launch_rung<T, 32, 4, 3>(a, m, st);
@@ -568,8 +569,11 @@ int launch_bwd(BwdArgs<T> a, bool columns, bool rows, cudaStream_t st) {
     if (n <= 16) return launch_rung<T, 8, 2, 0>(a, m, st);
     if (n <= 32) return launch_rung<T, 8, 4, 2>(a, m, st);
     if (n <= 64) return launch_rung<T, 8, 8, 4>(a, m, st);
-    if (n <= 80) return launch_rung<T, 8, 10, 8>(a, m, st);
-    return n <= 104 ? launch_rung<T, 8, 13, 10>(a, m, st) : launch_rung<T, 8, 16, 13>(a, m, st);
+    const int rc = n <= 80 ? launch_rung<T, 8, 10, 8>(a, m, st) : n <= 104 ? launch_rung<T, 8, 13, 10>(a, m, st)
+                   : launch_rung<T, 8, 16, 13>(a, m, st);
+    if (rc != kInTurn) return rc;
+    const int first = launch_bwd<T>(a, true, false, st);      // lines of one length: their own rung
+    return first != T2FW_OK ? first : launch_bwd<T>(a, false, true, st);
   }
 }
 
