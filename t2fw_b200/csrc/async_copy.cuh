@@ -22,9 +22,13 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 constexpr uint32_t kSpinLimit = 1u << 19;   // polls, each may suspend for up to ~2 us
 // bounded wait for the phase with the given parity; false on timeout
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
+#pragma unroll 1
   for (uint32_t i = 0; i < kSpinLimit; ++i) {
     uint32_t ok;
     asm volatile(

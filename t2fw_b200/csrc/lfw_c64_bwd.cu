@@ -33,14 +33,19 @@
 // sums over time are register-local plus one exchange between the four threads of a feature.  The d side's
 // rows are rotated by 16 features against the k side's so that the two half warps touch different banks.
 //
-// What bounds it: the latency of its phases at one CTA of 16 warps per SM.  Issue slots are 45 % busy (25.5 k warp
-// instructions per chunk; 53 k in the version that ran the two sides one after the other), the tensor pipe 18 %, DRAM 18 %; a
-// warp waits for barriers, fixed latencies, shared memory and instructions about equally.  B*H = 96, T = 1024 (1536 chunks):
-// 151 -> 99 us per launch with cold caches.
+// One persistent CTA per SM: 16 warps that compute and four that only issue (products, the next chunk's inputs, the finished
+// chunk's results).  What runs once per chunk or rarely is kept in rolled loops: a launch starts with cold instruction caches,
+// and the first chunk waits for every line of the code (156 KB, unrolled throughout: 31 k cycles; a chunk afterwards 12 k).
+// A computing warp reports "my part is in place" on an mbarrier and goes on; whoever needs all parts waits
+// for the barrier.  With the issuing done by computing warps, those fell behind by up to 3 k cycles per chunk and the others
+// waited for them at the next step.  Inputs arrive and results leave by bulk copies; the results are staged over the operand
+// tiles.  (A bulk copy costs its issuing warp about 70 cycles whatever its size.)
 //
-// One persistent CTA of 16 warps per SM; six raw 8 KB input blocks per chunk by bulk asynchronous copy (the
-// next chunk's are requested once this chunk's operands are built); operand tiles in shared memory (TF32,
-// 128-byte swizzle), accumulators in tensor memory.  Every wait is bounded.
+// What bounds it: the phases of the computing warps (gates and operands 3.1 k cycles, state operands 2.0 k, Z 1.2 k, sums and
+// results 4.5 k of 11 k per chunk), in which all warps want the same unit at the same time; products and copies run under them.
+// Whole training step, start of this arrangement -> now: 96 rows x 1024 steps 200 -> 177 us (N(0,1) gates, of which 0.4 per chunk
+// are tiny: their listing and sums took 6 k cycles, now 0.5 k), fused layer 8 x 12 heads x 1024 258 -> 206 us, 16 x 16384 with
+// 128 x 128 states 2213 -> 2035 us.
 #include "lfw_c64.cuh"
 #include "seq_layout.cuh"
 
@@ -54,28 +59,35 @@ int lfw_chunk_sm_count(int *out);
 
 namespace {
 
-constexpr int kThreadsB = 512;
+constexpr int kThreadsB = 512;         // computing threads
+constexpr int kWarpsB = kThreadsB / 32;
+constexpr int kThreadsAll = kThreadsB + 128;
+// Registers per thread after the split; the block is launched with 96 for each (the largest multiple of eight of which 640
+// threads get one), and 512 * 112 + 128 * 24 is less than 640 * 96.
+constexpr int kRegsCompute = 112, kRegsIssue = 24;
+static_assert(kThreadsB * kRegsCompute + 128 * kRegsIssue <= kThreadsAll * 96, "register split");
 constexpr int kFixCap = 128;           // tiny-gate entries per chunk
-constexpr int kFixRows = 16;           // features with tiny gates per chunk whose operand rows are kept
+constexpr int kFixParts = 512;         // partial sums of all entries together
 constexpr int kS0Ld = 144;             // row stride (bytes) of the start-state landing zone (64 x 16-bit + pad)
-constexpr int kRLd = 272;              // row stride (bytes) of the end-gradient landing zone (64 x fp32 + pad)
+constexpr int kRLd = 256;              // row stride (bytes) of the end-gradient landing zone (64 x fp32)
 // shared-memory map (bytes from the 1024-byte aligned base); side 0 = k, 1 = d
-constexpr int oT = 0;                               // [side][2] tiles [step][feature]: Mm (q pm | dO pm), Vm (k / pm | x / pm)
-constexpr int oZ = oT + 4 * kTile;                  // [own side][2] tiles: Z [t][s], Z^T [s][t]
-constexpr int oS0L = oZ + 4 * kTile;                // start state of the chunk, [64][kS0Ld]
+// Two buffers of four tiles that change places with every chunk: operands [side][2] tiles [step][feature]: Mm (q pm | dO pm),
+// Vm (k / pm | x / pm), over which the results are staged once TQ1 and T7 have read them; and Z [own side][2] tiles: Z [t][s],
+// Z^T [s][t].  So the next chunk's operands never meet results that are still on their way out.
+constexpr int kTiles = 4 * kTile;
+constexpr int oS0L = 2 * kTiles;                    // start state of the chunk, [64][kS0Ld]
 constexpr int oRL = oS0L + kDim * kS0Ld;            // end state gradient of the chunk, [64][kRLd]
 constexpr int oQt = oRL + kDim * kRLd;              // quarter products [side][4][64]
-constexpr int oPrd = oQt + 2 * 4 * kDim * 4;        // [side][2][64]: product up to the anchor, after the anchor
-constexpr int oXc = oPrd + 2 * 2 * kDim * 4;        // partial sums [3][4 quarters][side][64]
+constexpr int oXc = oQt + 2 * 4 * kDim * 4;         // partial sums [3][4 quarters][side][64]
 constexpr int oBnd = oXc + 3 * 4 * 2 * kDim * 4;    // boundary-term partials [side][4][64]
 constexpr int oFixCode = oBnd + 2 * 4 * kDim * 4;   // [kFixCap] int: step << 8 | side << 6 | feature
-constexpr int oFixVal = oFixCode + kFixCap * 4;     // [kFixCap] float
-constexpr int oFixMask = oFixVal + kFixCap * 4;     // [side][64] one bit per step
-constexpr int oFixSlot = oFixMask + 2 * kDim * 8;   // [side][64] int: row slot of a feature, -1 = none
-constexpr int oFixRow = oFixSlot + 2 * kDim * 4;    // [kFixRows][2][64] floats: operand rows Mw, Vw
-constexpr int oRaw = oFixRow + kFixRows * 2 * kDim * 4;   // x, f (fused layer: gate pre-activations), q, k, fk, dO
+constexpr int oFixPart = oFixCode + kFixCap * 4;    // [kFixParts] float
+constexpr int oDer0 = oFixPart + kFixParts * 4;     // fused layer: derivatives of the gates, [32 steps][64] floats; the other
+constexpr int oRaw = oDer0 + kRawBytes;             //   32 steps where the forget gates, which it does not have, would arrive
+constexpr int oDer1 = oRaw + kRawBytes;             // raw blocks: x, f, q, k, fk, dO
 constexpr int kSmemB = oRaw + 6 * kRawBytes + 1024; // + slack for the 1024-byte alignment
-static_assert(oRaw % 128 == 0 && oFixMask % 8 == 0 && oS0L % 16 == 0 && oRL % 16 == 0, "alignment");
+static_assert(oRaw % 128 == 0 && oS0L % 16 == 0 && oRL % 16 == 0, "alignment");
+static_assert(kFixCap * 4 <= kFixParts, "at least four parts per entry");
 static_assert(kSmemB + 256 <= 227 * 1024, "shared memory limit");
 
 // tensor-memory columns, both lane sets: four A operands, then the accumulators.  T2 takes Z's columns over
@@ -84,9 +96,10 @@ constexpr int cS2 = 0, cR2 = 64, cVw = 128, cMw = 192;
 constexpr int cZ = 256, cT2 = 256, cTQ1 = 320, cTQ2 = 384, cT7 = 448;
 constexpr int kTmemCols = 512;
 
-// kMode: 0 the plain operator, 1 the fused layer, 2 a grid of blocks (gradients summed over the blocks of the other axis)
+// kMode: 0 the plain operator, 1 the fused layer (forget gate 1, k-side gates from pre-activations), 2 a grid of blocks
+// (gradients summed over the blocks of the other axis)
 template <typename T, int kMode>
-__global__ void __launch_bounds__(kThreadsB, 1)
+__global__ void __launch_bounds__(kThreadsAll, 1)
 lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ state, const T *__restrict__ ckpt,
                    const float *__restrict__ Rend, const seq::Out<T> dx, const seq::Out<T> df, const seq::Out<T> dq,
                    const seq::Out<T> dk, const seq::Out<T> dfk, int *__restrict__ rowflag, int *__restrict__ status,
@@ -94,9 +107,9 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   constexpr bool kFused = kMode == 1, kGrid = kMode == 2;
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);
-  __shared__ __align__(8) uint64_t barRaw, barG, barZ, barM1, barM2;
+  __shared__ __align__(8) uint64_t barRaw, barState, barT, barA, barZs, barZ, barM1, barM2, barOut;
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_fail, s_bad2[2], fix_n2[2], fix_rows_n;
+  __shared__ int s_bad2[2], fix_n2[2];
 
   const int tid = threadIdx.x, warp = uniform_warp_idx(), lane = tid & 31;
   // lane quarter of tensor memory, 16-step quarter of the chunk, side (0 k, 1 d), row in the quarter
@@ -105,139 +118,243 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   const int t0 = 16 * tq;                             // first own step; also the first own column of the state blocks
 
   float *qtot = reinterpret_cast<float *>(sm + oQt);
-  float *prd = reinterpret_cast<float *>(sm + oPrd);
   float *xc = reinterpret_cast<float *>(sm + oXc);
   float *bndp = reinterpret_cast<float *>(sm + oBnd);
   int *fix_code = reinterpret_cast<int *>(sm + oFixCode);
-  float *fix_val = reinterpret_cast<float *>(sm + oFixVal);
-  unsigned long long *fix_mask = reinterpret_cast<unsigned long long *>(sm + oFixMask);
-  int *fix_slot = reinterpret_cast<int *>(sm + oFixSlot);
-  float *fix_rows = reinterpret_cast<float *>(sm + oFixRow);
   T *raw = reinterpret_cast<T *>(sm + oRaw);     // [6][64][64]: x, f, q, k, fk, dO
 
   // tensors: 0 x, 1 f, 2 q, 3 k, 4 fk, 5 dO
-  const bool unit_forget = kFused && (mp.flags & seq::kUnitForget) != 0;
-  const bool sigmoid_gate = kFused && (mp.flags & seq::kSigmoidGate) != 0;
   const float q_scale = kFused ? mp.q_scale : 1.f;
-  auto issue_raw = [&](const ItemWalk &w) {     // thread 0 only: one copy per tensor
+  auto valid_steps = [&](const ItemWalk &w) {
+    const int64_t left = T_ - (int64_t)w.c * kC;
+    return (int)(left < kC ? left : kC);
+  };
+  auto issue_raw = [&](const ItemWalk &w) {     // one thread: one copy per tensor
     int b, hc;
     w.item(mp.heads, &b, &hc);
-    const int row = (int)(b * T_ + w.c * kC);
-    const int nv = (int)((T_ - (int64_t)w.c * kC < kC) ? T_ - (int64_t)w.c * kC : kC);
+    const int row = (int)(b * T_ + w.c * kC), nv = valid_steps(w);
     const uint32_t per = (mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes;
-    acp::mbar_expect_tx(&barRaw, (unit_forget ? 5u : 6u) * per);
-#pragma unroll
+    acp::mbar_expect_tx(&barRaw, (kFused ? 5u : 6u) * per);
+#pragma unroll 1
     for (int i = 0; i < 6; ++i)
-      if (!(i == 1 && unit_forget)) seq::fetch_block<T>(mp, i, sm + oRaw + i * kRawBytes, row, hc, nv, &barRaw);
+      if (!(i == 1 && kFused)) seq::fetch_block<T>(mp, i, sm + oRaw + i * kRawBytes, row, hc, nv, &barRaw);
   };
-  // fused layer: the gate pre-activations once more, into the block that the constant forget gate leaves free.
-  // The epilogue reads them, after the raw blocks have been handed to the next chunk.
-  auto issue_preact = [&](const ItemWalk &w) {
-    int b, hc;
-    w.item(mp.heads, &b, &hc);
-    const int nv = (int)((T_ - (int64_t)w.c * kC < kC) ? T_ - (int64_t)w.c * kC : kC);
-    acp::mbar_expect_tx(&barG, (mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
-    seq::fetch_block<T>(mp, 4, sm + oRaw + kRawBytes, (int)(b * T_ + w.c * kC), hc, nv, &barG);
-  };
-  // start state (16-bit, 8 KB) and end state gradient (fp32, 16 KB) of a chunk into the padded
-  // landing zones: three 16-byte asynchronous copies per thread
-  auto issue_state = [&](const ItemWalk &w) {   // every thread
+  // one warp: start state of a chunk (16-bit, 8 KB; row by row into the padded landing zone) and end state gradient (fp32,
+  // 16 KB, pieces XOR-ed by row as the carry left them)
+  auto issue_state = [&](const ItemWalk &w) {
     const T *s0p = (w.c == 0) ? state + seq::state_off(mp, w.row, w.sub, 0, 1) : ckpt + seq::state_off(mp, w.row, w.sub, w.c - 1, nc);
-    const float *rp = Rend + ((size_t)w.bh() * nc + w.c) * kDim * kDim;
-    cp_async16(sm + oS0L + (tid >> 3) * kS0Ld + (tid & 7) * 16, s0p + (size_t)(tid >> 3) * mp.state_ld + (tid & 7) * 8);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int c16 = tid + i * kThreadsB;
-      cp_async16(sm + oRL + (c16 >> 4) * kRLd + (c16 & 15) * 16, rp + (c16 >> 4) * kDim + (c16 & 15) * 4);
+    if (lane == 0) {
+      acp::mbar_expect_tx(&barState, kDim * kDim * (uint32_t)(sizeof(float) + sizeof(T)));
+      acp::bulk_g2s(sm + oRL, Rend + ((size_t)w.bh() * nc + w.c) * kDim * kDim, kDim * kDim * (uint32_t)sizeof(float), &barState);
     }
-    cp_async_commit();
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kDim; r += 32)
+      acp::bulk_g2s(sm + oS0L + (lane + r) * kS0Ld, s0p + (size_t)(lane + r) * mp.state_ld, kDim * (uint32_t)sizeof(T), &barState);
+  };
+  // this warp's writes are complete: tiles (for the tensor core) and tensor memory
+  auto report = [&](uint64_t *bar) {
+    umma::fence_async_smem();
+    umma::fence_before_sync();
+    __syncwarp();
+    if (lane == 0) acp::mbar_arrive(bar);
   };
 
   if (tid == 0) {
     umma::mbar_init(&barRaw, 1);
-    umma::mbar_init(&barG, 1);
-    umma::mbar_init(&barZ, 2);       // one commit per side
-    umma::mbar_init(&barM1, 4);      // TQ1 and T7 of both sides
-    umma::mbar_init(&barM2, 4);      // TQ2 and T2 of both sides
+    umma::mbar_init(&barState, 1);
+    umma::mbar_init(&barT, kWarpsB + 1);  // operand tiles, and the results before have left the other buffer
+    umma::mbar_init(&barA, kWarpsB);      // state operands
+    umma::mbar_init(&barZs, kWarpsB);     // Z tiles
+    umma::mbar_init(&barZ, 1);
+    umma::mbar_init(&barM1, 1);           // TQ1 and T7 of both sides
+    umma::mbar_init(&barM2, 1);           // TQ2 and T2 of both sides
+    umma::mbar_init(&barOut, kWarpsB);    // results staged
     umma::mbar_fence_init();
-    s_fail = 0;
-    s_bad2[0] = s_bad2[1] = fix_n2[0] = fix_n2[1] = fix_rows_n = 0;
+    s_bad2[0] = s_bad2[1] = fix_n2[0] = fix_n2[1] = 0;
   }
-  if (tid < 2 * kDim) fix_mask[tid] = 0ull;
-  for (int i = tid; i < 4 * kTile / 16; i += kThreadsB)      // the blocks above the diagonal of Z are never written again
-    *reinterpret_cast<float4 *>(sm + oZ + 16 * i) = make_float4(0.f, 0.f, 0.f, 0.f);
   if (warp == 0) umma::tmem_alloc(&tmem_slot, kTmemCols);
   sync_all();
   dependency_wait();
   const uint32_t tb = __shfl_sync(0xffffffffu, tmem_slot, 0);
-  const uint32_t tl = umma::tmem_addr(tb, 32 * q4, 0);
-  bool raw_pending = false, pre_pending = false;      // thread 0
-  ItemWalk wi(blockIdx.x, gridDim.x, nc, kGrid ? mp.nsub : 1), wn = wi;           // this chunk and the next one
-  if (wi.unit < total) {
-    if (tid == 0) {
-      issue_raw(wi);
-      raw_pending = true;
+  ItemWalk wn(blockIdx.x, gridDim.x, nc, kGrid ? mp.nsub : 1);
+  uint32_t it = 0;
+  int fail = 0;
+  if (warp >= kWarpsB) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
+    if (warp == kWarpsB) {      // ---- products ----
+      const uint32_t aSm = umma::smem_u32(sm);
+      for (; wn.unit < total && !fail; ++it, wn.step()) {
+        const uint32_t ph = it & 1u;
+        const uint32_t aT = aSm + ph * kTiles, aZ = aSm + (ph ^ 1u) * kTiles;
+        const uint32_t ls = tb, ls1 = umma::tmem_addr(tb, 16, 0);      // lane sets of the k side and the d side
+        // The chains of dependent instructions of the two sides and of the two results take turns: the tensor core
+        // executes in issue order.
+        if (!umma::mbar_wait(&barT, ph)) fail = 1;
+        umma::fence_after_sync();
+        if (elect_one()) {      // Z of either side from the other side's tiles
+          const uint64_t k0 = desc_sw128(aT), k1 = desc_sw128(aT + kTile), d0 = desc_sw128(aT + 2 * kTile), d1 = desc_sw128(aT + 3 * kTile);
+#pragma unroll 1
+          for (int ks = 0; ks < 8; ++ks) {
+            umma::mma_tf32(ls + cZ, d0 + kstep(ks), d1 + kstep(ks), kIdesc64, ks > 0);
+            umma::mma_tf32(ls1 + cZ, k0 + kstep(ks), k1 + kstep(ks), kIdesc64, ks > 0);
+          }
+          umma::mma_commit(&barZ);
+        }
+        __syncwarp();
+        if (!umma::mbar_wait(&barA, ph)) fail = 1;
+        umma::fence_after_sync();
+        if (elect_one()) {
+          const uint64_t k0 = desc_sw128(aT), k1 = desc_sw128(aT + kTile), d0 = desc_sw128(aT + 2 * kTile), d1 = desc_sw128(aT + 3 * kTile);
+#pragma unroll 1
+          for (int ks = 0; ks < 8; ++ks) {
+            mma_tf32_ts(ls + cTQ1, ls + cS2 + 8 * ks, d0 + kstep(ks), kIdesc64, ks > 0);
+            mma_tf32_ts(ls1 + cTQ1, ls1 + cS2 + 8 * ks, k0 + kstep(ks), kIdesc64, ks > 0);
+            mma_tf32_ts(ls + cT7, ls + cR2 + 8 * ks, d1 + kstep(ks), kIdesc64, ks > 0);
+            mma_tf32_ts(ls1 + cT7, ls1 + cR2 + 8 * ks, k1 + kstep(ks), kIdesc64, ks > 0);
+          }
+          umma::mma_commit(&barM1);
+        }
+        __syncwarp();
+        if (!umma::mbar_wait(&barZs, ph)) fail = 1;
+        umma::fence_after_sync();
+        if (elect_one()) {      // TQ2 = Vw Z^T, T2 = Mw Z
+          const uint64_t k0 = desc_sw128(aZ), k1 = desc_sw128(aZ + kTile), d0 = desc_sw128(aZ + 2 * kTile), d1 = desc_sw128(aZ + 3 * kTile);
+#pragma unroll 1
+          for (int ks = 0; ks < 8; ++ks) {
+            mma_tf32_ts(ls + cTQ2, ls + cVw + 8 * ks, k0 + kstep(ks), kIdesc64, ks > 0);
+            mma_tf32_ts(ls1 + cTQ2, ls1 + cVw + 8 * ks, d0 + kstep(ks), kIdesc64, ks > 0);
+            mma_tf32_ts(ls + cT2, ls + cMw + 8 * ks, k1 + kstep(ks), kIdesc64, ks > 0);
+            mma_tf32_ts(ls1 + cT2, ls1 + cMw + 8 * ks, d1 + kstep(ks), kIdesc64, ks > 0);
+          }
+          umma::mma_commit(&barM2);
+        }
+        __syncwarp();
+      }
+    } else if (warp == kWarpsB + 1) {      // ---- raw blocks ----
+      int item = 0;
+      for (;; ++it, wn.step()) {
+        if (it > 0) {
+          if (!umma::mbar_wait(&barT, (it - 1) & 1u)) fail = 1;      // every warp has read its raw values
+          if (lane == 0 && s_bad2[(it - 1) & 1u]) atomicExch(rowflag + item, 1);      // the scan kernels redo this row
+        }
+        if (wn.unit >= total || fail) break;
+        item = wn.row;
+        if (lane == 0) issue_raw(wn);
+      }
+      // after a wait that gave up, copies may still be on their way into this CTA: bounded, let them land
+      if (it > 0) acp::mbar_wait(&barRaw, (it - 1) & 1u);
+    } else if (warp == kWarpsB + 2) {      // ---- state blocks ----
+      for (;; ++it, wn.step()) {
+        if (it > 0 && !umma::mbar_wait(&barA, (it - 1) & 1u)) fail = 1;      // the landing zones have been read
+        if (wn.unit >= total || fail) break;
+        issue_state(wn);
+      }
+      if (it > 0) acp::mbar_wait(&barState, (it - 1) & 1u);
+    } else {      // ---- results ----
+      if (lane == 0) acp::mbar_arrive(&barT);
+      for (; wn.unit < total && !fail; ++it, wn.step()) {
+        if (!umma::mbar_wait(&barOut, it & 1u)) fail = 1;
+        if (lane == 0 && !fail) {
+          const unsigned char *const uT = sm + (it & 1u) * kTiles;
+          int ob, oh;
+          wn.item(mp.heads, &ob, &oh);
+          const int64_t row0 = (int64_t)ob * T_ + (int64_t)wn.c * kC;
+          const int nvalid = valid_steps(wn);
+          if (kMode == 0) {      // dense [rows][64] arrays: one linear copy per tensor
+            const uint32_t bytes = (uint32_t)nvalid * kDim * sizeof(T);
+            acp::bulk_s2g(dq.p + row0 * kDim, uT, bytes);
+            acp::bulk_s2g(dk.p + row0 * kDim, uT + kRawBytes, bytes);
+            acp::bulk_s2g(dfk.p + row0 * kDim, uT + 2 * kRawBytes, bytes);
+            acp::bulk_s2g(dx.p + row0 * kDim, uT + 3 * kRawBytes, bytes);
+            acp::bulk_s2g(df.p + row0 * kDim, uT + 4 * kRawBytes, bytes);
+          } else if (kFused && nvalid == kC) {      // boxes of the gradient of the projection output
+            seq::store_block(&mp.out, dq.col + oh * kDim, (int)row0, uT);
+            seq::store_block(&mp.out, dk.col + oh * kDim, (int)row0, uT + kRawBytes);
+            seq::store_block(&mp.out, dfk.col + oh * kDim, (int)row0, uT + 2 * kRawBytes);
+            seq::store_block(&mp.out, dx.col + oh * kDim, (int)row0, uT + 3 * kRawBytes);
+          }
+          acp::bulk_commit();
+          acp::bulk_wait_read<0>();
+          acp::mbar_arrive(&barT);      // the buffer is free for the next chunk's Z
+        }
+      }
+      if (lane == 0) acp::bulk_wait_all();
     }
-    issue_state(wi);
-  }
-  const uint32_t aT = umma::smem_u32(sm);
+    if (fail) atomicExch(status, 1);
+  } else {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsCompute));
+  const uint32_t tl = umma::tmem_addr(tb, 32 * q4, 0);
   // tile column offset of the own feature: row r of the swizzled tile adds r * 128 and XORs r % 8 into bits 4-6
   const int tcol = (feat >> 5) * kColBlock + ((feat & 3) << 2), tswz = ((feat >> 2) & 7) << 4;
   // Z tiles of the own side: row 16 q4 + fl, columns t0 .. (16-byte pieces XOR-ed with the row); and column
   // 16 q4 + fl of the transposed tile, rows t0 .., the second half warp four rows on
   const int zt_row = 16 * q4 + fl;
-  unsigned char *const zrow = sm + oZ + h * 2 * kTile + (t0 >> 5) * kColBlock + zt_row * 128;
+  const int zrow = h * 2 * kTile + (t0 >> 5) * kColBlock + zt_row * 128;
   const int zsw = (((t0 >> 2) & 7) ^ (zt_row & 7)) << 4;
-  unsigned char *const zt_lo = sm + oZ + (h * 2 + 1) * kTile + (zt_row >> 5) * kColBlock + t0 * 128 + ((zt_row & 3) << 2) + 512 * h;
-  unsigned char *const zt_hi = zt_lo - 1024 * h;
+  const int zt_lo = (h * 2 + 1) * kTile + (zt_row >> 5) * kColBlock + t0 * 128 + ((zt_row & 3) << 2) + 512 * h;
+  const int zt_hi = zt_lo - 1024 * h;
   const int ztsw = (((zt_row >> 2) & 7) ^ (4 * h)) << 4;
+  // column of the end gradient: as in a tile, a row's pieces are XOR-ed with (row % 8)
+  const int rcol = ((feat >> 5) << 7) + ((feat & 3) << 2), rswz = tswz;
   const T *gcol = raw + (h ? 1 : 4) * kC * kDim + t0 * kDim + feat;
   const T *mcol = raw + (h ? 5 : 2) * kC * kDim + t0 * kDim + feat;
   const T *vcol = raw + (h ? 0 : 3) * kC * kDim + t0 * kDim + feat;
+  // fused layer: the gates' derivatives of the quarter, steps 0 .. 31 and 32 .. 63 in different places
+  float *const der = reinterpret_cast<float *>(sm + (tq < 2 ? oDer0 : oDer1)) + (t0 & 31) * kDim + 16 * q4 + fl;
 
-  uint32_t it = 0;
   for (; wn.unit < total; ++it) {
-    wi = wn;
+    const ItemWalk wi = wn;
     wn.step();
-    const int64_t t0c = (int64_t)wi.c * kC;
-    const int nvalid = (int)((T_ - t0c < kC) ? T_ - t0c : kC);
+    const uint32_t ph = it & 1u;
+    const int nvalid = valid_steps(wi);
     // first row and column windows of the chunk in the output arrays
     int ob, oh;
     wi.item(mp.heads, &ob, &oh);
-    const int64_t row0 = (int64_t)ob * T_ + t0c;
+    const int64_t row0 = (int64_t)ob * T_ + (int64_t)wi.c * kC;
     // grid: block (i, j) holds d-side window i and k-side window j; `add`: not the first block of the sum over the other axis
     const int gi = kGrid ? oh / mp.nk : 0, gj = kGrid ? oh - gi * mp.nk : 0;
-    const int hcol = (kGrid ? (h ? gi : gj) : oh) * kDim;
     const bool add = kGrid && (h ? gj : gi) != 0;
-    int &fix_n = fix_n2[it & 1], &s_bad = s_bad2[it & 1];
+    int &fix_n = fix_n2[ph], &s_bad = s_bad2[ph];
+    // this chunk's operand tiles (then its results) and its Z tiles
+    unsigned char *const uT = sm + ph * kTiles, *const uZ = sm + (ph ^ 1u) * kTiles;
 
-    if (!acp::mbar_wait(&barRaw, it & 1u)) s_fail = 1;
-    if (tid == 0) raw_pending = false;
+    if (!acp::mbar_wait(&barRaw, ph)) fail = 1;
 
     // ---- gates of the own feature and quarter, product of the quarter ----
     float g[16];
     float g_min = kRangeHi;
+    if (kFused) {      // the two half warps share the activations of the k side's feature; the d side's gates are 1
+      float a[8];
+      const T *p = raw + 4 * kC * kDim + (t0 + 8 * h) * kDim + 16 * q4 + fl;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) g[j] = Elem<T>::ld(gcol + j * kDim);
-    if (kFused) {
-      if (sigmoid_gate && h == 0) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) g[j] = seq::sigmoid_gate<T>(g[j]);
+      for (int j = 0; j < 8; ++j) {
+        const float e = seq::exp_neg(Elem<T>::ld(p + j * kDim)), sg = seq::rcp1p(e);
+        a[j] = seq::round_to<T>(fmaxf(sg, seq::kGateFloor));
+        // d gate / d pre-activation in fp32: s (1 - s) = s^2 e^-g
+        der[(8 * h + j) * kDim] = sg > seq::kGateFloor ? sg * sg * e : 0.f;
       }
-      if (unit_forget && h == 1) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) g[j] = 1.f;
+      for (int j = 0; j < 8; ++j) {
+        const float o = __shfl_xor_sync(0xffffffffu, a[j], 16);
+        g[j] = h ? 1.f : a[j];
+        g[8 + j] = h ? 1.f : o;
       }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) g[j] = Elem<T>::ld(gcol + j * kDim);
     }
     if (nvalid < kC) {      // partial chunk: identity steps beyond the valid ones
 #pragma unroll
       for (int j = 0; j < 16; ++j) g[j] = t0 + j < nvalid ? g[j] : 1.f;
     }
+    if (!kFused) {          // (the fused layer's gates are at least 1/8)
 #pragma unroll
-    for (int j = 0; j < 16; ++j) g_min = fminf(g_min, fabsf(g[j]));
-    if (!(g_min >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+      for (int j = 0; j < 16; ++j) g_min = fminf(g_min, fabsf(g[j]));
+      if (!(g_min >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
 #pragma unroll
-      for (int j = 0; j < 16; ++j) g[j] = sanitize_gate(g[j]);
+        for (int j = 0; j < 16; ++j) g[j] = sanitize_gate(g[j]);
+      }
     }
     {
       float p0 = g[0], p1 = g[1];      // two chains
@@ -245,7 +362,8 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       for (int j = 2; j < 16; j += 2) { p0 *= g[j]; p1 *= g[j + 1]; }
       qtot[(h * 4 + tq) * kDim + feat] = p0 * p1;
     }
-    umma::named_barrier(1 + q4, 128);      // the four warps that hold the quarters of the same features
+    if (umma::named_barrier_or(5, kThreadsB, fail)) break;      // (the whole group leaves together)
+    unsigned tiny = 0;                     // steps of the quarter with tiny gates
     float pm[16], up, after, pm_prev;      // ratios to the anchor; products up to and after it; ratio of the step before
     {
       const float *qt = qtot + h * 4 * kDim + feat;
@@ -253,10 +371,6 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       up = q0 * q1;
       after = q2 * q3;
       pm_prev = tq == 0 ? rcp_fast(up) : tq == 1 ? rcp_fast(q1) : tq == 2 ? 1.f : q2;
-      if (tq == 1) {
-        prd[(h * 2) * kDim + feat] = up;
-        prd[(h * 2 + 1) * kDim + feat] = after;
-      }
       const float carry = tq == 0 ? q1 : tq == 3 ? q2 : 1.f;
       float mw[16], vw[16];
 #pragma unroll
@@ -264,9 +378,9 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         mw[j] = Elem<T>::ld(mcol + j * kDim);
         vw[j] = Elem<T>::ld(vcol + j * kDim);
       }
-      if (kFused && q_scale != 1.f && h == 0) {
+      if (kFused) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) mw[j] = seq::round_to<T>(mw[j] * q_scale);
+        for (int j = 0; j < 16; ++j) mw[j] = h ? mw[j] : seq::round_to<T>(mw[j] * q_scale);
       }
       if (nvalid < kC) {
 #pragma unroll
@@ -275,17 +389,23 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
           vw[j] = t0 + j < nvalid ? vw[j] : 0.f;
         }
       }
-      // the walk away from the anchor: downwards for the first two quarters (s = 1 / pm), upwards for the others
-      float s = carry, lo = fabsf(carry), hi = lo;
+      // The walk away from the anchor: downwards for the first two quarters (s = 1 / pm), upwards for the others; and back
+      // with the reciprocal of the product at the far end, which the gates on the way turn into that of every step.
+      float s = carry, lo = fabsf(carry), hi = lo, r;
       if (tq < 2) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
-          pm[j] = rcp_fast(s);
-          mw[j] = rna_tf32(mw[j] * pm[j]);
           vw[j] = rna_tf32(vw[j] * s);
+          if (j == 0) r = rcp_fast(s);
           s *= g[j];
           lo = fminf(lo, fabsf(s));
           hi = fmaxf(hi, fabsf(s));
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (j > 0) r *= g[j];
+          pm[j] = r;
+          mw[j] = rna_tf32(mw[j] * r);
         }
       } else {
 #pragma unroll
@@ -295,91 +415,48 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
           hi = fmaxf(hi, fabsf(s));
           pm[j] = s;
           mw[j] = rna_tf32(mw[j] * s);
-          vw[j] = rna_tf32(vw[j] * rcp_fast(s));
+        }
+        r = rcp_fast(s);
+#pragma unroll
+        for (int j = 15; j >= 0; --j) {
+          vw[j] = rna_tf32(vw[j] * r);
+          r *= g[j];
         }
       }
       if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad = 1;      // also NaN
       umma::tmem_st16(tl + cMw + t0, mw);
       umma::tmem_st16(tl + cVw + t0, vw);
-      unsigned char *tp = sm + oT + h * 2 * kTile + tcol + t0 * 128;
+      unsigned char *tp = uT + h * 2 * kTile + tcol + t0 * 128;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         unsigned char *p = tp + (tswz ^ ((j & 7) << 4)) + j * 128;
         *reinterpret_cast<float *>(p) = mw[j];
         *reinterpret_cast<float *>(p + kTile) = vw[j];
       }
-      if (g_min < kTinyGate) {      // rare: some gate of this quarter is tiny; exact pair sums for those later
+      if (!kFused && g_min < kTinyGate) {      // rare: exact pair sums for these steps, listed further down
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (fabsf(g[j]) < kTinyGate && t0 + j < nvalid) {
-            const int slot = atomicAdd(&fix_n, 1);
-            if (slot < kFixCap) {
-              fix_code[slot] = ((t0 + j) << 8) | (h << 6) | feat;
-              if (atomicOr(&fix_mask[h * kDim + feat], 1ull << (t0 + j)) == 0ull) {      // first entry of this feature
-                const int rs = atomicAdd(&fix_rows_n, 1);
-                fix_slot[h * kDim + feat] = rs < kFixRows ? rs : -1;
-                if (rs >= kFixRows) s_bad = 1;
-              }
-            } else {
-              s_bad = 1;
-            }
-          }
-        }
+        for (int j = 0; j < 16; ++j) tiny |= (fabsf(g[j]) < kTinyGate && t0 + j < nvalid ? 1u : 0u) << j;
       }
     }
-    cp_async_wait_all();       // this thread's share of the start state and end gradient
-    umma::fence_async_smem();
-    sync_all();                // tiles, anchor products and state blocks of all threads
-    if (s_fail) break;
+    umma::tmem_st_wait();
+    report(&barT);
 
-    // ---- Z of both sides: each a chain of eight dependent instructions, issued by lanes of two warps so that
-    //      the chains interleave in the tensor core, which executes in issue order ----
-    if (warp < 2) {
-      const uint32_t d = umma::tmem_addr(tb, 16 * warp, cZ);
-      const uint32_t other = aT + oT + (warp ^ 1) * 2 * kTile;
-      const uint64_t da = desc_sw128(other), db = desc_sw128(other + kTile);
-      if (elect_one()) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) umma::mma_tf32(d, da + kstep(ks), db + kstep(ks), kIdesc64, ks > 0);
-        umma::mma_commit(&barZ);
-      }
-      __syncwarp();
-    }
-    if (kFused && sigmoid_gate && tid == 0) {      // every thread is past the epilogue of the chunk before
-      issue_preact(wi);
-      pre_pending = true;
-    }
-    if (fix_n > 0 && fix_mask[h * kDim + feat] != 0ull) {      // rare: the direct pair sums of this feature read its operand rows
-      const int rs = fix_slot[h * kDim + feat];
-      if (rs >= 0) {
-        float *row = fix_rows + rs * 2 * kDim + t0;
-        float a[16], b[16];
-        // (a divergent tensor-memory load is not possible: the values come back from the tile)
-        const unsigned char *tp = sm + oT + h * 2 * kTile + tcol + t0 * 128;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const unsigned char *p = tp + (tswz ^ ((j & 7) << 4)) + j * 128;
-          a[j] = *reinterpret_cast<const float *>(p);
-          b[j] = *reinterpret_cast<const float *>(p + kTile);
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          row[j] = a[j];
-          row[kDim + j] = b[j];
-        }
-      }
+    if (tid == 0) {      // (the other chunk's; read by nobody any more, written behind the next barrier)
+      s_bad2[ph ^ 1u] = 0;
+      fix_n2[ph ^ 1u] = 0;
     }
 
     // ---- state blocks as A operands: row = own feature, columns t0 .. t0 + 15 of the other side, scaled by the
     //      other side's anchor products; their elementwise product is the boundary term ----
+    if (!acp::mbar_wait(&barState, ph)) fail = 1;
     {
-      const float *oref = prd + (h ^ 1) * 2 * kDim + t0;
+      const float *oq = qtot + (h ^ 1) * 4 * kDim + t0;
       float sv[16], rv[16];
       if (h == 0) {         // S(own = k, other = d = t0 + j): a column of the stored blocks
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           sv[j] = Elem<T>::ld(reinterpret_cast<const T *>(sm + oS0L + (t0 + j) * kS0Ld) + feat);
-          rv[j] = *(reinterpret_cast<const float *>(sm + oRL + (t0 + j) * kRLd) + feat);
+          rv[j] = *reinterpret_cast<const float *>(sm + oRL + (t0 + j) * kRLd + rcol + (rswz ^ ((j & 7) << 4)));
         }
       } else {              // S(own = d, other = k = t0 + j): a row segment
 #pragma unroll
@@ -391,7 +468,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float4 r4 = *reinterpret_cast<const float4 *>(sm + oRL + feat * kRLd + t0 * 4 + 16 * i);
+          const float4 r4 = *reinterpret_cast<const float4 *>(sm + oRL + feat * kRLd + (((4 * tq + i) ^ (feat & 7)) << 4));
           rv[4 * i] = r4.x; rv[4 * i + 1] = r4.y; rv[4 * i + 2] = r4.z; rv[4 * i + 3] = r4.w;
         }
       }
@@ -399,8 +476,10 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       float acc = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float4 a = *reinterpret_cast<const float4 *>(oref + 4 * i), b = *reinterpret_cast<const float4 *>(oref + kDim + 4 * i);
-        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+        const float4 q0 = *reinterpret_cast<const float4 *>(oq + 4 * i), q1 = *reinterpret_cast<const float4 *>(oq + kDim + 4 * i);
+        const float4 q2 = *reinterpret_cast<const float4 *>(oq + 2 * kDim + 4 * i), q3 = *reinterpret_cast<const float4 *>(oq + 3 * kDim + 4 * i);
+        const float av[4] = {q0.x * q1.x, q0.y * q1.y, q0.z * q1.z, q0.w * q1.w};
+        const float bv[4] = {q2.x * q3.x, q2.y * q3.y, q2.z * q3.z, q2.w * q3.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float s2 = sv[4 * i + j] * av[j], r2 = rv[4 * i + j] * bv[j];
@@ -414,113 +493,50 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       bndp[(h * 4 + tq) * kDim + feat] = acc;
     }
     umma::tmem_st_wait();
-    sync_all();       // all operands in place; raw blocks and landing zones are consumed
-
-    if (warp >= 2 && warp < 6) {      // TQ1 (warps 2, 3) and T7 (warps 4, 5) of side warp & 1
-      const int side = warp & 1, is7 = (warp - 2) >> 1;
-      const uint32_t ls = umma::tmem_addr(tb, 16 * side, 0);
-      const uint32_t d = ls + (is7 ? cT7 : cTQ1), a = ls + (is7 ? cR2 : cS2);
-      const uint64_t db = desc_sw128(aT + oT + ((side ^ 1) * 2 + is7) * kTile);
-      if (elect_one()) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) mma_tf32_ts(d, a + 8 * ks, db + kstep(ks), kIdesc64, ks > 0);
-        umma::mma_commit(&barM1);
+    report(&barA);
+    if (!kFused) {
+      for (; tiny != 0; tiny &= tiny - 1) {
+        const int slot = atomicAdd(&fix_n, 1);
+        if (slot < kFixCap) fix_code[slot] = ((t0 + __ffs(tiny) - 1) << 8) | (h << 6) | feat;
+        else atomicExch(rowflag + wi.row, 1);      // the scan kernels redo this row
       }
       __syncwarp();
-    }
-    if (wn.unit < total) {      // the next chunk's inputs and state blocks
-      if (tid == 0) {
-        issue_raw(wn);
-        raw_pending = true;
-      }
-      issue_state(wn);
-    }
-    if (tid == 0) {
-      if (s_bad) atomicExch(rowflag + wi.row, 1);      // the scan kernels redo this row
-      s_bad2[(it & 1) ^ 1] = 0;
-      fix_n2[(it & 1) ^ 1] = 0;
     }
 
     // ---- Z: mask, round, store as [t][s] and [s][t].  A warp holds rows 16 q4 .. + 15 and columns t0 .. t0 + 15: on
-    //      the diagonal it masks, below it nothing is masked, above it the blocks stay zero ----
-    if (!umma::mbar_wait(&barZ, it & 1u)) s_fail = 1;
+    //      the diagonal it masks, below it nothing is masked, above it all is zero ----
+    if (!umma::mbar_wait(&barZ, ph)) fail = 1;
     umma::fence_after_sync();
-    if (tq <= q4) {
+    {
       float v[16];
-      umma::tmem_ld16(tl + cZ + t0, v);
-      umma::tmem_ld_wait();
-      if (tq == q4) {
+      if (tq <= q4) {
+        umma::tmem_ld16(tl + cZ + t0, v);
+        umma::tmem_ld_wait();
+        if (tq == q4) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = j <= fl ? bias_tf32(v[j]) : 0.f;
+          for (int j = 0; j < 16; ++j) v[j] = j <= fl ? bias_tf32(v[j]) : 0.f;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = bias_tf32(v[j]);
+        }
       } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = bias_tf32(v[j]);
+        for (int j = 0; j < 16; ++j) v[j] = 0.f;
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<float4 *>(zrow + (zsw ^ (j << 4))) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        *reinterpret_cast<float4 *>(uZ + zrow + (zsw ^ (j << 4))) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
       // transposed: the half warps take rows four apart, which lie in different halves of the swizzle
 #pragma unroll
       for (int j = 0; j < 16; ++j)
-        *reinterpret_cast<float *>(((j & 4) ? zt_hi : zt_lo) + j * 128 + (ztsw ^ ((j & 7) << 4))) = h ? v[j ^ 4] : v[j];
+        *reinterpret_cast<float *>(uZ + ((j & 4) ? zt_hi : zt_lo) + j * 128 + (ztsw ^ ((j & 7) << 4))) = h ? v[j ^ 4] : v[j];
     }
-    umma::fence_async_smem();
-    sync_all();
-    if (s_fail) break;
-
-    if (warp >= 2 && warp < 6) {      // TQ2 = Vw Z^T (warps 2, 3), T2 = Mw Z (warps 4, 5)
-      const int side = warp & 1, is2 = (warp - 2) >> 1;
-      const uint32_t ls = umma::tmem_addr(tb, 16 * side, 0);
-      const uint32_t d = ls + (is2 ? cT2 : cTQ2), a = ls + (is2 ? cMw : cVw);
-      const uint64_t db = desc_sw128(aT + oZ + (side * 2 + is2) * kTile);
-      if (elect_one()) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) mma_tf32_ts(d, a + 8 * ks, db + kstep(ks), kIdesc64, ks > 0);
-        umma::mma_commit(&barM2);
-      }
-      __syncwarp();
-    }
-    // ---- tiny gates: pair terms i < t <= s summed directly (runs under the MMAs), one warp per
-    //      entry, from the feature's operand rows ----
-    const int n_fix = fix_n < kFixCap ? fix_n : kFixCap;
-    if (n_fix > 0) {
-      // the tile holds Z with the rounding increment but unmasked: the value the tensor core uses
-      auto zval = [](const unsigned char *p) {
-        return __uint_as_float(*reinterpret_cast<const uint32_t *>(p) & 0xffffe000u);
-      };
-      for (int e = warp - 8; e >= 0 && e < n_fix; e += 8) {
-        const int code = fix_code[e], t = code >> 8, sf = code & 127, rs = fix_slot[sf];
-        if (rs < 0) continue;      // no row slot: the batch row is flagged
-        const unsigned char *zt = sm + oZ + (sf >> 6) * 2 * kTile;
-        const float *row = fix_rows + rs * 2 * kDim;
-        // sum_{s >= t} Mw[s] sum_{i < t} Z[s][i] Vw[i]: lanes over i, independent loads over s
-        float acc = 0.f;
-        for (int i = lane; i < t; i += 32) {
-          const unsigned char *zcol = zt + (i >> 5) * kColBlock + ((i & 3) << 2);      // tile offset of (s, i) without the s terms
-          const int ic = (i >> 2) & 7;
-          float a0 = 0.f, a1 = 0.f;      // two chains: the sums are latency-bound
-          int s = t;
-          if ((kC - t) & 1) {
-            a0 = row[s] * zval(zcol + s * 128 + ((ic ^ (s & 7)) << 4));
-            ++s;
-          }
-#pragma unroll 4
-          for (; s < kC; s += 2) {
-            a0 = fmaf(row[s], zval(zcol + s * 128 + ((ic ^ (s & 7)) << 4)), a0);
-            a1 = fmaf(row[s + 1], zval(zcol + (s + 1) * 128 + ((ic ^ ((s + 1) & 7)) << 4)), a1);
-          }
-          acc = fmaf(a0 + a1, row[kDim + i], acc);
-        }
-        acc = warp_sum(acc);
-        if (lane == 0) fix_val[e] = acc;
-      }
-      __syncthreads();      // the direct sums are visible (fix_n is final since the operand stage)
-    }
+    report(&barZs);
 
     // ---- epilogue: own feature, steps t0 .. t0 + 15 ----
     // state terms first, while the in-chunk products run: H = inclusive suffix of Mw TQ1 + exclusive prefix of Vw T7
     float H[16], tot_a, tot_p;
-    if (!umma::mbar_wait(&barM1, it & 1u)) s_fail = 1;
+    if (!umma::mbar_wait(&barM1, ph)) fail = 1;
     umma::fence_after_sync();
     {
       float a[16], b[16];
@@ -545,17 +561,59 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       }
       tot_a = run * up;
     }
-    // element pointers of step t0; one row pitch further per step.  The plain operator writes
-    // dense [rows][64] arrays.
-    const seq::Out<T> &o_dv = h ? dx : dk, &o_gt = h ? df : dfk;
-    const int64_t ld_mu = kMode ? dq.ld : kDim, ld_dv = kMode ? o_dv.ld : kDim, ld_gt = kMode ? o_gt.ld : kDim;
-    T *p_mu = dq.p + (size_t)(row0 + t0) * dq.ld + dq.col + hcol + feat;
-    T *p_dv = o_dv.p + (size_t)(row0 + t0) * o_dv.ld + o_dv.col + hcol + feat;
-    const int n_own = nvalid - t0;      // valid own steps (may be negative)
-    const bool full = n_own >= 16;
 
-    if (!umma::mbar_wait(&barM2, it & 1u)) s_fail = 1;
+    // ---- tiny gates: pair terms i < t <= s summed directly (runs under the MMAs) from the tiles, an entry's sum over s by
+    //      several warps ----
+    if (!kFused && !umma::mbar_wait(&barZs, ph)) fail = 1;      // the entries and Z tiles of all warps
+    const int n_fix = kFused ? 0 : fix_n < kFixCap ? fix_n : kFixCap;
+    const int parts_log = n_fix <= kFixParts / 16 ? 4 : n_fix <= kFixParts / 8 ? 3 : 2, n_parts = 1 << parts_log;
+    float *const fix_part = reinterpret_cast<float *>(sm + oFixPart);      // [entry][n_parts]
+    if (n_fix > 0) {
+#pragma unroll 1
+      for (int task = warp; task < n_fix * n_parts; task += kWarpsB) {
+        const int code = fix_code[task >> parts_log], t = code >> 8, sf = code & 127, f = sf & 63;
+        const unsigned char *const mt = uT + (sf >> 6) * 2 * kTile + (f >> 5) * kColBlock + ((f & 3) << 2);      // column of Mw
+        const unsigned char *const zt = uZ + (sf >> 6) * 2 * kTile + ((lane & 3) << 2);
+        auto at = [](const unsigned char *p, int r, int piece) {      // row r of a tile's column; as the tensor core reads it
+          return __uint_as_float(*reinterpret_cast<const uint32_t *>(p + r * 128 + ((piece ^ (r & 7)) << 4)) & 0xffffe000u);
+        };
+        // sum_{s >= t} Mw[s] sum_{i < t} Z[s][i] Vw[i]: lanes over i and i + 32, this part's s
+        float a0 = 0.f, a1 = 0.f;
+#pragma unroll 2
+        for (int r = t + (task & (n_parts - 1)); r < kC; r += n_parts) {
+          const float m = at(mt, r, (f >> 2) & 7);
+          a0 = fmaf(m, at(zt, r, lane >> 2), a0);
+          a1 = fmaf(m, at(zt + kColBlock, r, lane >> 2), a1);
+        }
+        float acc = lane < t ? a0 * at(mt + kTile, lane, (f >> 2) & 7) : 0.f;
+        if (lane + 32 < t) acc = fmaf(a1, at(mt + kTile, lane + 32, (f >> 2) & 7), acc);
+        acc = warp_sum(acc);
+        if (lane == 0) fix_part[task] = acc;
+      }
+      umma::named_barrier(5, kThreadsB);      // the direct sums are visible, the tiles are free
+    }
+
+    if (!umma::mbar_wait(&barM2, ph)) fail = 1;
     umma::fence_after_sync();
+    // Every warp is past its last read of the operand tiles: the results are staged there as [5][64 steps][64 features]
+    // blocks (d_q, d_k, d_f_key, d_x, d_f) and leave in whole rows.
+    T *const stage = reinterpret_cast<T *>(uT) + t0 * kDim + feat;
+    T *const s_dv = stage + (h ? 3 : 1) * kC * kDim, *const s_gt = stage + (h ? 4 : 2) * kC * kDim;
+    const int rr = tid >> 3, rp = tid & 7;      // row and 16-byte piece of this thread where rows leave by plain stores
+    auto place = [&](const seq::Out<T> &o, int col) { return o.p + (size_t)(row0 + rr) * o.ld + o.col + col + rp * 8; };
+    if (kGrid && (gi | gj) != 0) {      // this thread's own sums over the blocks before
+      uint4 old[5];
+      if (rr < nvalid) {
+        const seq::Out<T> *const o[5] = {&dq, &dk, &dfk, &dx, &df};
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+          if ((i < 3 ? gi : gj) != 0) old[i] = *reinterpret_cast<const uint4 *>(place(*o[i], (i < 3 ? gj : gi) * kDim));
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+          if ((i < 3 ? gi : gj) != 0) reinterpret_cast<uint4 *>(uT)[i * 512 + tid] = old[i];
+      }
+      umma::named_barrier(5, kThreadsB);
+    }
     float sb[16], run_b = 0.f;
 #pragma unroll
     for (int half = 1; half >= 0; --half) {
@@ -573,19 +631,6 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
           sb[8 * half + j] = run_b;
         }
       }
-      // grid: this thread's own sums over the blocks before, as stored.  All loads of a batch before the first use or
-      // store, none behind a branch of its own: each would be a round trip to L2.
-      T old_mu[8] = {}, old_dv[8] = {};
-      if (kGrid && add && n_own > 0) {
-        const T *pm_old = h == 0 ? p_mu : p_dv;      // (the d side has no such result: any valid address)
-        const int64_t ld_old = h == 0 ? ld_mu : ld_dv;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int jj = 8 * half + j < n_own ? 8 * half + j : 0;
-          old_mu[j] = pm_old[jj * ld_old];
-          old_dv[j] = p_dv[jj * ld_dv];
-        }
-      }
       float tq1[8], t7[8];
       umma::tmem_ld8(tl + cTQ1 + t0 + 8 * half, tq1);
       umma::tmem_ld8(tl + cT7 + t0 + 8 * half, t7);
@@ -596,17 +641,9 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         const float ip = rcp_fast(pm[jj]);
         const float dmu = pm[jj] * fmaf(up, tq1[j], tq2[j]), ddv = ip * fmaf(after, t7[j], t2[j]);
         pm[jj] = (jj > 0 ? pm[jj > 0 ? jj - 1 : 0] : pm_prev) * ip;      // from here on: 1 / gate of the step
-        if (full || jj < n_own) {
-          if (h == 0) p_mu[jj * ld_mu] = (T)(kFused ? dmu * q_scale : kGrid ? dmu + Elem<T>::ld(&old_mu[j]) : dmu);
-          p_dv[jj * ld_dv] = (T)(kGrid ? ddv + Elem<T>::ld(&old_dv[j]) : ddv);
-        }
+        if (h == 0) stage[jj * kDim] = (T)(kFused ? dmu * q_scale : kGrid && add ? dmu + Elem<T>::ld(stage + jj * kDim) : dmu);
+        s_dv[jj * kDim] = (T)(kGrid && add ? ddv + Elem<T>::ld(s_dv + jj * kDim) : ddv);
       }
-    }
-    T *p_gt = o_gt.p == nullptr ? nullptr : o_gt.p + (size_t)(row0 + t0) * o_gt.ld + o_gt.col + hcol + feat;
-    T old_gt[16] = {};
-    if (kGrid && add && n_own > 0) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) old_gt[j] = p_gt[(j < n_own ? j : 0) * ld_gt];
     }
     {
       const int o = h * kDim + feat;
@@ -634,42 +671,39 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         for (int e = 0; e < n_fix; ++e) {
           const int code = fix_code[e], jj = (code >> 8) - t0;
           if ((code & 127) == o && (unsigned)jj < 16u) {
-            const float v = fix_val[e];
+            float v = 0.f;
+            for (int i = 0; i < n_parts; ++i) v += fix_part[e * n_parts + i];
 #pragma unroll
             for (int j = 0; j < 16; ++j) sb[j] = (jj == j) ? v : sb[j];
           }
         }
-        __syncthreads();      // everybody has read the entries: clear them for the next chunk
-        if (tid < 2 * kDim) fix_mask[tid] = 0ull;
-        if (tid == 0) fix_rows_n = 0;
-        __syncthreads();
       }
-      if (kFused && sigmoid_gate) {
-        if (!acp::mbar_wait(&barG, it & 1u)) s_fail = 1;
-        if (tid == 0) pre_pending = false;
-      }
-      if (o_gt.p != nullptr) {
-        const T *pre = raw + kC * kDim + t0 * kDim + feat;     // fused layer: pre-activations
+      if (!(kFused && h == 1)) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           float dg = (H[j] + base + sb[j]) * pm[j];
-          if (kFused && sigmoid_gate && h == 0) {      // d gate / d pre-activation, from the pre-activation itself in fp32
-            const float e = seq::exp_neg(Elem<T>::ld(pre + j * kDim)), sg = seq::rcp1p(e);
-            dg *= sg > seq::kGateFloor ? sg * sg * e : 0.f;      // s (1 - s) = s^2 e^{-g}
-          }
-          if (full || j < n_own) p_gt[j * ld_gt] = (T)(kGrid ? dg + Elem<T>::ld(&old_gt[j]) : dg);
+          if (kFused) dg *= der[j * kDim];
+          s_gt[j * kDim] = (T)(kGrid && add ? dg + Elem<T>::ld(s_gt + j * kDim) : dg);
         }
       }
       __syncwarp();
     }
-    umma::fence_before_sync();      // this chunk's accumulator reads are ordered before the next barrier
+    // ---- own part of the results staged ----
+    if (kGrid || (kFused && nvalid < kC)) {      // rows that no bulk copy can take: 16 bytes per thread
+      const int kcol = (kGrid ? gj : oh) * kDim, dcol = (kGrid ? gi : oh) * kDim;
+      umma::named_barrier(5, kThreadsB);
+      if (rr < nvalid) {
+        const uint4 *v = reinterpret_cast<const uint4 *>(uT) + tid;
+        *reinterpret_cast<uint4 *>(place(dq, kcol)) = v[0];
+        *reinterpret_cast<uint4 *>(place(dk, kcol)) = v[512];
+        *reinterpret_cast<uint4 *>(place(dfk, kcol)) = v[2 * 512];
+        *reinterpret_cast<uint4 *>(place(dx, dcol)) = v[3 * 512];
+        if (!kFused) *reinterpret_cast<uint4 *>(place(df, dcol)) = v[4 * 512];
+      }
+    }
+    report(&barOut);
   }
-  cp_async_wait_all();
-  __syncthreads();      // s_fail of the last chunk is visible
-  if (tid == 0 && s_fail) {
-    atomicExch(status, 1);
-    if (raw_pending) acp::mbar_wait(&barRaw, it & 1u);   // bounded: let the copies in flight land
-    if (pre_pending) acp::mbar_wait(&barG, it & 1u);
+  if (fail) atomicExch(status, 1);
   }
   sync_all();
   if (warp == 0) umma::tmem_dealloc(tb, kTmemCols);
@@ -694,7 +728,7 @@ int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ck
   do {                                                                                                \
     auto *const kern1 = &lfw_c64_bwd_kernel<TT, FF>; \
     T2FW_ALLOW_SMEM(kern1, kSmemB);       \
-    T2FW_CHECK_CUDA(launch_dependent(lfw_c64_bwd_kernel<TT, FF>, dim3(grid), dim3(kThreadsB), kSmemB, st, mp,   \
+    T2FW_CHECK_CUDA(launch_dependent(lfw_c64_bwd_kernel<TT, FF>, dim3(grid), dim3(kThreadsAll), kSmemB, st, mp,   \
                                      (const TT *)state, (const TT *)ckpt, Rend, T2FW_OUT(TT, 0), T2FW_OUT(TT, 1), \
                                      T2FW_OUT(TT, 2), T2FW_OUT(TT, 3), T2FW_OUT(TT, 4), rowflag, status, T_, nc,  \
                                      total));                                                         \

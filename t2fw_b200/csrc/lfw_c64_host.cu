@@ -12,7 +12,7 @@
 //   2. lfw_c64_carry_kernel<.., false>  from the last chunk down: R_end(c-1) = (Ac Gc^T) .* R_end(c) + G_c,
 //      stored in place of G_c (fp32); what is left after chunk 0 is d_state
 //   3. lfw_c64_bwd_kernel               per (row, chunk): d_x, d_f, d_q, d_k, d_f_key
-// Scratch (floats): M[B][nc][64][64] | Ac[B][nc][64] | Gc[B][nc][64] | flags[B][nc] (int) |
+// Scratch (floats): M[B][nc][64][64], 16-byte pieces of a row XOR-ed with (row % 8) | Ac[B][nc][64] | Gc[B][nc][64] | flags[B][nc] (int) |
 // rowflag[B] (int).  A flagged row (gate products outside the range of the factored form) is recomputed by the
 // scan kernels afterwards.
 // States larger than 64 x 64 (D, K multiples of 64): the recurrence never mixes state rows or columns, so a D x K state
@@ -124,7 +124,8 @@ lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const fl
   dependency_wait();
   const int64_t b = blockIdx.x / (kDim / kCarryRows);
   const int d0 = (int)(blockIdx.x % (kDim / kCarryRows)) * kCarryRows;
-  const int dl = tid / (kDim / 4), d = d0 + dl, k0 = (tid % (kDim / 4)) * 4;
+  // (M's rows lie with their 16-byte pieces XOR-ed with (row % 8): a thread's piece of M holds columns k0 ..)
+  const int dl = tid / (kDim / 4), d = d0 + dl, k0 = ((tid % (kDim / 4)) ^ (d & 7)) * 4;
   // where this block of the states lies: item, offset inside one state, row stride
   const int item = gr.nsub == 1 ? (int)b : (int)b / gr.nsub, sub = (int)b - item * gr.nsub;
   const int in_state = (sub / gr.nk * kDim + d) * gr.ld + sub % gr.nk * kDim + k0, whole = gr.item;
@@ -134,7 +135,7 @@ lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const fl
   const int n = (int)nc;
   T *op = out + (size_t)item * (kFwd ? nc : 1) * whole + in_state;      // forward: the block's next checkpoint
   // this thread's four values of the first chunk of the walk; one chunk further along it per step
-  float *mp = M + (((size_t)b * nc + (kFwd ? 0 : nc - 1)) * kDim + d) * kDim + k0;
+  float *mp = M + (((size_t)b * nc + (kFwd ? 0 : nc - 1)) * kDim + d) * kDim + (tid % (kDim / 4)) * 4;
   constexpr int kNext = (kFwd ? 1 : -1) * kDim * kDim;
   const float *ac = Ac + (size_t)b * nc * kDim + d0, *gc = Gc + (size_t)b * nc * kDim;
   for (int c0 = 0; c0 < n; c0 += kBatch) {
@@ -314,6 +315,10 @@ int backward_typed(const Call &c, const void *gs, const void *state, const void 
   rc = build_maps(mp, all, 6, rows, c.heads, c.flags, c.q_scale);
   if (rc != T2FW_OK) return rc;
   set_grid(mp, c.grid);
+  if (c.f.p == nullptr) {      // fused layer: the four gradients are column windows of one array
+    rc = seq::make_map(&mp.out, outs[0], (uint64_t)rows, (uint64_t)out_ld[0], (uint64_t)out_ld[0]);
+    if (rc != T2FW_OK) return rc;
+  }
   return lfw_c64_backward_main(mp, state, ckpt, s.M, outs, out_ld, out_col, s.rowflag, BH, c.T_, dtype, st);
 }
 

@@ -245,7 +245,8 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
     {
       // Row d = own feature, columns k = t0 .. t0 + 15.  Stored straight from here, the lanes of a warp would write 32
       // different lines with every instruction; so the rows of a quarter pass through the k-side tile (consumed), its
-      // 16-byte pieces XOR-ed with the row, and leave as whole rows.
+      // 16-byte pieces XOR-ed with the row, and leave as whole rows, in memory with their pieces XOR-ed with (row % 8) too
+      // (the gradient kernel reads them along rows and along columns).
       float v[16];
       umma::tmem_ld16(tl + cD + t0, v);
       umma::tmem_ld_wait();
@@ -258,7 +259,7 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
       for (int i = 0; i < 4; ++i) {      // two rows per instruction: rows 8 (tq & 1) .. of this quarter's 16 in chunk tq >> 1
         const int e = tq >> 1, r = 16 * ((q4 + e) & 3) + 8 * (tq & 1) + 2 * i + h;
         const float4 o = *reinterpret_cast<const float4 *>(sm + oTk + e * kTile + r * 256 + ((fl ^ (r & 7)) << 4));
-        if (e == 0 || nv1 > 0) *reinterpret_cast<float4 *>(M + ((size_t)(ci + e) * kDim + r) * kDim + 4 * fl) = o;
+        if (e == 0 || nv1 > 0) *reinterpret_cast<float4 *>(M + ((size_t)(ci + e) * kDim + r) * kDim + 4 * (fl ^ (r & 7))) = o;
       }
     }
     // No full barrier here: before the next one the next pair writes only products of quarters, which nobody reads any

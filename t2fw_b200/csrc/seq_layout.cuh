@@ -29,6 +29,7 @@ constexpr float kGateFloor = 0.125f;   // with gates >= 1/8 no 32-step product l
 
 struct Maps {
   CUtensorMap m[kMaxTensors];    // one per input tensor of the kernel
+  CUtensorMap out;               // fused layer, backward: the gradient of the projection output
   const void *base[kMaxTensors]; // the arrays themselves (used for the linear copies of dense [rows][64] arrays)
   int col[kMaxTensors];          // column of sub-item 0 in a row of that tensor (elements)
   int hdiv[kMaxTensors];         // sub-item h of a batch item reads the 64-column window number
@@ -65,6 +66,14 @@ __device__ __forceinline__ void load_block(void *dst, const CUtensorMap *map, in
           acp::smem_u32(dst)),
       "l"(map), "r"(col), "r"(row), "r"(acp::smem_u32(bar))
       : "memory");
+}
+
+// dense [64][64] block in shared memory -> box whose first row is `row` and first column `col` (neither negative); the
+// caller commits the group
+__device__ __forceinline__ void store_block(const CUtensorMap *map, int col, int row, const void *src) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(col), "r"(row),
+               "r"(acp::smem_u32(src))
+               : "memory");
 }
 
 // ---- activations of the fused layer: gate = max(sigmoid(g), 1/8), rounded to the storage type (what a separate

@@ -144,8 +144,10 @@ __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
 }
 __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 constexpr uint32_t kSpinLimit = 1u << 19;
-// bounded wait for the phase with the given parity; false on timeout
+// bounded wait for the phase with the given parity; false on timeout.  Rolled: unrolled by the compiler, the polls of one
+// kernel's ten waits were half of its code, which a launch fetches through cold instruction caches.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t limit = kSpinLimit) {
+#pragma unroll 1
   for (uint32_t i = 0; i < limit; ++i) {
     uint32_t ok;
     asm volatile(
@@ -209,6 +211,21 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 // barrier among `nthreads` threads (a multiple of 32) that all name the same id (1..15)
 __device__ __forceinline__ void named_barrier(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+// the same, and whether any of them brought a non-zero value
+__device__ __forceinline__ bool named_barrier_or(int id, int nthreads, int v) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.s32 p, %3, 0;\n"
+      "barrier.cta.red.or.pred q, %1, %2, p;\n"
+      "selp.u32 %0, 1, 0, q;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(id), "r"(nthreads), "r"(v)
+      : "memory");
+  return r != 0;
 }
 
 }  // namespace umma
