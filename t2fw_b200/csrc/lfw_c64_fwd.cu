@@ -54,7 +54,7 @@ static_assert(kSmemF + 256 <= 227 * 1024, "shared memory limit");
 constexpr int cS2 = 0, cX = 64, cP = 128, cO1 = 192, cO2 = 256;
 constexpr int kTmemColsF = 512;
 
-// kMode: 0 the plain operator, 1 the fused layer, 2 a grid of blocks (outputs summed over the blocks of a row)
+// kMode: 0 the plain operator, 1 the fused layer (forget gate 1, k-side gates from pre-activations), 2 a grid of blocks (outputs summed over the blocks of a row)
 template <typename T, int kMode>
 __global__ void __launch_bounds__(kThreadsF, 1)
 lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ state, const T *__restrict__ ckpt,
@@ -75,8 +75,6 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   float *qtot = reinterpret_cast<float *>(sm + oQt) + h * 2 * 4 * kDim;      // of the own chunk
 
   // tensors: 0 x, 1 f, 2 q, 3 k, 4 fk
-  const bool unit_forget = kFused && (mp.flags & seq::kUnitForget) != 0;
-  const bool sigmoid_gate = kFused && (mp.flags & seq::kSigmoidGate) != 0;
   const float q_scale = kFused ? mp.q_scale : 1.f;
   auto valid_steps = [&](const ItemWalk &w) {
     if (w.unit >= total) return 0;
@@ -86,7 +84,7 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
   // Two groups with a barrier each: the gate blocks (f, fk) are free again after the products of the quarters, the value
   // blocks (x, q, k) only once the operands are built, so the next pair's gates are requested that much earlier.
   auto issue_raw = [&](const ItemWalk *w, bool gates) {     // thread 0 only: one copy per tensor and chunk
-    const uint32_t n = gates ? (unit_forget ? 1u : 2u) : 3u;
+    const uint32_t n = gates ? (kFused ? 1u : 2u) : 3u;
     uint64_t *bar = gates ? &barG : &barV;
     uint32_t bytes = 0;
 #pragma unroll
@@ -104,7 +102,7 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       const int row = (int)(b * T_ + w[e].c * kC);
 #pragma unroll
       for (int i = 0; i < 5; ++i)
-        if ((i == 1 || i == 4) == gates && !(i == 1 && unit_forget))
+        if ((i == 1 || i == 4) == gates && !(i == 1 && kFused))
           seq::fetch_block<T>(mp, i, sm + oRaw + (e * 5 + i) * kRawBytes, row, hc, nv, bar);
     }
   };
@@ -176,8 +174,8 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       gk[j] = rawv(4, j);
-      if (kFused && sigmoid_gate) gk[j] = seq::sigmoid_gate<T>(gk[j]);
-      gd[j] = kFused && unit_forget ? 1.f : rawv(1, j);
+      if (kFused) gk[j] = seq::sigmoid_gate<T>(gk[j]);
+      gd[j] = kFused ? 1.f : rawv(1, j);
     }
     if (partial) {
 #pragma unroll
@@ -186,10 +184,12 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         gd[j] = t0 + j < nvalid ? gd[j] : 1.f;
       }
     }
-    float mn = kRangeHi;
+    float mn = kRangeHi;      // (the fused layer's gates are at least 1/8)
+    if (!kFused) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) mn = fminf(mn, fminf(fabsf(gk[j]), fabsf(gd[j])));
-    if (!(mn >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+      for (int j = 0; j < 16; ++j) mn = fminf(mn, fminf(fabsf(gk[j]), fabsf(gd[j])));
+    }
+    if (!kFused && !(mn >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         gk[j] = sanitize_gate(gk[j]);
@@ -220,7 +220,7 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         mw[j] = rawv(2, j);
         vw[j] = rawv(3, j);
       }
-      if (kFused && q_scale != 1.f) {
+      if (kFused) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) mw[j] = seq::round_to<T>(mw[j] * q_scale);
       }
@@ -261,7 +261,7 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     float up;                  // A_REF of the own feature; gd[j] becomes pm_a[j]
     {   // d side: x / pm_a into tensor memory
       const float q0 = qtot[4 * kDim + feat], q1 = qtot[5 * kDim + feat];
-      up = q0 * q1;
+      up = kFused ? 1.f : q0 * q1;
       float s = tq == 0 ? q1 : tq == 3 ? qtot[6 * kDim + feat] : 1.f;
       float vw[16];
 #pragma unroll
@@ -270,9 +270,8 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
 #pragma unroll
         for (int j = 0; j < 16; ++j) vw[j] = t0 + j < nvalid ? vw[j] : 0.f;
       }
-      lo = fminf(lo, fabsf(s));
-      hi = fmaxf(hi, fabsf(s));
-      if (tq < 2) {
+      if (kFused) {      // gates 1: the values as they are (exact in TF32)
+      } else if (lo = fminf(lo, fabsf(s)), hi = fmaxf(hi, fabsf(s)), tq < 2) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
           const float a = gd[j];

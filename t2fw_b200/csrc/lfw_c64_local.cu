@@ -68,8 +68,6 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
   float *qtot = reinterpret_cast<float *>(sm + oQtL) + h * 2 * 4 * kDim + feat;      // own chunk and feature
 
   // tensors: 0 val_d, 1 gate_d, 2 val_k, 3 gate_k
-  const bool unit_forget = kFused && (mp.flags & seq::kUnitForget) != 0;
-  const bool sigmoid_gate = kFused && (mp.flags & seq::kSigmoidGate) != 0;
   const float k_scale = kFused ? mp.q_scale : 1.f;
   auto valid_steps = [&](const ItemWalk &w, int64_t ci) {
     if (ci >= total) return 0;
@@ -81,7 +79,7 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int nv = valid_steps(w[e], ci + e);
-      if (nv > 0) bytes += (unit_forget ? 3u : 4u) * ((mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
+      if (nv > 0) bytes += (kFused ? 3u : 4u) * ((mp.flags & seq::kContiguous) ? (uint32_t)nv * kDim * sizeof(T) : (uint32_t)kRawBytes);
     }
     acp::mbar_expect_tx(&barRaw, bytes);
 #pragma unroll
@@ -93,7 +91,7 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
       const int row = (int)(b * T_ + w[e].c * kC);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (!(i == 1 && unit_forget)) seq::fetch_block<T>(mp, i, sm + oRawL + (e * 4 + i) * kRawBytes, row, hc, nv, &barRaw);
+        if (!(i == 1 && kFused)) seq::fetch_block<T>(mp, i, sm + oRawL + (e * 4 + i) * kRawBytes, row, hc, nv, &barRaw);
     }
   };
 
@@ -141,14 +139,15 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
     auto gates = [&](int blk, bool kside, float (&g)[16]) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        if (kFused && !kside && unit_forget) g[j] = 1.f;
+        if (kFused && !kside) g[j] = 1.f;
         else g[j] = rawv(blk, j);
-        if (kFused && kside && sigmoid_gate) g[j] = seq::sigmoid_gate<T>(g[j]);
+        if (kFused && kside) g[j] = seq::sigmoid_gate<T>(g[j]);
       }
       if (partial) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) g[j] = t0 + j < nvalid ? g[j] : 1.f;
       }
+      if (kFused) return;             // (at least 1/8)
       float mn = kRangeHi;
 #pragma unroll
       for (int j = 0; j < 16; ++j) mn = fminf(mn, fabsf(g[j]));
@@ -167,13 +166,17 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
     auto walk = [&](int blk, bool kside, const float (&g)[16], const float *qt, float *tot, float (&w)[16]) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) w[j] = rawv(blk, j);
-      if (kFused && kside && k_scale != 1.f) {
+      if (kFused && kside) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) w[j] = seq::round_to<T>(w[j] * k_scale);
       }
       if (partial) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) w[j] = t0 + j < nvalid ? w[j] : 0.f;
+      }
+      if (kFused && !kside) {         // gates 1: the values as they are (exact in TF32)
+        if (tq == (kSuffix ? 0 : 3) && nvalid > 0) tot[(size_t)(ci + h) * kDim + feat] = 1.f;
+        return;
       }
       float s = 1.f, hi = 0.f;
 #pragma unroll
@@ -201,8 +204,10 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
     float gk[16], gd[16];
     gates(3, true, gk);
     qtot[(4 + tq) * kDim] = product(gk);
-    gates(1, false, gd);
-    qtot[tq * kDim] = product(gd);
+    if (!kFused) {
+      gates(1, false, gd);
+      qtot[tq * kDim] = product(gd);
+    }
     umma::named_barrier(1 + q4, 128);      // the four warps that hold the quarters of the same features
     {
       float w[16];
