@@ -36,6 +36,8 @@ int lfw_c64_forward_out(const seq::Maps &mp, const void *state, const void *ckpt
 int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ckpt, const float *Rend,
                           void *const outs[5], const int64_t out_ld[5], const int out_col[5], int *rowflag,
                           int64_t BH, int64_t T_, int dtype, cudaStream_t st);
+int lfw_wide_forward_out(const seq::Maps &mp, const void *state, const void *ckpt, void *out, int *rowflag, int64_t items,
+                         int64_t T_, int64_t D, int64_t K, int dtype, cudaStream_t st);      // lfw_wide_fwd.cu
 
 namespace {
 
@@ -239,6 +241,9 @@ struct Call {
   float q_scale;
   Grid2D grid{1, 1, kDim * kDim, kDim};
 };
+// States of up to 128 x 128 have kernels of their own that take a chunk of all blocks as one problem (lfw_wide_*.cu).
+// 16 x 16384, 128 x 128: outputs 180 us against 433 as a grid of blocks.
+bool wide(const Grid2D &g) { return g.nsub > 1 && g.nk <= 2 && g.nsub / g.nk <= 2; }
 void set_grid(seq::Maps &mp, const Grid2D &g) {
   mp.nsub = g.nsub; mp.nk = g.nk; mp.state_item = g.item; mp.state_ld = (int)g.ld;
 }
@@ -276,7 +281,8 @@ int forward_typed(const Call &c, const void *state, void *out, int64_t out_ld, i
   rc = build_maps(mp, all, 5, rows, c.heads, c.flags, c.q_scale);
   if (rc != T2FW_OK) return rc;
   set_grid(mp, c.grid);
-  rc = lfw_c64_forward_out(mp, state, ck_all, out, out_ld, out_col, s.rowflag, BH, c.T_, dtype, st);
+  rc = wide(c.grid) ? lfw_wide_forward_out(mp, state, ck_all, out, s.rowflag, c.B, c.T_, out_ld, c.grid.ld, dtype, st)
+                    : lfw_c64_forward_out(mp, state, ck_all, out, out_ld, out_col, s.rowflag, BH, c.T_, dtype, st);
   if (rc != T2FW_OK || m == 1) return rc;
   const int64_t items = BH / c.grid.nsub, slots = ceil_div64(c.T_, ckpt_every), n = items * slots * (c.grid.item / 8);
   const int64_t blocks = ceil_div64(n, 256);
