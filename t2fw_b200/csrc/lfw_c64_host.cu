@@ -38,6 +38,8 @@ int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ck
                           int64_t BH, int64_t T_, int dtype, cudaStream_t st);
 int lfw_wide_forward_out(const seq::Maps &mp, const void *state, const void *ckpt, void *out, int *rowflag, int64_t items,
                          int64_t T_, int64_t D, int64_t K, int dtype, cudaStream_t st);      // lfw_wide_fwd.cu
+int lfw_wide_backward_main(const seq::Maps &mp, const void *state, const void *ckpt, const float *Rend, void *const outs[5],
+                           int *rowflag, int64_t items, int64_t T_, int64_t D, int64_t K, int dtype, cudaStream_t st);
 
 namespace {
 
@@ -242,7 +244,7 @@ struct Call {
   Grid2D grid{1, 1, kDim * kDim, kDim};
 };
 // States of up to 128 x 128 have kernels of their own that take a chunk of all blocks as one problem (lfw_wide_*.cu).
-// 16 x 16384, 128 x 128: outputs 180 us against 433 as a grid of blocks.
+// 16 x 16384, 128 x 128: outputs 180 us against 433 as a grid of blocks, gradients 557 against 1052.
 bool wide(const Grid2D &g) { return g.nsub > 1 && g.nk <= 2 && g.nsub / g.nk <= 2; }
 void set_grid(seq::Maps &mp, const Grid2D &g) {
   mp.nsub = g.nsub; mp.nk = g.nk; mp.state_item = g.item; mp.state_ld = (int)g.ld;
@@ -325,6 +327,8 @@ int backward_typed(const Call &c, const void *gs, const void *state, const void 
     rc = seq::make_map(&mp.out, outs[0], (uint64_t)rows, (uint64_t)out_ld[0], (uint64_t)out_ld[0]);
     if (rc != T2FW_OK) return rc;
   }
+  if (wide(c.grid))
+    return lfw_wide_backward_main(mp, state, ckpt, s.M, outs, s.rowflag, c.B, c.T_, out_ld[0], out_ld[2], dtype, st);
   return lfw_c64_backward_main(mp, state, ckpt, s.M, outs, out_ld, out_col, s.rowflag, BH, c.T_, dtype, st);
 }
 
