@@ -70,39 +70,36 @@ inline Scratch carve(void *scratch, int64_t B, int64_t nc) {
   return s;
 }
 
-constexpr int kBatch = 16;         // chunks whose loads are in flight together
-constexpr int kCarryThreads = 256; // one block = 16 state rows (d) of one batch row, 4 columns (k) per thread
-constexpr int kCarryRows = kCarryThreads / (kDim / 4);
+constexpr int kCarryThreads = 256;
 
-template <typename T> struct Quad;
-template <> struct Quad<__half> {
-  static __device__ __forceinline__ float4 ld(const __half *p) {
-    const uint2 u = *reinterpret_cast<const uint2 *>(p);
-    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u.x));
-    const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
-    return make_float4(a.x, a.y, b.x, b.y);
+// kCols consecutive values of a row: fp32 scratch and 16-bit states
+template <int kCols> struct Piece;
+template <> struct Piece<4> { using F = float4; using H = uint2; };
+template <> struct Piece<2> { using F = float2; using H = uint32_t; };
+__device__ __forceinline__ float2 widen(__half2 v) { return __half22float2(v); }
+__device__ __forceinline__ float2 widen(__nv_bfloat162 v) { return __bfloat1622float2(v); }
+__device__ __forceinline__ void narrow(__half2 *p, float a, float b) { *p = __floats2half2_rn(a, b); }
+__device__ __forceinline__ void narrow(__nv_bfloat162 *p, float a, float b) { *p = __floats2bfloat162_rn(a, b); }
+template <typename T> struct Two;
+template <> struct Two<__half> { using type = __half2; };
+template <> struct Two<__nv_bfloat16> { using type = __nv_bfloat162; };
+template <typename T, int kCols>
+__device__ __forceinline__ void load16(float (&v)[kCols], const T *p) {
+  const typename Piece<kCols>::H u = *reinterpret_cast<const typename Piece<kCols>::H *>(p);
+#pragma unroll
+  for (int i = 0; i < kCols / 2; ++i) {
+    const float2 w = widen(reinterpret_cast<const typename Two<T>::type *>(&u)[i]);
+    v[2 * i] = w.x;
+    v[2 * i + 1] = w.y;
   }
-  static __device__ __forceinline__ void st(__half *p, float4 v) {
-    uint2 u;
-    *reinterpret_cast<__half2 *>(&u.x) = __floats2half2_rn(v.x, v.y);
-    *reinterpret_cast<__half2 *>(&u.y) = __floats2half2_rn(v.z, v.w);
-    *reinterpret_cast<uint2 *>(p) = u;
-  }
-};
-template <> struct Quad<__nv_bfloat16> {
-  static __device__ __forceinline__ float4 ld(const __nv_bfloat16 *p) {
-    const uint2 u = *reinterpret_cast<const uint2 *>(p);
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&u.y));
-    return make_float4(a.x, a.y, b.x, b.y);
-  }
-  static __device__ __forceinline__ void st(__nv_bfloat16 *p, float4 v) {
-    uint2 u;
-    *reinterpret_cast<__nv_bfloat162 *>(&u.x) = __floats2bfloat162_rn(v.x, v.y);
-    *reinterpret_cast<__nv_bfloat162 *>(&u.y) = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2 *>(p) = u;
-  }
-};
+}
+template <typename T, int kCols>
+__device__ __forceinline__ void store16(T *p, const float (&v)[kCols]) {
+  typename Piece<kCols>::H u;
+#pragma unroll
+  for (int i = 0; i < kCols / 2; ++i) narrow(reinterpret_cast<typename Two<T>::type *>(&u) + i, v[2 * i], v[2 * i + 1]);
+  *reinterpret_cast<typename Piece<kCols>::H *>(p) = u;
+}
 
 // States of the call: one 64 x 64 block per problem row (nsub = 1), or a grid of nsub blocks per item
 struct Grid2D {
@@ -110,18 +107,21 @@ struct Grid2D {
   int item, ld;          // elements of a state, row stride
 };
 
-// One thread per (row, d, four consecutive k); a block covers 16 state rows of one batch row.  The
+// One thread per (row, d, kCols consecutive k); a block covers 4 kCols state rows of one batch row.  The
 // recurrence over the chunks is a dependent chain, so the loads of up to 16 chunks are all issued
 // before the chain starts (one round of memory latency per 16 chunks); the decay vectors of those
 // chunks are shared by the block and go through shared memory.
 //   kFwd:  S_{c+1} = (Ac Gc^T) S_c + L_c from the caller's state; checkpoint slot c = S_{c+1}
 //   !kFwd: R_end(c-1) = (Ac Gc^T) R_end(c) + G_c from grad_state, last chunk first; G_c is
 //          overwritten with R_end(c); the value left after chunk 0 is d_state
-template <typename T, bool kFwd>
-__global__ void __launch_bounds__(kCarryThreads, 3)
+template <typename T, bool kFwd, int kCols>
+__global__ void __launch_bounds__(kCarryThreads, kCols == 4 ? 3 : 5)
 lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const float *__restrict__ Ac,
                      const float *__restrict__ Gc, const int *__restrict__ flags, int *__restrict__ rowflag,
                      T *__restrict__ out, const Grid2D gr, int64_t nc) {
+  using F = typename Piece<kCols>::F;
+  constexpr int kBatch = 16;                                 // chunks whose loads are in flight together
+  constexpr int kCarryRows = kCarryThreads / (kDim / kCols);         // state rows of the block
   __shared__ float a_s[kBatch][kCarryRows];
   __shared__ __align__(16) float g_s[kBatch][kDim];
   const int tid = threadIdx.x;
@@ -129,24 +129,25 @@ lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const fl
   const int64_t b = blockIdx.x / (kDim / kCarryRows);
   const int d0 = (int)(blockIdx.x % (kDim / kCarryRows)) * kCarryRows;
   // (M's rows lie with their 16-byte pieces XOR-ed with (row % 8): a thread's piece of M holds columns k0 ..)
-  const int dl = tid / (kDim / 4), d = d0 + dl, k0 = ((tid % (kDim / 4)) ^ (d & 7)) * 4;
+  const int dl = tid / (kDim / kCols), d = d0 + dl, kp = tid % (kDim / kCols) * kCols, k0 = kp ^ ((d & 7) << 2);
   // where this block of the states lies: item, offset inside one state, row stride
   const int item = gr.nsub == 1 ? (int)b : (int)b / gr.nsub, sub = (int)b - item * gr.nsub;
   const int in_state = (sub / gr.nk * kDim + d) * gr.ld + sub % gr.nk * kDim + k0, whole = gr.item;
   // init may be null: the carry then starts from zero (the summary of a sequence segment)
-  float4 S = init != nullptr ? Quad<T>::ld(init + (size_t)item * whole + in_state) : make_float4(0.f, 0.f, 0.f, 0.f);
+  alignas(16) float S[kCols] = {};
+  if (init != nullptr) load16<T, kCols>(S, init + (size_t)item * whole + in_state);
   int any = 0;
   const int n = (int)nc;
   T *op = out + (size_t)item * (kFwd ? nc : 1) * whole + in_state;      // forward: the block's next checkpoint
-  // this thread's four values of the first chunk of the walk; one chunk further along it per step
-  float *mp = M + (((size_t)b * nc + (kFwd ? 0 : nc - 1)) * kDim + d) * kDim + (tid % (kDim / 4)) * 4;
+  // this thread's values of the first chunk of the walk; one chunk further along it per step
+  float *mp = M + (((size_t)b * nc + (kFwd ? 0 : nc - 1)) * kDim + d) * kDim + kp;
   constexpr int kNext = (kFwd ? 1 : -1) * kDim * kDim;
   const float *ac = Ac + (size_t)b * nc * kDim + d0, *gc = Gc + (size_t)b * nc * kDim;
   for (int c0 = 0; c0 < n; c0 += kBatch) {
-    float4 l[kBatch];
+    F l[kBatch];
 #pragma unroll
     for (int j = 0; j < kBatch; ++j)
-      l[j] = *reinterpret_cast<const float4 *>(mp + (c0 + j < n ? j : 0) * kNext);
+      l[j] = *reinterpret_cast<const F *>(mp + (c0 + j < n ? j : 0) * kNext);
     __syncthreads();      // the previous batch's decay vectors are no longer read
     for (int i = tid; i < kBatch * (kCarryRows + kDim); i += kCarryThreads) {
       const int j = i / (kCarryRows + kDim), r = i % (kCarryRows + kDim);
@@ -160,23 +161,34 @@ lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const fl
 #pragma unroll
     for (int j = 0; j < kBatch; ++j) {
       if (c0 + j < n) {
-        if (!kFwd) *reinterpret_cast<float4 *>(mp) = S;
+        if (!kFwd) *reinterpret_cast<F *>(mp) = *reinterpret_cast<const F *>(S);
         const float a = a_s[j][dl];
-        const float4 g = *reinterpret_cast<const float4 *>(&g_s[j][k0]);
-        S.x = a * g.x * S.x + l[j].x;
-        S.y = a * g.y * S.y + l[j].y;
-        S.z = a * g.z * S.z + l[j].z;
-        S.w = a * g.w * S.w + l[j].w;
+        const F g = *reinterpret_cast<const F *>(&g_s[j][k0]);
+#pragma unroll
+        for (int i = 0; i < kCols; ++i) S[i] = a * reinterpret_cast<const float *>(&g)[i] * S[i] + reinterpret_cast<const float *>(&l[j])[i];
         if (kFwd) {
-          Quad<T>::st(op, S);
+          store16<T, kCols>(op, S);
           op += whole;
         }
         mp += kNext;
       }
     }
   }
-  if (!kFwd) Quad<T>::st(op, S);
+  if (!kFwd) store16<T, kCols>(op, S);
   if (any) atomicExch(rowflag + item, 1);
+}
+
+// The carry of BH problem rows.  Two values per thread make twice as many blocks, so that one block's loads run under
+// another's chain; where one round of loads holds all chunks, or the rows alone fill the chip, their smaller accesses cost more
+// than that gives.  Two / four values: 64 rows x 256 chunks 141 / 164 us, 96 rows x 16 chunks 11.3 / 10.3.
+template <typename T, bool kFwd>
+cudaError_t launch_carry(const T *init, float *M, const float *Ac, const float *Gc, const int *flags, int *rowflag, T *out,
+                         const Grid2D &gr, int64_t BH, int64_t nc, cudaStream_t st) {
+  if (nc > 16 && BH <= 128)
+    return launch_dependent(lfw_c64_carry_kernel<T, kFwd, 2>, dim3((unsigned)(BH * 8)), dim3(kCarryThreads), 0, st, init, M, Ac,
+                            Gc, flags, rowflag, out, gr, nc);
+  return launch_dependent(lfw_c64_carry_kernel<T, kFwd, 4>, dim3((unsigned)(BH * 4)), dim3(kCarryThreads), 0, st, init, M, Ac, Gc,
+                          flags, rowflag, out, gr, nc);
 }
 
 // Checkpoint interval of m chunks: slot j of the caller's checkpoints = state after chunk
@@ -261,9 +273,7 @@ int chunk_states(const Call &c, const Scratch &s, const void *state, T *ck_all, 
   set_grid(mp, c.grid);
   rc = lfw_chunk_local_umma(false, mp, s.M, s.Ac, s.Gc, s.flags, s.rowflag, BH, c.T_, dtype, st);
   if (rc != T2FW_OK) return rc;
-  T2FW_CHECK_CUDA(launch_dependent(lfw_c64_carry_kernel<T, true>, dim3((unsigned)(BH * (kDim / kCarryRows))),
-                                   dim3(kCarryThreads), 0, st, (const T *)state, s.M, (const float *)s.Ac,
-                                   (const float *)s.Gc, (const int *)s.flags, s.rowflag, ck_all, c.grid, nc));
+  T2FW_CHECK_CUDA((launch_carry<T, true>((const T *)state, s.M, s.Ac, s.Gc, s.flags, s.rowflag, ck_all, c.grid, BH, nc, st)));
   T2FW_CHECK_LAUNCH(1);
   return T2FW_OK;
 }
@@ -314,10 +324,7 @@ int backward_typed(const Call &c, const void *gs, const void *state, const void 
   set_grid(mp, c.grid);
   rc = lfw_chunk_local_umma(true, mp, s.M, s.Ac, s.Gc, s.flags, m > 1 ? nullptr : s.rowflag, BH, c.T_, dtype, st);
   if (rc != T2FW_OK) return rc;
-  T2FW_CHECK_CUDA(launch_dependent(lfw_c64_carry_kernel<T, false>, dim3((unsigned)(BH * (kDim / kCarryRows))),
-                                   dim3(kCarryThreads), 0, st, (const T *)gs, s.M, (const float *)s.Ac,
-                                   (const float *)s.Gc, (const int *)s.flags, s.rowflag, (T *)ds, c.grid,
-                                   nc));
+  T2FW_CHECK_CUDA((launch_carry<T, false>((const T *)gs, s.M, s.Ac, s.Gc, s.flags, s.rowflag, (T *)ds, c.grid, BH, nc, st)));
   T2FW_CHECK_LAUNCH(1);
   const Tensor2D all[6] = {c.x, c.f, c.q, c.k, c.fk, c.go};
   rc = build_maps(mp, all, 6, rows, c.heads, c.flags, c.q_scale);
@@ -472,15 +479,10 @@ int summary_typed(bool backward, const void *val_d, const void *gate_d, const vo
   set_grid(mp, one);
   rc = lfw_chunk_local_umma(backward, mp, s.M, s.Ac, s.Gc, s.flags, s.rowflag, B, T_, dtype, st);
   if (rc != T2FW_OK) return rc;
-  const dim3 grid((unsigned)(B * (kDim / kCarryRows)));
   if (backward) {      // the state gradient at the segment start that the segment's own output gradients cause
-    T2FW_CHECK_CUDA(launch_dependent(lfw_c64_carry_kernel<T, false>, grid, dim3(kCarryThreads), 0, st, (const T *)nullptr,
-                                     s.M, (const float *)s.Ac, (const float *)s.Gc, (const int *)s.flags, s.rowflag,
-                                     (T *)end_state, one, nc));
+    T2FW_CHECK_CUDA((launch_carry<T, false>(nullptr, s.M, s.Ac, s.Gc, s.flags, s.rowflag, (T *)end_state, one, B, nc, st)));
   } else {             // the state at the segment end that the segment's own inputs cause
-    T2FW_CHECK_CUDA(launch_dependent(lfw_c64_carry_kernel<T, true>, grid, dim3(kCarryThreads), 0, st, (const T *)nullptr,
-                                     s.M, (const float *)s.Ac, (const float *)s.Gc, (const int *)s.flags, s.rowflag,
-                                     (T *)s.ck_all, one, nc));
+    T2FW_CHECK_CUDA((launch_carry<T, true>(nullptr, s.M, s.Ac, s.Gc, s.flags, s.rowflag, (T *)s.ck_all, one, B, nc, st)));
     lfw_c64_pick_ckpt_kernel<T><<<(unsigned)ceil_div64(B * (kDim * kDim / 8), 256), 256, 0, st>>>(
         (const T *)s.ck_all, (T *)end_state, B, nc, nc, 1, (int64_t)(kDim * kDim / 8));
   }
