@@ -17,7 +17,7 @@
 // (and the right-hand side) split in two, everything else is TF32 with fp32 accumulation.
 //
 // What bounds it is latency at few warps, no pipe.  B*H = 96, T = 1024, fp16, cold caches: prep 60 us, tensor pipe 50 %,
-// issue slots 35 %, 11 warps per SM; carry 28 us, 4 warps on each of 96 SMs, tensor 19 %; gradients 78 us, tensor 40 %,
+// issue slots 35 %, 11 warps per SM; carry 26 us, 4 warps on each of 96 SMs, tensor 19 %; gradients 78 us, tensor 40 %,
 // issue slots 30 %, 15 warps per SM that wait most for the other group at the five meetings, then for global memory
 // (252 bytes of spills per thread among it).  Whole backward 188 -> 165 us.
 #include "dfw_frag.cuh"
@@ -207,40 +207,44 @@ dfw_prep_bwd_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *
   mma_kt_b<T, true, false>(Gimg + img, aK, Ds, 1.f, w, lane);       // (Dl^T K)^T = K^T Dl
 }
 
-// ---- carry: one CTA per row, chunks in reverse; warp w = rows 16 w .. of R [d][m] and of S^T [m][d] -------------
-// Qb^T, Nb and (Dl^T K)^T of a chunk arrive together, two chunks ahead; R_end (row-major) replaces Nb and S0^T (an
-// image) replaces (Dl^T K)^T.
-constexpr int kStages = 3;
-constexpr int kSmemCarry = kStages * 3 * kImg * 4;
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
+// ---- carry, chunks in reverse: blocks of 16 rows of R [d][m] and of S^T [m][d], spread over CTAs and warps as in the forward ----
+// Qb^T and the CTA's parts of Nb and (Dl^T K)^T of a chunk arrive together by bulk copies; R_end (row-major) replaces Nb and
+// S0^T (an image) replaces (Dl^T K)^T.
+template <typename T, int kW, int kH, int kStages>
+__global__ void __launch_bounds__(32 * kH * kW)
 dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state, const float *__restrict__ Qimg,
-                     float *__restrict__ NR, float *__restrict__ GS, T *__restrict__ ds, int nc) {
+                     float *__restrict__ NR, float *__restrict__ GS, T *__restrict__ ds, int nc, int *__restrict__ status) {
   extern __shared__ __align__(128) unsigned char sm[];
+  __shared__ __align__(8) uint64_t full[kStages];
+  __shared__ uint4 xs[kH == 2 ? 2 : 1][kH == 2 ? kW : 1][8][32];      // operands of the block's rows, by step parity
+  constexpr int kN = 8 / kH;                                            // 8-column tiles of a warp
+  constexpr int kPart = kW * kImg / 4, kStage = kImg + 2 * kPart;      // floats
   float *ring = reinterpret_cast<float *>(sm);
-  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int64_t b = blockIdx.x;
+  const int tid = threadIdx.x, wl = tid / (32 * kH), ch = kH == 1 ? 0 : (tid >> 5) & 1, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int64_t b = blockIdx.x / (4 / kW);
+  const int w0 = (int)(blockIdx.x % (4 / kW)) * kW, w = w0 + wl;
   const size_t img0 = (size_t)b * nc * kImg;
+  init_ring<kStages>(full, tid);
   dependency_wait();
-  auto fetch = [&](int i) {      // i-th chunk from the end
-    if (i < nc) {
-      const size_t o = img0 + (size_t)(nc - 1 - i) * kImg;
-      float *dst = ring + (i % kStages) * 3 * kImg;
-      load_image(dst, Qimg + o, tid);
-      load_image(dst + kImg, NR + o, tid);
-      load_image(dst + 2 * kImg, GS + o, tid);
-    }
-    commit();
+  auto fetch = [&](int i) {      // i-th chunk from the end; one thread
+    if (i >= nc) return;
+    const size_t o = img0 + (size_t)(nc - 1 - i) * kImg;
+    uint64_t *bar = &full[i % kStages];
+    float *dst = ring + (i % kStages) * kStage;
+    acp::mbar_expect_tx(bar, (uint32_t)(kStage * sizeof(float)));
+    acp::bulk_g2s(dst, Qimg + o, kImg * (uint32_t)sizeof(float), bar);
+    acp::bulk_g2s(dst + kImg, NR + o + w0 * (kImg / 4), kPart * (uint32_t)sizeof(float), bar);
+    acp::bulk_g2s(dst + kImg + kPart, GS + o + w0 * (kImg / 4), kPart * (uint32_t)sizeof(float), bar);
   };
-#pragma unroll
-  for (int i = 0; i < kStages - 1; ++i) fetch(i);
-  float R[8][4], S[8][4];
+  if (tid == 0) {
+    for (int i = 0; i < kStages - 1; ++i) fetch(i);
+  }
+  float R[kN][4], S[kN][4];
   {
-    const T *rp = gs + ((size_t)b * kDim + 16 * w + g) * kDim + 2 * t;
-    const T *sp = final_state + (size_t)b * kDim * kDim + (2 * t) * kDim + 16 * w + g;      // S^T[m = 16 w + g][d]
+    const T *rp = gs + ((size_t)b * kDim + 16 * w + g) * kDim + 32 * ch + 2 * t;
+    const T *sp = final_state + (size_t)b * kDim * kDim + (32 * ch + 2 * t) * kDim + 16 * w + g;      // S^T[m = 16 w + g][d]
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
+    for (int n = 0; n < kN; ++n) {
       const uint32_t u = *reinterpret_cast<const uint32_t *>(rp + 8 * n), x = *reinterpret_cast<const uint32_t *>(rp + 8 * kDim + 8 * n);
       R[n][0] = __uint_as_float(lo16<T>(u)); R[n][1] = __uint_as_float(hi16<T>(u));
       R[n][2] = __uint_as_float(lo16<T>(x)); R[n][3] = __uint_as_float(hi16<T>(x));
@@ -248,34 +252,58 @@ dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state
       S[n][2] = Elem<T>::ld(sp + 8 * n * kDim + 8); S[n][3] = Elem<T>::ld(sp + (8 * n + 1) * kDim + 8);
     }
   }
+  int fail = acp::mbar_wait(&full[0], 0) ? 0 : 1;
+  float4 bq[8][4 / kH];
+  carry_load_b<kH>(bq, ring, ch, lane);
   for (int i = 0; i < nc; ++i) {
-    wait<kStages - 2>();
-    __syncthreads();             // chunk i has landed for all; the buffer refilled next is no longer read
-    fetch(i + kStages - 1);
-    const float *buf = ring + (i % kStages) * 3 * kImg;
+    uint32_t own[kN][4], oth[4][4];
+#pragma unroll
+    for (int n = 0; n < kN; ++n) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) own[n][e] = op(R[n][e]);
+      if (kH == 2) xs[i & 1][wl][4 * ch + n][lane] = make_uint4(own[n][0], own[n][1], own[n][2], own[n][3]);
+    }
+    const int in = i + 1 < nc ? i + 1 : i;      // (the last chunk's matrix once more: nobody uses it)
+    if (!acp::mbar_wait(&full[in % kStages], (uint32_t)(in / kStages) & 1u)) fail = 1;
+    if (__syncthreads_or(fail)) break;      // the halves are exchanged; the buffer refilled next is no longer read
+    if (tid == 0) fetch(i + kStages - 1);
+    const float *buf = ring + (i % kStages) * kStage;
     const size_t o = img0 + (size_t)(nc - 1 - i) * kImg;
-    uint32_t a[8][4];
-    float *rp = NR + o + (16 * w + g) * kDim + 2 * t;
+    float *rp = NR + o + (16 * w + g) * kDim + 32 * ch + 2 * t;
+    float4 *const img = reinterpret_cast<float4 *>(GS + o) + (w * 8 + 4 * ch) * 32 + lane;
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      const float4 gx = image_at(buf + 2 * kImg, w, n, lane), nx = image_at(buf + kImg, w, n, lane);
+    for (int n = 0; n < kN; ++n) {
+      if (kH == 2) {
+        const uint4 u = xs[i & 1][wl][4 * (ch ^ 1) + (n & 3)][lane];
+        oth[n & 3][0] = u.x; oth[n & 3][1] = u.y; oth[n & 3][2] = u.z; oth[n & 3][3] = u.w;
+      }
+      const float4 gx = image_at(buf + kImg + kPart, wl, 4 * ch + n, lane), nx = image_at(buf + kImg, wl, 4 * ch + n, lane);
       S[n][0] -= gx.x; S[n][1] -= gx.y; S[n][2] -= gx.z; S[n][3] -= gx.w;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) a[n][e] = op(R[n][e]);
+      img[n * 32] = make_float4(rnd(S[n][0]), rnd(S[n][1]), rnd(S[n][2]), rnd(S[n][3]));
       *reinterpret_cast<float2 *>(rp + 8 * n) = make_float2(rnd(R[n][0]), rnd(R[n][1]));
       *reinterpret_cast<float2 *>(rp + 8 * kDim + 8 * n) = make_float2(rnd(R[n][2]), rnd(R[n][3]));
       R[n][0] += nx.x; R[n][1] += nx.y; R[n][2] += nx.z; R[n][3] += nx.w;
     }
-    store_rows<true>(GS + o, S, w, lane);
-    mma_image(R, a, buf, lane);
+    carry_product<kH>(R, own, oth, bq, ring + (in % kStages) * kStage, ch, lane);
   }
-  T *dp = ds + ((size_t)b * kDim + 16 * w + g) * kDim + 2 * t;
+  if (fail) atomicExch(status, 1);
+  T *dp = ds + ((size_t)b * kDim + 16 * w + g) * kDim + 32 * ch + 2 * t;
 #pragma unroll
-  for (int n = 0; n < 8; ++n) {
+  for (int n = 0; n < kN; ++n) {
     *reinterpret_cast<uint32_t *>(dp + 8 * n) = pack16<T>(R[n][0], R[n][1]);
     *reinterpret_cast<uint32_t *>(dp + 8 * kDim + 8 * n) = pack16<T>(R[n][2], R[n][3]);
   }
-  wait<0>();
+}
+
+template <typename T, int kW, int kH, int kStages>
+int launch_carry_bwd(const void *gs, const void *final_state, const float *Qb, float *NR, float *GS, void *ds, int64_t B, int nc,
+                     int *status, cudaStream_t st) {
+  constexpr int kSmem = kStages * (kImg + 2 * kW * kImg / 4) * 4;
+  auto *const carry = &dfw_carry_bwd_kernel<T, kW, kH, kStages>;
+  T2FW_ALLOW_SMEM(carry, kSmem);
+  T2FW_CHECK_CUDA(launch_dependent(carry, dim3((unsigned)(B * (4 / kW))), dim3(32 * kH * kW), kSmem, st, (const T *)gs,
+                                   (const T *)final_state, Qb, NR, GS, (T *)ds, nc, status));
+  return T2FW_OK;
 }
 
 // ---- gradients: grid = B * nc, eight warps ---------------------------------------------------------------------
@@ -305,9 +333,10 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
   float *Ds = reinterpret_cast<float *>(sm + oDg), *Rs = reinterpret_cast<float *>(sm + oRg), *Es = Rs;
   float *Ss = reinterpret_cast<float *>(sm + oSg);
   const uint32_t aK = smem_u32(sm + oKg), aQ = smem_u32(sm + oQg), aG = smem_u32(sm + oGg);
-  const int64_t b = blockIdx.x / (uint32_t)nc, t0 = (int64_t)(blockIdx.x - (uint32_t)b * nc) * kC;
+  const uint32_t blk = gridDim.x - 1 - blockIdx.x;      // last first: what prep wrote last is still in L2
+  const int64_t b = blk / (uint32_t)nc, t0 = (int64_t)(blk - (uint32_t)b * nc) * kC;
   const int nvalid = (int)(T_ - t0 < kC ? T_ - t0 : kC);
-  const size_t base = ((size_t)b * T_ + t0) * kDim, img = (size_t)blockIdx.x * kImg;
+  const size_t base = ((size_t)b * T_ + t0) * kDim, img = (size_t)blk * kImg;
   dependency_wait();
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -520,10 +549,15 @@ int backward_typed(const void *go, const void *gs, const void *q, const void *k,
   T2FW_ALLOW_SMEM(prep, kSmemPrep);
   T2FW_CHECK_CUDA(launch_dependent(prep, dim3((unsigned)n), dim3(kThreads), kSmemPrep, st, (const T *)go, (const T *)q, (const T *)k,
                                    (const float *)delta, W, U, Qb, NR, GS, T_, (int)nc));
-  auto *const carry = &dfw_carry_bwd_kernel<T>;
-  T2FW_ALLOW_SMEM(carry, kSmemCarry);
-  T2FW_CHECK_CUDA(launch_dependent(carry, dim3((unsigned)B), dim3(kThreads), kSmemCarry, st, (const T *)gs, (const T *)final_state,
-                                   (const float *)Qb, NR, GS, (T *)ds, (int)nc));
+  int *status = nullptr;
+  int rc = lfw_chunk_status_ptr(&status);
+  if (rc != T2FW_OK) return rc;
+  const CarryPlan plan = carry_plan(B);
+  rc = plan == kSpread1   ? launch_carry_bwd<T, 1, 2, 9>(gs, final_state, Qb, NR, GS, ds, B, (int)nc, status, st)
+       : plan == kSpread2 ? launch_carry_bwd<T, 2, 2, 6>(gs, final_state, Qb, NR, GS, ds, B, (int)nc, status, st)
+       : plan == kDeep    ? launch_carry_bwd<T, 4, 1, 4>(gs, final_state, Qb, NR, GS, ds, B, (int)nc, status, st)
+                          : launch_carry_bwd<T, 4, 1, 4>(gs, final_state, Qb, NR, GS, ds, B, (int)nc, status, st);
+  if (rc != T2FW_OK) return rc;
   auto *const grad = &dfw_grad_kernel<T>;
   T2FW_ALLOW_SMEM(grad, kSmemGrad);
   T2FW_CHECK_CUDA(launch_dependent(grad, dim3((unsigned)n), dim3(kThreadsG), kSmemGrad, st, (const T *)go, (const T *)q, (const T *)k,

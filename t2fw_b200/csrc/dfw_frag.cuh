@@ -17,6 +17,7 @@
 // value is exact in TF32), those of a TF32 product in the order above.
 #pragma once
 
+#include "async_copy.cuh"
 #include "common.cuh"
 
 namespace t2fw {
@@ -337,5 +338,50 @@ __device__ __forceinline__ void gram_lower(float *Ls, uint32_t x, uint32_t y, in
   }
 }
 
+// ---- the carries: 16 rows of a state per warp or pair of warps, a ring of stages filled by bulk copies ------------------------------------------------
+constexpr int kMaxStages = 11;
+template <int kStages>
+__device__ __forceinline__ void init_ring(uint64_t *full, int tid) {
+  if (tid == 0) {
+    for (int i = 0; i < kStages; ++i) acp::mbar_init(&full[i], 1);
+    acp::mbar_fence_init();
+  }
+  __syncthreads();
+}
+// One step's product for a warp of 16 rows and 1 / kH of the columns (part ch) of X += A B^T: A = all 64 columns of X as
+// operands, the own ones first (own), then the partner's (oth, kH = 2); B in registers, which take the next step's B as they
+// are used: its loads run under this product.
+template <int kH>
+__device__ __forceinline__ int carry_col(int jj, int ch) { return kH == 1 ? jj : (jj & 3) + 4 * (jj < 4 ? ch : ch ^ 1); }
+template <int kH>
+__device__ __forceinline__ void carry_load_b(float4 (&bq)[8][4 / kH], const float *img, int ch, int lane) {
+#pragma unroll
+  for (int jj = 0; jj < 8; ++jj)
+#pragma unroll
+    for (int np = 0; np < 4 / kH; ++np) bq[jj][np] = image_at(img, 4 / kH * ch + np, carry_col<kH>(jj, ch), lane);
+}
+template <int kH>
+__device__ __forceinline__ void carry_product(float (&c)[8 / kH][4], const uint32_t (&own)[8 / kH][4], const uint32_t (&oth)[4][4],
+                                              float4 (&bq)[8][4 / kH], const float *next, int ch, int lane) {
+#pragma unroll
+  for (int jj = 0; jj < 8; ++jj)
+#pragma unroll
+    for (int np = 0; np < 4 / kH; ++np) {
+      const float4 b = bq[jj][np];
+      mma_acc_a(c[2 * np], jj < 8 / kH ? own[jj % (8 / kH)] : oth[jj & 3], bits(b.x), bits(b.y));
+      mma_acc_a(c[2 * np + 1], jj < 8 / kH ? own[jj % (8 / kH)] : oth[jj & 3], bits(b.z), bits(b.w));
+      bq[jj][np] = image_at(next, 4 / kH * ch + np, carry_col<kH>(jj, ch), lane);
+    }
+}
+// How B rows are spread: one or two of a row's four blocks per CTA with a pair of warps each, while that leaves a CTA an SM of
+// its own (every CTA fetches the whole transition matrix of a chunk); else a row per CTA with a warp per block, the ring as deep as
+// shared memory allows as long as an SM holds one CTA.  Training calls, fp16, a warp per block in one CTA with three stages that
+// all threads copy -> now: 1 row x 4096 steps 161 -> 117 us, 8 x 4096 212 -> 162, 32 x 4096 418 -> 346, 48 x 1333 186 -> 167,
+// 74 x 1333 257 -> 244, 96 x 1024 242 -> 236, 200 x 512 253 -> 244, 384 x 341 347 -> 342; pairs of warps instead at 96 and 200
+// rows: 240, 250.
+enum CarryPlan { kSpread1, kSpread2, kDeep, kDense };
+inline CarryPlan carry_plan(int64_t B) { return B <= 37 ? kSpread1 : B <= 74 ? kSpread2 : B <= 148 ? kDeep : kDense; }
+
 }  // namespace frag
+int lfw_chunk_status_ptr(int **out);      // lfw_c64_local.cu
 }  // namespace t2fw

@@ -139,63 +139,91 @@ dfw_prep_fwd_kernel(const T *__restrict__ k, const T *__restrict__ v, float *__r
   mma_kt_b<T, false, true>(Qimg + img, aK, Ls, -1.f, w, lane);      // Qc^T = -K^T W
 }
 
-// ---- carry: one CTA per row, warp w = state rows 16 w .. ------------------------------------------------
-// Qc^T and N of a chunk arrive together, two chunks ahead.  Start states replace N: a chunk's N is in shared memory
-// before its start state is written.
-constexpr int kStages = 3;
-constexpr int kSmemCarry = kStages * 2 * kImg * 4;
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
+// ---- carry: the 16-row blocks of a state never meet, so a row's four may be spread over 4 / kW CTAs; kH warps per block, each
+// 1 / kH of the columns ----
+// Qc^T and the CTA's part of N of a chunk arrive together by bulk copies.  Start states replace N: a chunk's N is in shared
+// memory before its start state is written.  A step is a chain: operands, exchange of the halves (kH = 2), products (a warp's 64 take
+// about 1 k cycles, hence the halves where SMs are free), next operands.
+template <typename T, int kW, int kH, int kStages>
+__global__ void __launch_bounds__(32 * kH * kW)
 dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg, float *__restrict__ NSimg,
-                     T *__restrict__ final_state, int nc) {
+                     T *__restrict__ final_state, int nc, int *__restrict__ status) {
   extern __shared__ __align__(128) unsigned char sm[];
+  __shared__ __align__(8) uint64_t full[kStages];
+  __shared__ uint4 xs[kH == 2 ? 2 : 1][kH == 2 ? kW : 1][8][32];      // operands of the block's rows, by step parity
+  constexpr int kN = 8 / kH;                                            // 8-column tiles of a warp
+  constexpr int kPart = kW * kImg / 4, kStage = kImg + kPart;      // floats
   float *ring = reinterpret_cast<float *>(sm);
-  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int64_t b = blockIdx.x;
+  const int tid = threadIdx.x, wl = tid / (32 * kH), ch = kH == 1 ? 0 : (tid >> 5) & 1, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int64_t b = blockIdx.x / (4 / kW);
+  const int w0 = (int)(blockIdx.x % (4 / kW)) * kW, w = w0 + wl;
   const size_t img0 = (size_t)b * nc * kImg;
+  init_ring<kStages>(full, tid);
   dependency_wait();
-  auto fetch = [&](int c) {
-    if (c < nc) {
-      float *dst = ring + (c % kStages) * 2 * kImg;
-      load_image(dst, Qimg + img0 + (size_t)c * kImg, tid);
-      load_image(dst + kImg, NSimg + img0 + (size_t)c * kImg, tid);
-    }
-    commit();
+  auto fetch = [&](int c) {      // one thread
+    if (c >= nc) return;
+    float *dst = ring + (c % kStages) * kStage;
+    acp::mbar_expect_tx(&full[c % kStages], (uint32_t)(kStage * sizeof(float)));
+    acp::bulk_g2s(dst, Qimg + img0 + (size_t)c * kImg, kImg * (uint32_t)sizeof(float), &full[c % kStages]);
+    acp::bulk_g2s(dst + kImg, NSimg + img0 + (size_t)c * kImg + w0 * (kImg / 4), kPart * (uint32_t)sizeof(float), &full[c % kStages]);
   };
+  if (tid == 0) {
+    for (int c = 0; c < kStages - 1; ++c) fetch(c);
+  }
+  float S[kN][4];
+  const T *sp = state + ((size_t)b * kDim + 16 * w + g) * kDim + 32 * ch + 2 * t;
 #pragma unroll
-  for (int c = 0; c < kStages - 1; ++c) fetch(c);
-  float S[8][4];
-  const T *sp = state + ((size_t)b * kDim + 16 * w + g) * kDim + 2 * t;
-#pragma unroll
-  for (int n = 0; n < 8; ++n) {
+  for (int n = 0; n < kN; ++n) {
     const uint32_t u = *reinterpret_cast<const uint32_t *>(sp + 8 * n), x = *reinterpret_cast<const uint32_t *>(sp + 8 * kDim + 8 * n);
     S[n][0] = __uint_as_float(lo16<T>(u)); S[n][1] = __uint_as_float(hi16<T>(u));
     S[n][2] = __uint_as_float(lo16<T>(x)); S[n][3] = __uint_as_float(hi16<T>(x));
   }
+  int fail = acp::mbar_wait(&full[0], 0) ? 0 : 1;
+  float4 bq[8][4 / kH];
+  carry_load_b<kH>(bq, ring, ch, lane);
   for (int c = 0; c < nc; ++c) {
-    wait<kStages - 2>();
-    __syncthreads();             // chunk c has landed for all; the buffer refilled next is no longer read
-    fetch(c + kStages - 1);
-    const float *buf = ring + (c % kStages) * 2 * kImg;
-    store_rows<true>(NSimg + img0 + (size_t)c * kImg, S, w, lane);
-    uint32_t a[8][4];
+    uint32_t own[kN][4], oth[4][4];
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      const float4 nx = image_at(buf + kImg, w, n, lane);
+    for (int n = 0; n < kN; ++n) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) a[n][e] = op(S[n][e]);
+      for (int e = 0; e < 4; ++e) own[n][e] = op(S[n][e]);
+      if (kH == 2) xs[c & 1][wl][4 * ch + n][lane] = make_uint4(own[n][0], own[n][1], own[n][2], own[n][3]);
+    }
+    const int cn = c + 1 < nc ? c + 1 : c;      // (the last chunk's matrix once more: nobody uses it)
+    if (!acp::mbar_wait(&full[cn % kStages], (uint32_t)(cn / kStages) & 1u)) fail = 1;
+    if (__syncthreads_or(fail)) break;      // the halves are exchanged; the buffer refilled next is no longer read
+    if (tid == 0) fetch(c + kStages - 1);
+    const float *buf = ring + (c % kStages) * kStage;
+    float4 *const img = reinterpret_cast<float4 *>(NSimg + img0 + (size_t)c * kImg) + (w * 8 + 4 * ch) * 32 + lane;
+#pragma unroll
+    for (int n = 0; n < kN; ++n) {
+      if (kH == 2) {
+        const uint4 u = xs[c & 1][wl][4 * (ch ^ 1) + (n & 3)][lane];
+        oth[n & 3][0] = u.x; oth[n & 3][1] = u.y; oth[n & 3][2] = u.z; oth[n & 3][3] = u.w;
+      }
+      img[n * 32] = make_float4(rnd(S[n][0]), rnd(S[n][1]), rnd(S[n][2]), rnd(S[n][3]));
+      const float4 nx = image_at(buf + kImg, wl, 4 * ch + n, lane);
       S[n][0] += nx.x; S[n][1] += nx.y; S[n][2] += nx.z; S[n][3] += nx.w;
     }
-    mma_image(S, a, buf, lane);
+    carry_product<kH>(S, own, oth, bq, ring + (cn % kStages) * kStage, ch, lane);
   }
-  T *fp = final_state + ((size_t)b * kDim + 16 * w + g) * kDim + 2 * t;
+  if (fail) atomicExch(status, 1);
+  T *fp = final_state + ((size_t)b * kDim + 16 * w + g) * kDim + 32 * ch + 2 * t;
 #pragma unroll
-  for (int n = 0; n < 8; ++n) {
+  for (int n = 0; n < kN; ++n) {
     *reinterpret_cast<uint32_t *>(fp + 8 * n) = pack16<T>(S[n][0], S[n][1]);
     *reinterpret_cast<uint32_t *>(fp + 8 * kDim + 8 * n) = pack16<T>(S[n][2], S[n][3]);
   }
-  wait<0>();
+}
+
+template <typename T, int kW, int kH, int kStages>
+int launch_carry_fwd(const void *state, const float *Qc, float *NS, void *final_state, int64_t B, int nc, int *status, cudaStream_t st) {
+  constexpr int kSmem = kStages * (kImg + kW * kImg / 4) * 4;
+  auto *const carry = &dfw_carry_fwd_kernel<T, kW, kH, kStages>;
+  T2FW_ALLOW_SMEM(carry, kSmem);
+  T2FW_CHECK_CUDA(launch_dependent(carry, dim3((unsigned)(B * (4 / kW))), dim3(32 * kH * kW), kSmem, st, (const T *)state, Qc, NS,
+                                   (T *)final_state, nc, status));
+  return T2FW_OK;
 }
 
 // ---- outputs: grid = B * nc, four warps ------------------------------------------------------------------
@@ -322,10 +350,15 @@ int forward_typed(const void *q, const void *k, const void *v, const void *state
   auto *const prep = &dfw_prep_fwd_kernel<T>;
   T2FW_ALLOW_SMEM(prep, kSmemPrep);
   T2FW_CHECK_CUDA(launch_dependent(prep, dim3((unsigned)n), dim3(kThreads), kSmemPrep, st, (const T *)k, (const T *)v, W, U, Qc, NS, T_, (int)nc));
-  auto *const carry = &dfw_carry_fwd_kernel<T>;
-  T2FW_ALLOW_SMEM(carry, kSmemCarry);
-  T2FW_CHECK_CUDA(launch_dependent(carry, dim3((unsigned)B), dim3(kThreads), kSmemCarry, st, (const T *)state, (const float *)Qc, NS,
-                                   (T *)final_state, (int)nc));
+  int *status = nullptr;
+  int rc = lfw_chunk_status_ptr(&status);
+  if (rc != T2FW_OK) return rc;
+  const CarryPlan plan = carry_plan(B);
+  rc = plan == kSpread1   ? launch_carry_fwd<T, 1, 2, 10>(state, Qc, NS, final_state, B, (int)nc, status, st)
+       : plan == kSpread2 ? launch_carry_fwd<T, 2, 2, 8>(state, Qc, NS, final_state, B, (int)nc, status, st)
+       : plan == kDeep    ? launch_carry_fwd<T, 4, 1, 7>(state, Qc, NS, final_state, B, (int)nc, status, st)
+                          : launch_carry_fwd<T, 4, 1, 3>(state, Qc, NS, final_state, B, (int)nc, status, st);
+  if (rc != T2FW_OK) return rc;
   auto *const outk = &dfw_out_fwd_kernel<T>;
   T2FW_ALLOW_SMEM(outk, kSmemOut);
   T2FW_CHECK_CUDA(launch_dependent(outk, dim3((unsigned)n), dim3(kThreads), kSmemOut, st, (const T *)q, (const T *)k, (const float *)W,
