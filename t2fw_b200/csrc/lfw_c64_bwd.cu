@@ -362,6 +362,12 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       for (int j = 2; j < 16; j += 2) { p0 *= g[j]; p1 *= g[j + 1]; }
       qtot[(h * 4 + tq) * kDim + feat] = p0 * p1;
     }
+    float mw[16], vw[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      mw[j] = Elem<T>::ld(mcol + j * kDim);
+      vw[j] = Elem<T>::ld(vcol + j * kDim);
+    }
     if (umma::named_barrier_or(5, kThreadsB, fail)) break;      // (the whole group leaves together)
     unsigned tiny = 0;                     // steps of the quarter with tiny gates
     float pm[16], up, after, pm_prev;      // ratios to the anchor; products up to and after it; ratio of the step before
@@ -372,12 +378,6 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       after = q2 * q3;
       pm_prev = tq == 0 ? rcp_fast(up) : tq == 1 ? rcp_fast(q1) : tq == 2 ? 1.f : q2;
       const float carry = tq == 0 ? q1 : tq == 3 ? q2 : 1.f;
-      float mw[16], vw[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        mw[j] = Elem<T>::ld(mcol + j * kDim);
-        vw[j] = Elem<T>::ld(vcol + j * kDim);
-      }
       if (kFused) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) mw[j] = h ? mw[j] : seq::round_to<T>(mw[j] * q_scale);
