@@ -38,6 +38,8 @@ int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ck
                           int64_t BH, int64_t T_, int dtype, cudaStream_t st);
 int lfw_wide_forward_out(const seq::Maps &mp, const void *state, const void *ckpt, void *out, int *rowflag, int64_t items,
                          int64_t T_, int64_t D, int64_t K, int dtype, cudaStream_t st);      // lfw_wide_fwd.cu
+int lfw_wide_local(bool backward, const seq::Maps &mp, float *M, float *Ac, float *Gc, int *flags, int *rowflag, int64_t items,
+                   int64_t T_, int64_t D, int64_t K, int dtype, cudaStream_t st);
 int lfw_wide_backward_main(const seq::Maps &mp, const void *state, const void *ckpt, const float *Rend, void *const outs[5],
                            int *rowflag, int64_t items, int64_t T_, int64_t D, int64_t K, int dtype, cudaStream_t st);
 
@@ -256,7 +258,8 @@ struct Call {
   Grid2D grid{1, 1, kDim * kDim, kDim};
 };
 // States of up to 128 x 128 have kernels of their own that take a chunk of all blocks as one problem (lfw_wide_*.cu).
-// 16 x 16384, 128 x 128: outputs 180 us against 433 as a grid of blocks, gradients 557 against 1052.
+// 16 x 16384, 128 x 128: chunk-local 136 us against 162 as a grid of blocks, outputs 180 against 433,
+// gradients 557 against 1052.
 bool wide(const Grid2D &g) { return g.nsub > 1 && g.nk <= 2 && g.nsub / g.nk <= 2; }
 void set_grid(seq::Maps &mp, const Grid2D &g) {
   mp.nsub = g.nsub; mp.nk = g.nk; mp.state_item = g.item; mp.state_ld = (int)g.ld;
@@ -271,7 +274,8 @@ int chunk_states(const Call &c, const Scratch &s, const void *state, T *ck_all, 
   int rc = build_maps(mp, loc, 4, rows, c.heads, c.flags, 1.f);
   if (rc != T2FW_OK) return rc;
   set_grid(mp, c.grid);
-  rc = lfw_chunk_local_umma(false, mp, s.M, s.Ac, s.Gc, s.flags, s.rowflag, BH, c.T_, dtype, st);
+  rc = wide(c.grid) ? lfw_wide_local(false, mp, s.M, s.Ac, s.Gc, s.flags, s.rowflag, c.B, c.T_, c.x.width, c.k.width, dtype, st)
+                    : lfw_chunk_local_umma(false, mp, s.M, s.Ac, s.Gc, s.flags, s.rowflag, BH, c.T_, dtype, st);
   if (rc != T2FW_OK) return rc;
   T2FW_CHECK_CUDA((launch_carry<T, true>((const T *)state, s.M, s.Ac, s.Gc, s.flags, s.rowflag, ck_all, c.grid, BH, nc, st)));
   T2FW_CHECK_LAUNCH(1);
@@ -322,7 +326,9 @@ int backward_typed(const Call &c, const void *gs, const void *state, const void 
   int rc = build_maps(mp, loc, 4, rows, c.heads, c.flags, c.q_scale);
   if (rc != T2FW_OK) return rc;
   set_grid(mp, c.grid);
-  rc = lfw_chunk_local_umma(true, mp, s.M, s.Ac, s.Gc, s.flags, m > 1 ? nullptr : s.rowflag, BH, c.T_, dtype, st);
+  int *const flag0 = m > 1 ? nullptr : s.rowflag;
+  rc = wide(c.grid) ? lfw_wide_local(true, mp, s.M, s.Ac, s.Gc, s.flags, flag0, c.B, c.T_, c.x.width, c.k.width, dtype, st)
+                    : lfw_chunk_local_umma(true, mp, s.M, s.Ac, s.Gc, s.flags, flag0, BH, c.T_, dtype, st);
   if (rc != T2FW_OK) return rc;
   T2FW_CHECK_CUDA((launch_carry<T, false>((const T *)gs, s.M, s.Ac, s.Gc, s.flags, s.rowflag, (T *)ds, c.grid, BH, nc, st)));
   T2FW_CHECK_LAUNCH(1);
