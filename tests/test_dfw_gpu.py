@@ -115,6 +115,17 @@ def test_chunked_path_lengths(cuda, dtype, B, T, keys, state_std):
     check_against_oracle(dev, got, dtype)
 
 
+@pytest.mark.parametrize("B", [1, 37, 38, 74, 75, 148, 149])
+@pytest.mark.parametrize("T", [65, 839])
+def test_carry_plans(cuda, B, T):
+    """The chain over the chunks spreads its rows by how many there are: either side of every line, fewer and more chunks
+    than any ring has stages."""
+    dev = to_dev(dfw_inputs(B, T, 64, 64, "scaled", 0.3, B + T), torch.float16, cuda)
+    got = run_cabi(*dev)
+    assert all(torch.isfinite(t).all() for t in (got[0], got[1], *got[2]))
+    check_against_oracle(dev, got, torch.float16, rows=[0, B - 1])
+
+
 def test_scan_forward_pairs_with_chunked_backward(cuda):
     """The scratch-free forward (scan kernels) and the forward with scratch (chunked kernels) save
     the same delta, so either can feed the backward."""

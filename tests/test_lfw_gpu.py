@@ -239,6 +239,37 @@ def test_blocked_state_shapes(cuda, D, K):
     check_against_oracle(dev, run_cabi(*dev), torch.float16)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,K,T", [(128, 128, 64), (128, 64, 65), (64, 128, 127), (128, 128, 191), (128, 64, 128), (64, 128, 193)])
+def test_wide_state_lengths(cuda, dtype, D, K, T):
+    """States of up to 128 x 128 take a chunk of all blocks as one problem: whole and ragged chunks, either side with one or
+    two windows of features."""
+    dev = to_dev(lfw_inputs(3, T, D, K, "sigmoid", 0.5, D + K + T), dtype, cuda)
+    check_against_oracle(dev, run_cabi(*dev), dtype)
+
+
+@pytest.mark.parametrize("B,T,D,K", [(2, 1093, 64, 64), (128, 1088, 64, 64), (129, 1093, 64, 64), (3, 2113, 128, 64)])
+def test_carry_over_more_chunks_than_one_round(cuda, B, T, D, K):
+    """More than 16 chunks: with few rows the carry takes two values per thread, with more four; whole and partial rounds."""
+    dev = to_dev(lfw_inputs(B, T, D, K, "sigmoid", 0.5, B + T), torch.float16, cuda)
+    got = run_cabi(*dev)
+    assert all(torch.isfinite(t).all() for t in (got[0], got[1], *got[2]))
+    check_against_oracle(dev, got, torch.float16, rows=[0, B - 1])
+
+
+@pytest.mark.parametrize("D,K", [(64, 64), (128, 128), (64, 128)])
+@pytest.mark.parametrize("n", [1, 32, 33, 64, 65, 128, 129])
+def test_tiny_gate_list_lengths(cuda, n, D, K):
+    """n gates below 2^-13 in one chunk: their sums are split into 16, 8 or 4 parts by how many there are, and beyond 128 the
+    row is left to the scan kernels."""
+    x, f, q, k, fk, s, go, gs = lfw_inputs(2, 130, D, K, "sigmoid", 0.5, 500 + n)
+    for i in range(n):
+        gate, feat = (fk, (i // 2) % K) if i % 2 else (f, (i // 2) % D)
+        gate[1, 66 + 5 * (i % 11) + i // 128, feat] = 5e-5 if i % 3 else -6e-5
+    dev = to_dev((x, f, q, k, fk, s, go, gs), torch.float16, cuda)
+    check_against_oracle(dev, run_cabi(*dev), torch.float16)
+
+
 def test_blocked_extreme_gates(cuda):
     """Flagged blocks of a D=K=128 problem fall back to the scan kernels block by block."""
     x, f, q, k, fk, s, go, gs = lfw_inputs(2, 100, 128, 128, "sigmoid", 0.5, 71)
