@@ -17,7 +17,7 @@
 // (and the right-hand side) split in two, everything else is TF32 with fp32 accumulation.
 //
 // What bounds it is latency at few warps, no pipe.  B*H = 96, T = 1024, fp16, cold caches: prep 60 us, tensor pipe 50 %,
-// issue slots 35 %, 11 warps per SM; carry 26 us, 4 warps on each of 96 SMs, tensor 19 %; gradients 78 us, tensor 40 %,
+// issue slots 35 %, 11 warps per SM; carry 28 us, 4 warps on each of 96 SMs, tensor 18 %; gradients 78 us, tensor 40 %,
 // issue slots 30 %, 15 warps per SM that wait most for the other group at the five meetings, then for global memory
 // (252 bytes of spills per thread among it).  Whole backward 188 -> 165 us.
 #include "dfw_frag.cuh"

@@ -20,8 +20,8 @@
 // path converted every operand to tiles and walked the whole chunk sequentially per row, 7.2 k cycles each on at
 // most one SM per row.  What bounds it now is latency at few warps, no pipe: with
 // cold caches (B*H = 96, T = 1024, fp16) prep 39 us, tensor pipe 52 %, issue slots 39 %, 14 warps per SM that wait for
-// fixed latencies, the tensor pipe and barriers; carry 19 us, 4 warps on each of 96 SMs, tensor 29 %, waiting for the
-// images and for its own chain; out 33 us, tensor 32 %, DRAM 42 %, waiting for the images.  Whole forward 108 -> 91 us;
+// fixed latencies, the tensor pipe and barriers; carry 20 us, 4 warps on each of 96 SMs, tensor 29 %, waiting for its own
+// chain; out 33 us, tensor 32 %, DRAM 42 %, waiting for the images.  Whole forward 108 -> 91 us;
 // 48 rows of 1333 steps, bf16, the whole call 110 -> 61 us.
 #include "dfw_frag.cuh"
 

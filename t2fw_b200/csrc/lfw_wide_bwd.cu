@@ -16,6 +16,7 @@
 // d side's ratios wait there for its turn.  Shared memory: raw values land where tiles will be (a thread takes its values into
 // registers before the barrier that precedes the tiles' first write), Z tiles and staged results share one area.
 //
+// Issue slots 45 % busy (68 k warp instructions per chunk of four blocks), tensor pipe 11 %, DRAM 16 %.
 // 16 rows x 16384 steps, 128 x 128 (4096 chunks): 1052 us as a grid of blocks -> 557 us.  Bound by the latency of its phases, as
 // the 64 x 64 kernel was before its issuing warps: block barriers, and state blocks that are loaded when they are needed.
 #include "lfw_c64.cuh"
