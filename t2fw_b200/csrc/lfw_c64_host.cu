@@ -259,7 +259,7 @@ struct Call {
 };
 // States of up to 128 x 128 have kernels of their own that take a chunk of all blocks as one problem (lfw_wide_*.cu).
 // 16 x 16384, 128 x 128: chunk-local 136 us against 162 as a grid of blocks, outputs 180 against 433,
-// gradients 557 against 1052.
+// gradients 515 against 1052.
 bool wide(const Grid2D &g) { return g.nsub > 1 && g.nk <= 2 && g.nsub / g.nk <= 2; }
 void set_grid(seq::Maps &mp, const Grid2D &g) {
   mp.nsub = g.nsub; mp.nk = g.nk; mp.state_item = g.item; mp.state_ld = (int)g.ld;

@@ -17,8 +17,9 @@
 // registers before the barrier that precedes the tiles' first write), Z tiles and staged results share one area.
 //
 // Issue slots 45 % busy (68 k warp instructions per chunk of four blocks), tensor pipe 11 %, DRAM 16 %.
-// 16 rows x 16384 steps, 128 x 128 (4096 chunks): 1052 us as a grid of blocks -> 557 us.  Bound by the latency of its phases, as
-// the 64 x 64 kernel was before its issuing warps: block barriers, and state blocks that are loaded when they are needed.
+// 16 rows x 16384 steps, 128 x 128 (4096 chunks): 1052 us as a grid of blocks -> 515 us (557 with the end gradients
+// loaded by the threads that use them: the d side's rows are 256 bytes apart, 9 k of 37 k cycles per chunk).  Bound by the latency of
+// its phases, as the 64 x 64 kernel was before its issuing warps: block barriers, and state blocks that are loaded when they are needed.
 #include "lfw_c64.cuh"
 #include "seq_layout.cuh"
 
@@ -39,7 +40,7 @@ constexpr int kFixParts = 512;         // partial sums of all entries of a chunk
 // shared-memory map (bytes from the 1024-byte aligned base); side 0 = k, 1 = d
 constexpr int kSideTiles = 4 * kTile;               // of a side: [Mm, Vm][window] tiles [step][feature]
 constexpr int oTw = 0;                              // [side]; raw values of the next chunk over Mm: q, k / dO, x [window]
-constexpr int oXw = oTw + 2 * kSideTiles;           // Z [t][s], Z^T [s][t] of the side at work; then its results
+constexpr int oXw = oTw + 2 * kSideTiles;           // end gradients, Z [t][s], Z^T [s][t] of the side at work; then its results
 constexpr int oGw = oXw + 3 * kTile;                // raw gates: f, fk [window]
 constexpr int oQtw = oGw + 4 * kRawBytes;           // [side][4][128] products of the quarters
 constexpr int oXcw = oQtw + 2 * 4 * kWide * 4;      // partial sums [3][4 quarters][128]
@@ -67,7 +68,7 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
                     int64_t T_, int64_t nc, int64_t total, int D, int K) {
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   unsigned char *sm = sm_raw + ((1024u - (umma::smem_u32(sm_raw) & 1023u)) & 1023u);
-  __shared__ __align__(8) uint64_t barG, barV, barZ, barM1, barM2;
+  __shared__ __align__(8) uint64_t barG, barV, barR, barZ, barM1, barM2;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_bad2[2], fix_n2[2];
 
@@ -109,6 +110,7 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
   if (tid == 0) {
     umma::mbar_init(&barG, 1);
     umma::mbar_init(&barV, 1);
+    umma::mbar_init(&barR, 1);
     umma::mbar_init(&barZ, 2);       // one commit per side
     umma::mbar_init(&barM1, 2);      // TQ1, T7 of one window
     umma::mbar_init(&barM2, 2);      // TQ2, T2
@@ -141,6 +143,15 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
 
   int fail = 0;                         // a wait of this thread gave up
   uint32_t it = 0, n1 = 0, n2 = 0;      // chunks; rounds of TQ1 / T7 and of TQ2 / T2
+  uint32_t nr = 0, nr_issued = 0;       // rounds of end gradients, (thread 0) requested
+  // thread 0: end gradients of window v of the other side and all windows of this one, blocks of 16 KB at r0, nc chunks apart
+  auto issue_r = [&](const float *r0, int side, int v) {
+    const int n = side ? nd : nk;
+    acp::mbar_expect_tx(&barR, (uint32_t)n * kTile);
+    for (int o = 0; o < n; ++o)
+      acp::bulk_g2s(sm + oXw + o * kTile, r0 + (size_t)(side ? o * nk + v : v * nk + o) * nc * kDim * kDim, kTile, &barR);
+    ++nr_issued;
+  };
   for (; wn.unit < total; ++it) {
     const ItemWalk w = wn;
     wn.step();
@@ -196,9 +207,13 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
     values(0, feat < K);
     umma::fence_async_smem();
     if (__syncthreads_or(fail)) break;      // products complete; the k side's values are in registers
-    if (tid == 0 && wn.unit < total) {
-      issue_gates(wn);
-      gates_pending = true;
+    const float *const r0 = Rend + ((size_t)w.row * nd * nk * nc + w.c) * kDim * kDim;      // block 0; nc chunks per block
+    if (tid == 0) {
+      issue_r(r0, 0, 0);      // the results before have left
+      if (wn.unit < total) {
+        issue_gates(wn);
+        gates_pending = true;
+      }
     }
     // The walk away from the anchor: downwards for the first two quarters (s = 1 / pm), upwards for the others; and back with
     // the reciprocal of the product at the far end, which the gates on the way turn into that of every step.
@@ -290,7 +305,6 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
     const int n_fix = fix_n < kFixCap ? fix_n : kFixCap;
     const int parts_log = n_fix <= kFixParts / 16 ? 4 : n_fix <= kFixParts / 8 ? 3 : 2, n_parts = 1 << parts_log;
     const T *const s0 = (w.c == 0) ? state + (size_t)w.row * D * K : ckpt + ((size_t)w.row * nc + w.c - 1) * D * K;
-    const float *const r0 = Rend + ((size_t)w.row * nd * nk * nc + w.c) * kDim * kDim;      // block 0; nc chunks per block
 
 #pragma unroll 1
     for (int side = 0; side < 2; ++side) {
@@ -305,6 +319,10 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
         pm_prev = tq == 0 ? rcp_fast(up) : tq == 1 ? rcp_fast(q1) : tq == 2 ? 1.f : q2;
       }
       if (side == 1) {      // the d side's own operands from its tiles, its ratios from where they wait
+        if (tid == 0) {
+          acp::bulk_wait_read<0>();      // the k side's results have left
+          issue_r(r0, 1, 0);
+        }
         const unsigned char *tp = sm + oTw + kSideTiles + tcol;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -327,15 +345,10 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
 #pragma unroll
         for (int j = 0; j < 16; ++j) sv[j] = rv[j] = 0.f;
         if (has) {
-          // block (i, j) of the grid: windows of the d side and of the k side; pieces of a row XOR-ed with (row % 8)
-          const float *rb = r0 + (size_t)(side ? win * nk + v : v * nk + win) * nc * kDim * kDim;
           if (side == 0) {         // a column of the stored state, own = k
             const T *sp = s0 + (size_t)(64 * v + t0) * K + feat;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              sv[j] = Elem<T>::ld(sp + (size_t)j * K);
-              rv[j] = rb[(t0 + j) * kDim + (((wf >> 2) ^ (j & 7)) << 2) + (wf & 3)];
-            }
+            for (int j = 0; j < 16; ++j) sv[j] = Elem<T>::ld(sp + (size_t)j * K);
           } else {                 // a row segment, own = d
             const T *sp = s0 + (size_t)feat * K + 64 * v + t0;
 #pragma unroll
@@ -345,9 +358,20 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
 #pragma unroll
               for (int j = 0; j < 8; ++j) sv[8 * i + j] = Elem<T>::ld(e + j);
             }
+          }
+        }
+        // end gradients: rows d of a block, 16-byte pieces of a row XOR-ed with (row % 8)
+        if (!acp::mbar_wait(&barR, nr++ & 1u)) fail = 1;
+        if (has) {
+          const unsigned char *rb = sm + oXw + win * kTile;
+          if (side == 0) {
+            rb += t0 * 256 + ((wf >> 5) << 7) + ((wf & 3) << 2);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) rv[j] = *reinterpret_cast<const float *>(rb + j * 256 + (tswz ^ ((j & 7) << 4)));
+          } else {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const float4 r4 = *reinterpret_cast<const float4 *>(rb + wf * kDim + (((4 * tq + i) ^ (wf & 7)) << 2));
+              const float4 r4 = *reinterpret_cast<const float4 *>(rb + wf * 256 + (((4 * tq + i) ^ (wf & 7)) << 4));
               rv[4 * i] = r4.x; rv[4 * i + 1] = r4.y; rv[4 * i + 2] = r4.z; rv[4 * i + 3] = r4.w;
             }
           }
@@ -375,9 +399,9 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
         umma::tmem_st16(tl + cS2 + t0, sv);
         umma::tmem_st16(tl + cR2 + t0, rv);
         umma::tmem_st_wait();
-        // (before the first of these barriers of the d side thread 0 sees the k side's results leave, before their place is Z's)
-        if (side == 1 && tid == 0) acp::bulk_wait_read<0>();
-        sync_all();
+        umma::fence_async_smem();
+        sync_all();      // also: the end gradients have been read
+        if (tid == 0 && v + 1 < n_oth) issue_r(r0, side, v + 1);
         if (warp == 2 || warp == 4) {      // TQ1 from Mm, T7 from Vm of the other side
           const int is7 = warp >> 2;
           const uint64_t db = desc_sw128(aT + (side ^ 1) * kSideTiles + (2 * is7 + v) * kTile);
@@ -587,6 +611,7 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
   if (tid == 0) {      // after a wait that gave up, copies may still be on their way into this CTA: bounded, let them land
     if (gates_pending) acp::mbar_wait(&barG, it & 1u);
     if (values_pending) acp::mbar_wait(&barV, it & 1u);
+    if (nr_issued > 0) acp::mbar_wait(&barR, (nr_issued - 1) & 1u);
   }
   sync_all();
   if (warp == 0) umma::tmem_dealloc(tb, kTmemColsW);
