@@ -270,8 +270,13 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
 #pragma unroll
         for (int j = 0; j < 16; ++j) vw[j] = t0 + j < nvalid ? vw[j] : 0.f;
       }
-      if (kFused) {      // gates 1: the values as they are (exact in TF32)
-      } else if (lo = fminf(lo, fabsf(s)), hi = fmaxf(hi, fabsf(s)), tq < 2) {
+      if (!kFused) {
+        lo = fminf(lo, fabsf(s));
+        hi = fmaxf(hi, fabsf(s));
+      }
+      if (kFused) {
+        // gates 1: the values as they are (exact in TF32)
+      } else if (tq < 2) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
           const float a = gd[j];
