@@ -255,7 +255,8 @@ dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state
   int fail = acp::mbar_wait(&full[0], 0) ? 0 : 1;
   float4 bq[8][4 / kH];
   carry_load_b<kH>(bq, ring, ch, lane);
-  for (int i = 0; i < nc; ++i) {
+  int i = 0;
+  for (; i < nc; ++i) {
     uint32_t own[kN][4], oth[4][4];
 #pragma unroll
     for (int n = 0; n < kN; ++n) {
@@ -287,6 +288,7 @@ dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state
     carry_product<kH>(R, own, oth, bq, ring + (in % kStages) * kStage, ch, lane);
   }
   if (fail) atomicExch(status, 1);
+  if (i < nc && tid == 0) drain_ring<kStages>(full, i, nc);
   T *dp = ds + ((size_t)b * kDim + 16 * w + g) * kDim + 32 * ch + 2 * t;
 #pragma unroll
   for (int n = 0; n < kN; ++n) {

@@ -348,6 +348,12 @@ __device__ __forceinline__ void init_ring(uint64_t *full, int tid) {
   }
   __syncthreads();
 }
+// A chain that gave up at step i of n, with the stages up to i + kStages - 2 requested: they land (a bounded wait each) before
+// the block leaves its shared memory to the next one.
+template <int kStages>
+__device__ __forceinline__ void drain_ring(uint64_t *full, int i, int n) {
+  for (int j = i; j < n && j < i + kStages - 1; ++j) acp::mbar_wait(&full[j % kStages], (uint32_t)(j / kStages) & 1u);
+}
 // One step's product for a warp of 16 rows and 1 / kH of the columns (part ch) of X += A B^T: A = all 64 columns of X as
 // operands, the own ones first (own), then the partner's (oth, kH = 2); B in registers, which take the next step's B as they
 // are used: its loads run under this product.

@@ -181,7 +181,8 @@ dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg
   int fail = acp::mbar_wait(&full[0], 0) ? 0 : 1;
   float4 bq[8][4 / kH];
   carry_load_b<kH>(bq, ring, ch, lane);
-  for (int c = 0; c < nc; ++c) {
+  int c = 0;
+  for (; c < nc; ++c) {
     uint32_t own[kN][4], oth[4][4];
 #pragma unroll
     for (int n = 0; n < kN; ++n) {
@@ -208,6 +209,7 @@ dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg
     carry_product<kH>(S, own, oth, bq, ring + (cn % kStages) * kStage, ch, lane);
   }
   if (fail) atomicExch(status, 1);
+  if (c < nc && tid == 0) drain_ring<kStages>(full, c, nc);
   T *fp = final_state + ((size_t)b * kDim + 16 * w + g) * kDim + 32 * ch + 2 * t;
 #pragma unroll
   for (int n = 0; n < kN; ++n) {

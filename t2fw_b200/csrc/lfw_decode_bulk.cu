@@ -115,7 +115,8 @@ lfw_decode_bulk_kernel(const T *__restrict__ x, const T *__restrict__ f, const T
   if (threadIdx.x == 0)
     for (int i = 0; i < kStages - 1 && i < n_items; ++i) issue_load(i);
 
-  for (int item = 0; item < n_items; ++item) {
+  int item = 0;
+  for (; item < n_items; ++item) {
     const int s = item % kStages;
     const uint32_t parity = (uint32_t)(item / kStages) & 1u;
     if (!mbar_wait(&full[s], parity)) s_fail = 1;   // benign race: every writer stores 1
@@ -165,6 +166,8 @@ lfw_decode_bulk_kernel(const T *__restrict__ x, const T *__restrict__ f, const T
   if (threadIdx.x == 0) {
     bulk_wait_all();
     if (s_fail) atomicExch(status, 1);
+    // gave up at `item`: the rows requested so far land before the block leaves (nothing is left to wait for otherwise)
+    for (int i = item; i < n_items && i < item + kStages - 1; ++i) mbar_wait(&full[i % kStages], (uint32_t)(i / kStages) & 1u);
   }
 }
 

@@ -63,3 +63,23 @@ def test_dependent_launches_wait_first(path):
         before = body[:body.index("dependency_wait()")]
         assert before.count("{") - before.count("}") == 1, m.group(1) + ": not in the outermost block"
         assert re.search(r"[;{}]\s*$", before), m.group(1) + ": under a condition"
+
+
+def _kernels(text):
+    """(name, body) of every kernel."""
+    for m in re.finditer(r"__global__[^;{]*?\b(\w+_kernel)\([^;{]*\{", text):
+        yield m.group(1), _block(text, m.end() - 1)[0]
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_copies_in_flight_are_waited_for_on_the_way_out(path):
+    """Bulk copies that a kernel asked for may still be on their way when it gives up, into shared memory that the next block
+    gets: behind the last place where it asks for more it waits once more for every barrier that they arrive on."""
+    for name, body in _kernels(_text(path)):
+        for m in re.finditer(r"auto (\w+) = \[&\]\([^)]*\) \{", body):
+            fetch, _ = _block(body, m.end() - 1)
+            if "mbar_expect_tx(" not in fetch:
+                continue
+            last = [c.end() for c in re.finditer(r"\b%s\(" % m.group(1), body)][-1]
+            for bar in set(re.findall(r"&(bar\w+|full)\b", fetch)):
+                assert re.search(r"\bmbar_wait\(&%s\b|\bdrain_ring<[^(]*\(%s\b" % (bar, bar), body[last:]), (name, m.group(1), bar)
