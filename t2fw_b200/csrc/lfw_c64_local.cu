@@ -132,8 +132,8 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
     const bool partial = nv0 < kC || nv1 < kC;      // steps beyond the valid ones become identity steps
     int *s_bad = s_bad2[it & 1];
 
-    if (!acp::mbar_wait(&barRaw, it & 1u)) s_fail = 1;
-    if (tid == 0) raw_pending = false;
+    if (acp::mbar_wait(&barRaw, it & 1u)) raw_pending = false;
+    else s_fail = 1;
 
     // gates of one side, own feature and quarter
     auto gates = [&](int blk, bool kside, float (&g)[16]) {

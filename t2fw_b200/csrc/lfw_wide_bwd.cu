@@ -160,8 +160,8 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
     int &s_bad = s_bad2[it & 1], &fix_n = fix_n2[it & 1];
 
     // ---- gates of the own feature and quarter on both sides, products of the quarters; raw values of the k side ----
-    if (!acp::mbar_wait(&barG, it & 1u)) fail = 1;
-    if (tid == 0) gates_pending = false;
+    if (acp::mbar_wait(&barG, it & 1u)) gates_pending = false;
+    else fail = 1;
     float g[2][16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -193,8 +193,8 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
       for (int j = 2; j < 16; j += 2) { p0 *= g[sd][j]; p1 *= g[sd][j + 1]; }
       qtot[(sd * 4 + tq) * kWide + feat] = p0 * p1;
     }
-    if (!acp::mbar_wait(&barV, it & 1u)) fail = 1;
-    if (tid == 0) values_pending = false;
+    if (acp::mbar_wait(&barV, it & 1u)) values_pending = false;
+    else fail = 1;
     float mw[16], vw[16], pm[16];
     auto values = [&](int sd, bool has) {
       const T *p = rawm + sd * (kSideTiles / 2);

@@ -95,8 +95,8 @@ lfw_wide_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ 
     const int nvalid = (int)(left < kC ? left : kC);      // steps beyond the valid ones become identity steps
     int &s_bad = s_bad2[it & 1];
 
-    if (!acp::mbar_wait(&barRaw, it & 1u)) fail = 1;
-    if (tid == 0) raw_pending = false;
+    if (acp::mbar_wait(&barRaw, it & 1u)) raw_pending = false;
+    else fail = 1;
 
     auto gates = [&](int blk, bool has, float (&g)[16]) {
       const T *p = raw + 2 * blk * kC * kDim;

@@ -83,3 +83,11 @@ def test_copies_in_flight_are_waited_for_on_the_way_out(path):
             last = [c.end() for c in re.finditer(r"\b%s\(" % m.group(1), body)][-1]
             for bar in set(re.findall(r"&(bar\w+|full)\b", fetch)):
                 assert re.search(r"\bmbar_wait\(&%s\b|\bdrain_ring<[^(]*\(%s\b" % (bar, bar), body[last:]), (name, m.group(1), bar)
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_copies_count_as_landed_only_after_a_wait_that_succeeded(path):
+    """A wait that gave up says nothing about the copies it stood for: they are still due on the way out."""
+    for m in re.finditer(r"[^;{}]*\b\w+_pending = false;", _text(path)):
+        s = m.group(0).strip()
+        assert s.startswith("bool ") or re.match(r"if \((acp::)?mbar_wait\(", s), s
