@@ -150,6 +150,10 @@ dfw_prep_bwd_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *
         }
       }
     }
+    float z0 = 0.f, z1 = 0.f;      // a NaN in Ub^T (which op has dropped) or in a column of c
+    row_nonfinite(u, z0, z1);
+    row_nonfinite(c, z0, z1);
+    spread_nonfinite(c, z0, z1);
     store_rows<false>(Nimg + img, c, w, lane);
   }
   float wb[8][4];      // Wb = T^T K, rows t = 16 w ..
@@ -252,6 +256,7 @@ dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state
       S[n][2] = Elem<T>::ld(sp + 8 * n * kDim + 8); S[n][3] = Elem<T>::ld(sp + (8 * n + 1) * kDim + 8);
     }
   }
+  spread_start<kH>(R, reinterpret_cast<float *>(&xs[0][0][0][0]), wl, ch, lane);
   int fail = acp::mbar_wait(&full[0], 0) ? 0 : 1;
   float4 bq[8][4 / kH];
   carry_load_b<kH>(bq, ring, ch, lane);
@@ -272,6 +277,7 @@ dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state
     const size_t o = img0 + (size_t)(nc - 1 - i) * kImg;
     float *rp = NR + o + (16 * w + g) * kDim + 32 * ch + 2 * t;
     float4 *const img = reinterpret_cast<float4 *>(GS + o) + (w * 8 + 4 * ch) * 32 + lane;
+    const float z0 = R[0][0] * 0.f, z1 = R[0][2] * 0.f;
 #pragma unroll
     for (int n = 0; n < kN; ++n) {
       if (kH == 2) {
@@ -281,8 +287,9 @@ dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state
       const float4 gx = image_at(buf + kImg + kPart, wl, 4 * ch + n, lane), nx = image_at(buf + kImg, wl, 4 * ch + n, lane);
       S[n][0] -= gx.x; S[n][1] -= gx.y; S[n][2] -= gx.z; S[n][3] -= gx.w;
       img[n * 32] = make_float4(rnd(S[n][0]), rnd(S[n][1]), rnd(S[n][2]), rnd(S[n][3]));
-      *reinterpret_cast<float2 *>(rp + 8 * n) = make_float2(rnd(R[n][0]), rnd(R[n][1]));
-      *reinterpret_cast<float2 *>(rp + 8 * kDim + 8 * n) = make_float2(rnd(R[n][2]), rnd(R[n][3]));
+      const float4 r4 = with_rows(own[n], z0, z1);
+      *reinterpret_cast<float2 *>(rp + 8 * n) = make_float2(r4.x, r4.y);
+      *reinterpret_cast<float2 *>(rp + 8 * kDim + 8 * n) = make_float2(r4.z, r4.w);
       R[n][0] += nx.x; R[n][1] += nx.y; R[n][2] += nx.z; R[n][3] += nx.w;
     }
     carry_product<kH>(R, own, oth, bq, ring + (in % kStages) * kStage, ch, lane);
@@ -385,7 +392,7 @@ dfw_grad_kernel(const T *__restrict__ go, const T *__restrict__ q, const T *__re
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
 #pragma unroll
-      for (int x = 0; x < 4; ++x) ea[n][x] = op(-e[n][x]);
+      for (int x = 0; x < 4; ++x) ea[n][x] = bits(rnd(-e[n][x]));
       reinterpret_cast<uint4 *>(Es)[(w * 8 + n) * 32 + lane] = make_uint4(ea[n][0], ea[n][1], ea[n][2], ea[n][3]);
       *reinterpret_cast<uint32_t *>(sm + oEg + raw_off(r0, n) + 4 * t) = pack16<T>(e[n][0], e[n][1]);
       *reinterpret_cast<uint32_t *>(sm + oEg + raw_off(r1, n) + 4 * t) = pack16<T>(e[n][2], e[n][3]);

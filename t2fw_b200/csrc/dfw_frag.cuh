@@ -56,15 +56,15 @@ __device__ __forceinline__ void mma_16<__nv_bfloat16>(float (&c)[4], const uint3
 }
 
 // ---- operand values --------------------------------------------------------------------------------
-// TF32 rounding (nearest, ties away) of a value that only feeds a product: the tensor core drops the low 13 bits
+// TF32 rounding (nearest, ties away) of a value that only feeds products: the tensor core drops the low 13 bits, so half a
+// unit of the last kept place is added.  rnd: in floating point, for a NaN to stay one.  op: one integer addition, which makes
+// a zero of the NaN that arithmetic gives (0x7fffffff), where another operand brings the NaN along as well.
+__device__ __forceinline__ float rnd(float v) { return fmaf(__uint_as_float(__float_as_uint(v) & 0xff800000u), 0x1p-11f, v); }
 __device__ __forceinline__ uint32_t op(float v) { return __float_as_uint(v) + 0x1000u; }
-// the rounded value itself
-__device__ __forceinline__ float rnd(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u); }
-// v = hi + lo with both parts TF32 operands: together 22 bits
+// v = hi + lo with both parts TF32 operands: together 22 bits (of a NaN, lo is one)
 __device__ __forceinline__ void split(float v, uint32_t &hi, uint32_t &lo) {
-  const float h = rnd(v);
-  hi = __float_as_uint(h);
-  lo = __float_as_uint(v - h);
+  hi = op(v) & 0xffffe000u;
+  lo = __float_as_uint(v - __uint_as_float(hi));
 }
 // the two 16-bit values of a register as TF32 operands (exact)
 template <typename T> __device__ __forceinline__ uint32_t lo16(uint32_t u);
@@ -353,6 +353,53 @@ __device__ __forceinline__ void init_ring(uint64_t *full, int tid) {
 template <int kStages>
 __device__ __forceinline__ void drain_ring(uint64_t *full, int i, int n) {
   for (int j = i; j < n && j < i + kStages - 1; ++j) acp::mbar_wait(&full[j % kStages], (uint32_t)(j / kStages) & 1u);
+}
+// A state row with a NaN or an infinity in one column has them in all columns after the next step.  The rows that the carries
+// start from and add are made so at once: then the products of the chain need not round with care (op), and one element tells
+// of its row.  c: rows g and g + 8 of a warp's 16, the four lanes of a row hold its columns.  z0, z1: 0, or NaN.
+template <int kN>
+__device__ __forceinline__ void row_nonfinite(const float (&c)[kN][4], float &z0, float &z1) {
+#pragma unroll
+  for (int n = 0; n < kN; ++n) {
+    z0 = fmaf(c[n][0], 0.f, fmaf(c[n][1], 0.f, z0));
+    z1 = fmaf(c[n][2], 0.f, fmaf(c[n][3], 0.f, z1));
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    z0 += __shfl_xor_sync(0xffffffffu, z0, o);
+    z1 += __shfl_xor_sync(0xffffffffu, z1, o);
+  }
+}
+template <int kN>
+__device__ __forceinline__ void spread_nonfinite(float (&c)[kN][4], float z0, float z1) {
+  if (z0 == 0.f && z1 == 0.f) return;
+#pragma unroll
+  for (int n = 0; n < kN; ++n) {
+    c[n][0] += z0; c[n][1] += z0;
+    c[n][2] += z1; c[n][3] += z1;
+  }
+}
+// the carries' start: with kH = 2 a row's other columns are the partner warp's (x: [kW][2][2][8] floats)
+template <int kH>
+__device__ __forceinline__ void spread_start(float (&c)[8 / kH][4], float *x, int wl, int ch, int lane) {
+  float z0 = 0.f, z1 = 0.f;
+  row_nonfinite(c, z0, z1);
+  if (kH == 2) {
+    float *own = x + ((wl * 2 + ch) * 2) * 8 + (lane >> 2), *oth = x + ((wl * 2 + (ch ^ 1)) * 2) * 8 + (lane >> 2);
+    if ((lane & 3) == 0) {
+      own[0] = z0;
+      own[8] = z1;
+    }
+    __syncthreads();
+    z0 += oth[0];
+    z1 += oth[8];
+    __syncthreads();      // x is used again
+  }
+  spread_nonfinite(c, z0, z1);
+}
+// operands as a part of an image, with their rows' 0 or NaN
+__device__ __forceinline__ float4 with_rows(const uint32_t (&a)[4], float z0, float z1) {
+  return make_float4(__uint_as_float(a[0]) + z0, __uint_as_float(a[1]) + z0, __uint_as_float(a[2]) + z1, __uint_as_float(a[3]) + z1);
 }
 // One step's product for a warp of 16 rows and 1 / kH of the columns (part ch) of X += A B^T: A = all 64 columns of X as
 // operands, the own ones first (own), then the partner's (oth, kH = 2); B in registers, which take the next step's B as they

@@ -122,7 +122,7 @@ dfw_prep_fwd_kernel(const T *__restrict__ k, const T *__restrict__ v, float *__r
 #pragma unroll
       for (int s = 0; s < 2; ++s)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) a[s][e] = op(c[2 * kk + s][e]);
+        for (int e = 0; e < 4; ++e) a[s][e] = bits(rnd(c[2 * kk + s][e]));
 #pragma unroll
       for (int np = 0; np < 4; ++np) {
         uint32_t r[4];
@@ -178,6 +178,7 @@ dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg
     S[n][0] = __uint_as_float(lo16<T>(u)); S[n][1] = __uint_as_float(hi16<T>(u));
     S[n][2] = __uint_as_float(lo16<T>(x)); S[n][3] = __uint_as_float(hi16<T>(x));
   }
+  spread_start<kH>(S, reinterpret_cast<float *>(&xs[0][0][0][0]), wl, ch, lane);
   int fail = acp::mbar_wait(&full[0], 0) ? 0 : 1;
   float4 bq[8][4 / kH];
   carry_load_b<kH>(bq, ring, ch, lane);
@@ -196,13 +197,14 @@ dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg
     if (tid == 0) fetch(c + kStages - 1);
     const float *buf = ring + (c % kStages) * kStage;
     float4 *const img = reinterpret_cast<float4 *>(NSimg + img0 + (size_t)c * kImg) + (w * 8 + 4 * ch) * 32 + lane;
+    const float z0 = S[0][0] * 0.f, z1 = S[0][2] * 0.f;
 #pragma unroll
     for (int n = 0; n < kN; ++n) {
       if (kH == 2) {
         const uint4 u = xs[c & 1][wl][4 * (ch ^ 1) + (n & 3)][lane];
         oth[n & 3][0] = u.x; oth[n & 3][1] = u.y; oth[n & 3][2] = u.z; oth[n & 3][3] = u.w;
       }
-      img[n * 32] = make_float4(rnd(S[n][0]), rnd(S[n][1]), rnd(S[n][2]), rnd(S[n][3]));
+      img[n * 32] = with_rows(own[n], z0, z1);
       const float4 nx = image_at(buf + kImg, wl, 4 * ch + n, lane);
       S[n][0] += nx.x; S[n][1] += nx.y; S[n][2] += nx.z; S[n][3] += nx.w;
     }
@@ -287,7 +289,7 @@ dfw_out_fwd_kernel(const T *__restrict__ q, const T *__restrict__ k, const float
 #pragma unroll
   for (int n = 0; n < 8; ++n)
     reinterpret_cast<float4 *>(Ws)[(w * 8 + n) * 32 + lane] =
-        make_float4(__uint_as_float(op(c[n][0])), __uint_as_float(op(c[n][1])), __uint_as_float(op(c[n][2])), __uint_as_float(op(c[n][3])));
+        make_float4(rnd(c[n][0]), rnd(c[n][1]), rnd(c[n][2]), rnd(c[n][3]));
   __syncthreads();
 
   uint32_t qa[4][4];

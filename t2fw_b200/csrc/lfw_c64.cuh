@@ -12,8 +12,11 @@
 // gradient at the chunk end: the 64 x 64 state block carries the anchor product of the side that is
 // contracted away, and the result is scaled by that of its own side.  (The chunk-local kernel alone
 // anchors its operands at the chunk's end or start, lfw_c64_local.cu.)
-// A batch row whose one-sided 32-step products leave [2^-100, 2^100] is flagged and recomputed by
-// the sequential scan kernels.
+// A batch row whose one-sided 32-step products leave [2^-100, 2^100], or that holds a NaN or an infinity, is flagged and
+// recomputed by the sequential scan kernels.  A call looks at every input on the way to its flags: the chunk-local kernel at the
+// gates and the two value tensors that it contracts, the carry at the states that it walks, the output kernel at the query, the
+// gradient kernel at x, k and the start states.
+// The fused layer has no gate products out of range and no scan behind it: its kernels round so that a NaN stays one.
 //
 // Operand tiles are 64 x 64 fp32 (TF32-rounded) in the K-major 128-byte-swizzle layout of the
 // tcgen05 shared-memory descriptor: two column blocks of 32 floats; inside a block row r is 128
@@ -44,16 +47,43 @@ constexpr float kRangeLo = 7.888609e-31f;       // 2^-100
 constexpr float kRangeHi = 1.267651e+30f;       // 2^100
 
 // Round to TF32 (10 mantissa bits), nearest with ties away from zero - what cvt.rna.tf32.f32 does -
-// as two integer instructions: the conversion instruction runs on the quarter-rate pipe and there
-// are hundreds of them per thread and chunk.  (Infinity becomes NaN; such rows are flagged anyway.)
+// as integer instructions: the conversion instruction runs on the quarter-rate pipe and there
+// are hundreds of them per thread and chunk.  For a value that is ONLY stored as a tensor-core operand the
+// mask can be left out: the tensor core ignores the low 13 bits of an fp32 operand (shared memory and tensor
+// memory alike; tests/test_umma_gpu.py checks it), so adding half a unit of the last kept place is enough.
+// The integer addition makes a zero of the NaN that arithmetic gives (0x7fffffff): without kNaN the row is one that
+// is flagged.  kNaN: the half unit is added in floating point, one instruction more (everywhere: 96 x 1024 training
+// 174 -> 183 us), with the same result for every other value.
+template <bool kNaN = false>
+__device__ __forceinline__ float bias_tf32(float v) {
+  if (kNaN) return fmaf(__uint_as_float(__float_as_uint(v) & 0xff800000u), 0x1p-11f, v);
+  return __uint_as_float(__float_as_uint(v) + 0x1000u);
+}
+template <bool kNaN = false>
 __device__ __forceinline__ float rna_tf32(float v) {
-  return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);
+  return __uint_as_float(__float_as_uint(bias_tf32<kNaN>(v)) & 0xffffe000u);
 }
 
-// The same rounding for a value that is ONLY stored as a tensor-core operand: the tensor core ignores
-// the low 13 bits of an fp32 operand (shared memory and tensor memory alike; tests/test_umma_gpu.py checks it),
-// so adding half a unit of the last kept place is enough and the mask can be left out.
-__device__ __forceinline__ float bias_tf32(float v) { return __uint_as_float(__float_as_uint(v) + 0x1000u); }
+// The largest magnitude of three values, NaN if one of them is none (fmaxf would drop it): the range tests take the values
+// along with the products, for no more instructions than without
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3_abs(float a, float b, float c) {      // (drops a NaN)
+  float r;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// whether all n values are finite numbers
+template <int n>
+__device__ __forceinline__ bool all_finite(const float (&v)[n]) {
+  float m = 0.f;
+#pragma unroll
+  for (int j = 0; j < n; j += 2) m = max3_abs(m, v[j], v[j + 1]);
+  return m <= 3.4028235e38f;
+}
 
 // 1 / v as the hardware's approximation (about 1 ulp; denormals count as zero, which every caller has excluded)
 __device__ __forceinline__ float rcp_fast(float v) {

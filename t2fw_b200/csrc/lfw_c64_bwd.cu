@@ -332,7 +332,7 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float e = seq::exp_neg(Elem<T>::ld(p + j * kDim)), sg = seq::rcp1p(e);
-        a[j] = seq::round_to<T>(fmaxf(sg, seq::kGateFloor));
+        a[j] = seq::round_to<T>(seq::floored(sg));
         // d gate / d pre-activation in fp32: s (1 - s) = s^2 e^-g
         der[(8 * h + j) * kDim] = sg > seq::kGateFloor ? sg * sg * e : 0.f;
       }
@@ -352,8 +352,8 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     }
     if (!kFused) {          // (the fused layer's gates are at least 1/8)
 #pragma unroll
-      for (int j = 0; j < 16; ++j) g_min = fminf(g_min, fabsf(g[j]));
-      if (!(g_min >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+      for (int j = 0; j < 16; j += 2) g_min = min3_abs(g_min, g[j], g[j + 1]);
+      if (!(g_min >= kTinyState)) {      // rare: some gate needs the clamp
 #pragma unroll
         for (int j = 0; j < 16; ++j) g[j] = sanitize_gate(g[j]);
       }
@@ -397,35 +397,36 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       if (tq < 2) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
-          vw[j] = rna_tf32(vw[j] * s);
+          const float e = vw[j];
+          vw[j] = rna_tf32<kFused>(e * s);
           if (j == 0) r = rcp_fast(s);
           s *= g[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, e);      // x and k too
         }
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           if (j > 0) r *= g[j];
           pm[j] = r;
-          mw[j] = rna_tf32(mw[j] * r);
+          mw[j] = rna_tf32<kFused>(mw[j] * r);
         }
       } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           s *= g[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, vw[j]);
           pm[j] = s;
-          mw[j] = rna_tf32(mw[j] * s);
+          mw[j] = rna_tf32<kFused>(mw[j] * s);
         }
         r = rcp_fast(s);
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
-          vw[j] = rna_tf32(vw[j] * r);
+          vw[j] = rna_tf32<kFused>(vw[j] * r);
           r *= g[j];
         }
       }
-      if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad = 1;      // also NaN
+      if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad = 1;
       umma::tmem_st16(tl + cMw + t0, mw);
       umma::tmem_st16(tl + cVw + t0, vw);
       unsigned char *tp = uT + h * 2 * kTile + tcol + t0 * 128;
@@ -486,13 +487,14 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         for (int j = 0; j < 4; ++j) {
           const float s2 = sv[4 * i + j] * av[j], r2 = rv[4 * i + j] * bv[j];
           acc = fmaf(s2, r2, acc);
-          sv[4 * i + j] = bias_tf32(s2);
-          rv[4 * i + j] = bias_tf32(r2);
+          sv[4 * i + j] = bias_tf32<kFused>(s2);
+          rv[4 * i + j] = bias_tf32<kFused>(r2);
         }
       }
       umma::tmem_st16(tl + cS2 + t0, sv);
       umma::tmem_st16(tl + cR2 + t0, rv);
       bndp[(h * 4 + tq) * kDim + feat] = acc;
+      if (!kFused && !(fabsf(acc) <= 3.4028235e38f)) atomicExch(rowflag + wi.row, 1);      // no finite number in a state
     }
     umma::tmem_st_wait();
     report(&barA);
@@ -516,10 +518,10 @@ lfw_c64_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         umma::tmem_ld_wait();
         if (tq == q4) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = j <= fl ? bias_tf32(v[j]) : 0.f;
+          for (int j = 0; j < 16; ++j) v[j] = j <= fl ? bias_tf32<kFused>(v[j]) : 0.f;
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = bias_tf32(v[j]);
+          for (int j = 0; j < 16; ++j) v[j] = bias_tf32<kFused>(v[j]);
         }
       } else {
 #pragma unroll

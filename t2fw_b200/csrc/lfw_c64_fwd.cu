@@ -187,9 +187,9 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
     float mn = kRangeHi;      // (the fused layer's gates are at least 1/8)
     if (!kFused) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) mn = fminf(mn, fminf(fabsf(gk[j]), fabsf(gd[j])));
+      for (int j = 0; j < 16; ++j) mn = min3_abs(mn, gk[j], gd[j]);
     }
-    if (!kFused && !(mn >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+    if (!kFused && !(mn >= kTinyState)) {      // rare: some gate needs the clamp
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         gk[j] = sanitize_gate(gk[j]);
@@ -235,20 +235,21 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       if (tq < 2) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
-          mw[j] = bias_tf32(mw[j] * rcp_fast(s));
-          vw[j] = bias_tf32(vw[j] * s);
+          const float e = mw[j];
+          mw[j] = bias_tf32<kFused>(e * rcp_fast(s));
+          vw[j] = bias_tf32<kFused>(vw[j] * s);
           s *= gk[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, e);      // the query's values too
         }
       } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           s *= gk[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
-          mw[j] = bias_tf32(mw[j] * s);
-          vw[j] = bias_tf32(vw[j] * rcp_fast(s));
+          hi = max3_abs(hi, s, mw[j]);
+          mw[j] = bias_tf32<kFused>(mw[j] * s);
+          vw[j] = bias_tf32<kFused>(vw[j] * rcp_fast(s));
         }
       }
 #pragma unroll
@@ -272,7 +273,7 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       }
       if (!kFused) {
         lo = fminf(lo, fabsf(s));
-        hi = fmaxf(hi, fabsf(s));
+        hi = max3_abs(hi, s, s);
       }
       if (kFused) {
         // gates 1: the values as they are (exact in TF32)
@@ -281,24 +282,24 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         for (int j = 15; j >= 0; --j) {
           const float a = gd[j];
           gd[j] = rcp_fast(s);
-          vw[j] = bias_tf32(vw[j] * s);
+          vw[j] = bias_tf32<kFused>(vw[j] * s);
           s *= a;
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, s);
         }
       } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           s *= gd[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, s);
           gd[j] = s;
-          vw[j] = bias_tf32(vw[j] * rcp_fast(s));
+          vw[j] = bias_tf32<kFused>(vw[j] * rcp_fast(s));
         }
       }
       umma::tmem_st16(tl + cX + t0, vw);
     }
-    if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad[h] = 1;      // also NaN
+    if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad[h] = 1;
     {   // state: row d = own feature, columns k = t0 .. t0 + 15, scaled by G_REF
       float sv[16];
 #pragma unroll
@@ -312,10 +313,10 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
       for (int i = 0; i < 4; ++i) {
         const float4 a = *reinterpret_cast<const float4 *>(qtot + t0 + 4 * i);
         const float4 b = *reinterpret_cast<const float4 *>(qtot + kDim + t0 + 4 * i);
-        sv[4 * i] = bias_tf32(sv[4 * i] * (a.x * b.x));
-        sv[4 * i + 1] = bias_tf32(sv[4 * i + 1] * (a.y * b.y));
-        sv[4 * i + 2] = bias_tf32(sv[4 * i + 2] * (a.z * b.z));
-        sv[4 * i + 3] = bias_tf32(sv[4 * i + 3] * (a.w * b.w));
+        sv[4 * i] = bias_tf32<kFused>(sv[4 * i] * (a.x * b.x));
+        sv[4 * i + 1] = bias_tf32<kFused>(sv[4 * i + 1] * (a.y * b.y));
+        sv[4 * i + 2] = bias_tf32<kFused>(sv[4 * i + 2] * (a.z * b.z));
+        sv[4 * i + 3] = bias_tf32<kFused>(sv[4 * i + 3] * (a.w * b.w));
       }
       umma::tmem_st16(tl + cS2 + t0, sv);
     }
@@ -366,10 +367,10 @@ lfw_c64_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ s
         umma::tmem_ld_wait();
         if (tq == q4) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = j <= fl ? bias_tf32(v[j]) : 0.f;
+          for (int j = 0; j < 16; ++j) v[j] = j <= fl ? bias_tf32<kFused>(v[j]) : 0.f;
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = bias_tf32(v[j]);
+          for (int j = 0; j < 16; ++j) v[j] = bias_tf32<kFused>(v[j]);
         }
       } else {
 #pragma unroll

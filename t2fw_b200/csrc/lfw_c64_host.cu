@@ -13,8 +13,8 @@
 //      stored in place of G_c (fp32); what is left after chunk 0 is d_state
 //   3. lfw_c64_bwd_kernel               per (row, chunk): d_x, d_f, d_q, d_k, d_f_key
 // Scratch (floats): M[B][nc][64][64], 16-byte pieces of a row XOR-ed with (row % 8) | Ac[B][nc][64] | Gc[B][nc][64] | flags[B][nc] (int) |
-// rowflag[B] (int).  A flagged row (gate products outside the range of the factored form) is recomputed by the
-// scan kernels afterwards.
+// rowflag[B] (int).  A flagged row (gate products outside the range of the factored form, values that are no
+// finite numbers) is recomputed by the scan kernels afterwards.
 // States larger than 64 x 64 (D, K multiples of 64): the recurrence never mixes state rows or columns, so a D x K state
 // is a (D/64) x (K/64) grid of independent blocks, problem rows of their own for the kernels (B above counts them);
 // block (i, j) reads the d-side vectors' window i and the k-side vectors' window j in place, states and checkpoints are
@@ -177,7 +177,7 @@ lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const fl
     }
   }
   if (!kFwd) store16<T, kCols>(op, S);
-  if (any) atomicExch(rowflag + item, 1);
+  if (any || !all_finite(S)) atomicExch(rowflag + item, 1);      // (a NaN or an infinity that has got into a state stays in it)
 }
 
 // The carry of BH problem rows.  Two values per thread make twice as many blocks, so that one block's loads run under

@@ -150,8 +150,8 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
       if (kFused) return;             // (at least 1/8)
       float mn = kRangeHi;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) mn = fminf(mn, fabsf(g[j]));
-      if (!(mn >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+      for (int j = 0; j < 16; j += 2) mn = min3_abs(mn, g[j], g[j + 1]);
+      if (!(mn >= kTinyState)) {      // rare: some gate needs the clamp
 #pragma unroll
         for (int j = 0; j < 16; ++j) g[j] = sanitize_gate(g[j]);
       }
@@ -185,19 +185,20 @@ lfw_c64_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ M
       if (kSuffix) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
-          w[j] = bias_tf32(w[j] * s);
+          const float e = w[j];
+          w[j] = bias_tf32<kFused>(e * s);
           s *= g[j];
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, e);
         }
       } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           s *= g[j];
-          hi = fmaxf(hi, fabsf(s));
-          w[j] = bias_tf32(w[j] * s);
+          hi = max3_abs(hi, s, w[j]);
+          w[j] = bias_tf32<kFused>(w[j] * s);
         }
       }
-      if (!(hi <= kRangeHi)) s_bad[h] = 1;     // also catches NaN
+      if (!(hi <= kRangeHi)) s_bad[h] = 1;     // a product out of range, a gate or a value that is no finite number
       if (tq == (kSuffix ? 0 : 3) && nvalid > 0) tot[(size_t)(ci + h) * kDim + feat] = s;
     };
 

@@ -170,7 +170,7 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
     }
     float g_min = kRangeHi;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) g_min = fminf(g_min, fminf(fabsf(g[0][j]), fabsf(g[1][j])));
+    for (int j = 0; j < 16; ++j) g_min = min3_abs(g_min, g[0][j], g[1][j]);
     unsigned tiny = 0;      // steps of the quarter with tiny gates, k side in the low half
     if (g_min < kTinyGate) {
 #pragma unroll
@@ -179,7 +179,7 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
         tiny |= (fabsf(g[1][j]) < kTinyGate ? 0x10000u : 0u) << j;
       }
     }
-    if (!(g_min >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+    if (!(g_min >= kTinyState)) {      // rare: some gate needs the clamp
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         g[0][j] = sanitize_gate(g[0][j]);
@@ -223,11 +223,12 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
       if (tq < 2) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
-          vw[j] = rna_tf32(vw[j] * s);
+          const float e = vw[j];
+          vw[j] = rna_tf32(e * s);
           if (j == 0) r = rcp_fast(s);
           s *= gg[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, e);      // x and k too
         }
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -240,7 +241,7 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
         for (int j = 0; j < 16; ++j) {
           s *= gg[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, vw[j]);
           pm[j] = s;
           mw[j] = rna_tf32(mw[j] * s);
         }
@@ -251,7 +252,7 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
           r *= gg[j];
         }
       }
-      if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad = 1;      // also NaN
+      if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad = 1;
       unsigned char *tp = sm + oTw + sd * kSideTiles + tcol;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
@@ -415,6 +416,7 @@ lfw_wide_bwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
         }
       }
       bndp[tq * kWide + feat] = acc;
+      if (!(fabsf(acc) <= 3.4028235e38f)) atomicExch(rowflag + w.row, 1);      // no finite number in a state
 
       // ---- Z: mask, round, store as [t][s] and [s][t].  A warp holds rows 16 q4 .. + 15 and columns t0 .. t0 + 15: on the
       //      diagonal it masks, below it nothing is masked, above it all is zero ----

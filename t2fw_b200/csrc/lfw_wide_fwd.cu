@@ -135,8 +135,8 @@ lfw_wide_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
     }
     float mn = kRangeHi;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) mn = fminf(mn, fminf(fabsf(gk[j]), fabsf(gd[j])));
-    if (!(mn >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+    for (int j = 0; j < 16; ++j) mn = min3_abs(mn, gk[j], gd[j]);
+    if (!(mn >= kTinyState)) {      // rare: some gate needs the clamp
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         gk[j] = sanitize_gate(gk[j]);
@@ -178,18 +178,19 @@ lfw_wide_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
       if (tq < 2) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
-          mw[j] = bias_tf32(mw[j] * rcp_fast(s));
+          const float e = mw[j];
+          mw[j] = bias_tf32(e * rcp_fast(s));
           vw[j] = bias_tf32(vw[j] * s);
           s *= gk[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, e);      // the query's values too
         }
       } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           s *= gk[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, mw[j]);
           mw[j] = bias_tf32(mw[j] * s);
           vw[j] = bias_tf32(vw[j] * rcp_fast(s));
         }
@@ -210,7 +211,7 @@ lfw_wide_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
 #pragma unroll
       for (int j = 0; j < 16; ++j) vw[j] = has_d && t0 + j < nvalid ? rawv(0, j) : 0.f;
       lo = fminf(lo, fabsf(s));
-      hi = fmaxf(hi, fabsf(s));
+      hi = max3_abs(hi, s, s);
       if (tq < 2) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
@@ -219,21 +220,21 @@ lfw_wide_fwd_kernel(const __grid_constant__ seq::Maps mp, const T *__restrict__ 
           vw[j] = bias_tf32(vw[j] * s);
           s *= a;
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, s);
         }
       } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           s *= gd[j];
           lo = fminf(lo, fabsf(s));
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, s);
           gd[j] = s;
           vw[j] = bias_tf32(vw[j] * rcp_fast(s));
         }
       }
       umma::tmem_st16(tl + cXw + t0, vw);
     }
-    if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad = 1;      // also NaN
+    if (!(lo >= kRangeLo && hi <= kRangeHi)) s_bad = 1;
     for (int c = 0; c < nk; ++c) {   // state: row d = own feature, a quarter of the columns k, scaled by G_REF
       const int k0 = nk * t0 + 16 * c;
       float sv[16];

@@ -104,9 +104,9 @@ lfw_wide_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ 
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         g[j] = has && t0 + j < nvalid ? Elem<T>::ld(p + j * kDim) : 1.f;
-        mn = fminf(mn, fabsf(g[j]));
+        if (j & 1) mn = min3_abs(mn, g[j - 1], g[j]);
       }
-      if (!(mn >= kTinyState)) {      // rare (also NaN): some gate needs the clamp
+      if (!(mn >= kTinyState)) {      // rare: some gate needs the clamp
 #pragma unroll
         for (int j = 0; j < 16; ++j) g[j] = sanitize_gate(g[j]);
       }
@@ -127,19 +127,20 @@ lfw_wide_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ 
       if (kSuffix) {
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
-          v[j] = bias_tf32(v[j] * s);
+          const float e = v[j];
+          v[j] = bias_tf32(e * s);
           s *= g[j];
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, e);
         }
       } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           s *= g[j];
-          hi = fmaxf(hi, fabsf(s));
+          hi = max3_abs(hi, s, v[j]);
           v[j] = bias_tf32(v[j] * s);
         }
       }
-      if (!(hi <= kRangeHi)) s_bad = 1;     // also catches NaN
+      if (!(hi <= kRangeHi)) s_bad = 1;     // a product out of range, a gate or a value that is no finite number
       return s;
     };
     const bool edge = tq == (kSuffix ? 0 : 3);      // this quarter ends with the chunk's total

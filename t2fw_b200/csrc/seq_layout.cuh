@@ -95,9 +95,14 @@ __device__ __forceinline__ float rcp1p(float e) {      // 1 / (1 + e)
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
   return r;
 }
+__device__ __forceinline__ float floored(float s) {      // NaN stays NaN (fmaxf would give the floor)
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(s), "f"(kGateFloor));
+  return r;
+}
 template <typename T>
 __device__ __forceinline__ float sigmoid_gate(float g) {
-  return round_to<T>(fmaxf(rcp1p(exp_neg(g)), kGateFloor));
+  return round_to<T>(floored(rcp1p(exp_neg(g))));
 }
 // The block of tensor i for the chunk whose first row is `row` (nv valid rows), sub-item h.
 // Dense [rows][64] arrays: one linear bulk copy of the valid rows; otherwise the tiled copy of the
