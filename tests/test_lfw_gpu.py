@@ -233,10 +233,31 @@ def test_decode_shapes(cuda, B, D, K):
 
 @pytest.mark.parametrize("D,K", [(128, 64), (64, 128), (128, 128), (192, 64), (64, 256)])
 def test_blocked_state_shapes(cuda, D, K):
-    """D x K states that are grids of 64 x 64 blocks run on the tensor-core path as a virtual
-    batch; outputs and gradients are sums over the other axis' blocks."""
+    """States larger than 64 x 64 on the tensor-core path: up to 128 x 128 a chunk is one problem, beyond that the state is a
+    grid of 64 x 64 blocks, whose outputs and gradients are sums over the other axis' blocks."""
     dev = to_dev(lfw_inputs(2, 150, D, K, "sigmoid", 0.5, D + K), torch.float16, cuda)
     check_against_oracle(dev, run_cabi(*dev), torch.float16)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,K,T", [(192, 128, 192), (128, 192, 150), (256, 256, 130)])
+def test_grid_of_blocks_along_both_axes(cuda, dtype, D, K, T):
+    """Blocks that are neither in the first row nor in the first column of the grid add to sums of both axes; whole and ragged
+    last chunks; 110 rows of three chunks, so that every kernel has CTAs that take more than they begin with."""
+    dev = to_dev(lfw_inputs(110, T, D, K, "sigmoid", 0.5, D + K + T), dtype, cuda)
+    got = run_cabi(*dev)
+    assert all(torch.isfinite(t).all() for t in (got[0], got[1], *got[2]))
+    check_against_oracle(dev, got, dtype, rows=[0, 54, 109])
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,K", [(128, 64), (64, 128)])
+def test_wide_rectangles_on_further_chunks(cuda, dtype, D, K):
+    """More chunks than any kernel has CTAs: some take a second one, with one side's upper features unused."""
+    dev = to_dev(lfw_inputs(32, 640, D, K, "sigmoid", 0.5, D + 2 * K), dtype, cuda)
+    got = run_cabi(*dev)
+    assert all(torch.isfinite(t).all() for t in (got[0], got[1], *got[2]))
+    check_against_oracle(dev, got, dtype, rows=[0, 15, 31])
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
@@ -257,24 +278,27 @@ def test_carry_over_more_chunks_than_one_round(cuda, B, T, D, K):
     check_against_oracle(dev, got, torch.float16, rows=[0, B - 1])
 
 
-@pytest.mark.parametrize("D,K", [(64, 64), (128, 128), (64, 128)])
+@pytest.mark.parametrize("D,K", [(64, 64), (128, 128), (64, 128), (192, 128)])
 @pytest.mark.parametrize("n", [1, 32, 33, 64, 65, 128, 129])
 def test_tiny_gate_list_lengths(cuda, n, D, K):
-    """n gates below 2^-13 in one chunk: their sums are split into 16, 8 or 4 parts by how many there are, and beyond 128 the
-    row is left to the scan kernels."""
+    """n gates of 2^-19 in one chunk: their sums are split into 16, 8 or 4 parts by how many there are, and beyond 128 the
+    row is left to the scan kernels.  (The factored form of the sum alone is 4e-2 of the largest gradient off at 2^-18.5,
+    twice the tolerance: an entry that is left out shows.)"""
     x, f, q, k, fk, s, go, gs = lfw_inputs(2, 130, D, K, "sigmoid", 0.5, 500 + n)
     for i in range(n):
         gate, feat = (fk, (i // 2) % K) if i % 2 else (f, (i // 2) % D)
-        gate[1, 66 + 5 * (i % 11) + i // 128, feat] = 5e-5 if i % 3 else -6e-5
+        gate[1, 66 + 5 * (i % 11) + i // 128, feat] = 2e-6 if i % 3 else -2e-6
     dev = to_dev((x, f, q, k, fk, s, go, gs), torch.float16, cuda)
     check_against_oracle(dev, run_cabi(*dev), torch.float16)
 
 
-def test_blocked_extreme_gates(cuda):
-    """Flagged blocks of a D=K=128 problem fall back to the scan kernels block by block."""
-    x, f, q, k, fk, s, go, gs = lfw_inputs(2, 100, 128, 128, "sigmoid", 0.5, 71)
+@pytest.mark.parametrize("D,K", [(128, 128), (192, 128)])
+def test_blocked_extreme_gates(cuda, D, K):
+    """Rows whose gates leave the range in some of the state's blocks are redone by the scan kernels, others are not touched."""
+    x, f, q, k, fk, s, go, gs = lfw_inputs(4, 100, D, K, "sigmoid", 0.5, 71)
     fk[1, :, 64:] = 1e-3
     f[0, 30, :] = 0.0
+    f[3, :, 64:128] = 1e-3
     dev = to_dev((x, f, q, k, fk, s, go, gs), torch.float16, cuda)
     check_against_oracle(dev, run_cabi(*dev), torch.float16)
 
@@ -294,7 +318,7 @@ def test_many_tiny_gates_in_one_chunk(cuda):
     check_against_oracle(dev, run_cabi(*dev), torch.float16)
 
 
-@pytest.mark.parametrize("D,T,ckpt_every", [(64, 300, 128), (64, 256, 128), (64, 500, 192), (64, 70, 256), (128, 330, 128)])
+@pytest.mark.parametrize("D,T,ckpt_every", [(64, 300, 128), (64, 256, 128), (64, 500, 192), (64, 70, 256), (128, 330, 128), (192, 330, 128)])
 def test_checkpoint_intervals_of_several_chunks(cuda, D, T, ckpt_every):
     """Checkpoint intervals that are multiples of 64 (BASELINE config 4 names 128) stay on the
     tensor-core path: the per-chunk states live in scratch, the caller's checkpoints hold every
