@@ -36,6 +36,7 @@ int lfw_c64_forward_out(const seq::Maps &mp, const void *state, const void *ckpt
 int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ckpt, const float *Rend,
                           void *const outs[5], const int64_t out_ld[5], const int out_col[5], int *rowflag,
                           int64_t BH, int64_t T_, int dtype, cudaStream_t st);
+int lfw_chunk_sm_count(int *out);   // lfw_c64_local.cu
 int lfw_wide_forward_out(const seq::Maps &mp, const void *state, const void *ckpt, void *out, int *rowflag, int64_t items,
                          int64_t T_, int64_t D, int64_t K, int dtype, cudaStream_t st);      // lfw_wide_fwd.cu
 int lfw_wide_local(bool backward, const seq::Maps &mp, float *M, float *Ac, float *Gc, int *flags, int *rowflag, int64_t items,
@@ -180,13 +181,20 @@ lfw_c64_carry_kernel(const T *__restrict__ init, float *__restrict__ M, const fl
   if (any || !all_finite(S)) atomicExch(rowflag + item, 1);      // (a NaN or an infinity that has got into a state stays in it)
 }
 
-// The carry of BH problem rows.  Two values per thread make twice as many blocks, so that one block's loads run under
-// another's chain; where one round of loads holds all chunks, or the rows alone fill the chip, their smaller accesses cost more
-// than that gives.  Two / four values: 64 rows x 256 chunks 141 / 164 us, 96 rows x 16 chunks 11.3 / 10.3.
+// The carry of BH problem rows.  Two values per thread make twice as many blocks (five of them share an SM, of the others three),
+// so that one block's loads run under another's chain; where one round of loads holds all chunks, or the rows alone fill the
+// chip, their smaller accesses cost more than that gives, and with few rounds so does a second wave of blocks that four values do
+// not need.  The kernel with two / four values, us: 64 rows x 256 chunks 141 / 164, 96 x 16 11.3 / 10.3.  Training calls, 64 x 64, fp16: rows x chunks
+//     16 x 64   148.8 / 151.0     64 x 20  155.8 / 156.6     96 x 20  212.5 / 205.8     128 x 20  271.1 / 272.6
+//     64 x 64   418.9 / 426.8     96 x 32  310.4 / 311.0    128 x 64  789.3 / 817.1     192 x 64 1156.4 / 1151.4
+// (148 SMs: rows 93 to 111 have the second wave; beyond 128 rows neither is ahead by more than 2 %).
 template <typename T, bool kFwd>
 cudaError_t launch_carry(const T *init, float *M, const float *Ac, const float *Gc, const int *flags, int *rowflag, T *out,
                          const Grid2D &gr, int64_t BH, int64_t nc, cudaStream_t st) {
-  if (nc > 16 && BH <= 128)
+  int n_sm = 0;
+  if (lfw_chunk_sm_count(&n_sm) != T2FW_OK) return cudaErrorUnknown;
+  const bool second_wave = BH * 8 > 5 * n_sm && BH * 4 <= 3 * n_sm;      // with two values only
+  if (nc > 16 && BH <= 128 && !(second_wave && nc < 32))
     return launch_dependent(lfw_c64_carry_kernel<T, kFwd, 2>, dim3((unsigned)(BH * 8)), dim3(kCarryThreads), 0, st, init, M, Ac,
                             Gc, flags, rowflag, out, gr, nc);
   return launch_dependent(lfw_c64_carry_kernel<T, kFwd, 4>, dim3((unsigned)(BH * 4)), dim3(kCarryThreads), 0, st, init, M, Ac, Gc,
@@ -259,7 +267,8 @@ struct Call {
 };
 // States of up to 128 x 128 have kernels of their own that take a chunk of all blocks as one problem (lfw_wide_*.cu).
 // 16 x 16384, 128 x 128: chunk-local 136 us against 162 as a grid of blocks, outputs 180 against 433,
-// gradients 515 against 1052.
+// gradients 515 against 1052.  Rectangles, whole training call, against the grid: 128 x 64, 16 x 16384 1038 / 1097, 96 x 1024
+// 379 / 388; 64 x 128 1077 / 1102, 394 / 397; 3 x 777 and 24 x 160 as fast; forward alone, 12 x 1500, 40.0 / 41.8, 41.6 / 42.5.
 bool wide(const Grid2D &g) { return g.nsub > 1 && g.nk <= 2 && g.nsub / g.nk <= 2; }
 void set_grid(seq::Maps &mp, const Grid2D &g) {
   mp.nsub = g.nsub; mp.nk = g.nk; mp.state_item = g.item; mp.state_ld = (int)g.ld;

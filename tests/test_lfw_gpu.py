@@ -269,9 +269,9 @@ def test_wide_state_lengths(cuda, dtype, D, K, T):
     check_against_oracle(dev, run_cabi(*dev), dtype)
 
 
-@pytest.mark.parametrize("B,T,D,K", [(2, 1093, 64, 64), (128, 1088, 64, 64), (129, 1093, 64, 64), (3, 2113, 128, 64)])
+@pytest.mark.parametrize("B,T,D,K", [(2, 1093, 64, 64), (128, 1088, 64, 64), (96, 1093, 64, 64), (129, 1093, 64, 64), (3, 2113, 128, 64)])
 def test_carry_over_more_chunks_than_one_round(cuda, B, T, D, K):
-    """More than 16 chunks: with few rows the carry takes two values per thread, with more four; whole and partial rounds."""
+    """More than 16 chunks: the carry takes two or four values per thread, by rows and chunks; whole and partial rounds."""
     dev = to_dev(lfw_inputs(B, T, D, K, "sigmoid", 0.5, B + T), torch.float16, cuda)
     got = run_cabi(*dev)
     assert all(torch.isfinite(t).all() for t in (got[0], got[1], *got[2]))
