@@ -220,7 +220,7 @@ dfw_carry_bwd_kernel(const T *__restrict__ gs, const T *__restrict__ final_state
                      float *__restrict__ NR, float *__restrict__ GS, T *__restrict__ ds, int nc, int *__restrict__ status) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ __align__(8) uint64_t full[kStages];
-  __shared__ uint4 xs[kH == 2 ? 2 : 1][kH == 2 ? kW : 1][8][32];      // operands of the block's rows, by step parity
+  __shared__ uint4 xs[kH == 2 ? 2 : 1][kH == 2 ? kW : 1][kH == 2 ? 8 : 1][kH == 2 ? 32 : 1];      // operands of the block's rows, by step parity
   constexpr int kN = 8 / kH;                                            // 8-column tiles of a warp
   constexpr int kPart = kW * kImg / 4, kStage = kImg + 2 * kPart;      // floats
   float *ring = reinterpret_cast<float *>(sm);
@@ -308,6 +308,7 @@ template <typename T, int kW, int kH, int kStages>
 int launch_carry_bwd(const void *gs, const void *final_state, const float *Qb, float *NR, float *GS, void *ds, int64_t B, int nc,
                      int *status, cudaStream_t st) {
   constexpr int kSmem = kStages * (kImg + 2 * kW * kImg / 4) * 4;
+  static_assert(kSmem + kCarryStatic<kW, kH, kStages> <= kSharedLimit, "shared memory limit");
   auto *const carry = &dfw_carry_bwd_kernel<T, kW, kH, kStages>;
   T2FW_ALLOW_SMEM(carry, kSmem);
   T2FW_CHECK_CUDA(launch_dependent(carry, dim3((unsigned)(B * (4 / kW))), dim3(32 * kH * kW), kSmem, st, (const T *)gs,
@@ -561,10 +562,12 @@ int backward_typed(const void *go, const void *gs, const void *q, const void *k,
   int *status = nullptr;
   int rc = lfw_chunk_status_ptr(&status);
   if (rc != T2FW_OK) return rc;
-  const CarryPlan plan = carry_plan(B);
+  int n_sm = 0;
+  rc = lfw_chunk_sm_count(&n_sm);
+  if (rc != T2FW_OK) return rc;
+  const CarryPlan plan = carry_plan(B, n_sm);
   rc = plan == kSpread1   ? launch_carry_bwd<T, 1, 2, 9>(gs, final_state, Qb, NR, GS, ds, B, (int)nc, status, st)
        : plan == kSpread2 ? launch_carry_bwd<T, 2, 2, 6>(gs, final_state, Qb, NR, GS, ds, B, (int)nc, status, st)
-       : plan == kDeep    ? launch_carry_bwd<T, 4, 1, 4>(gs, final_state, Qb, NR, GS, ds, B, (int)nc, status, st)
                           : launch_carry_bwd<T, 4, 1, 4>(gs, final_state, Qb, NR, GS, ds, B, (int)nc, status, st);
   if (rc != T2FW_OK) return rc;
   auto *const grad = &dfw_grad_kernel<T>;

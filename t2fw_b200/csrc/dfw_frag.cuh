@@ -339,7 +339,6 @@ __device__ __forceinline__ void gram_lower(float *Ls, uint32_t x, uint32_t y, in
 }
 
 // ---- the carries: 16 rows of a state per warp or pair of warps, a ring of stages filled by bulk copies ------------------------------------------------
-constexpr int kMaxStages = 11;
 template <int kStages>
 __device__ __forceinline__ void init_ring(uint64_t *full, int tid) {
   if (tid == 0) {
@@ -433,8 +432,12 @@ __device__ __forceinline__ void carry_product(float (&c)[8 / kH][4], const uint3
 // 74 x 1333 257 -> 244, 96 x 1024 242 -> 236, 200 x 512 253 -> 244, 384 x 341 347 -> 342; pairs of warps instead at 96 and 200
 // rows: 240, 250.
 enum CarryPlan { kSpread1, kSpread2, kDeep, kDense };
-inline CarryPlan carry_plan(int64_t B) { return B <= 37 ? kSpread1 : B <= 74 ? kSpread2 : B <= 148 ? kDeep : kDense; }
+inline CarryPlan carry_plan(int64_t B, int n_sm) { return 4 * B <= n_sm ? kSpread1 : 2 * B <= n_sm ? kSpread2 : B <= n_sm ? kDeep : kDense; }
+// shared memory of a carry besides its ring of stages: barriers, and the halves' exchange
+template <int kW, int kH, int kStages> constexpr int kCarryStatic = kStages * 8 + (kH == 2 ? 2 * kW * 8 * 32 * 16 : 16);
+constexpr int kSharedLimit = 227 * 1024;
 
 }  // namespace frag
 int lfw_chunk_status_ptr(int **out);      // lfw_c64_local.cu
+int lfw_chunk_sm_count(int *out);
 }  // namespace t2fw

@@ -150,7 +150,7 @@ dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg
                      T *__restrict__ final_state, int nc, int *__restrict__ status) {
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ __align__(8) uint64_t full[kStages];
-  __shared__ uint4 xs[kH == 2 ? 2 : 1][kH == 2 ? kW : 1][8][32];      // operands of the block's rows, by step parity
+  __shared__ uint4 xs[kH == 2 ? 2 : 1][kH == 2 ? kW : 1][kH == 2 ? 8 : 1][kH == 2 ? 32 : 1];      // operands of the block's rows, by step parity
   constexpr int kN = 8 / kH;                                            // 8-column tiles of a warp
   constexpr int kPart = kW * kImg / 4, kStage = kImg + kPart;      // floats
   float *ring = reinterpret_cast<float *>(sm);
@@ -223,6 +223,7 @@ dfw_carry_fwd_kernel(const T *__restrict__ state, const float *__restrict__ Qimg
 template <typename T, int kW, int kH, int kStages>
 int launch_carry_fwd(const void *state, const float *Qc, float *NS, void *final_state, int64_t B, int nc, int *status, cudaStream_t st) {
   constexpr int kSmem = kStages * (kImg + kW * kImg / 4) * 4;
+  static_assert(kSmem + kCarryStatic<kW, kH, kStages> <= kSharedLimit, "shared memory limit");
   auto *const carry = &dfw_carry_fwd_kernel<T, kW, kH, kStages>;
   T2FW_ALLOW_SMEM(carry, kSmem);
   T2FW_CHECK_CUDA(launch_dependent(carry, dim3((unsigned)(B * (4 / kW))), dim3(32 * kH * kW), kSmem, st, (const T *)state, Qc, NS,
@@ -357,7 +358,10 @@ int forward_typed(const void *q, const void *k, const void *v, const void *state
   int *status = nullptr;
   int rc = lfw_chunk_status_ptr(&status);
   if (rc != T2FW_OK) return rc;
-  const CarryPlan plan = carry_plan(B);
+  int n_sm = 0;
+  rc = lfw_chunk_sm_count(&n_sm);
+  if (rc != T2FW_OK) return rc;
+  const CarryPlan plan = carry_plan(B, n_sm);
   rc = plan == kSpread1   ? launch_carry_fwd<T, 1, 2, 10>(state, Qc, NS, final_state, B, (int)nc, status, st)
        : plan == kSpread2 ? launch_carry_fwd<T, 2, 2, 8>(state, Qc, NS, final_state, B, (int)nc, status, st)
        : plan == kDeep    ? launch_carry_fwd<T, 4, 1, 7>(state, Qc, NS, final_state, B, (int)nc, status, st)

@@ -737,7 +737,7 @@ int lfw_c64_backward_main(const seq::Maps &mp, const void *state, const void *ck
                                      T2FW_OUT(TT, 2), T2FW_OUT(TT, 3), T2FW_OUT(TT, 4), rowflag, status, T_, nc,  \
                                      total));                                                         \
   } while (0)
-  const bool fused = (mp.flags & (seq::kUnitForget | seq::kSigmoidGate)) != 0 || mp.q_scale != 1.f;
+  const bool fused = (mp.flags & seq::kFusedLayer) != 0;
 #define T2FW_MODES(TT)                                                                              \
   do {                                                                                              \
     if (mp.nsub > 1) T2FW_LAUNCH(TT, 2); else if (fused) T2FW_LAUNCH(TT, 1); else T2FW_LAUNCH(TT, 0); \

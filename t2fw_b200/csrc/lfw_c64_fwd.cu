@@ -463,7 +463,7 @@ int lfw_c64_forward_out(const seq::Maps &mp, const void *state, const void *ckpt
                                      (const TT *)state, (const TT *)ckpt, seq::Out<TT>{(TT *)out, out_ld, out_col}, \
                                      rowflag, status, T_, nc, total));                               \
   } while (0)
-  const bool fused = (mp.flags & (seq::kUnitForget | seq::kSigmoidGate)) != 0 || mp.q_scale != 1.f;
+  const bool fused = (mp.flags & seq::kFusedLayer) != 0;
 #define T2FW_MODES(TT)                                                                              \
   do {                                                                                              \
     if (mp.nsub > 1) T2FW_LAUNCH(TT, 2); else if (fused) T2FW_LAUNCH(TT, 1); else T2FW_LAUNCH(TT, 0); \

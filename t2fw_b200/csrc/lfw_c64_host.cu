@@ -12,16 +12,17 @@
 //   2. lfw_c64_carry_kernel<.., false>  from the last chunk down: R_end(c-1) = (Ac Gc^T) .* R_end(c) + G_c,
 //      stored in place of G_c (fp32); what is left after chunk 0 is d_state
 //   3. lfw_c64_bwd_kernel               per (row, chunk): d_x, d_f, d_q, d_k, d_f_key
-// Scratch (floats): M[B][nc][64][64], 16-byte pieces of a row XOR-ed with (row % 8) | Ac[B][nc][64] | Gc[B][nc][64] | flags[B][nc] (int) |
-// rowflag[B] (int).  A flagged row (gate products outside the range of the factored form, values that are no
+// Scratch (floats): M[B][nc][64][64], 16-byte pieces of a row XOR-ed with (row % 8) | Ac[B][nc][64] | Gc[B][nc][64] |
+// flags[B][nc] (int) | rowflag[B] (int).  A flagged row (gate products outside the range of the factored form, values that are no
 // finite numbers) is recomputed by the scan kernels afterwards.
-// States larger than 64 x 64 (D, K multiples of 64): the recurrence never mixes state rows or columns, so a D x K state
+// States of up to 128 x 128 (D, K = 64 or 128) have kernels of their own for 1. and 3. (lfw_wide_*.cu) and share the carry, whose
+// rows are their 64 x 64 blocks.
+// Larger ones (D, K multiples of 64): the recurrence never mixes state rows or columns, so a D x K state
 // is a (D/64) x (K/64) grid of independent blocks, problem rows of their own for the kernels (B above counts them);
 // block (i, j) reads the d-side vectors' window i and the k-side vectors' window j in place, states and checkpoints are
 // read and written in place too, and what leaves the state is summed over the other axis' blocks by the output and
-// gradient kernels, whose CTAs walk all blocks of a chunk: a thread adds to what it wrote itself (per-block results and
-// separate summing and re-layout passes took 0.4 of 2.4 ms at B = 16, T = 16384, D = K = 128).  Flags are then per
-// batch item.
+// gradient kernels, whose CTAs walk all blocks of a chunk: a thread adds to what it wrote itself.  Flags are then per batch
+// item.
 #include "lfw_c64.cuh"
 #include "seq_layout.cuh"
 
@@ -384,7 +385,7 @@ Call fused_call(const void *qkvg, const void *go, int64_t B, int64_t T_, int H) 
   c.fk = {qkvg, 4 * C, (int)(3 * C)};
   c.f = {nullptr, 0, 0};
   c.go = {go, C, 0};
-  c.B = B; c.T_ = T_; c.heads = H; c.flags = seq::kUnitForget | seq::kSigmoidGate; c.q_scale = 0.125f;   // 1 / sqrt(64)
+  c.B = B; c.T_ = T_; c.heads = H; c.flags = seq::kFusedLayer; c.q_scale = 0.125f;   // 1 / sqrt(64)
   return c;
 }
 

@@ -350,7 +350,7 @@ int lfw_chunk_local_umma(bool backward, const seq::Maps &mp, float *M, float *Ac
     T2FW_CHECK_CUDA(launch_dependent(lfw_c64_local_kernel<TT, SUF, FF>, dim3(grid), dim3(kThreadsL), kSmemL, st, mp, M, \
                                      Ac, Gc, flags, rowflag, (int)(BH / mp.nsub), status, T_, nc, total));                         \
   } while (0)
-  const bool fused = (mp.flags & (seq::kUnitForget | seq::kSigmoidGate)) != 0 || mp.q_scale != 1.f;
+  const bool fused = (mp.flags & seq::kFusedLayer) != 0;
 #define T2FW_FUSED(TT, SUF)                                                   \
   do {                                                                        \
     if (fused) T2FW_LAUNCH(TT, SUF, true); else T2FW_LAUNCH(TT, SUF, false);  \

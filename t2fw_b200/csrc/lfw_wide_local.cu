@@ -213,9 +213,8 @@ lfw_wide_local_kernel(const __grid_constant__ seq::Maps mp, float *__restrict__ 
       }
       umma::named_barrier(1 + q4, 128);
     }
-    // No full barrier here: before the next one the next chunk writes only products of quarters, which nobody reads any
-    // more, and tile rows of its quarter's features, behind the quarter's own barriers - in a place where another quarter's
-    // results may still be on their way: the tile's rows are 128 bytes, the results' 256.
+    // A full barrier: the next chunk's tile rows are 128 bytes, these results' 256, so that a quarter's operands go where
+    // another quarter's results may still be on their way out.
     umma::fence_before_sync();
     __syncthreads();
   }

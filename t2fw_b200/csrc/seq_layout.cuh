@@ -21,9 +21,9 @@ namespace seq {
 constexpr int kMaxTensors = 6;
 
 enum : int {
-  kUnitForget = 1,     // the d-side gate is the constant 1: nothing is read for it
-  kSigmoidGate = 2,    // the k-side gate tensor holds pre-activations: gate = max(sigmoid(g), 1/8)
-  kContiguous = 4,     // every tensor is a dense [rows][64] array: a chunk's block is one linear 8 KB copy
+  kFusedLayer = 1,     // the d-side gate is the constant 1 (nothing is read for it), the k-side gate tensor holds
+                       //   pre-activations, gate = max(sigmoid(g), 1/8), and the query is scaled
+  kContiguous = 2,     // every tensor is a dense [rows][64] array: a chunk's block is one linear 8 KB copy
 };
 constexpr float kGateFloor = 0.125f;   // with gates >= 1/8 no 32-step product leaves the safe range
 
@@ -42,7 +42,7 @@ struct Maps {
   int64_t state_item;            // elements of one state of a batch item (or problem row without a grid), and the
   int state_ld;                  //   stride of its rows
   int flags;
-  float q_scale;                 // factor on the query tensor (1 for the plain operators)
+  float q_scale;                 // fused layer: factor on the query tensor
 };
 
 // element offset of the 64 x 64 block of sub-item `sub` of item `b` (problem row without a grid), state number c of S
