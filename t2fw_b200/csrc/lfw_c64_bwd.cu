@@ -43,11 +43,11 @@
 //
 // What bounds it: the phases of the computing warps (gates and operands 3.1 k cycles, state operands 2.0 k, Z 1.2 k, sums and
 // results 4.5 k of 11 k per chunk), in which all warps want the same unit at the same time; products and copies run under them.
-// Issue slots 58 % busy (27.9 k warp instructions per chunk, polling included), tensor pipe 21 %, DRAM 21 %; B*H = 96, T = 1024
-// (1536 chunks): 99 -> 79 us per launch with cold caches.
-// Whole training step, start of this arrangement -> now: 96 rows x 1024 steps 200 -> 177 us (N(0,1) gates, of which 0.4 per chunk
-// are tiny: their listing and sums took 6 k cycles, now 0.5 k), fused layer 8 x 12 heads x 1024 258 -> 206 us, 16 x 16384 with
-// 128 x 128 states 2213 -> 2035 us.
+// Issue slots 58 % busy (28.2 k warp instructions per chunk, polling included), tensor pipe 21 %, DRAM 21 %; B*H = 96, T = 1024
+// (1536 chunks): 99 us per launch with cold caches before the issuing warps, 79 to 81 with them.
+// Whole training step, without issuing warps -> with them: 96 rows x 1024 steps 200 -> 175 to 181 us from box to box (N(0,1)
+// gates, of which 0.4 per chunk are tiny: their listing and sums took 6 k cycles, now 0.5 k), fused layer 8 x 12 heads x 1024
+// 258 -> 197 us.
 #include "lfw_c64.cuh"
 #include "seq_layout.cuh"
 

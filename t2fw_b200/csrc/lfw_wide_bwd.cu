@@ -16,7 +16,7 @@
 // d side's ratios wait there for its turn.  Shared memory: raw values land where tiles will be (a thread takes its values into
 // registers before the barrier that precedes the tiles' first write), Z tiles and staged results share one area.
 //
-// Issue slots 45 % busy (68 k warp instructions per chunk of four blocks), tensor pipe 11 %, DRAM 16 %.
+// Issue slots 50 % busy (70 k warp instructions per chunk of four blocks), tensor pipe 12 %, DRAM 17 % (16 rows x 2048 steps).
 // 16 rows x 16384 steps, 128 x 128 (4096 chunks): 1052 us as a grid of blocks -> 515 us (557 with the end gradients
 // loaded by the threads that use them: the d side's rows are 256 bytes apart, 9 k of 37 k cycles per chunk).  Bound by the latency of
 // its phases, as the 64 x 64 kernel was before its issuing warps: block barriers, and state blocks that are loaded when they are needed.

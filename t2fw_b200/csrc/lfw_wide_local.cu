@@ -7,7 +7,8 @@
 // Results and decay vectors leave in the layout of the blocks, which the carry goes through as before.
 //
 // Persistent CTAs of 16 warps, two per SM; thread (feature, 16-step quarter) serves the feature with its number on both sides.
-// 16 rows x 16384 steps, 128 x 128 (4096 chunks): 162 us as a grid of blocks -> 136 us; the results alone are 268 MB.
+// 16 rows x 16384 steps, 128 x 128 (4096 chunks): 162 us as a grid of blocks -> 136 us; the results alone are 268 MB.  The range
+// test's look at the values costs 2 (142 -> 144, in turn on one box).
 #include "lfw_c64.cuh"
 #include "seq_layout.cuh"
 
